@@ -31,7 +31,7 @@ extern "C" {
 #pragma GCC visibility push(default) /* the entry points below are the library's only exports */
 #endif
 
-#define KDA_B200_ABI_VERSION 9
+#define KDA_B200_ABI_VERSION 10
 #define KDA_CHUNK 64 /* tokens per chunk of the chunked kernels */
 
 /* io_dtype of q, k, v, o and of their gradients */
@@ -155,8 +155,8 @@ int kda_recurrent_bwd(const kda_recurrent_bwd_args* args, void* stream);
  * The caller passes one scratch buffer ("workspace") of at least kda_chunk_workspace_bytes(...).
  * When save_for_backward != 0 the forward leaves in it what kda_chunk_bwd needs; the caller keeps the
  * buffer alive and unmodified until the backward call and passes the same pointer.
- * cu_seqlens is always required (for equal lengths pass 0, T, 2T, ...); chunks restart at every
- * sequence start and the last chunk of a sequence may be partial.
+ * cu_seqlens == NULL: N sequences of tokens / N tokens each (KDA_E_SHAPE if N does not divide tokens); the chunk geometry is
+ * then arithmetic and no table is built.  Chunks restart at every sequence start and the last chunk of a sequence may be partial.
  * ------------------------------------------------------------------------------------------------ */
 typedef struct kda_chunk_args {
   /* forward inputs */
@@ -166,7 +166,7 @@ typedef struct kda_chunk_args {
   const float* g;              /* [tokens, H, K] fp32 log-decay */
   const float* beta;           /* [tokens, H]    fp32 */
   const float* h0;             /* [N, H, K, V] fp32 or NULL */
-  const int32_t* cu_seqlens;   /* device [N+1] int32 */
+  const int32_t* cu_seqlens;   /* device [N+1] int32, or NULL: equal lengths */
   /* forward outputs */
   void* o;                     /* [tokens, H, V] bf16 */
   float* ht;                   /* [N, H, K, V] fp32 or NULL */

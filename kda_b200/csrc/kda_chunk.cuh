@@ -30,6 +30,7 @@ constexpr size_t TILE_GL = size_t(KD) * 4;        // 512 B
 struct ChunkWs {
   int* seq_chunk_off;   // [N+1] first chunk of each sequence; [N] = total chunks
   int* chunk_seq;       // [max_chunks] sequence of each chunk
+  int* seq_order;       // [N] sequences by falling number of chunks: the order in which the state scans start them
   unsigned* status;     // [4] device status word (first bytes of the workspace): KDA_STATUS_* bits, 0 = nothing to report
   unsigned char *W, *UT, *KG, *QG, *AQK, *GL;          // always
   unsigned char *TI, *RKK, *HS, *VNEWT;                // save_for_backward only
@@ -55,6 +56,7 @@ inline ChunkWs carve_ws(unsigned char* base, unsigned char* bwd_base, int64_t to
   w.status = reinterpret_cast<unsigned*>(take(16));      // first, so that its address does not depend on the sizes
   w.seq_chunk_off = reinterpret_cast<int*>(take(sizeof(int) * (static_cast<size_t>(N) + 1)));
   w.chunk_seq = reinterpret_cast<int*>(take(sizeof(int) * (NTmax + 1)));
+  w.seq_order = reinterpret_cast<int*>(take(sizeof(int) * (static_cast<size_t>(N) + 1)));
   w.W = take(tiles * TILE_TK);
   w.UT = take(tiles * TILE_VT);
   w.KG = take(tiles * TILE_TK);
@@ -90,20 +92,39 @@ inline ChunkWs carve_ws(unsigned char* base, unsigned char* bwd_base, int64_t to
   return w;
 }
 
-// Chunk geometry read from the tables: which sequence, first token, valid rows.
+// Chunk geometry: which sequence, first token, valid rows.
 struct ChunkInfo {
   int seq;
   long long tok0;
   int len;
 };
-__device__ __forceinline__ ChunkInfo chunk_info(const int* seq_chunk_off, const int* chunk_seq, const int* cu, int c) {
-  ChunkInfo ci;
-  ci.seq = chunk_seq[c];
-  const int cis = c - seq_chunk_off[ci.seq];
-  ci.tok0 = static_cast<long long>(cu[ci.seq]) + static_cast<long long>(cis) * C;
-  const long long rem = static_cast<long long>(cu[ci.seq + 1]) - ci.tok0;
-  ci.len = rem < C ? static_cast<int>(rem) : C;
-  return ci;
+// Which chunks a call has.  Sequences of equal length (T > 0: cu_seqlens was NULL) need no tables: everything is arithmetic, and
+// the call saves the tables kernel (4 us) in front of prepare.  Otherwise the tables kernel has filled the arrays.
+struct ChunkMap {
+  const int *cu, *seq_chunk_off, *chunk_seq, *seq_order;
+  int N, T, per_seq;      // per_seq = chunks per sequence (T > 0)
+
+  __device__ __forceinline__ int total() const { return T > 0 ? N * per_seq : seq_chunk_off[N]; }
+  __device__ __forceinline__ int first_chunk(int seq) const { return T > 0 ? seq * per_seq : seq_chunk_off[seq]; }
+  __device__ __forceinline__ long long first_token(int seq) const { return T > 0 ? static_cast<long long>(seq) * T : cu[seq]; }
+  __device__ __forceinline__ int started(int i) const { return T > 0 ? i : seq_order[i]; }      // the i-th sequence that a scan starts
+  __device__ __forceinline__ ChunkInfo info(int c) const {
+    ChunkInfo ci;
+    ci.seq = T > 0 ? c / per_seq : chunk_seq[c];
+    ci.tok0 = first_token(ci.seq) + static_cast<long long>(c - first_chunk(ci.seq)) * C;
+    const long long rem = first_token(ci.seq + 1) - ci.tok0;
+    ci.len = rem < C ? static_cast<int>(rem) : C;
+    return ci;
+  }
+};
+// the map of a call on its workspace; with cu == NULL every sequence has tokens / N tokens
+inline ChunkMap chunk_map(const ChunkWs& w, const int32_t* cu, int64_t tokens, int N) {
+  ChunkMap m{cu, w.seq_chunk_off, w.chunk_seq, w.seq_order, N, 0, 0};
+  if (!cu) {
+    m.T = static_cast<int>(tokens / N);
+    m.per_seq = (m.T + C - 1) / C;
+  }
+  return m;
 }
 
 // byte offset of element (v, k) of a [128 v][128 k] state tile: span k/64, then the 128-byte-row swizzle

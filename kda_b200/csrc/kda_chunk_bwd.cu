@@ -152,11 +152,11 @@ extern "C" int kda_chunk_bwd(const kda_chunk_args* args, void* stream) {
   }
 
   RScanParams rp{};
-  rp.cu = a.cu_seqlens; rp.seq_chunk_off = w.seq_chunk_off; rp.chunk_seq = w.chunk_seq;
+  rp.map = chunk_map(w, a.cu_seqlens, a.tokens, a.N);
   rp.W = w.W; rp.KG = w.KG; rp.QG = w.QG; rp.AQK = w.AQK; rp.GL = w.GL;
   rp.DH = w.DH; rp.DVNEWT = w.DVNEWT;
   rp.d_o = static_cast<const __nv_bfloat16*>(a.d_o); rp.d_ht = a.d_ht; rp.dh0 = a.dh0; rp.status = w.status; rp.dbg = g_dbg_clocks;
-  rp.N = a.N; rp.H = a.H;
+  rp.H = a.H;
   if (make_rows_tmap(&rp.tm_do, a.d_o, false, a.tokens, a.H, VD, 64, C, true)) return KDA_E_TMAP;
   const int slices = scan_slices_for(a.N * a.H, a.scan_slices);
   if ((rc = slices > 1 ? launch_bwd_scan_vs(rp, a.N * a.H, st) : launch_bwd_scan_tc(rp, a.N * a.H, st)) != KDA_OK) return rc;
@@ -164,7 +164,7 @@ extern "C" int kda_chunk_bwd(const kda_chunk_args* args, void* stream) {
 
   MainParams mp{};
   mp.q = q; mp.k = k; mp.v = static_cast<const __nv_bfloat16*>(a.v); mp.d_o = static_cast<const __nv_bfloat16*>(a.d_o);
-  mp.g = a.g; mp.beta = a.beta; mp.cu = a.cu_seqlens; mp.seq_chunk_off = w.seq_chunk_off; mp.chunk_seq = w.chunk_seq;
+  mp.g = a.g; mp.beta = a.beta; mp.map = rp.map;
   mp.TI = w.TI; mp.RKK = w.RKK; mp.HS = w.HS; mp.VNEWT = w.VNEWT; mp.DH = w.DH; mp.DVNEWT = w.DVNEWT;
   mp.dv = static_cast<__nv_bfloat16*>(a.dv);
   // grouped value heads: every value head writes its own dq, dk; a second kernel sums each group
@@ -176,7 +176,7 @@ extern "C" int kda_chunk_bwd(const kda_chunk_args* args, void* stream) {
       make_rows_tmap(&mp.tm_v, a.v, false, a.tokens, a.H, VD, 64, C, true) ||
       make_rows_tmap(&mp.tm_do, a.d_o, false, a.tokens, a.H, VD, 64, C, true))
     return KDA_E_TMAP;
-  mp.N = a.N; mp.H = a.H; mp.scale = a.scale; mp.grp = grp;
+  mp.H = a.H; mp.scale = a.scale; mp.grp = grp;
   // without grouped heads the normalisation's backward is applied by bwd_main's own epilogue
   const bool fused_l2 = l2 && grp == 1;
   mp.rstd = fused_l2 ? w.RSTD : nullptr; mp.qrows = rows;

@@ -9,14 +9,13 @@ namespace kda {
 struct MainParams {
   const __nv_bfloat16 *q, *k, *v, *d_o;
   const float *g, *beta;
-  const int* cu;
-  const int *seq_chunk_off, *chunk_seq;
+  ChunkMap map;
   const unsigned char *TI, *RKK, *HS, *VNEWT, *DH, *DVNEWT;
   __nv_bfloat16 *dv, *dq, *dk;
   float *dbeta, *dg;
   unsigned* status;
   long long* dbg;
-  int N, H;
+  int H;
   float scale;
   int grp;          // value heads per q/k head (grouped value heads): the q, k maps have H / grp heads
   const float* rstd;    // [2][qrows] reciprocal norms of the q, k rows, or NULL.  Not NULL (only with grp == 1): q, k are the
@@ -27,8 +26,7 @@ struct MainParams {
 };
 
 struct RScanParams {
-  const int* cu;
-  const int *seq_chunk_off, *chunk_seq;
+  ChunkMap map;
   const unsigned char *W, *KG, *QG, *AQK, *GL;
   unsigned char *DH, *DVNEWT;
   const __nv_bfloat16* d_o;
@@ -36,7 +34,7 @@ struct RScanParams {
   float* dh0;
   unsigned* status;
   long long* dbg;       // development aid: phase clocks
-  int N, H;
+  int H;
   alignas(64) CUtensorMap tm_do;   // 64-column boxes of dO in the 128-byte-swizzled operand layout
 };
 

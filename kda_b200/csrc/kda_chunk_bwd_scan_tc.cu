@@ -52,10 +52,10 @@ __global__ void __launch_bounds__(RNT, 1) kda_chunk_bwd_scan_tc_kernel(const __g
   TcRScanSmem& s = *reinterpret_cast<TcRScanSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int q4 = warp & 3, half = warp >> 2;
-  const int seq = blockIdx.x / p.H, h = blockIdx.x % p.H;
-  const int c_begin = p.seq_chunk_off[seq], c_end = p.seq_chunk_off[seq + 1];
+  const int seq = p.map.started(blockIdx.x / p.H), h = blockIdx.x % p.H;
+  const int c_begin = p.map.first_chunk(seq), c_end = p.map.first_chunk(seq + 1);
   const int nchunks = c_end - c_begin;
-  const long long seq_tok0 = p.cu[seq];
+  const long long seq_tok0 = p.map.first_token(seq);
   const int v = 32 * q4 + lane;
 
   if (tid == 0) {

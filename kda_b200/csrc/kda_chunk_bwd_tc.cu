@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
   TcSmem& s = *reinterpret_cast<TcSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int q4 = warp & 3, part = warp >> 2;          // TMEM lane quadrant of this warp; which 16 of the 64 columns
-  const long long total_tiles = static_cast<long long>(p.seq_chunk_off[p.N]) * p.H;
+  const long long total_tiles = static_cast<long long>(p.map.total()) * p.H;
 
   // aliases inside the tile regions
   unsigned char* const sKG = s.HS;
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
   // thread 0: first token and length of tile idx's chunk into slot (two dependent global loads: done early, off the
   // critical path, while phase B2 executes and the other warps build operands)
   auto stash_chunk = [&](long long idx, int slot) {
-    const ChunkInfo cn = chunk_info(p.seq_chunk_off, p.chunk_seq, p.cu, static_cast<int>(idx / p.H));
+    const ChunkInfo cn = p.map.info(static_cast<int>(idx / p.H));
     s.ci_tok0[slot] = cn.tok0;
     s.ci_len[slot] = cn.len;
   };

@@ -25,46 +25,87 @@ namespace kda {
 // nothing; no device->host synchronisation is needed for the check.
 __global__ void __launch_bounds__(1024) kda_chunk_tables_kernel(const int* __restrict__ cu, int N, long long tokens, int max_chunks,
                                                                 int* __restrict__ seq_chunk_off, int* __restrict__ chunk_seq,
-                                                                unsigned* __restrict__ status) {
-  __shared__ int part[1024];
-  const int tid = threadIdx.x;
+                                                                int* __restrict__ seq_order, unsigned* __restrict__ status) {
+  __shared__ int warp_sum_[32];
+  __shared__ int offs[1025];      // chunk offsets of the first 1,024 sequences (all of them in ordinary calls)
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int per = (N + 1023) / 1024;
   const int n0 = min(N, tid * per), n1 = min(N, n0 + per);
+  // a partial sum that would overflow is certainly beyond max_chunks: sums saturate there instead of wrapping
+  const int cap = max_chunks + 1;
   int sum = 0;
   bool bad = (tid == 0) && (cu[0] < 0 || static_cast<long long>(cu[N]) > tokens);
   for (int n = n0; n < n1; ++n) {
     const int len = cu[n + 1] - cu[n];
     bad |= len < 0;
-    // a partial sum that would overflow is certainly beyond max_chunks; saturate instead of wrapping
     const int nc = (len > 0) ? (len + C - 1) / C : 0;
-    sum = (sum > max_chunks || nc > max_chunks) ? max_chunks + 1 : sum + nc;
+    sum = min(cap, sum + min(cap, nc));
   }
-  part[tid] = sum;
+  int incl = sum;                 // inclusive scan over the block: within the warp, then over the warps' totals
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl = min(cap, incl + x);
+  }
+  if (lane == 31) warp_sum_[warp] = incl;
   __syncthreads();
-  for (int off = 1; off < 1024; off <<= 1) {   // inclusive Hillis-Steele scan (saturating)
-    int x = (tid >= off) ? part[tid - off] : 0;
-    __syncthreads();
-    const int y = part[tid] + x;
-    part[tid] = (y > max_chunks || y < 0) ? max_chunks + 1 : y;
-    __syncthreads();
+  if (warp == 0) {
+    int x = warp_sum_[lane];
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, off);
+      if (lane >= off) x = min(cap, x + y);
+    }
+    warp_sum_[lane] = x;
   }
-  bad |= part[tid] > max_chunks;
+  __syncthreads();
+  if (warp > 0) incl = min(cap, incl + warp_sum_[warp - 1]);
+  const int total = warp_sum_[31];
+  bad |= total > max_chunks;
   bad = __syncthreads_or(bad) != 0;
   if (tid < 4) status[tid] = (tid == 0 && bad) ? KDA_STATUS_BAD_CU_SEQLENS : 0u;
   if (bad) {
-    for (int n = n0; n < n1; ++n) seq_chunk_off[n] = 0;
+    for (int n = n0; n < n1; ++n) {
+      seq_chunk_off[n] = 0;
+      seq_order[n] = n;
+    }
     if (tid == 1023) seq_chunk_off[N] = 0;
     return;
   }
-  int run = part[tid] - sum;   // exclusive prefix
+  int run = incl - sum;           // exclusive prefix
   for (int n = n0; n < n1; ++n) {
     const int len = cu[n + 1] - cu[n];
-    const int nc = (len > 0) ? (len + C - 1) / C : 0;
     seq_chunk_off[n] = run;
-    for (int c = 0; c < nc; ++c) chunk_seq[run + c] = n;
-    run += nc;
+    if (n < 1024) offs[n] = run;
+    run += (len > 0) ? (len + C - 1) / C : 0;
   }
-  if (tid == 1023) seq_chunk_off[N] = part[1023];
+  if (tid == 1023) seq_chunk_off[N] = total;
+  if (tid == 0 && N <= 1024) offs[N] = total;
+  __syncthreads();
+  // sequence of every chunk: a thread per chunk, binary search over the offsets (a thread per SEQUENCE would write a long
+  // prompt's whole range alone: 512 chunks took 5.8 us)
+  const int* table = N <= 1024 ? offs : seq_chunk_off;
+  for (int c = tid; c < total; c += 1024) {
+    int lo = 0, hi = N;           // the last n with offset <= c
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (table[mid] <= c) lo = mid; else hi = mid;
+    }
+    chunk_seq[c] = lo;
+  }
+  // Longest first for the state scans, whose CTAs each walk one sequence: with more (sequence, head) units than SMs a long
+  // sequence that starts last would run on alone.  Rank by counting; beyond 1,024 sequences the tail is short anyway.
+  if (N > 1024) {
+    for (int n = n0; n < n1; ++n) seq_order[n] = n;
+  } else if (tid < N) {
+    const int mine = offs[tid + 1] - offs[tid];
+    int rank = 0;
+    for (int n = 0; n < N; ++n) {
+      const int other = offs[n + 1] - offs[n];
+      rank += (other > mine || (other == mine && n < tid)) ? 1 : 0;
+    }
+    seq_order[rank] = tid;
+  }
 }
 
 // =================================================================================================
@@ -91,11 +132,11 @@ static_assert(TILE_VT + TILE_TK <= C * GS * 4, "staged tiles must fit the G buff
 struct PrepParams {
   const __nv_bfloat16 *q, *k, *v;
   const float *g, *beta;
-  const int* cu;
-  const int *seq_chunk_off, *chunk_seq;
+  ChunkMap map;
+  unsigned* status;   // cleared here when there is no tables kernel in front (equal lengths), else NULL
   unsigned char *W, *UT, *KG, *QG, *AQK, *GL, *TI, *RKK;   // TI, RKK may be NULL
   long long* dbg;
-  int N, H;
+  int H;
   int use_l2norm;
   float scale;
   int HQ, grp;      // q/k heads and value heads per q/k head (grouped value heads); H counts value heads
@@ -250,8 +291,9 @@ __global__ void __launch_bounds__(256, 2) kda_chunk_prepare_kernel(const PrepPar
   PrepSmem& s = *reinterpret_cast<PrepSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
   const int c = blockIdx.x, h = blockIdx.y;
-  if (c >= p.seq_chunk_off[p.N]) return;
-  const ChunkInfo ci = chunk_info(p.seq_chunk_off, p.chunk_seq, p.cu, c);
+  if (p.status && c == 0 && h == 0 && tid < 4) p.status[tid] = 0u;
+  if (c >= p.map.total()) return;
+  const ChunkInfo ci = p.map.info(c);
   const int len = ci.len;
   const size_t tile = static_cast<size_t>(c) * p.H + h;
   KDA_DBG_CLOCK(p.dbg, 16);
@@ -681,7 +723,8 @@ int validate_chunk_args(const kda_chunk_args& a, bool backward) {
   if (a.io_dtype != KDA_BF16) return KDA_E_DTYPE;
   if (a.tokens / C + a.N > 0x3fffffffLL) return KDA_E_SHAPE;
   if (a.tokens == 0 || a.N == 0) return KDA_OK;
-  if (!a.q || !a.k || !a.v || !a.g || !a.beta || !a.cu_seqlens || !a.workspace) return KDA_E_NULL;
+  if (!a.q || !a.k || !a.v || !a.g || !a.beta || !a.workspace) return KDA_E_NULL;
+  if (!a.cu_seqlens && a.tokens % a.N != 0) return KDA_E_SHAPE;
   if (!backward && !a.o) return KDA_E_NULL;
   uintptr_t bits = reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v) |
                    reinterpret_cast<uintptr_t>(a.g) | reinterpret_cast<uintptr_t>(a.o) | reinterpret_cast<uintptr_t>(a.h0) |
@@ -733,22 +776,24 @@ extern "C" int kda_chunk_fwd(const kda_chunk_args* args, void* stream) {
   const int NTmax = static_cast<int>(a.tokens / C + a.N);
 
   ProfCall* prof = prof_begin(st);
-  kda_chunk_tables_kernel<<<1, 1024, 0, st>>>(a.cu_seqlens, a.N, a.tokens, NTmax, w.seq_chunk_off, w.chunk_seq, w.status);
-  if ((e = cudaGetLastError()) != cudaSuccess) return static_cast<int>(e);
+  const ChunkMap map = chunk_map(w, a.cu_seqlens, a.tokens, a.N);
+  if (a.cu_seqlens) {
+    kda_chunk_tables_kernel<<<1, 1024, 0, st>>>(a.cu_seqlens, a.N, a.tokens, NTmax, w.seq_chunk_off, w.chunk_seq, w.seq_order, w.status);
+    if ((e = cudaGetLastError()) != cudaSuccess) return static_cast<int>(e);
+  }
   prof_mark(prof, KDA_STAGE_TABLES, st);
 
   PrepParams pp{};
   pp.q = static_cast<const __nv_bfloat16*>(a.q);
   pp.k = static_cast<const __nv_bfloat16*>(a.k);
   pp.v = static_cast<const __nv_bfloat16*>(a.v);
-  pp.g = a.g; pp.beta = a.beta; pp.cu = a.cu_seqlens;
-  pp.seq_chunk_off = w.seq_chunk_off; pp.chunk_seq = w.chunk_seq;
+  pp.g = a.g; pp.beta = a.beta; pp.map = map; pp.status = a.cu_seqlens ? nullptr : w.status;
   pp.W = w.W; pp.UT = w.UT; pp.KG = w.KG; pp.QG = w.QG; pp.AQK = w.AQK; pp.GL = w.GL; pp.TI = save ? w.TI : nullptr; pp.RKK = save ? w.RKK : nullptr;
-  pp.dbg = g_dbg_clocks; pp.N = a.N; pp.H = a.H; pp.use_l2norm = a.use_qk_l2norm; pp.scale = a.scale;
+  pp.dbg = g_dbg_clocks; pp.H = a.H; pp.use_l2norm = a.use_qk_l2norm; pp.scale = a.scale;
   pp.HQ = a.HQ > 0 ? a.HQ : a.H; pp.grp = a.H / pp.HQ;
   pp.QN = keep_qn ? w.QN : nullptr; pp.KN = keep_qn ? w.KN : nullptr; pp.RSTD = keep_qn ? w.RSTD : nullptr;
   pp.qrows = static_cast<long long>(a.tokens) * pp.HQ;
-  const dim3 pgrid(NTmax, a.H);
+  const dim3 pgrid(map.T > 0 ? static_cast<unsigned>(a.N * map.per_seq) : static_cast<unsigned>(NTmax), a.H);
   if (a.safe_gate) {
     if (keep_qn) kda_chunk_prepare_kernel<true, true><<<pgrid, 256, sizeof(PrepSmem), st>>>(pp);
     else kda_chunk_prepare_kernel<false, true><<<pgrid, 256, sizeof(PrepSmem), st>>>(pp);
@@ -760,11 +805,11 @@ extern "C" int kda_chunk_fwd(const kda_chunk_args* args, void* stream) {
   prof_mark(prof, KDA_STAGE_PREPARE, st);
 
   ScanParams sp{};
-  sp.cu = a.cu_seqlens; sp.seq_chunk_off = w.seq_chunk_off; sp.chunk_seq = w.chunk_seq;
+  sp.map = map;
   sp.W = w.W; sp.UT = w.UT; sp.KG = w.KG; sp.QG = w.QG; sp.AQK = w.AQK; sp.GL = w.GL;
   sp.HS = save ? w.HS : nullptr; sp.VNEWT = save ? w.VNEWT : nullptr;
   sp.h0 = a.h0; sp.ht = a.ht; sp.o = static_cast<__nv_bfloat16*>(a.o); sp.status = w.status; sp.dbg = g_dbg_clocks;
-  sp.N = a.N; sp.H = a.H;
+  sp.H = a.H;
   const int slices = scan_slices_for(a.N * a.H, a.scan_slices);
   if ((rc = slices > 1 ? launch_scan_vs(sp, a.N * a.H, st) : launch_scan_tc(sp, a.N * a.H, st)) != KDA_OK) return rc;
   prof_mark(prof, KDA_STAGE_SCAN, st);

@@ -94,10 +94,10 @@ __global__ void __launch_bounds__(VS_THREADS, 1) kda_chunk_scan_vs_kernel(const 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int q4 = warp & 3, half = (warp >> 2) & 1;
   const int unit = blockIdx.x / NS, slice = blockIdx.x % NS;
-  const int seq = unit / p.H, h = unit % p.H;
-  const int c_begin = p.seq_chunk_off[seq], c_end = p.seq_chunk_off[seq + 1];
+  const int seq = p.map.started(unit / p.H), h = unit % p.H;
+  const int c_begin = p.map.first_chunk(seq), c_end = p.map.first_chunk(seq + 1);
   const int nchunks = c_end - c_begin;
-  const long long seq_tok0 = p.cu[seq], seq_tok1 = p.cu[seq + 1];
+  const long long seq_tok0 = p.map.first_token(seq), seq_tok1 = p.map.first_token(seq + 1);
   const int k = 32 * q4 + lane;          // compute thread: its key row = TMEM lane of the state
   const int t = 16 * q4 + lane;          // lanes 0..15 of a quadrant hold rows 16 q4 .. of an M = 64 accumulator
   const int v0 = VS * slice;             // first value column of the slice

@@ -6,8 +6,7 @@
 namespace kda {
 
 struct ScanParams {
-  const int* cu;
-  const int *seq_chunk_off, *chunk_seq;
+  ChunkMap map;
   const unsigned char *W, *UT, *KG, *QG, *AQK, *GL;
   unsigned char *HS, *VNEWT;    // NULL unless saving for backward
   const float* h0;
@@ -15,7 +14,7 @@ struct ScanParams {
   __nv_bfloat16* o;
   unsigned* status;
   long long* dbg;       // development aid: phase clocks (NULL unless built with the clock marks and a buffer is registered)
-  int N, H;
+  int H;
 };
 
 // tcgen05 / TMEM version (kda_chunk_scan_tc.cu); returns KDA_OK, a negative KDA_E_* or a positive cudaError_t
