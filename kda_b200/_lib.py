@@ -169,12 +169,33 @@ def chunk_status(workspace_ptr=None) -> int:
     return int(v.value)
 
 
+def raise_chunk_status(v: int, what: str) -> None:
+    why = "; ".join(t for b, t in STATUS_BITS.items() if v & b) or "unknown bits"
+    raise KdaError(f"{what}: device status 0x{v:x} ({why}); the outputs of this call are incomplete")
+
+
 def check_chunk_status(workspace_ptr, what: str) -> None:
     """Raises KdaError when the chunked kernels reported a problem for this workspace."""
     v = chunk_status(workspace_ptr)
     if v:
-        why = "; ".join(t for b, t in STATUS_BITS.items() if v & b) or "unknown bits"
-        raise KdaError(f"{what}: device status 0x{v:x} ({why}); the outputs of this call are incomplete")
+        raise_chunk_status(v, what)
+
+
+_native = None
+
+
+def native():
+    """The host path of the operators (_kda_torch.so, csrc/host/), loaded once; raises RuntimeError with a build hint."""
+    global _native
+    if _native is None:
+        load()
+        try:
+            from . import _kda_torch
+        except ImportError as e:
+            raise RuntimeError(f"_kda_torch.so is missing or does not load ({e}): build it with `python -m kda_b200.build`") from e
+        _kda_torch.set_errors(KdaError, raise_chunk_status)
+        _native = _kda_torch
+    return _native
 
 
 def profile_read(reset: bool = True) -> dict:

@@ -1,16 +1,19 @@
-"""Builds libkda_b200.so in-tree with nvcc for sm_100a.  `python -m kda_b200.build` or `build()`."""
+"""Builds libkda_b200.so in-tree with nvcc for sm_100a, and the host path on torch tensors (_kda_torch.so) with the C++
+compiler.  `python -m kda_b200.build` or `build()`."""
 from __future__ import annotations
 
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libkda_b200.so")
 DEBUG_LIB = os.path.join(PKG, "libkda_b200_debug.so")      # development checks (csrc/debug/): loaded by tests only
+HOST_LIB = os.path.join(PKG, "_kda_torch.so")                  # csrc/host/: the operators' host path, linked against LIB
 OBJ = os.path.join(PKG, "csrc", "_obj")
 
 NVCC_FLAGS = [
@@ -34,6 +37,19 @@ def sources() -> list[str]:
 def debug_sources() -> list[str]:
     d = os.path.join(CSRC, "debug")
     return sorted(os.path.join(d, f) for f in os.listdir(d) if f.endswith(".cu"))
+
+
+def _host_command() -> list[str]:
+    """g++ line of _kda_torch.so: torch's and Python's headers, libkda_b200.so found next to it at run time."""
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+    inc = include_paths() + [sysconfig.get_paths()["include"], os.path.join(ROOT, "include"),
+                             os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")]
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DNDEBUG",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    cmd += [f"-I{i}" for i in inc if i.startswith(ROOT)] + [a for i in inc if not i.startswith(ROOT) for a in ("-isystem", i)]
+    cmd += [os.path.join(CSRC, "host", "kda_torch.cpp"), "-o", HOST_LIB, f"-L{PKG}", "-l:libkda_b200.so", "-Wl,-rpath,$ORIGIN"]
+    return cmd + [f"-L{d}" for d in library_paths()] + ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
 
 
 def _stale(target: str, deps: list[str]) -> bool:
@@ -79,6 +95,11 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False, 
             if verbose:
                 print(" ".join(cmd), flush=True)
             subprocess.check_call(cmd)
+    if force or _stale(HOST_LIB, [os.path.join(CSRC, "host", "kda_torch.cpp"), os.path.join(ROOT, "include", "kda_b200.h")]):
+        cmd = _host_command()
+        if verbose:
+            print(" ".join(cmd), flush=True)
+        subprocess.check_call(cmd)
     return LIB
 
 

@@ -242,80 +242,9 @@ def fused_recurrent_kda_fwd(q, k, v, g, beta, A_log=None, dt_bias=None, initial_
     from the slot of its first token -- with `num_accepted_tokens` [N] (speculative decoding) from the slot of its
     last accepted token -- and the state after token t lands in slot `ssm_state_indices[n, t]`.
     `transpose_state_layout`: states are [N, H, V, K] instead of [N, H, K, V] (K = 64 or 128)."""
-    B, T, H, K, V = _check_common(q, k, v, g, beta, None, cu_seqlens)
-    if transpose_state_layout and K not in (64, 128):
-        raise NotImplementedError(f"kda_b200: transpose_state_layout needs K = 64 or 128, got {K}")
-    if scale is None:
-        scale = K ** -0.5
-    dev = q.device
-    # the gate activation and the beta sigmoid run inside the recurrent kernels (no separate pass over g and beta)
-    gate_kw = {}
-    if use_gate_in_kernel:
-        assert A_log is not None, "A_log must be provided when use_gate_in_kernel=True."
-        if g.dtype not in _DT:
-            g = g.float()
-        a_log = A_log.detach().to(device=dev, dtype=torch.float32).contiguous()
-        bias = dt_bias.detach().to(device=dev, dtype=torch.float32).contiguous() if dt_bias is not None else None
-        if a_log.numel() != H or (bias is not None and bias.numel() != H * K):
-            raise ValueError(f"A_log must have {H} elements and dt_bias {H * K}")
-        gate_kw.update(A_log=_ptr(a_log), dt_bias=_ptr(bias), g_raw_dtype=_DT[g.dtype],
-                       lower_bound=float(lower_bound) if lower_bound is not None else 0.0,
-                       use_lower_bound=int(lower_bound is not None))
-        g = g.detach().contiguous()
-    else:
-        g = g.contiguous().float()
-    if use_beta_sigmoid_in_kernel:
-        if beta.dtype not in _DT:
-            beta = beta.float()
-        gate_kw.update(beta_sigmoid=1, beta_raw_dtype=_DT[beta.dtype])
-        beta = beta.detach().contiguous()
-    else:
-        beta = beta.contiguous().float()
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    N = B if cu_seqlens is None else len(cu_seqlens) - 1
-    cu = _as_i32(cu_seqlens, dev) if cu_seqlens is not None else None
-    h0 = initial_state.contiguous() if initial_state is not None else None
-    if inplace_final_state:
-        assert initial_state is not None
-        if h0.data_ptr() != initial_state.data_ptr() or h0.dtype != torch.float32:
-            raise ValueError("inplace_final_state needs a contiguous fp32 initial_state")
-        ht = h0
-    elif output_final_state:
-        ht = torch.empty((N, H, V, K) if transpose_state_layout else (N, H, K, V), dtype=torch.float32, device=dev)
-    else:
-        ht = None
-    idx, acc, stride = None, None, 0
-    if ssm_state_indices is not None:
-        if not inplace_final_state:
-            raise ValueError("ssm_state_indices requires inplace_final_state=True")
-        idx = ssm_state_indices.to(device=dev, dtype=torch.int32).contiguous()
-        stride = 1 if idx.ndim == 1 else idx.stride(0)
-        if idx.ndim == 1 and cu_seqlens is None and T > 1:
-            raise ValueError("ssm_state_indices must be [N, T] when a sequence has more than one token")
-        if num_accepted_tokens is not None:
-            acc = num_accepted_tokens.to(device=dev, dtype=torch.int32).contiguous()
-    elif num_accepted_tokens is not None:
-        raise ValueError("num_accepted_tokens requires ssm_state_indices")
-    if out is None:
-        o = torch.empty_like(v)
-    else:
-        assert out.shape == v.shape
-        if not out.is_contiguous() or out.dtype != v.dtype:
-            raise ValueError("`out` must be contiguous and of v's dtype")
-        o = out
-    args = _lib.RecurrentArgs(
-        q=_ptr(q), k=_ptr(k), v=_ptr(v), g=_ptr(g), beta=_ptr(beta), h0=_ptr(h0), ht=_ptr(ht), o=_ptr(o),
-        cu_seqlens=_ptr(cu), state_indices=_ptr(idx), tokens=B * T, N=N, T=T, H=H, K=K, V=V,
-        io_dtype=_DT[q.dtype], use_qk_l2norm=int(bool(use_qk_l2norm_in_kernel)), scale=float(scale),
-        num_accepted_tokens=_ptr(acc), state_indices_stride=stride, transpose_state=int(bool(transpose_state_layout)),
-        HQ=q.shape[2], **gate_kw)
-    with torch.cuda.device(dev):
-        _lib.check(_lib.load().kda_recurrent_fwd(C.byref(args), _stream(dev)), "kda_recurrent_fwd")
-        if _checked():
-            st = _lib.recurrent_status()
-            if st:
-                raise _lib.KdaError(f"kda_recurrent_fwd: device status 0x{st:x} (a bounded wait gave up); the outputs are incomplete")
-    return o, ht
+    return (_lib._native or _lib.native()).recurrent_fwd(
+        q, k, v, g, beta, A_log, dt_bias, initial_state, scale, output_final_state, inplace_final_state, cu_seqlens, ssm_state_indices,
+        num_accepted_tokens, use_qk_l2norm_in_kernel, use_gate_in_kernel, use_beta_sigmoid_in_kernel, lower_bound, out, transpose_state_layout)
 
 
 @torch.no_grad()
@@ -563,6 +492,12 @@ def chunk_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_sta
     chunk_size = kwargs.pop("chunk_size", 64)
     if chunk_size not in (32, 64):
         raise ValueError(f"`chunk_size` must be either 32 or 64 for KDA, got {chunk_size}.")
+    if not return_intermediate_states:
+        r = (_lib._native or _lib.native()).chunk_kda(
+            q, k, v, g, beta, kwargs.get("A_log"), kwargs.get("dt_bias"), initial_state, scale, output_final_state, cu_seqlens, use_qk_l2norm_in_kernel,
+            use_gate_in_kernel, use_beta_sigmoid_in_kernel, lower_bound, safe_gate, transpose_state_layout, SCAN_SLICES)
+        if r is not None:
+            return r
     # chunk_size only selects how the same recurrence is tiled: o, the final state and every gradient are the same
     # function of the inputs for 32 and 64, so both run on the 64-token tiles.  Only the intermediate states depend on
     # it (one state per chunk of that size, see _chunk_fwd_with_states).
