@@ -47,4 +47,11 @@ struct DeviceOnce {
   }
 };
 
+// SMs of the current device
+inline int sm_count() {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
 }  // namespace kda

@@ -60,4 +60,9 @@ __device__ __forceinline__ void tma_load_rows(void* dst_smem, const CUtensorMap*
                : "memory");
 }
 
+// the same box into L2 only
+__device__ __forceinline__ void tma_prefetch_rows(const CUtensorMap* map, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(map), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+
 }  // namespace kda
