@@ -59,7 +59,7 @@ static_assert(UT_OFF % 128 == 0 && TI_OFF + C * TS * 2 <= OP_ROWS * QS * 2, "the
 static_assert(TILE_TK <= C * AS * 4, "the staged W tile must fit Akk");
 static_assert(2 * (sizeof(PrepSmem) + 1024) <= 227 * 1024, "two CTAs per SM");
 
-// Sum over the 32 lanes of N per-lane values at once (N = 8, 16): afterwards lane L holds the total of slot L % N.
+// Sum over the 32 lanes of N per-lane values at once (N = 4, 8): afterwards lane L holds the total of slot L % N.
 template <int N>
 __device__ __forceinline__ float butterfly(float (&v)[N], int lane) {
 #pragma unroll
@@ -221,36 +221,74 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
       }
     }
   }
+  // k waits in this thread's own part of the k Gam tile (its final value replaces it there): eight registers less
+#pragma unroll
+  for (int i = 0; i < 4; ++i) *reinterpret_cast<uint2*>(&s.kG[(t0 + i) * QS + kk]) = k[i];
+  auto key = [&](int i) { return widen(*reinterpret_cast<const uint2*>(&s.kG[(t0 + i) * QS + kk])); };
   __nv_bfloat16* const mine = s.op + op_base(blk) * QS + kk;      // this block's operand rows, this thread's columns
   auto put = [&](int row, const F4& x) { *reinterpret_cast<uint2*>(mine + row * QS) = narrow(x); };
+  // keeps the compiler from carrying widened (fp32) q, k or products of lam from one use to the next: they would not fit the registers
+  auto forget = [&] {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      asm volatile("" : "+r"(q[i].x), "+r"(q[i].y), "+f"(lam[i].a.x), "+f"(lam[i].a.y), "+f"(lam[i].b.x), "+f"(lam[i].b.y));
+  };
   __syncthreads();      // T; Aqk, Akk are cleared
   KDA_DBG_CLOCK(p.dbg, 18);
 
   if constexpr (!SAFE) {
-    // ---- P3a: the 4 x 4 diagonal block of these rows pairwise.  Rows upwards while E_j = k_j prod(j+1 .. t) is carried per column j.
-    // Row t gives t + 1 values q_t.E_j (slots t*t + j) and t values k_t.E_j (slots t*t + t + 1 + j): 16, summed over the lanes at once.
+    // ---- P3a: the 4 x 4 diagonal block of these rows pairwise: E = k_j prod(j+1 .. t) is carried upwards per column j and dotted with
+    // q_t and k_t.  The 16 values are summed over the lanes four at a time (all at once they do not fit the registers beside lam, q,
+    // k, and spills miss the small L1: 2 k cycles of the tile).
     {
-      float val[16];
-      F4 E[4];
+      float val[4];
+      F4 E = key(0), F;
       auto dot = [](const F4& x, const F4& y) { return fmaf(x.b.y, y.b.y, fmaf(x.b.x, y.b.x, fmaf(x.a.y, y.a.y, x.a.x * y.a.x))); };
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const F4 qt = widen(q[t]), kt = widen(k[t]);
-#pragma unroll
-        for (int j = 0; j < t; ++j) E[j] = mul4c(E[j], lam[t]);
-        E[t] = kt;
-#pragma unroll
-        for (int j = 0; j <= t; ++j) val[t * t + j] = dot(qt, E[j]);
-#pragma unroll
-        for (int j = 0; j < t; ++j) val[t * t + t + 1 + j] = dot(kt, E[j]);
+      val[0] = dot(widen(q[0]), E);
+      E = mul4c(E, lam[1]);
+      F = key(1);
+      val[2] = dot(F, E);
+      {
+        const F4 qt = widen(q[1]);
+        val[1] = dot(qt, E);
+        val[3] = dot(qt, F);
       }
-      const float x = butterfly<16>(val, lane);
-      if (lane < 16) {
-        const int t = (lane >= 9) ? 3 : (lane >= 4) ? 2 : (lane >= 1) ? 1 : 0, off = lane - t * t;
-        if (off > t) s.Akk[(t0 + t) * AS + t0 + off - t - 1] = x;                            // raw; beta_t is applied later
-        else s.Aqk[(t0 + t) * TS + t0 + off] = __float2bfloat16_rn(p.scale * x);
+      float x = butterfly<4>(val, lane);
+      auto two_rows = [&] {            // rows 2 and 3 against the column carried in E
+        E = mul4c(E, lam[2]);
+        val[0] = dot(widen(q[2]), E);
+        val[1] = dot(key(2), E);
+        E = mul4c(E, lam[3]);
+        val[2] = dot(widen(q[3]), E);
+        val[3] = dot(key(3), E);
+        return butterfly<4>(val, lane);
+      };
+      float y = two_rows();
+      x = (lane & 4) ? y : x;
+      forget();
+      E = key(1);
+      y = two_rows();
+      x = (lane & 12) == 8 ? y : x;
+      forget();
+      E = key(2);
+      val[0] = dot(widen(q[2]), E);
+      E = mul4c(E, lam[3]);
+      F = key(3);
+      val[3] = dot(F, E);
+      {
+        const F4 qt = widen(q[3]);
+        val[1] = dot(qt, F);
+        val[2] = dot(qt, E);
+      }
+      y = butterfly<4>(val, lane);
+      x = (lane & 12) == 12 ? y : x;
+      if (lane < 16) {      // row, column (two bits per lane) and matrix of the lane's value
+        const int r = t0 + ((0xfefafa54u >> (2 * lane)) & 3), cl = t0 + ((0xae550040u >> (2 * lane)) & 3);
+        if ((0x8aa4u >> lane) & 1) s.Akk[r * AS + cl] = x;                            // raw; beta_t is applied later
+        else s.Aqk[r * TS + cl] = __float2bfloat16_rn(p.scale * x);
       }
     }
+    forget();
     // ---- P3b: operands of levels 8 and 4
     if (quad >= 2) {                                    // rows 8..15: prod(8 .. i)
       F4 f = quad == 3 ? mul4c(lds4(&s.T[warp - 1][kk]), lam[0]) : lam[0];
@@ -258,16 +296,17 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
       for (int i = 0; i < 4; ++i) {
         if (i > 0) f = mul4c(f, lam[i]);
         put(4 * (quad - 2) + i, mul4c(widen(q[i]), f));
-        put(8 + 4 * (quad - 2) + i, mul4c(widen(k[i]), f));
+        put(8 + 4 * (quad - 2) + i, mul4c(key(i), f));
       }
     } else {                                            // columns 0..7: prod(j+1 .. 7)
       F4 f = quad == 0 ? lds4(&s.T[warp + 1][kk]) : splat(1.f);
 #pragma unroll
       for (int j = 3; j >= 0; --j) {
         if (j < 3) f = mul4c(f, lam[j + 1]);
-        put(OP_B8 + 4 * quad + j, mul4c(widen(k[j]), f));
+        put(OP_B8 + 4 * quad + j, mul4c(key(j), f));
       }
     }
+    forget();
     const int u = quad >> 1;
     if (quad & 1) {                                     // rows 4..7, 12..15: prod from row 4, 12
       F4 f = lam[0];
@@ -275,15 +314,15 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
       for (int i = 0; i < 4; ++i) {
         if (i > 0) f = mul4c(f, lam[i]);
         put(OP_A4 + 8 * u + i, mul4c(widen(q[i]), f));
-        put(OP_A4 + 8 * u + 4 + i, mul4c(widen(k[i]), f));
+        put(OP_A4 + 8 * u + 4 + i, mul4c(key(i), f));
       }
     } else {                                            // columns 0..3, 8..11: prod up to row 3, 11
-      put(OP_B4 + 4 * u + 3, widen(k[3]));
+      put(OP_B4 + 4 * u + 3, key(3));
       F4 f = lam[3];
 #pragma unroll
       for (int j = 2; j >= 0; --j) {
         if (j < 2) f = mul4c(f, lam[j + 1]);
-        put(OP_B4 + 4 * u + j, mul4c(widen(k[j]), f));
+        put(OP_B4 + 4 * u + j, mul4c(key(j), f));
       }
     }
   } else {
@@ -298,8 +337,8 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
       for (int i = 0; i < 4; ++i) {
         if (i > 0) f = mul4c(f, lam[i]);
         put(4 * quad + i, mul4c(widen(q[i]), f));
-        put(16 + 4 * quad + i, mul4c(widen(k[i]), f));
-        put(32 + 4 * quad + i, mul4c(widen(k[i]), inv(f)));
+        put(16 + 4 * quad + i, mul4c(key(i), f));
+        put(32 + 4 * quad + i, mul4c(key(i), inv(f)));
       }
     } else {
       F4 f = quad == 0 ? lds4(&s.T[warp + 1][kk]) : splat(1.f);
@@ -308,13 +347,14 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
         if (i < 3) f = mul4c(f, lam[i + 1]);
         const F4 r = inv(f);
         put(4 * quad + i, mul4c(widen(q[i]), r));
-        put(16 + 4 * quad + i, mul4c(widen(k[i]), r));
-        put(32 + 4 * quad + i, mul4c(widen(k[i]), f));
+        put(16 + 4 * quad + i, mul4c(key(i), r));
+        put(32 + 4 * quad + i, mul4c(key(i), f));
       }
     }
   }
   asm volatile("bar.sync %0, 128;" ::"r"(1 + blk) : "memory");      // the four warps of this 16-row block
   KDA_DBG_CLOCK(p.dbg, 19);
+  forget();
   const __nv_bfloat16* const part = s.op + op_base(blk) * QS;
   if constexpr (!SAFE) {
     float a[1][4];
@@ -359,9 +399,31 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
     unsigned char* const gQG = p.QG + tile * TILE_TK + toff;
     unsigned char* const gKG = p.KG + tile * TILE_TK + toff;
     const uint32_t piece = (lane & 15) >> 1;
-    // decay over the rows of the block in front of these and behind them; over the blocks in front and behind
-    F4 f = lam[0], pre = splat(1.f);
+    // columns seen from the blocks behind: distance 1 needs only this block's rest, 2 and 3 the blocks in between
+    F4 f = splat(1.f);
+    for (int w = warp + 1; w < 4 * blk + 4; ++w) f = mul4c(f, lds4(&s.T[w][kk]));
+    {
+      F4 post = splat(1.f), m2 = splat(1.f), m3 = splat(1.f);
+      for (int b = blk + 1; b < 4; ++b) {
+        if (b == blk + 2) m2 = post;
+        if (b == blk + 3) m3 = post;
+        post = mul4c(post, lds4(&s.TB[b][kk]));
+      }
+      const int cb = (blk > 0 ? 32 : 0) + 4 * quad;
+#pragma unroll
+      for (int i = 3; i >= 0; --i) {                    // f = prod(i+1 .. last row of the block)
+        if (i < 3) f = mul4c(f, lam[i + 1]);
+        const F4 kf = mul4c(key(i), f);
+        *reinterpret_cast<uint2*>(gKG + i * 128 + ((piece ^ ((t0 + i) & 7)) << 4)) = narrow(mul4c(kf, post));
+        if (blk < 3) put(cb + i, kf);
+        if (blk < 2) put(cb + 16 + i, mul4c(kf, m2));
+        if (blk < 1) put(cb + 32 + i, mul4c(kf, m3));
+      }
+    }
+    // decay over the rows of the block in front of these; over the blocks in front
+    f = lam[0];
     for (int w = 4 * blk; w < warp; ++w) f = mul4c(f, lds4(&s.T[w][kk]));
+    F4 pre = splat(1.f);
     for (int b = 0; b < blk; ++b) pre = mul4c(pre, lds4(&s.TB[b][kk]));
     if (warp == 15) {
       const F4 gl = mul4c(pre, lds4(&s.TB[3][kk]));
@@ -371,32 +433,13 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
 #pragma unroll
     for (int i = 0; i < 4; ++i) {                       // f = prod(first row of the block .. i)
       if (i > 0) f = mul4c(f, lam[i]);
-      const F4 qf = mul4c(widen(q[i]), f), kf = mul4c(widen(k[i]), f);
+      const F4 qf = mul4c(widen(q[i]), f), kf = mul4c(key(i), f);
       if (blk > 0) {
         put(4 * quad + i, qf);
         put(16 + 4 * quad + i, kf);
       }
       *reinterpret_cast<uint2*>(gQG + i * 128 + ((piece ^ ((t0 + i) & 7)) << 4)) = narrow(mul4c(qf, preq));
       *reinterpret_cast<uint2*>(&s.kG[(t0 + i) * QS + kk]) = narrow(mul4c(kf, pre));
-    }
-    // columns seen from the blocks behind: distance 1 needs only this block's rest, 2 and 3 the blocks in between
-    f = splat(1.f);
-    for (int w = warp + 1; w < 4 * blk + 4; ++w) f = mul4c(f, lds4(&s.T[w][kk]));
-    F4 post = splat(1.f), m2 = splat(1.f), m3 = splat(1.f);
-    for (int b = blk + 1; b < 4; ++b) {
-      if (b == blk + 2) m2 = post;
-      if (b == blk + 3) m3 = post;
-      post = mul4c(post, lds4(&s.TB[b][kk]));
-    }
-    const int cb = (blk > 0 ? 32 : 0) + 4 * quad;
-#pragma unroll
-    for (int i = 3; i >= 0; --i) {                      // f = prod(i+1 .. last row of the block)
-      if (i < 3) f = mul4c(f, lam[i + 1]);
-      const F4 kf = mul4c(widen(k[i]), f);
-      *reinterpret_cast<uint2*>(gKG + i * 128 + ((piece ^ ((t0 + i) & 7)) << 4)) = narrow(mul4c(kf, post));
-      if (blk < 3) put(cb + i, kf);
-      if (blk < 2) put(cb + 16 + i, mul4c(kf, m2));
-      if (blk < 1) put(cb + 32 + i, mul4c(kf, m3));
     }
   }
   __syncthreads();
