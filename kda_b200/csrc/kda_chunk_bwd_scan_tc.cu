@@ -49,7 +49,7 @@ __device__ __forceinline__ unsigned char* swq(unsigned char* tile, int row, int 
 
 __global__ void __launch_bounds__(RNT, 1) kda_chunk_bwd_scan_tc_kernel(const __grid_constant__ RScanParams p) {
   extern __shared__ unsigned char smem_raw[];
-  TcRScanSmem& s = *reinterpret_cast<TcRScanSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  TcRScanSmem& s = *reinterpret_cast<TcRScanSmem*>(smem_raw + pad_to_1024(smem_raw));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int q4 = warp & 3, half = warp >> 2;
   const int seq = p.map.started(blockIdx.x / p.H), h = blockIdx.x % p.H;

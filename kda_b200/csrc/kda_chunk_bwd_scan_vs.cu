@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(RVS_THREADS, 1) kda_chunk_bwd_scan_vs_kernel(c
   constexpr int C_H = 0, C_VN = VS;      // TMEM columns
   constexpr uint32_t TM_COLS = 2 * VS < 32 ? 32 : 2 * VS;
   extern __shared__ unsigned char smem_raw[];
-  RvsSmem<VS>& s = *reinterpret_cast<RvsSmem<VS>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  RvsSmem<VS>& s = *reinterpret_cast<RvsSmem<VS>*>(smem_raw + pad_to_1024(smem_raw));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int q4 = warp & 3, half = (warp >> 2) & 1;
   const int unit = blockIdx.x / NS, slice = blockIdx.x % NS;

@@ -93,7 +93,7 @@ __device__ __forceinline__ unsigned char* sw_piece(unsigned char* tile, int row,
 template <bool L2>
 __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __grid_constant__ MainParams p) {
   extern __shared__ unsigned char smem_raw[];
-  TcSmem& s = *reinterpret_cast<TcSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  TcSmem& s = *reinterpret_cast<TcSmem*>(smem_raw + pad_to_1024(smem_raw));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int q4 = warp & 3, part = warp >> 2;          // TMEM lane quadrant of this warp; which 16 of the 64 columns
   const long long total_tiles = static_cast<long long>(p.map.total()) * p.H;

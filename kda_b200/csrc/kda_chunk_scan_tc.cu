@@ -54,7 +54,7 @@ __device__ __forceinline__ unsigned char* swp(unsigned char* tile, int row, int 
 
 __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanParams p) {
   extern __shared__ unsigned char smem_raw[];
-  TcScanSmem& s = *reinterpret_cast<TcScanSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  TcScanSmem& s = *reinterpret_cast<TcScanSmem*>(smem_raw + pad_to_1024(smem_raw));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int q4 = warp & 3, half = warp >> 2;
   const int seq = p.map.started(blockIdx.x / p.H), h = blockIdx.x % p.H;

@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(VS_THREADS, 1) kda_chunk_scan_vs_kernel(const 
   constexpr int HC = VS / 2;             // columns per compute thread (two column halves)
   constexpr int C_H = 0, C_VN = VS, C_O = 2 * VS;      // TMEM columns; o double buffered: C_O + VS * (chunk & 1)
   extern __shared__ unsigned char smem_raw[];
-  VsSmem<VS>& s = *reinterpret_cast<VsSmem<VS>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  VsSmem<VS>& s = *reinterpret_cast<VsSmem<VS>*>(smem_raw + pad_to_1024(smem_raw));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int q4 = warp & 3, half = (warp >> 2) & 1;
   const int unit = blockIdx.x / NS, slice = blockIdx.x % NS;

@@ -74,6 +74,11 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// Bytes from `p` (dynamic shared memory) to the next multiple of 1024.  Used as an offset on the array itself: rounding the pointer's
+// integer value up instead hides from the compiler that it points to shared memory, and every access through it becomes a
+// generic one (64-bit address, longer latency): the per-chunk backward took 3.78 instead of 3.51 ms, the sliced scan 867 instead of 759 us.
+__device__ __forceinline__ uint32_t pad_to_1024(const void* p) { return (1024u - (smem_u32(p) & 1023u)) & 1023u; }
+
 __device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));

@@ -70,7 +70,7 @@ __device__ __forceinline__ float butterfly_sum16(float (&v)[16], int lane) {
 template <typename IO, bool TR, bool GATE>
 __global__ void __launch_bounds__(DEC_THREADS, 1) kda_decode_bulk_kernel(const kda_recurrent_args a) {
   extern __shared__ unsigned char smem_raw[];
-  DecSmem& s = *reinterpret_cast<DecSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+  DecSmem& s = *reinterpret_cast<DecSmem*>(smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const long long total = static_cast<long long>(a.N) * a.H;
   const int HQ = a.HQ > 0 ? a.HQ : a.H, grp = a.H / HQ;
