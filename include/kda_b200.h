@@ -231,6 +231,7 @@ int kda_chunk_bwd(const kda_chunk_args* args, void* stream);
 #define KDA_STATUS_SCAN_MMA_WAIT 0x2u       /* forward scan: a product did not complete */
 #define KDA_STATUS_BWD_SCAN_LOAD_WAIT 0x4u  /* reverse scan: operand tiles of a chunk did not arrive */
 #define KDA_STATUS_BWD_SCAN_MMA_WAIT 0x8u   /* reverse scan: a product did not complete */
+#define KDA_STATUS_PREP_LOAD_WAIT 0x10u     /* per-chunk preparation: v did not arrive */
 #define KDA_STATUS_BWD_MAIN_LOAD_WAIT 0x20u /* per-chunk backward: a tile's loads did not arrive */
 #define KDA_STATUS_BWD_MAIN_MMA_WAIT 0x40u  /* per-chunk backward: a product did not complete */
 #define KDA_STATUS_BAD_CU_SEQLENS 0x100u    /* cu_seqlens is not a non-decreasing sequence within [0, tokens]: nothing was computed */

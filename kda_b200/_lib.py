@@ -157,6 +157,7 @@ def recurrent_status() -> int:
 
 STATUS_BITS = {0x1: "forward scan: operand tiles did not arrive", 0x2: "forward scan: a product did not complete",
                0x4: "reverse scan: operand tiles did not arrive", 0x8: "reverse scan: a product did not complete",
+               0x10: "per-chunk preparation: v did not arrive",
                0x20: "per-chunk backward: a tile's loads did not arrive", 0x40: "per-chunk backward: a product did not complete",
                0x100: "cu_seqlens is inconsistent with the number of tokens: nothing was computed"}
 

@@ -180,7 +180,7 @@ extern "C" int kda_chunk_fwd(const kda_chunk_args* args, void* stream) {
   pp.q = static_cast<const __nv_bfloat16*>(a.q);
   pp.k = static_cast<const __nv_bfloat16*>(a.k);
   pp.v = static_cast<const __nv_bfloat16*>(a.v);
-  pp.g = a.g; pp.beta = a.beta; pp.map = map; pp.status = a.cu_seqlens ? nullptr : w.status;
+  pp.g = a.g; pp.beta = a.beta; pp.map = map; pp.status = w.status; pp.clear_status = a.cu_seqlens == nullptr;
   pp.W = w.W; pp.UT = w.UT; pp.KG = w.KG; pp.QG = w.QG; pp.AQK = w.AQK; pp.GL = w.GL; pp.TI = save ? w.TI : nullptr; pp.RKK = save ? w.RKK : nullptr;
   pp.dbg = g_dbg_clocks; pp.H = a.H; pp.use_l2norm = a.use_qk_l2norm; pp.scale = a.scale;
   pp.HQ = a.HQ > 0 ? a.HQ : a.H; pp.grp = a.H / pp.HQ;

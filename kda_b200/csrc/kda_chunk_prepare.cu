@@ -33,7 +33,8 @@ constexpr int DS = 20;    // floats per row of a 16 x 16 fp32 block
 //   levels 8 and 4:  A8 16 rows (q 8..15, k 8..15) | B8 8 | A4 16 (q 4..7, k 4..7, q 12..15, k 12..15) | B4 8
 //   SAFE diagonal:   q 16 | k 16 (row side) | k 16 (column side)
 //   level 16:        blocks 1..3: q 16 | k 16; then columns for the blocks at distance 1, 2, 3 (16 rows each)
-// Afterwards the region holds v (64 rows), the staged UT tile and Tm as bf16 (times beta: TB; plain: TI).
+// Afterwards the region holds v (two 64-column tiles in the 128-byte swizzle), the staged UT tile and Tm as bf16 (times beta: TB;
+// plain: TI, in its tile image).
 constexpr int OP_ROWS = 208;
 constexpr int OP_B8 = 16, OP_A4 = 24, OP_B4 = 40;
 __device__ __forceinline__ int op_base(int blk) { return blk == 0 ? 0 : 48 * blk + (blk > 1 ? 16 : 0); }      // 48, 64, 48, 48 rows
@@ -41,9 +42,9 @@ __device__ __forceinline__ int op_cols(int blk, int dist) { return op_base(blk) 
 
 struct PrepSmem {
   __nv_bfloat16 op[OP_ROWS * QS];
-  __nv_bfloat16 kG[C * QS];    // k * Gam
-  float Akk[C * AS];           // raw <k_t D, k_j>; at the end the staged W tile
-  __nv_bfloat16 Aqk[C * TS];   // scale <q_t D, k_j>, lower triangle incl. diagonal
+  __nv_bfloat16 kG[C * QS];    // k, then k * Gam
+  float Akk[C * AS];           // raw <k_t D, k_j> below the diagonal (nothing else is written); at the end the staged W tile
+  unsigned char Aqk[TILE_TT];  // scale <q_t D, k_j>, lower triangle incl. diagonal: the tile image that leaves by a bulk store
   union {
     float T[16][KD];             // decay over every four rows (P2, P3)
     struct {
@@ -53,11 +54,13 @@ struct PrepSmem {
   };
   float TB[4][KD];               // decay over every 16-row block
   float beta[C];
+  uint64_t barV;
 };
-constexpr int UT_OFF = C * QS * 2, TB_OFF = UT_OFF + static_cast<int>(TILE_VT), TI_OFF = TB_OFF + C * TS * 2;      // bytes, behind v
-static_assert(UT_OFF % 128 == 0 && TI_OFF + C * TS * 2 <= OP_ROWS * QS * 2, "the last phase's tiles must fit the operand region");
+constexpr int UT_OFF = static_cast<int>(TILE_TK), TI_OFF = UT_OFF + static_cast<int>(TILE_VT), TB_OFF = TI_OFF + static_cast<int>(TILE_TT);      // bytes, behind v
+static_assert(TB_OFF + C * TS * 2 <= OP_ROWS * QS * 2, "the last phase's tiles must fit the operand region");
 static_assert(TILE_TK <= C * AS * 4, "the staged W tile must fit Akk");
-static_assert(2 * (sizeof(PrepSmem) + 1024) <= 227 * 1024, "two CTAs per SM");
+constexpr int PREP_SMEM = static_cast<int>(sizeof(PrepSmem)) + 1024;      // 1024-byte alignment for the swizzled v tiles
+static_assert(2 * (PREP_SMEM + 1024) <= 227 * 1024, "two CTAs per SM");
 
 // Sum over the 32 lanes of N per-lane values at once (N = 4, 8): afterwards lane L holds the total of slot L % N.
 template <int N>
@@ -77,23 +80,51 @@ __device__ __forceinline__ float butterfly(float (&v)[N], int lane) {
   return v[0];
 }
 
-// two fp32 products in one instruction (sm_100: packed fp32 pairs)
-__device__ __forceinline__ float2 mul2(const float2 a, const float2 b) {
-  float2 d;
-  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mul.rn.ftz.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}\n"
-      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+// Four adjacent key columns in fp32, as two packed pairs (sm_100 multiplies a pair in one instruction).
+using f32x2 = unsigned long long;
+struct F4 { f32x2 a, b; };
+__device__ __forceinline__ f32x2 pair(float x, float y) {
+  f32x2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
   return d;
 }
-// four adjacent key columns in fp32
-struct F4 { float2 a, b; };
-__device__ __forceinline__ F4 mul4c(const F4& x, const F4& y) { return {mul2(x.a, y.a), mul2(x.b, y.b)}; }
-__device__ __forceinline__ F4 widen(const uint2 u) { return {unpack_bf16(u.x), unpack_bf16(u.y)}; }
-__device__ __forceinline__ uint2 narrow(const F4& x) { return make_uint2(pack_bf16(x.a.x, x.a.y), pack_bf16(x.b.x, x.b.y)); }
-__device__ __forceinline__ F4 lds4(const float* p) {
-  const float4 v = *reinterpret_cast<const float4*>(p);
-  return {make_float2(v.x, v.y), make_float2(v.z, v.w)};
+__device__ __forceinline__ float2 halves(f32x2 v) {
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(v));
+  return d;
 }
-__device__ __forceinline__ F4 splat(float x) { return {make_float2(x, x), make_float2(x, x)}; }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ F4 mul4c(const F4& x, const F4& y) { return {mul2(x.a, y.a), mul2(x.b, y.b)}; }
+__device__ __forceinline__ f32x2 widen2(uint32_t u) {      // two bf16 -> two fp32
+  f32x2 d;
+  asm("{\n .reg .b32 lo, hi;\n shl.b32 lo, %1, 16;\n and.b32 hi, %1, 0xffff0000;\n mov.b64 %0, {lo, hi};\n}\n" : "=l"(d) : "r"(u));
+  return d;
+}
+__device__ __forceinline__ uint32_t narrow2(f32x2 v) {
+  const float2 f = halves(v);
+  return pack_bf16(f.x, f.y);
+}
+__device__ __forceinline__ F4 widen(const uint2 u) { return {widen2(u.x), widen2(u.y)}; }
+__device__ __forceinline__ uint2 narrow(const F4& x) { return make_uint2(narrow2(x.a), narrow2(x.b)); }
+__device__ __forceinline__ F4 lds4(const float* p) {
+  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+  return {v.x, v.y};
+}
+__device__ __forceinline__ void sts4(float* p, const F4& x) { *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(x.a, x.b); }
+__device__ __forceinline__ F4 splat(float x) { return {pair(x, x), pair(x, x)}; }
+__device__ __forceinline__ float dot(const F4& x, const F4& y) {
+  const float2 v = halves(fma2(x.b, y.b, mul2(x.a, y.a)));
+  return v.x + v.y;
+}
 // read-once global loads: no L1 allocation
 __device__ __forceinline__ uint2 ldg_u2(const void* p) {
   uint2 r;
@@ -141,12 +172,12 @@ __device__ __forceinline__ void prep_mma(float (&acc)[NB][4], const __nv_bfloat1
 // SAFE: the caller promises bounded gates (safe_gate: at least -5 per token), see above.
 template <bool KEEP_QN, bool SAFE>
 __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(const __grid_constant__ PrepParams p) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  PrepSmem& s = *reinterpret_cast<PrepSmem*>(smem_raw);
+  extern __shared__ unsigned char smem_raw[];
+  PrepSmem& s = *reinterpret_cast<PrepSmem*>(smem_raw + pad_to_1024(smem_raw));
   const int tid = threadIdx.x, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);      // warp-uniform for the compiler: role branches need no reconvergence code
   const int c = blockIdx.x / p.H, h = blockIdx.x % p.H;        // neighbouring CTAs take neighbouring heads: contiguous rows and tiles
-  if (p.status && blockIdx.x == 0 && tid < 4) p.status[tid] = 0u;
+  if (p.clear_status && blockIdx.x == 0 && tid < 4) p.status[tid] = 0u;
   if (c >= p.map.total()) return;
   const ChunkInfo ci = p.map.info(c);
   const int len = ci.len;
@@ -167,12 +198,14 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
     for (int i = 0; i < 4; ++i) {
       const bool ok = t0 + i < len;      // warp-uniform
       const float4 g4 = ok ? ldg_f4(gp + i * gs) : make_float4(0.f, 0.f, 0.f, 0.f);
-      lam[i] = {make_float2(g4.x, g4.y), make_float2(g4.z, g4.w)};
+      lam[i] = {pair(g4.x, g4.y), pair(g4.z, g4.w)};
       q[i] = ok ? ldg_u2(qp + i * qs) : make_uint2(0u, 0u);
       k[i] = ok ? ldg_u2(kp + i * qs) : make_uint2(0u, 0u);
     }
-    // the tile that will run here next: its inputs into L2 (four tiled prefetches by one thread)
+    // the tile that will run here next: its inputs into L2 (tiled prefetches by one thread)
     if (tid == 0) {
+      mbar_init(&s.barV, 1);
+      fence_mbar_init();
       const long long nt = static_cast<long long>(blockIdx.x) + p.ahead;
       if (nt < static_cast<long long>(p.map.total()) * p.H) {
         const int tok = static_cast<int>(p.map.info(static_cast<int>(nt / p.H)).tok0), hn = static_cast<int>(nt % p.H);
@@ -180,23 +213,23 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
         tma_prefetch_rows(&p.tm_q, 0, hn / p.grp, tok);
         tma_prefetch_rows(&p.tm_k, 0, hn / p.grp, tok);
         tma_prefetch_rows(&p.tm_v, 0, hn, tok);
+        tma_prefetch_rows(&p.tm_v, 64, hn, tok);
       }
     }
-    for (int i = tid; i < C * AS / 4; i += PREP_THREADS) reinterpret_cast<float4*>(s.Akk)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int i = tid; i < C * TS / 8; i += PREP_THREADS) reinterpret_cast<uint4*>(s.Aqk)[i] = make_uint4(0u, 0u, 0u, 0u);
+    static_assert(TILE_TT == 16 * PREP_THREADS, "one piece per thread");
+    reinterpret_cast<uint4*>(s.Aqk)[tid] = make_uint4(0u, 0u, 0u, 0u);
     if (tid < C) s.beta[tid] = tid < len ? __ldg(p.beta + static_cast<size_t>(ci.tok0 + tid) * p.H + h) : 0.f;
   }
   KDA_DBG_CLOCK(p.dbg, 17);
   // ---- P2: lam, the decay over these four rows -------------------------------------------------------------------------
   {
-    const float2 le = make_float2(LOG2E, LOG2E);
+    const f32x2 le = pair(LOG2E, LOG2E);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const float2 x = mul2(lam[i].a, le), y = mul2(lam[i].b, le);
-      lam[i] = {make_float2(ex2(x.x), ex2(x.y)), make_float2(ex2(y.x), ex2(y.y))};
+      const float2 x = halves(mul2(lam[i].a, le)), y = halves(mul2(lam[i].b, le));
+      lam[i] = {pair(ex2(x.x), ex2(x.y)), pair(ex2(y.x), ex2(y.y))};
     }
-    const F4 tot = mul4c(mul4c(lam[0], lam[1]), mul4c(lam[2], lam[3]));
-    *reinterpret_cast<float4*>(&s.T[warp][kk]) = make_float4(tot.a.x, tot.a.y, tot.b.x, tot.b.y);
+    sts4(&s.T[warp][kk], mul4c(mul4c(lam[0], lam[1]), mul4c(lam[2], lam[3])));
   }
   // ---- P1b: optional L2 normalisation of q and k rows (result rounded to bf16, as the unfused op does)
   if (p.use_l2norm) {
@@ -204,8 +237,8 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const F4 x = widen(q[i]), y = widen(k[i]);
-      ss[i] = fmaf(x.a.x, x.a.x, fmaf(x.a.y, x.a.y, fmaf(x.b.x, x.b.x, x.b.y * x.b.y)));
-      ss[4 + i] = fmaf(y.a.x, y.a.x, fmaf(y.a.y, y.a.y, fmaf(y.b.x, y.b.x, y.b.y * y.b.y)));
+      ss[i] = dot(x, x);
+      ss[4 + i] = dot(y, y);
     }
     const float r = rsqrtf(butterfly<8>(ss, lane) + L2NORM_EPS);      // slots 0..3: q rows, 4..7: k rows
     const bool keep = KEEP_QN && p.QN != nullptr && h % p.grp == 0;      // once per q/k head
@@ -231,9 +264,9 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
   auto forget = [&] {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-      asm volatile("" : "+r"(q[i].x), "+r"(q[i].y), "+f"(lam[i].a.x), "+f"(lam[i].a.y), "+f"(lam[i].b.x), "+f"(lam[i].b.y));
+      asm volatile("" : "+r"(q[i].x), "+r"(q[i].y), "+l"(lam[i].a), "+l"(lam[i].b));
   };
-  __syncthreads();      // T; Aqk, Akk are cleared
+  __syncthreads();      // T; Aqk is cleared
   KDA_DBG_CLOCK(p.dbg, 18);
 
   if constexpr (!SAFE) {
@@ -243,7 +276,6 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
     {
       float val[4];
       F4 E = key(0), F;
-      auto dot = [](const F4& x, const F4& y) { return fmaf(x.b.y, y.b.y, fmaf(x.b.x, y.b.x, fmaf(x.a.y, y.a.y, x.a.x * y.a.x))); };
       val[0] = dot(widen(q[0]), E);
       E = mul4c(E, lam[1]);
       F = key(1);
@@ -285,7 +317,7 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
       if (lane < 16) {      // row, column (two bits per lane) and matrix of the lane's value
         const int r = t0 + ((0xfefafa54u >> (2 * lane)) & 3), cl = t0 + ((0xae550040u >> (2 * lane)) & 3);
         if ((0x8aa4u >> lane) & 1) s.Akk[r * AS + cl] = x;                            // raw; beta_t is applied later
-        else s.Aqk[r * TS + cl] = __float2bfloat16_rn(p.scale * x);
+        else *reinterpret_cast<__nv_bfloat16*>(s.Aqk + swz<128>(r, cl)) = __float2bfloat16_rn(p.scale * x);
       }
     }
     forget();
@@ -329,7 +361,8 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
     // ---- P3b, bounded gates: the diagonal 16 x 16 blocks whole, cut between rows 7 and 8: row side prod(8 .. t) above the cut and
     // 1 / prod(t+1 .. 7) below it, column side the reciprocals (every factor within 2^58 under the bound)
     auto inv = [](const F4& f) {
-      return F4{make_float2(__fdividef(1.f, f.a.x), __fdividef(1.f, f.a.y)), make_float2(__fdividef(1.f, f.b.x), __fdividef(1.f, f.b.y))};
+      const float2 a = halves(f.a), b = halves(f.b);
+      return F4{pair(__fdividef(1.f, a.x), __fdividef(1.f, a.y)), pair(__fdividef(1.f, b.x), __fdividef(1.f, b.y))};
     };
     if (quad >= 2) {
       F4 f = quad == 3 ? mul4c(lds4(&s.T[warp - 1][kk]), lam[0]) : lam[0];
@@ -361,13 +394,13 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
     if (quad == 0) {             // level 8: accumulator rows 0..7: q rows 8.., rows 8..15: k rows 8..
       prep_mma<1>(a, part, part + OP_B8 * QS, lane);
       const int row = b0 + 8 + gid, col = b0 + 2 * tig;
-      *reinterpret_cast<uint32_t*>(&s.Aqk[row * TS + col]) = pack_bf16(p.scale * a[0][0], p.scale * a[0][1]);
+      *reinterpret_cast<uint32_t*>(s.Aqk + swz<128>(row, col)) = pack_bf16(p.scale * a[0][0], p.scale * a[0][1]);
       *reinterpret_cast<float2*>(&s.Akk[row * AS + col]) = make_float2(a[0][2], a[0][3]);
     } else if (quad == 1) {      // level 4: accumulator rows 0..7 (q 4..7, k 4..7) go with columns 0..3, rows 8..15 (q, k 12..15) with columns 4..7
       prep_mma<1>(a, part + OP_A4 * QS, part + OP_B4 * QS, lane);
       const int u = tig >> 1, row = b0 + 8 * u + 4 + (gid & 3), col = b0 + 8 * u + 2 * (tig & 1);
       const float x = u ? a[0][2] : a[0][0], y = u ? a[0][3] : a[0][1];
-      if (gid < 4) *reinterpret_cast<uint32_t*>(&s.Aqk[row * TS + col]) = pack_bf16(p.scale * x, p.scale * y);
+      if (gid < 4) *reinterpret_cast<uint32_t*>(s.Aqk + swz<128>(row, col)) = pack_bf16(p.scale * x, p.scale * y);
       else *reinterpret_cast<float2*>(&s.Akk[row * AS + col]) = make_float2(x, y);
     }
   } else {
@@ -382,13 +415,12 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
       *reinterpret_cast<float2*>(&s.Akk[(b0 + ra) * AS + b0 + col]) = make_float2(v0, v1);
       *reinterpret_cast<float2*>(&s.Akk[(b0 + rb) * AS + b0 + col]) = make_float2(v2, v3);
     } else {
-      *reinterpret_cast<uint32_t*>(&s.Aqk[(b0 + ra) * TS + b0 + col]) = pack_bf16(p.scale * v0, p.scale * v1);
-      *reinterpret_cast<uint32_t*>(&s.Aqk[(b0 + rb) * TS + b0 + col]) = pack_bf16(p.scale * v2, p.scale * v3);
+      *reinterpret_cast<uint32_t*>(s.Aqk + swz<128>((b0 + ra), b0 + col)) = pack_bf16(p.scale * v0, p.scale * v1);
+      *reinterpret_cast<uint32_t*>(s.Aqk + swz<128>((b0 + rb), b0 + col)) = pack_bf16(p.scale * v2, p.scale * v3);
     }
   }
   if (quad == 3) {               // the decay over the whole block, for the next phase
-    const F4 tot = mul4c(mul4c(lds4(&s.T[warp - 3][kk]), lds4(&s.T[warp - 2][kk])), mul4c(lds4(&s.T[warp - 1][kk]), lds4(&s.T[warp][kk])));
-    *reinterpret_cast<float4*>(&s.TB[blk][kk]) = make_float4(tot.a.x, tot.a.y, tot.b.x, tot.b.y);
+    sts4(&s.TB[blk][kk], mul4c(mul4c(lds4(&s.T[warp - 3][kk]), lds4(&s.T[warp - 2][kk])), mul4c(lds4(&s.T[warp - 1][kk]), lds4(&s.T[warp][kk]))));
   }
   __syncthreads();      // the level 8 / 4 operands have been read; TB is there
   KDA_DBG_CLOCK(p.dbg, 20);
@@ -401,13 +433,19 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
     const uint32_t piece = (lane & 15) >> 1;
     // columns seen from the blocks behind: distance 1 needs only this block's rest, 2 and 3 the blocks in between
     F4 f = splat(1.f);
-    for (int w = warp + 1; w < 4 * blk + 4; ++w) f = mul4c(f, lds4(&s.T[w][kk]));
+    if (quad < 3) f = lds4(&s.T[4 * blk + 3][kk]);
+    if (quad < 2) f = mul4c(f, lds4(&s.T[4 * blk + 2][kk]));
+    if (quad < 1) f = mul4c(f, lds4(&s.T[4 * blk + 1][kk]));
     {
       F4 post = splat(1.f), m2 = splat(1.f), m3 = splat(1.f);
-      for (int b = blk + 1; b < 4; ++b) {
-        if (b == blk + 2) m2 = post;
-        if (b == blk + 3) m3 = post;
-        post = mul4c(post, lds4(&s.TB[b][kk]));
+      if (blk < 3) post = lds4(&s.TB[blk + 1][kk]);
+      if (blk < 2) {
+        m2 = post;
+        post = mul4c(post, lds4(&s.TB[blk + 2][kk]));
+      }
+      if (blk < 1) {
+        m3 = post;
+        post = mul4c(post, lds4(&s.TB[3][kk]));
       }
       const int cb = (blk > 0 ? 32 : 0) + 4 * quad;
 #pragma unroll
@@ -422,12 +460,15 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
     }
     // decay over the rows of the block in front of these; over the blocks in front
     f = lam[0];
-    for (int w = 4 * blk; w < warp; ++w) f = mul4c(f, lds4(&s.T[w][kk]));
+    if (quad > 0) f = mul4c(f, lds4(&s.T[4 * blk][kk]));
+    if (quad > 1) f = mul4c(f, lds4(&s.T[4 * blk + 1][kk]));
+    if (quad > 2) f = mul4c(f, lds4(&s.T[4 * blk + 2][kk]));
     F4 pre = splat(1.f);
-    for (int b = 0; b < blk; ++b) pre = mul4c(pre, lds4(&s.TB[b][kk]));
+    if (blk > 0) pre = lds4(&s.TB[0][kk]);
+    if (blk > 1) pre = mul4c(pre, lds4(&s.TB[1][kk]));
+    if (blk > 2) pre = mul4c(pre, lds4(&s.TB[2][kk]));
     if (warp == 15) {
-      const F4 gl = mul4c(pre, lds4(&s.TB[3][kk]));
-      *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.GL + tile * TILE_GL) + kk) = make_float4(gl.a.x, gl.a.y, gl.b.x, gl.b.y);
+      sts4(reinterpret_cast<float*>(p.GL + tile * TILE_GL) + kk, mul4c(pre, lds4(&s.TB[3][kk])));
     }
     const F4 preq = mul4c(pre, splat(p.scale));
 #pragma unroll
@@ -481,20 +522,27 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
         *reinterpret_cast<float2*>(&s.Akk[ra * AS + col]) = make_float2(a[nh][0], a[nh][1]);
         *reinterpret_cast<float2*>(&s.Akk[rb * AS + col]) = make_float2(a[nh][2], a[nh][3]);
       } else {
-        *reinterpret_cast<uint32_t*>(&s.Aqk[ra * TS + col]) = pack_bf16(p.scale * a[nh][0], p.scale * a[nh][1]);
-        *reinterpret_cast<uint32_t*>(&s.Aqk[rb * TS + col]) = pack_bf16(p.scale * a[nh][2], p.scale * a[nh][3]);
+        *reinterpret_cast<uint32_t*>(s.Aqk + swz<128>(ra, col)) = pack_bf16(p.scale * a[nh][0], p.scale * a[nh][1]);
+        *reinterpret_cast<uint32_t*>(s.Aqk + swz<128>(rb, col)) = pack_bf16(p.scale * a[nh][2], p.scale * a[nh][3]);
       }
     }
   }
+  fence_proxy_async();  // Aqk leaves by a bulk store, v arrives in the operand region
   __syncthreads();      // Aqk, Akk, TD complete; the operand region is free
   KDA_DBG_CLOCK(p.dbg, 22);
 
-  __nv_bfloat16* const sV = s.op;
+  if (tid == 128) {      // v, needed by the last phase; AQK
+    mbar_expect_tx(&s.barV, TILE_TK);
+    tma_load_rows(s.op, &p.tm_v, 0, h, static_cast<int>(ci.tok0), &s.barV);
+    tma_load_rows(reinterpret_cast<unsigned char*>(s.op) + 8192, &p.tm_v, 64, h, static_cast<int>(ci.tok0), &s.barV);
+    bulk_s2g(p.AQK + tile * TILE_TT, s.Aqk, TILE_TT);
+    bulk_commit();
+  }
   __nv_bfloat16* const sTB = reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<unsigned char*>(s.op) + TB_OFF);      // Tm diag(beta)
-  __nv_bfloat16* const sTI = reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<unsigned char*>(s.op) + TI_OFF);      // Tm
+  unsigned char* const sTI = reinterpret_cast<unsigned char*>(s.op) + TI_OFF;                                            // Tm
   auto put_tm = [&](int row, int col, float x, float y) {      // two adjacent entries of Tm = (I + diag(beta) Akk)^-1
     *reinterpret_cast<uint32_t*>(&sTB[row * TS + col]) = pack_bf16(x * s.beta[col], y * s.beta[col + 1]);
-    if (p.TI) *reinterpret_cast<uint32_t*>(&sTI[row * TS + col]) = pack_bf16(x, y);
+    if (p.TI) *reinterpret_cast<uint32_t*>(sTI + swz<128>(row, col)) = pack_bf16(x, y);
   };
   if (warp < 4) {
     // ---- P4b: the two levels of block merges  T21 = -T22 A21 T11  on tensor cores, every fp32 operand split into bf16 hi + lo
@@ -588,35 +636,36 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
       put_tm(56 + gid, col, -y1[2], -y1[3]);
     }
   } else {
-    // ---- the other twelve warps: v (needed by the last phase), AQK and the raw k-k products (for dbeta) to global, Tm's diagonal blocks
+    // ---- the other twelve warps: Tm's diagonal blocks; for the backward the raw k-k products (dbeta) and the zeros of Tm
     const int u = tid - 128;
-    for (int i = u; i < C * 16; i += PREP_THREADS - 128) {
-      const int r = i >> 4, pc = i & 15;
-      const bool ok = r < len;
-      const size_t row = (static_cast<size_t>(ci.tok0 + (ok ? r : 0)) * p.H + h) * KD + pc * 8;
-      cp_async16(&sV[r * QS + pc * 8], p.v + row, ok);
-    }
-    cp_async_commit();
-    unsigned char* gR = p.RKK ? p.RKK + tile * TILE_TT : nullptr;
-    unsigned char* gA = p.AQK + tile * TILE_TT;
-    for (int i = u; i < C * 8; i += PREP_THREADS - 128) {
-      const int r = i >> 3, pc = i & 7;
-      const uint32_t off = swz<128>(r, pc * 8);
-      *reinterpret_cast<uint4*>(gA + off) = *reinterpret_cast<const uint4*>(&s.Aqk[r * TS + pc * 8]);
-      if (gR) {
-        const float4 a0 = *reinterpret_cast<const float4*>(&s.Akk[r * AS + pc * 8]);
-        const float4 a1 = *reinterpret_cast<const float4*>(&s.Akk[r * AS + pc * 8 + 4]);
-        *reinterpret_cast<uint4*>(gR + off) =
-            make_uint4(pack_bf16(a0.x, a0.y), pack_bf16(a0.z, a0.w), pack_bf16(a1.x, a1.y), pack_bf16(a1.z, a1.w));
-      }
-      if (p.TI && (pc >> 1) > (r >> 4)) *reinterpret_cast<uint4*>(&sTI[r * TS + pc * 8]) = make_uint4(0u, 0u, 0u, 0u);      // above the diagonal
-    }
     for (int i = u; i < C * 8; i += PREP_THREADS - 128) {      // 64 rows x 8 column pairs of the diagonal blocks
       const int r = i >> 3, cp = (i & 7) * 2;
       const float2 x = *reinterpret_cast<const float2*>(&s.TD[r >> 4][(r & 15) * DS + cp]);
       put_tm(r, (r & 48) + cp, x.x, x.y);
     }
-    cp_async_wait<0>();   // v
+    if (p.RKK) {
+      unsigned char* const gR = p.RKK + tile * TILE_TT;
+      for (int i = u; i < C * 8; i += PREP_THREADS - 128) {
+        const int r = i >> 3, pc = i & 7, below = r - pc * 8;      // entries of the piece left of the diagonal
+        const uint32_t off = swz<128>(r, pc * 8);
+        uint4 o = make_uint4(0u, 0u, 0u, 0u);
+        if (below > 0) {
+          const float4 a0 = *reinterpret_cast<const float4*>(&s.Akk[r * AS + pc * 8]);
+          const float4 a1 = *reinterpret_cast<const float4*>(&s.Akk[r * AS + pc * 8 + 4]);
+          o = make_uint4(pack_bf16(a0.x, below > 1 ? a0.y : 0.f), pack_bf16(below > 2 ? a0.z : 0.f, below > 3 ? a0.w : 0.f),
+                         pack_bf16(below > 4 ? a1.x : 0.f, below > 5 ? a1.y : 0.f), pack_bf16(below > 6 ? a1.z : 0.f, below > 7 ? a1.w : 0.f));
+        }
+        *reinterpret_cast<uint4*>(gR + off) = o;
+        if ((pc >> 1) > (r >> 4)) *reinterpret_cast<uint4*>(sTI + off) = make_uint4(0u, 0u, 0u, 0u);      // block above the diagonal
+      }
+    }
+  }
+  if (!mbar_wait(&s.barV, 0) && tid == 0) atomicOr(p.status, KDA_STATUS_PREP_LOAD_WAIT);
+  if (len < C) {      // rows beyond the sequence hold the next one's tokens: clear them
+    for (int i = len * 8 + tid; i < C * 8; i += PREP_THREADS) {
+      reinterpret_cast<uint4*>(s.op)[i] = make_uint4(0u, 0u, 0u, 0u);
+      reinterpret_cast<uint4*>(s.op)[C * 8 + i] = make_uint4(0u, 0u, 0u, 0u);
+    }
   }
   __syncthreads();
   KDA_DBG_CLOCK(p.dbg, 23);
@@ -638,6 +687,7 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
       if (ks < 2 && ks <= pr) ldsm_x4(a[1][ks], ta1 + ks * 32);
     }
     {      // u^T: rows = value columns n0 .. n0 + 15, columns = tokens
+      const uint32_t av = smem_u32(s.op) + (static_cast<uint32_t>(n0 >> 6) << 13) + swz<128>((lane & 7) + ((lane >> 4) << 3), (n0 & 63) + (((lane >> 3) & 1) << 3));
       float acc[2][2][4];      // [row tile][8 tokens][fragment]
 #pragma unroll
       for (int i = 0; i < 16; ++i) (&acc[0][0][0])[i] = 0.f;
@@ -645,7 +695,7 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
       for (int ks = 0; ks < 4; ++ks) {
         if (ks <= 3 - pr) {
           uint32_t x[4];
-          ldsm_x4_t(x, smem_u32(&sV[(ks * 16 + (lane & 7) + ((lane >> 4) << 3)) * QS + n0 + (((lane >> 3) & 1) << 3)]));
+          ldsm_x4_t(x, av + ks * 2048);
           mma16816(acc[0][0], x, a[0][ks][0], a[0][ks][2]);
           mma16816(acc[0][1], x, a[0][ks][1], a[0][ks][3]);
           if (ks < 2 && ks <= pr) {
@@ -689,26 +739,23 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
           *reinterpret_cast<uint32_t*>(stW + tk_off(ta + 8, col)) = pack_bf16(acc[w][n][2], acc[w][n][3]);
         }
     }
-    if (p.TI) {            // Tm for the backward
-      unsigned char* gT = p.TI + tile * TILE_TT;
-      for (int i = tid; i < C * 8; i += PREP_THREADS)
-        *reinterpret_cast<uint4*>(gT + swz<128>(i >> 3, (i & 7) * 8)) = *reinterpret_cast<const uint4*>(&sTI[(i >> 3) * TS + (i & 7) * 8]);
-    }
     fence_proxy_async();   // the staged tiles (generic-proxy writes) are read next by the bulk-copy engine
     __syncthreads();
     if (tid == 0) {
       bulk_s2g(p.UT + tile * TILE_VT, stUT, TILE_VT);
       bulk_s2g(p.W + tile * TILE_TK, stW, TILE_TK);
+      if (p.TI) bulk_s2g(p.TI + tile * TILE_TT, sTI, TILE_TT);
       bulk_commit();
       bulk_wait_read<0>();   // shared memory must stay valid until the engine has read it
     }
+    if (tid == 128) bulk_wait_read<0>();
     KDA_DBG_CLOCK(p.dbg, 24);
   }
 }
 
 int launch_prepare(PrepParams& p, long long tiles, long long tokens, bool keep_qn, bool safe_gate, cudaStream_t st) {
   static DeviceOnce once;
-  const int smem = static_cast<int>(sizeof(PrepSmem));
+  const int smem = PREP_SMEM;
   const int rc = once.run([&] {
     cudaError_t e = cudaSuccess;
     for (auto fn : {kda_chunk_prepare_kernel<false, false>, kda_chunk_prepare_kernel<true, false>, kda_chunk_prepare_kernel<false, true>,
@@ -721,11 +768,11 @@ int launch_prepare(PrepParams& p, long long tiles, long long tokens, bool keep_q
   if (rc != KDA_OK) return rc;
   if (tiles > 0x7fffffffLL) return KDA_E_SHAPE;
   p.ahead = 2 * sm_count();
-  if (tiles > p.ahead) {
-    if (make_rows_tmap(&p.tm_q, p.q, false, tokens, p.HQ, KD, KD, C, false) || make_rows_tmap(&p.tm_k, p.k, false, tokens, p.HQ, KD, KD, C, false) ||
-        make_rows_tmap(&p.tm_v, p.v, false, tokens, p.H, VD, VD, C, false) || make_rows_tmap(&p.tm_g, p.g, true, tokens, p.H, KD, KD, C, false))
-      return KDA_E_TMAP;
-  }
+  if (make_rows_tmap(&p.tm_v, p.v, false, tokens, p.H, VD, 64, C, true)) return KDA_E_TMAP;
+  if (tiles > p.ahead &&
+      (make_rows_tmap(&p.tm_q, p.q, false, tokens, p.HQ, KD, KD, C, false) || make_rows_tmap(&p.tm_k, p.k, false, tokens, p.HQ, KD, KD, C, false) ||
+       make_rows_tmap(&p.tm_g, p.g, true, tokens, p.H, KD, KD, C, false)))
+    return KDA_E_TMAP;
   const unsigned grid = static_cast<unsigned>(tiles);
   if (safe_gate) {
     if (keep_qn) kda_chunk_prepare_kernel<true, true><<<grid, PREP_THREADS, smem, st>>>(p);

@@ -10,7 +10,8 @@ struct PrepParams {
   const __nv_bfloat16 *q, *k, *v;
   const float *g, *beta;
   ChunkMap map;
-  unsigned* status;   // cleared here when there is no tables kernel in front (equal lengths), else NULL
+  unsigned* status;
+  bool clear_status;  // there is no tables kernel in front (equal lengths): prepare clears the status word
   unsigned char *W, *UT, *KG, *QG, *AQK, *GL, *TI, *RKK;   // TI, RKK may be NULL
   long long* dbg;
   int H;
@@ -21,7 +22,8 @@ struct PrepParams {
   float* RSTD;              // [2][tokens * HQ] reciprocal norms of q, k
   long long qrows;          // tokens * HQ
   int ahead;                // tiles between a CTA and the one that will take its place: its inputs are fetched into L2 now
-  alignas(64) CUtensorMap tm_q, tm_k, tm_v, tm_g;      // [tokens, heads, 128] in boxes of 64 tokens of one head, for that prefetch
+  alignas(64) CUtensorMap tm_q, tm_k, tm_g;      // [tokens, heads, 128] in boxes of 64 tokens of one head, for that prefetch
+  alignas(64) CUtensorMap tm_v;                  // 64-column boxes in the 128-byte swizzle
 };
 
 // `tiles` = chunks x heads (an upper bound is fine); returns KDA_OK, a negative KDA_E_* or a positive cudaError_t
