@@ -205,6 +205,10 @@ typedef struct kda_chunk_args {
                                   blocks of the intra-chunk products on tensor cores too, factored around each block's middle row,
                                   instead of pairwise on CUDA cores.  With gates outside the bound the result may overflow; 0 is safe
                                   for any gate. */
+  int32_t k_cols, v_cols;      /* columns of the rows of q, k, g (and K of the states), of v, o (and V of the states) and of their
+                                  gradients when they are narrower than the kernels' K = V = 128: multiples of 8, 0 = 128.  The
+                                  missing columns count as zero (k = q = v = 0, g = 0), which leaves every result unchanged.  Backward
+                                  with narrow rows: no grouped heads; with use_qk_l2norm only with save_for_backward bit 1. */
 } kda_chunk_args;
 
 /* Upper bound on the number of chunks: every sequence adds at most one partial chunk. */

@@ -41,6 +41,7 @@ class ChunkArgs(C.Structure):
         ("tokens", C.c_int64), ("N", C.c_int32), ("H", C.c_int32), ("K", C.c_int32), ("V", C.c_int32),
         ("io_dtype", C.c_int32), ("use_qk_l2norm", C.c_int32), ("save_for_backward", C.c_int32),
         ("scale", C.c_float), ("HQ", C.c_int32), ("scan_slices", C.c_int32), ("safe_gate", C.c_int32),
+        ("k_cols", C.c_int32), ("v_cols", C.c_int32),
     ]
 
 

@@ -256,7 +256,7 @@ kda_chunk_args chunk_args(const ChunkSaved& s, const ChunkOpts& o, int save) {
   a.cu_seqlens = ptr<int32_t>(s.cu); a.workspace = ptr(s.ws); a.workspace_bytes = static_cast<size_t>(s.ws.numel());
   a.tokens = s.q.size(0) * s.q.size(1);
   a.N = static_cast<int32_t>(sequences(s)); a.H = static_cast<int32_t>(s.v.size(2)); a.HQ = static_cast<int32_t>(s.q.size(2));
-  a.K = static_cast<int32_t>(s.q.size(3)); a.V = static_cast<int32_t>(s.v.size(3)); a.io_dtype = KDA_BF16; a.use_qk_l2norm = o.l2norm;
+  a.K = a.V = 128; a.k_cols = static_cast<int32_t>(s.q.size(3)); a.v_cols = static_cast<int32_t>(s.v.size(3)); a.io_dtype = KDA_BF16; a.use_qk_l2norm = o.l2norm;
   a.save_for_backward = save; a.scale = static_cast<float>(o.scale); a.scan_slices = o.slices; a.safe_gate = o.safe_gate;
   return a;
 }
@@ -395,10 +395,13 @@ bool wants_grad(std::initializer_list<const Tensor*> ts) {
   return false;
 }
 
-// bf16 tensors with K = V = 128.  Returns false for a call that takes another path (float32, other heads).
+// bf16 tensors with K, V <= 128.  Returns false for a call that takes another path: float32, larger heads, and the narrow ones that
+// the kernels do not read in place (no multiple of eight columns; gradients with grouped value heads).
 bool chunk_kda(ChunkCall& c, Tensor& o, Tensor& ht) {
   const Sizes s = check_common(c.q, c.k, c.v, c.g, c.beta, c.h0, c.cu);
-  if (c.q.scalar_type() != at::kBFloat16 || s.K != 128 || s.V != 128) return false;
+  const bool grads = wants_grad({&c.q, &c.k, &c.v, &c.g, &c.beta, &c.h0, &c.A_log, &c.dt_bias});
+  if (c.q.scalar_type() != at::kBFloat16 || s.K > 128 || s.V > 128 || s.K % 8 || s.V % 8) return false;
+  if ((s.K < 128 || s.V < 128) && grads && s.HQ != s.H) return false;
   ChunkOpts opt;
   opt.scale = c.scale ? *c.scale : 1.0 / std::sqrt(static_cast<double>(s.K));
   opt.output_final = c.output_final; opt.l2norm = c.l2norm; opt.gate = c.gate; opt.beta_sigmoid = c.beta_sigmoid; opt.safe_gate = c.safe_gate;
@@ -422,7 +425,7 @@ bool chunk_kda(ChunkCall& c, Tensor& o, Tensor& ht) {
   const at::Device dev = c.q.device();
   if (c.transposed && c.h0.defined()) c.h0 = c.h0.transpose(-1, -2);
   const Tensor cu = i32(c.cu, dev);
-  if (wants_grad({&c.q, &c.k, &c.v, &c.g, &c.beta, &c.h0, &c.A_log, &c.dt_bias})) {
+  if (grads) {
     auto some = [](const Tensor& t) { return t.defined() ? std::optional<Tensor>(t) : std::nullopt; };
     const variable_list r = ChunkFunction::apply(c.q, c.k, c.v, c.g, c.beta, some(c.h0), some(c.A_log), some(c.dt_bias), some(cu), opt);
     o = r[0];

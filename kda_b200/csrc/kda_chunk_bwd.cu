@@ -123,7 +123,7 @@ extern "C" int kda_chunk_bwd(const kda_chunk_args* args, void* stream) {
   if (a.N == 0) return KDA_OK;
   if (a.tokens == 0) {
     if (a.dh0) {
-      const size_t bytes = static_cast<size_t>(a.N) * a.H * KD * VD * sizeof(float);
+      const size_t bytes = static_cast<size_t>(a.N) * a.H * (a.k_cols > 0 ? a.k_cols : KD) * (a.v_cols > 0 ? a.v_cols : VD) * sizeof(float);
       return static_cast<int>(a.d_ht ? cudaMemcpyAsync(a.dh0, a.d_ht, bytes, cudaMemcpyDeviceToDevice, st)
                                      : cudaMemsetAsync(a.dh0, 0, bytes, st));
     }
@@ -131,6 +131,9 @@ extern "C" int kda_chunk_bwd(const kda_chunk_args* args, void* stream) {
   }
   const bool l2 = a.use_qk_l2norm != 0;
   const int HQ = a.HQ > 0 ? a.HQ : a.H, grp = a.H / HQ;
+  const int kc = a.k_cols > 0 ? a.k_cols : KD, vc = a.v_cols > 0 ? a.v_cols : VD;
+  // narrow rows: the kernels read and write them as they are, except for the two detours through 128-wide scratch
+  if ((kc != KD || vc != VD) && (grp > 1 || (l2 && !(a.save_for_backward & 2)))) return KDA_E_SHAPE;
   const bool kept_qn = l2 && (a.save_for_backward & 2) != 0;      // the forward left the normalised q, k in its workspace
   ChunkWs w = carve_ws(static_cast<unsigned char*>(a.workspace), static_cast<unsigned char*>(a.bwd_workspace), a.tokens, a.N,
                        a.H, true, l2, grp > 1, (a.save_for_backward & 2) != 0);
@@ -156,8 +159,8 @@ extern "C" int kda_chunk_bwd(const kda_chunk_args* args, void* stream) {
   rp.W = w.W; rp.KG = w.KG; rp.QG = w.QG; rp.AQK = w.AQK; rp.GL = w.GL;
   rp.DH = w.DH; rp.DVNEWT = w.DVNEWT;
   rp.d_o = static_cast<const __nv_bfloat16*>(a.d_o); rp.d_ht = a.d_ht; rp.dh0 = a.dh0; rp.status = w.status; rp.dbg = g_dbg_clocks;
-  rp.H = a.H;
-  if (make_rows_tmap(&rp.tm_do, a.d_o, false, a.tokens, a.H, VD, 64, C, true)) return KDA_E_TMAP;
+  rp.H = a.H; rp.kc = kc; rp.vc = vc;
+  if (make_rows_tmap(&rp.tm_do, a.d_o, false, a.tokens, a.H, vc, 64, C, true)) return KDA_E_TMAP;
   const int slices = scan_slices_for(a.N * a.H, a.scan_slices);
   if ((rc = slices > 1 ? launch_bwd_scan_vs(rp, a.N * a.H, st) : launch_bwd_scan_tc(rp, a.N * a.H, st)) != KDA_OK) return rc;
   prof_mark(prof, KDA_STAGE_BWD_SCAN, st);
@@ -170,11 +173,12 @@ extern "C" int kda_chunk_bwd(const kda_chunk_args* args, void* stream) {
   // grouped value heads: every value head writes its own dq, dk; a second kernel sums each group
   mp.dq = grp > 1 ? w.DQH : static_cast<__nv_bfloat16*>(a.dq);
   mp.dk = grp > 1 ? w.DKH : static_cast<__nv_bfloat16*>(a.dk);
+  mp.kc = kc; mp.vc = vc; mp.qc = l2 ? KD : kc; mp.dqc = grp > 1 ? KD : kc;
   mp.dbeta = a.dbeta; mp.dg = a.dg; mp.status = w.status; mp.dbg = g_dbg_clocks;
-  if (make_rows_tmap(&mp.tm_q, q, false, a.tokens, HQ, KD, KD, C, false) || make_rows_tmap(&mp.tm_k, k, false, a.tokens, HQ, KD, KD, C, false) ||
-      make_rows_tmap(&mp.tm_g, a.g, true, a.tokens, a.H, KD, KD, C, false) ||
-      make_rows_tmap(&mp.tm_v, a.v, false, a.tokens, a.H, VD, 64, C, true) ||
-      make_rows_tmap(&mp.tm_do, a.d_o, false, a.tokens, a.H, VD, 64, C, true))
+  if (make_rows_tmap(&mp.tm_q, q, false, a.tokens, HQ, mp.qc, KD, C, false) || make_rows_tmap(&mp.tm_k, k, false, a.tokens, HQ, mp.qc, KD, C, false) ||
+      make_rows_tmap(&mp.tm_g, a.g, true, a.tokens, a.H, kc, KD, C, false) ||
+      make_rows_tmap(&mp.tm_v, a.v, false, a.tokens, a.H, vc, 64, C, true) ||
+      make_rows_tmap(&mp.tm_do, a.d_o, false, a.tokens, a.H, vc, 64, C, true))
     return KDA_E_TMAP;
   mp.H = a.H; mp.scale = a.scale; mp.grp = grp;
   // without grouped heads the normalisation's backward is applied by bwd_main's own epilogue

@@ -16,6 +16,9 @@ struct MainParams {
   unsigned* status;
   long long* dbg;
   int H;
+  int kc, vc;       // key and value columns of the tensors (<= 128; tiles are 128 wide, zero beyond)
+  int qc;           // columns of a row of q, k as the kernel reads them (kc, or 128 for the kept normalised rows)
+  int dqc;          // columns of a row of dq, dk as the kernel writes them (kc, or 128 for the per-value-head scratch)
   float scale;
   int grp;          // value heads per q/k head (grouped value heads): the q, k maps have H / grp heads
   const float* rstd;    // [2][qrows] reciprocal norms of the q, k rows, or NULL.  Not NULL (only with grp == 1): q, k are the
@@ -35,6 +38,7 @@ struct RScanParams {
   unsigned* status;
   long long* dbg;       // development aid: phase clocks
   int H;
+  int kc, vc;           // key and value columns of the tensors
   alignas(64) CUtensorMap tm_do;   // 64-column boxes of dO in the 128-byte-swizzled operand layout
 };
 

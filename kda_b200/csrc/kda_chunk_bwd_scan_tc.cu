@@ -91,14 +91,14 @@ __global__ void __launch_bounds__(RNT, 1) kda_chunk_bwd_scan_tc_kernel(const __g
   }
 
   {
-    const size_t sb = (static_cast<size_t>(seq) * p.H + h) * KD * VD;
+    const size_t sb = (static_cast<size_t>(seq) * p.H + h) * p.kc * p.vc;
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
       float x[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const int kk = 64 * half + 16 * g + i;
-        x[i] = p.d_ht ? __ldg(p.d_ht + sb + static_cast<size_t>(kk) * VD + v) : 0.f;
+        x[i] = p.d_ht && kk < p.kc && v < p.vc ? __ldg(p.d_ht + sb + static_cast<size_t>(kk) * p.vc + v) : 0.f;
       }
       umma::tmem_st16(tq + C_H + 64 * half + 16 * g, x);
     }
@@ -219,14 +219,17 @@ __global__ void __launch_bounds__(RNT, 1) kda_chunk_bwd_scan_tc_kernel(const __g
   alive = __syncthreads_and(alive);      // uniform: either every thread writes dh0 or none does
   if (alive && p.dh0) {
     umma::fence_after_sync();
-    const size_t sb = (static_cast<size_t>(seq) * p.H + h) * KD * VD;
+    const size_t sb = (static_cast<size_t>(seq) * p.H + h) * p.kc * p.vc;
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
       float x[16];
       umma::tmem_ld16(tq + C_H + 64 * half + 16 * g, x);
       umma::tmem_ld_wait();
 #pragma unroll
-      for (int e = 0; e < 16; ++e) p.dh0[sb + static_cast<size_t>(64 * half + 16 * g + e) * VD + v] = x[e];
+      for (int e = 0; e < 16; ++e) {
+        const int kk = 64 * half + 16 * g + e;
+        if (kk < p.kc && v < p.vc) p.dh0[sb + static_cast<size_t>(kk) * p.vc + v] = x[e];
+      }
     }
   }
   if (tid == 0) bulk_wait<0>();

@@ -130,13 +130,13 @@ __global__ void __launch_bounds__(RVS_THREADS, 1) kda_chunk_bwd_scan_vs_kernel(c
   }
 
   if (warp < 8) {                                     // gradient w.r.t. the final state -> TMEM: lane k, the slice's columns
-    const size_t sb = ((static_cast<size_t>(seq) * p.H + h) * KD + k) * VD + v0 + HC * half;
+    const size_t sb = ((static_cast<size_t>(seq) * p.H + h) * p.kc + k) * p.vc + v0 + HC * half;
 #pragma unroll
     for (int g = 0; g < HC / 16; ++g) {
       float x[16];
 #pragma unroll
       for (int e = 0; e < 16; e += 4) {
-        const float4 f = p.d_ht ? __ldg(reinterpret_cast<const float4*>(p.d_ht + sb + 16 * g + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 f = p.d_ht && k < p.kc && v0 + HC * half + 16 * g + e < p.vc ? __ldg(reinterpret_cast<const float4*>(p.d_ht + sb + 16 * g + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
         x[e] = f.x; x[e + 1] = f.y; x[e + 2] = f.z; x[e + 3] = f.w;
       }
       umma::tmem_st16(tq + C_H + HC * half + 16 * g, x);
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(RVS_THREADS, 1) kda_chunk_bwd_scan_vs_kernel(c
     if (__any_sync(0xffffffffu, s.dead != 0)) {
       if (lane == 0) atomicOr(p.status, KDA_STATUS_BWD_SCAN_MMA_WAIT);
     } else if (p.dh0) {
-      const size_t sb = ((static_cast<size_t>(seq) * p.H + h) * KD + k) * VD + v0 + HC * half;
+      const size_t sb = ((static_cast<size_t>(seq) * p.H + h) * p.kc + k) * p.vc + v0 + HC * half;
 #pragma unroll
       for (int g = 0; g < HC / 16; ++g) {
         float x[16];
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(RVS_THREADS, 1) kda_chunk_bwd_scan_vs_kernel(c
         umma::tmem_ld_wait();
 #pragma unroll
         for (int e = 0; e < 16; e += 4)
-          *reinterpret_cast<float4*>(p.dh0 + sb + 16 * g + e) = make_float4(x[e], x[e + 1], x[e + 2], x[e + 3]);
+          if (k < p.kc && v0 + HC * half + 16 * g + e < p.vc) *reinterpret_cast<float4*>(p.dh0 + sb + 16 * g + e) = make_float4(x[e], x[e + 1], x[e + 2], x[e + 3]);
       }
     }
   } else if (warp == RW_ISSUE) {

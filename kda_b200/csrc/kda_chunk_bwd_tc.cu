@@ -449,11 +449,11 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
       }
       {
         const int vcol = 32 * q4 + lane;
-        __nv_bfloat16* const dvp = p.dv + (static_cast<size_t>(ci.tok0 + 16 * part) * p.H + h) * VD + vcol;
-        const size_t tstride = static_cast<size_t>(p.H) * VD;
+        __nv_bfloat16* const dvp = p.dv + (static_cast<size_t>(ci.tok0 + 16 * part) * p.H + h) * p.vc + vcol;
+        const size_t tstride = static_cast<size_t>(p.H) * p.vc;
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          if (16 * part + i < len) dvp[i * tstride] = __float2bfloat16_rn(s.beta[16 * part + i] * v3[i]);
+          if (16 * part + i < len && vcol < p.vc) dvp[i * tstride] = __float2bfloat16_rn(s.beta[16 * part + i] * v3[i]);
       }
     }
     fence_proxy_async();
@@ -756,8 +756,8 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
         for (int u = 0; u < 2; ++u) {
           const int i = tid + u * NT, r = i >> 4, pc = i & 15;
           const size_t grow = static_cast<size_t>(ci.tok0 + (r < len ? r : 0)) * p.H + h;
-          yq2[u] = __ldg(reinterpret_cast<const uint4*>(p.q + grow * KD + pc * 8));
-          yk2[u] = __ldg(reinterpret_cast<const uint4*>(p.k + grow * KD + pc * 8));
+          yq2[u] = __ldg(reinterpret_cast<const uint4*>(p.q + grow * p.qc + pc * 8));
+          yk2[u] = __ldg(reinterpret_cast<const uint4*>(p.k + grow * p.qc + pc * 8));
           rq2[u] = __ldg(p.rstd + grow);
           rk2[u] = __ldg(p.rstd + p.qrows + grow);
         }
@@ -767,15 +767,15 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
         float add = 0.f;             // totals of the later blocks
 #pragma unroll
         for (int bb = 1; bb < 4; ++bb) add += (bb > blk) ? s.carry[bb][kk] : 0.f;
-        float* const dgp = p.dg + (static_cast<size_t>(ci.tok0 + t0) * p.H + h) * KD + kk;      // a warp stores 128 contiguous bytes
+        float* const dgp = p.dg + (static_cast<size_t>(ci.tok0 + t0) * p.H + h) * p.kc + kk;      // a warp stores 128 contiguous bytes
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          if (t0 + i < len) dgp[static_cast<size_t>(i) * p.H * KD] = dGv[i] + add;
+          if (t0 + i < len && kk < p.kc) dgp[static_cast<size_t>(i) * p.H * p.kc] = dGv[i] + add;
       }
 #pragma unroll
       for (int u = 0; u < C * 16 / NT; ++u) {
         const int i = tid + u * NT, r = i >> 4, pc = i & 15;
-        const size_t row = (static_cast<size_t>(ci.tok0 + (r < len ? r : 0)) * p.H + h) * KD + pc * 8;
+        const size_t row = (static_cast<size_t>(ci.tok0 + (r < len ? r : 0)) * p.H + h) * p.dqc + pc * 8;
         uint4 oq = *reinterpret_cast<const uint4*>(&stq[r * KD + pc * 8]);
         uint4 ok = *reinterpret_cast<const uint4*>(&stk[r * KD + pc * 8]);
         if constexpr (L2) {
@@ -809,7 +809,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
           oq = make_uint4(wq[0], wq[1], wq[2], wq[3]);
           ok = make_uint4(wk[0], wk[1], wk[2], wk[3]);
         }
-        if (r < len) {
+        if (r < len && pc * 8 < p.dqc) {
           *reinterpret_cast<uint4*>(p.dq + row) = oq;
           *reinterpret_cast<uint4*>(p.dk + row) = ok;
         }

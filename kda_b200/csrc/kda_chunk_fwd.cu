@@ -114,6 +114,7 @@ int validate_chunk_args(const kda_chunk_args& a, bool backward) {
   if (a.tokens < 0 || a.N < 0 || a.H <= 0) return KDA_E_SHAPE;
   if (a.HQ < 0 || (a.HQ > 0 && (a.HQ > a.H || a.H % a.HQ != 0))) return KDA_E_SHAPE;
   if (a.K != KD || a.V != VD) return KDA_E_SHAPE;
+  if (a.k_cols < 0 || a.k_cols > KD || a.k_cols % 8 || a.v_cols < 0 || a.v_cols > VD || a.v_cols % 8) return KDA_E_SHAPE;
   if (a.scan_slices != 0 && a.scan_slices != 1 && a.scan_slices != 4) return KDA_E_SHAPE;
   if (a.io_dtype != KDA_BF16) return KDA_E_DTYPE;
   if (a.tokens / C + a.N > 0x3fffffffLL) return KDA_E_SHAPE;
@@ -152,9 +153,10 @@ extern "C" int kda_chunk_fwd(const kda_chunk_args* args, void* stream) {
   if (rc != KDA_OK) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (a.N == 0) return KDA_OK;
+  const int kc = a.k_cols > 0 ? a.k_cols : KD, vc = a.v_cols > 0 ? a.v_cols : VD;
   if (a.tokens == 0) {
     if (a.ht && a.ht != a.h0) {
-      const size_t bytes = static_cast<size_t>(a.N) * a.H * KD * VD * sizeof(float);
+      const size_t bytes = static_cast<size_t>(a.N) * a.H * kc * vc * sizeof(float);
       return static_cast<int>(a.h0 ? cudaMemcpyAsync(a.ht, a.h0, bytes, cudaMemcpyDeviceToDevice, st)
                                    : cudaMemsetAsync(a.ht, 0, bytes, st));
     }
@@ -182,7 +184,7 @@ extern "C" int kda_chunk_fwd(const kda_chunk_args* args, void* stream) {
   pp.v = static_cast<const __nv_bfloat16*>(a.v);
   pp.g = a.g; pp.beta = a.beta; pp.map = map; pp.status = w.status; pp.clear_status = a.cu_seqlens == nullptr;
   pp.W = w.W; pp.UT = w.UT; pp.KG = w.KG; pp.QG = w.QG; pp.AQK = w.AQK; pp.GL = w.GL; pp.TI = save ? w.TI : nullptr; pp.RKK = save ? w.RKK : nullptr;
-  pp.dbg = g_dbg_clocks; pp.H = a.H; pp.use_l2norm = a.use_qk_l2norm; pp.scale = a.scale;
+  pp.dbg = g_dbg_clocks; pp.H = a.H; pp.kc = kc; pp.vc = vc; pp.use_l2norm = a.use_qk_l2norm; pp.scale = a.scale;
   pp.HQ = a.HQ > 0 ? a.HQ : a.H; pp.grp = a.H / pp.HQ;
   pp.QN = keep_qn ? w.QN : nullptr; pp.KN = keep_qn ? w.KN : nullptr; pp.RSTD = keep_qn ? w.RSTD : nullptr;
   pp.qrows = static_cast<long long>(a.tokens) * pp.HQ;
@@ -195,7 +197,7 @@ extern "C" int kda_chunk_fwd(const kda_chunk_args* args, void* stream) {
   sp.W = w.W; sp.UT = w.UT; sp.KG = w.KG; sp.QG = w.QG; sp.AQK = w.AQK; sp.GL = w.GL;
   sp.HS = save ? w.HS : nullptr; sp.VNEWT = save ? w.VNEWT : nullptr;
   sp.h0 = a.h0; sp.ht = a.ht; sp.o = static_cast<__nv_bfloat16*>(a.o); sp.status = w.status; sp.dbg = g_dbg_clocks;
-  sp.H = a.H;
+  sp.H = a.H; sp.kc = kc; sp.vc = vc;
   const int slices = scan_slices_for(a.N * a.H, a.scan_slices);
   if ((rc = slices > 1 ? launch_scan_vs(sp, a.N * a.H, st) : launch_scan_tc(sp, a.N * a.H, st)) != KDA_OK) return rc;
   prof_mark(prof, KDA_STAGE_SCAN, st);

@@ -186,17 +186,17 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
   const int kk = 4 * lane, t0 = 4 * warp, b0 = 16 * blk;
   KDA_DBG_CLOCK(p.dbg, 16);
 
-  // ---- P1: q, k, g of this thread's columns and rows; rows >= len: q = k = 0, no decay ---------------------------------
+  // ---- P1: q, k, g of this thread's columns and rows; rows >= len and columns >= kc: q = k = 0, no decay ---------------------------------
   F4 lam[4];
   uint2 q[4], k[4];
   {
-    const float* gp = p.g + (static_cast<size_t>(ci.tok0 + t0) * p.H + h) * KD + kk;
-    const size_t qoff = (static_cast<size_t>(ci.tok0 + t0) * p.HQ + h / p.grp) * KD + kk;
+    const float* gp = p.g + (static_cast<size_t>(ci.tok0 + t0) * p.H + h) * p.kc + kk;
+    const size_t qoff = (static_cast<size_t>(ci.tok0 + t0) * p.HQ + h / p.grp) * p.kc + kk;
     const __nv_bfloat16 *qp = p.q + qoff, *kp = p.k + qoff;
-    const size_t gs = static_cast<size_t>(p.H) * KD, qs = static_cast<size_t>(p.HQ) * KD;
+    const size_t gs = static_cast<size_t>(p.H) * p.kc, qs = static_cast<size_t>(p.HQ) * p.kc;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const bool ok = t0 + i < len;      // warp-uniform
+      const bool ok = t0 + i < len && kk < p.kc;
       const float4 g4 = ok ? ldg_f4(gp + i * gs) : make_float4(0.f, 0.f, 0.f, 0.f);
       lam[i] = {pair(g4.x, g4.y), pair(g4.z, g4.w)};
       q[i] = ok ? ldg_u2(qp + i * qs) : make_uint2(0u, 0u);
@@ -768,10 +768,10 @@ int launch_prepare(PrepParams& p, long long tiles, long long tokens, bool keep_q
   if (rc != KDA_OK) return rc;
   if (tiles > 0x7fffffffLL) return KDA_E_SHAPE;
   p.ahead = 2 * sm_count();
-  if (make_rows_tmap(&p.tm_v, p.v, false, tokens, p.H, VD, 64, C, true)) return KDA_E_TMAP;
+  if (make_rows_tmap(&p.tm_v, p.v, false, tokens, p.H, p.vc, 64, C, true)) return KDA_E_TMAP;
   if (tiles > p.ahead &&
-      (make_rows_tmap(&p.tm_q, p.q, false, tokens, p.HQ, KD, KD, C, false) || make_rows_tmap(&p.tm_k, p.k, false, tokens, p.HQ, KD, KD, C, false) ||
-       make_rows_tmap(&p.tm_g, p.g, true, tokens, p.H, KD, KD, C, false)))
+      (make_rows_tmap(&p.tm_q, p.q, false, tokens, p.HQ, p.kc, KD, C, false) || make_rows_tmap(&p.tm_k, p.k, false, tokens, p.HQ, p.kc, KD, C, false) ||
+       make_rows_tmap(&p.tm_g, p.g, true, tokens, p.H, p.kc, KD, C, false)))
     return KDA_E_TMAP;
   const unsigned grid = static_cast<unsigned>(tiles);
   if (safe_gate) {

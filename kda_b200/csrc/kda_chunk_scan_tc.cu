@@ -95,14 +95,14 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
 
   // initial state -> TMEM: lane v, columns k = 64 half .. +63
   if (!issuer) {
-    const size_t sb = (static_cast<size_t>(seq) * p.H + h) * KD * VD;
+    const size_t sb = (static_cast<size_t>(seq) * p.H + h) * p.kc * p.vc;
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
       float x[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const int kk = 64 * half + 16 * g + i;
-        x[i] = p.h0 ? __ldg(p.h0 + sb + static_cast<size_t>(kk) * VD + v) : 0.f;
+        x[i] = p.h0 && kk < p.kc && v < p.vc ? __ldg(p.h0 + sb + static_cast<size_t>(kk) * p.vc + v) : 0.f;
       }
       umma::tmem_st16(tq + C_H + 64 * half + 16 * g, x);
     }
@@ -267,8 +267,8 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
     asm volatile("bar.sync 1, 256;" ::: "memory");      // the eight compute warps only
     for (int e = tid; e < C * 16; e += SCT) {
       const int r = e >> 4, pc = e & 15;
-      if (r < ci.len)
-        *reinterpret_cast<uint4*>(p.o + (static_cast<size_t>(ci.tok0 + r) * p.H + h) * VD + pc * 8) =
+      if (r < ci.len && pc * 8 < p.vc)
+        *reinterpret_cast<uint4*>(p.o + (static_cast<size_t>(ci.tok0 + r) * p.H + h) * p.vc + pc * 8) =
             *reinterpret_cast<const uint4*>(&s.oS[r * VD + pc * 8]);
     }
     // (the next iteration's first barrier orders these reads of oS before it is rewritten)
@@ -279,14 +279,17 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
   // final state
   if (alive && p.ht && !issuer) {
     umma::fence_after_sync();
-    const size_t sb = (static_cast<size_t>(seq) * p.H + h) * KD * VD;
+    const size_t sb = (static_cast<size_t>(seq) * p.H + h) * p.kc * p.vc;
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
       float x[16];
       umma::tmem_ld16(tq + C_H + 64 * half + 16 * g, x);
       umma::tmem_ld_wait();
 #pragma unroll
-      for (int e = 0; e < 16; ++e) p.ht[sb + static_cast<size_t>(64 * half + 16 * g + e) * VD + v] = x[e];
+      for (int e = 0; e < 16; ++e) {
+        const int kk = 64 * half + 16 * g + e;
+        if (kk < p.kc && v < p.vc) p.ht[sb + static_cast<size_t>(kk) * p.vc + v] = x[e];
+      }
     }
   }
   if (lead) bulk_wait<0>();              // outstanding bulk stores read shared memory that dies with the CTA

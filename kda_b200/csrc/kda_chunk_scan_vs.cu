@@ -143,13 +143,13 @@ __global__ void __launch_bounds__(VS_THREADS, 1) kda_chunk_scan_vs_kernel(const 
 
   // initial state -> TMEM: lane k, the slice's columns
   if (warp < 8) {
-    const size_t sb = ((static_cast<size_t>(seq) * p.H + h) * KD + k) * VD + v0 + HC * half;
+    const size_t sb = ((static_cast<size_t>(seq) * p.H + h) * p.kc + k) * p.vc + v0 + HC * half;
 #pragma unroll
     for (int g = 0; g < HC / 16; ++g) {
       float x[16];
 #pragma unroll
       for (int e = 0; e < 16; e += 4) {
-        const float4 f = p.h0 ? __ldg(reinterpret_cast<const float4*>(p.h0 + sb + 16 * g + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 f = p.h0 && k < p.kc && v0 + HC * half + 16 * g + e < p.vc ? __ldg(reinterpret_cast<const float4*>(p.h0 + sb + 16 * g + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
         x[e] = f.x; x[e + 1] = f.y; x[e + 2] = f.z; x[e + 3] = f.w;
       }
       umma::tmem_st16(tq + C_H + HC * half + 16 * g, x);
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(VS_THREADS, 1) kda_chunk_scan_vs_kernel(const 
     if (__any_sync(0xffffffffu, s.dead != 0)) {
       if (lane == 0) atomicOr(p.status, KDA_STATUS_SCAN_MMA_WAIT);
     } else if (p.ht) {
-      const size_t sb = ((static_cast<size_t>(seq) * p.H + h) * KD + k) * VD + v0 + HC * half;
+      const size_t sb = ((static_cast<size_t>(seq) * p.H + h) * p.kc + k) * p.vc + v0 + HC * half;
 #pragma unroll
       for (int g = 0; g < HC / 16; ++g) {
         float x[16];
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(VS_THREADS, 1) kda_chunk_scan_vs_kernel(const 
         umma::tmem_ld_wait();
 #pragma unroll
         for (int e = 0; e < 16; e += 4)
-          *reinterpret_cast<float4*>(p.ht + sb + 16 * g + e) = make_float4(x[e], x[e + 1], x[e + 2], x[e + 3]);
+          if (k < p.kc && v0 + HC * half + 16 * g + e < p.vc) *reinterpret_cast<float4*>(p.ht + sb + 16 * g + e) = make_float4(x[e], x[e + 1], x[e + 2], x[e + 3]);
       }
     }
   } else if (warp == W_ISSUE) {
@@ -349,9 +349,10 @@ __global__ void __launch_bounds__(VS_THREADS, 1) kda_chunk_scan_vs_kernel(const 
       __syncwarp();
       if (lane == 0) mbar_arrive(&s.oFree[b]);          // the accumulator may be overwritten (chunk i + 2)
       if (lane < 16 && t < len) {
-        uint4* dst = reinterpret_cast<uint4*>(p.o + (static_cast<size_t>(tok0 + t) * p.H + h) * VD + v0);
+        uint4* dst = reinterpret_cast<uint4*>(p.o + (static_cast<size_t>(tok0 + t) * p.H + h) * p.vc + v0);
 #pragma unroll
-        for (int e = 0; e < VS / 8; ++e) dst[e] = out[e];
+        for (int e = 0; e < VS / 8; ++e)
+          if (v0 + 8 * e < p.vc) dst[e] = out[e];
       }
     }
   } else if (warp == W_STORE) {

@@ -15,6 +15,7 @@ struct PrepParams {
   unsigned char *W, *UT, *KG, *QG, *AQK, *GL, *TI, *RKK;   // TI, RKK may be NULL
   long long* dbg;
   int H;
+  int kc, vc;         // key and value columns of the tensors (<= 128, multiples of 8; tiles are 128 wide, zero beyond)
   int use_l2norm;
   float scale;
   int HQ, grp;      // q/k heads and value heads per q/k head (grouped value heads); H counts value heads

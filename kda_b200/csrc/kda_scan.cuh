@@ -15,6 +15,7 @@ struct ScanParams {
   unsigned* status;
   long long* dbg;       // development aid: phase clocks (NULL unless built with the clock marks and a buffer is registered)
   int H;
+  int kc, vc;           // key and value columns of the tensors (<= 128; tiles and state are 128 wide, zero beyond)
 };
 
 // tcgen05 / TMEM version (kda_chunk_scan_tc.cu); returns KDA_OK, a negative KDA_E_* or a positive cudaError_t
