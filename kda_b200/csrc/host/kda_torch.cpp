@@ -256,7 +256,7 @@ kda_chunk_args chunk_args(const ChunkSaved& s, const ChunkOpts& o, int save) {
   a.cu_seqlens = ptr<int32_t>(s.cu); a.workspace = ptr(s.ws); a.workspace_bytes = static_cast<size_t>(s.ws.numel());
   a.tokens = s.q.size(0) * s.q.size(1);
   a.N = static_cast<int32_t>(sequences(s)); a.H = static_cast<int32_t>(s.v.size(2)); a.HQ = static_cast<int32_t>(s.q.size(2));
-  a.K = a.V = 128; a.k_cols = static_cast<int32_t>(s.q.size(3)); a.v_cols = static_cast<int32_t>(s.v.size(3)); a.io_dtype = KDA_BF16; a.use_qk_l2norm = o.l2norm;
+  a.K = a.V = 128; a.k_cols = static_cast<int32_t>(s.q.size(3)); a.v_cols = static_cast<int32_t>(s.v.size(3)); a.io_dtype = dtype_code(s.q); a.use_qk_l2norm = o.l2norm;
   a.save_for_backward = save; a.scale = static_cast<float>(o.scale); a.scan_slices = o.slices; a.safe_gate = o.safe_gate;
   return a;
 }
@@ -293,7 +293,8 @@ std::pair<Tensor, Tensor> chunk_forward(ChunkSaved& s, const Tensor& q, const Te
   s.cu = cu;
   const int64_t N = sequences(s);
   const int save = need_grad ? save_bits(o) : 0;
-  s.ws = bytes(kda_chunk_workspace_bytes(tokens, static_cast<int32_t>(N), static_cast<int32_t>(H), static_cast<int32_t>(K), static_cast<int32_t>(V), save), dev);
+  const int fp32 = dtype_code(q) == KDA_FP32 ? 4 : 0;
+  s.ws = bytes(kda_chunk_workspace_bytes(tokens, static_cast<int32_t>(N), static_cast<int32_t>(H), static_cast<int32_t>(K), static_cast<int32_t>(V), save | fp32), dev);
   const Tensor out = empty(v.sizes(), v.scalar_type(), dev);
   const Tensor ht = o.output_final ? empty({N, H, K, V}, at::kFloat, dev) : Tensor();
   kda_chunk_args a = chunk_args(s, o, save);
@@ -343,7 +344,7 @@ class ChunkFunction : public torch::autograd::Function<ChunkFunction> {
     const Tensor dq = empty(s.q.sizes(), s.q.scalar_type(), dev), dk = empty(s.k.sizes(), s.k.scalar_type(), dev), dv = empty(s.v.sizes(), s.v.scalar_type(), dev);
     Tensor dg = empty(s.g.sizes(), at::kFloat, dev), dbeta = empty(s.beta.sizes(), at::kFloat, dev);
     const Tensor dh0 = s.h0.defined() ? empty(s.h0.sizes(), at::kFloat, dev) : Tensor();
-    const int flags = (o.l2norm ? 1 | 4 : 0) | (s.q.size(2) != H ? 2 : 0);
+    const int flags = (o.l2norm ? 1 | 4 : 0) | (s.q.size(2) != H ? 2 : 0) | (dtype_code(s.q) == KDA_FP32 ? 8 : 0);
     const Tensor bws = bytes(
         kda_chunk_bwd_workspace_bytes(tokens, static_cast<int32_t>(N), static_cast<int32_t>(H), static_cast<int32_t>(K), static_cast<int32_t>(V), flags), dev);
     kda_chunk_args a = chunk_args(s, o, save_bits(o));
@@ -395,13 +396,23 @@ bool wants_grad(std::initializer_list<const Tensor*> ts) {
   return false;
 }
 
-// bf16 tensors with K, V <= 128.  Returns false for a call that takes another path: float32, larger heads, and the narrow ones that
-// the kernels do not read in place (no multiple of eight columns; gradients with grouped value heads).
+// float32 gradients of a handful of tokens (fewer than four chunks in all: gradient checks) stay with the token-recurrent kernels, which
+// take the recurrence's own steps; anything longer takes the chunked ones (8 x 2048 tokens x 32 heads: 26 ms there).
+bool recurrent_backward(const Sizes& s) {
+  auto built = [](int64_t d) { return d == 32 || d == 64 || d == 128; };
+  return s.B * s.T < 256 && built(s.K) && built(s.V);
+}
+
+// Heads up to 128, bf16, and float32 with gradients.  Returns false for a call that takes another path: float32 without gradients
+// (token-recurrent kernel), larger heads, and the narrow ones that the kernels do not read in place (no multiple of eight columns; bf16
+// gradients with grouped value heads).
 bool chunk_kda(ChunkCall& c, Tensor& o, Tensor& ht) {
   const Sizes s = check_common(c.q, c.k, c.v, c.g, c.beta, c.h0, c.cu);
   const bool grads = wants_grad({&c.q, &c.k, &c.v, &c.g, &c.beta, &c.h0, &c.A_log, &c.dt_bias});
-  if (c.q.scalar_type() != at::kBFloat16 || s.K > 128 || s.V > 128 || s.K % 8 || s.V % 8) return false;
-  if ((s.K < 128 || s.V < 128) && grads && s.HQ != s.H) return false;
+  const bool fp32 = c.q.scalar_type() == at::kFloat;
+  if (s.K > 128 || s.V > 128 || s.K % 8 || s.V % 8) return false;
+  if (!fp32 && (s.K < 128 || s.V < 128) && grads && s.HQ != s.H) return false;
+  if (fp32 && (!grads || recurrent_backward(s))) return false;
   ChunkOpts opt;
   opt.scale = c.scale ? *c.scale : 1.0 / std::sqrt(static_cast<double>(s.K));
   opt.output_final = c.output_final; opt.l2norm = c.l2norm; opt.gate = c.gate; opt.beta_sigmoid = c.beta_sigmoid; opt.safe_gate = c.safe_gate;
