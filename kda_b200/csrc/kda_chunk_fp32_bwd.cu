@@ -192,7 +192,7 @@ struct MainSmem32 {
 constexpr int MAIN32_SMEM = static_cast<int>(sizeof(MainSmem32)) + 1024;
 static_assert(MAIN32_SMEM <= 227 * 1024, "MainSmem32 too large");
 // tensor-memory columns
-constexpr int M_DQG = 0, M_DKG = 64, M_DW = 128, M_DAQ = 192, M_DTM = 256, M_DBV = 320, M_DBK = 384, M_XY = 448;
+constexpr int M_DQG = 0, M_DW = 64, M_DKG = 128, M_DAQ = 192, M_DTM = 256, M_DBV = 320, M_DBK = 384, M_XY = 448;
 
 }  // namespace
 
@@ -250,14 +250,16 @@ __global__ void __launch_bounds__(NT, 1) kda_f32_bwd_main_kernel(const F32Params
         hd[i] += x[i].x * x[2 + i].x + x[i].y * x[2 + i].y + x[i].z * x[2 + i].z + x[i].w * x[2 + i].w;
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) put4(s.R + 65536 + 16384 * i, S64, r, pc, x[4 + i]);
+      for (int i = 0; i < 2; ++i) put4(s.R + 65536 + i * S64, 2 * S64, r, pc, x[4 + i]);
+#pragma unroll
+      for (int i = 2; i < 4; ++i) put4(s.R + 65536 + 16384 * i, S64, r, pc, x[4 + i]);
       staged();
       if (tid == 0) {
-        mma_slice(tb + M_DQG, aR, S128, aR + 65536, S64, idesc(128, 64), sl > 0);
-        mma_slice(tb + M_DW, aR, S128, aR + 81920, S64, idesc(128, 64), sl > 0);
+        // dO and dv_new stand one behind the other as one B operand of 128 rows: dqg^T and dw^T are one product, h is read once
+        mma_slice(tb + M_DQG, aR, S128, aR + 65536, 2 * S64, idesc(128, 128), sl > 0);
         mma_slice(tb + M_DKG, aR + 32768, S128, aR + 98304, S64, idesc(128, 64), sl > 0);
-        mma_slice(tb + M_DAQ, aR + 65536, S64, aR + 98304, S64, idesc(64, 64), sl > 0);
-        mma_slice(tb + M_DTM, aR + 81920, S64, aR + 114688, S64, idesc(64, 64), sl > 0);
+        mma_slice(tb + M_DAQ, aR + 65536, 2 * S64, aR + 98304, S64, idesc(64, 64), sl > 0);
+        mma_slice(tb + M_DTM, aR + 65536 + S64, 2 * S64, aR + 114688, S64, idesc(64, 64), sl > 0);
         umma::commit(&s.bar);
       }
       if (sl < 3) load(sl + 1);
@@ -385,18 +387,24 @@ __global__ void __launch_bounds__(NT, 1) kda_f32_bwd_main_kernel(const F32Params
     const bool okk = kk < p.kc;
     const size_t grow = (static_cast<size_t>(ci.tok0 + t0) * p.H + h) * p.kc + kk, qrow = (static_cast<size_t>(ci.tok0 + t0) * p.HQ + h / p.grp) * p.kc + kk;
     const size_t gs = static_cast<size_t>(p.H) * p.kc, qs = static_cast<size_t>(p.HQ) * p.kc;
+    // all 48 loads first: anything that waits for one of them in between would expose a latency per row
+    const float* qs_ = p.use_l2 ? p.w.QN + tTK + t0 * KD + kk : p.q + qrow;
+    const float* ks_ = p.use_l2 ? p.w.KN + tTK + t0 * KD + kk : p.k + qrow;
+    const size_t st = p.use_l2 ? static_cast<size_t>(KD) : qs;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const bool ok = okk && t0 + i < len;
-      lam[i] = ok ? expf(__ldg(p.g + grow + i * gs)) : 1.f;
-      if (p.use_l2) {
-        qv[i] = __ldg(p.w.QN + tTK + (t0 + i) * KD + kk);
-        kv[i] = __ldg(p.w.KN + tTK + (t0 + i) * KD + kk);
-      } else {
-        qv[i] = ok ? __ldg(p.q + qrow + i * qs) : 0.f;
-        kv[i] = ok ? __ldg(p.k + qrow + i * qs) : 0.f;
-      }
-    }
+    for (int i = 0; i < 16; ++i) lam[i] = okk && t0 + i < len ? __ldg(p.g + grow + i * gs) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) qv[i] = okk && t0 + i < len ? __ldg(qs_ + i * st) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) kv[i] = okk && t0 + i < len ? __ldg(ks_ + i * st) : 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) lam[i] = expf(lam[i]);
+  }
+  float rk[16];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float4 x = ld4(p.w.RKK + tTT + row * C + 16 * part + 4 * e, low);
+    rk[4 * e] = x.x; rk[4 * e + 1] = x.y; rk[4 * e + 2] = x.z; rk[4 * e + 3] = x.w;
   }
   wait_mma(&s.bar, ph, p.w.status, BIT);
   __syncthreads();      // every product is complete: the operand region becomes the last phase's arrays
@@ -412,7 +420,7 @@ __global__ void __launch_bounds__(NT, 1) kda_f32_bwd_main_kernel(const F32Params
       for (int e = 0; e < 16; ++e) {
         const int j = 16 * part + e;
         const float x = j < row ? -y[e] : 0.f;
-        pb = fmaf(x, __ldg(p.w.RKK + tTT + row * C + j), pb);
+        pb = fmaf(x, rk[e], pb);
         s.dA[row * DA + j] = make_float2(j <= row ? p.scale * a[e] : 0.f, b * x);
       }
       s.dbp[4 + part][row] = pb;

@@ -78,22 +78,48 @@ constexpr uint32_t S64 = 64 * 128, S128 = 128 * 128;      // bytes of one 32-col
 __host__ __device__ constexpr uint32_t idesc(int M, int N) {      // kind::tf32, fp32 accumulation, both operands K-major
   return (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(N >> 3) << 17) | (static_cast<uint32_t>(M >> 4) << 24);
 }
-__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t id, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d), "l"(a), "l"(b), "r"(id),
-      "r"(acc)
-      : "memory");
-}
-// D (+)= A B^T over one 32-column slice: a, b = shared-memory addresses of the hi tiles, alo, blo = bytes from there to the lo tiles
+// D (+)= A B^T over one 32-column slice: a, b = shared-memory addresses of the hi tiles, alo, blo = bytes from there to the lo tiles.
+// One asm block for the twelve products (hi hi + hi lo + lo hi of four k-steps): consecutive products then issue about 60 cycles apart,
+// as separate statements 88.
 __device__ __forceinline__ void mma_slice(uint32_t d, uint32_t a, uint32_t alo, uint32_t b, uint32_t blo, uint32_t id, bool acc) {
-  const uint64_t ah = umma::desc_kmajor(a, 0), al = umma::desc_kmajor(a + alo, 0), bh = umma::desc_kmajor(b, 0), bl = umma::desc_kmajor(b + blo, 0);
-#pragma unroll
-  for (int s = 0; s < 4; ++s) {
-    const uint64_t o = static_cast<uint64_t>(s) * 2u;
-    mma(d, ah + o, bh + o, id, acc || s > 0);
-    mma(d, ah + o, bl + o, id, 1);
-    mma(d, al + o, bh + o, id, 1);
-  }
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p0, p1;\n\t"
+      ".reg .b64 ah, al, bh, bl;\n\t"
+      "setp.ne.b32 p0, %6, 0;\n\t"
+      "setp.eq.b32 p1, %6, %6;\n\t"
+      "mov.b64 ah, %1;\n\t"
+      "mov.b64 al, %2;\n\t"
+      "mov.b64 bh, %3;\n\t"
+      "mov.b64 bl, %4;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], ah, bh, %5, p0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], ah, bl, %5, p1;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], al, bh, %5, p1;\n\t"
+      "add.u64 ah, ah, 2;\n\t"
+      "add.u64 al, al, 2;\n\t"
+      "add.u64 bh, bh, 2;\n\t"
+      "add.u64 bl, bl, 2;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], ah, bh, %5, p1;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], ah, bl, %5, p1;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], al, bh, %5, p1;\n\t"
+      "add.u64 ah, ah, 2;\n\t"
+      "add.u64 al, al, 2;\n\t"
+      "add.u64 bh, bh, 2;\n\t"
+      "add.u64 bl, bl, 2;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], ah, bh, %5, p1;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], ah, bl, %5, p1;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], al, bh, %5, p1;\n\t"
+      "add.u64 ah, ah, 2;\n\t"
+      "add.u64 al, al, 2;\n\t"
+      "add.u64 bh, bh, 2;\n\t"
+      "add.u64 bl, bl, 2;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], ah, bh, %5, p1;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], ah, bl, %5, p1;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], al, bh, %5, p1;\n\t"
+      "}\n" ::"r"(d),
+      "l"(umma::desc_kmajor(a, 0)), "l"(umma::desc_kmajor(a + alo, 0)), "l"(umma::desc_kmajor(b, 0)), "l"(umma::desc_kmajor(b + blo, 0)), "r"(id),
+      "r"(static_cast<uint32_t>(acc))
+      : "memory");
 }
 __device__ __forceinline__ float tf32_hi(float x) {
   uint32_t r;
