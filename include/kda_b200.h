@@ -212,6 +212,16 @@ typedef struct kda_chunk_args {
                                   gradients when they are narrower than the kernels' K = V = 128: multiples of 8, 0 = 128.  The
                                   missing columns count as zero (k = q = v = 0, g = 0), which leaves every result unchanged.  Backward
                                   with narrow rows: no grouped heads; with use_qk_l2norm only with save_for_backward bit 1. */
+  /* Gate front end inside the forward (KDA_BF16), all zero / NULL: g and beta are the activated fp32 values.  With g_raw (beta_raw)
+   * the forward activates them itself, with the formulas of kda_gate_fwd, and `g` (`beta`) is an OUTPUT: it receives the activated
+   * values, which kda_chunk_bwd reads; NULL in a forward-only call.  kda_gate_bwd turns dg, dbeta into the raw tensors' gradients. */
+  const void* g_raw;           /* [tokens, H, K] of g_raw_dtype, or NULL */
+  const void* beta_raw;        /* [tokens, H] logits of beta_raw_dtype, or NULL */
+  const float* A_log;          /* [H], required with g_raw */
+  const float* dt_bias;        /* [H * K] or NULL */
+  int32_t g_raw_dtype, beta_raw_dtype;      /* KDA_BF16 or KDA_FP32 */
+  int32_t use_lower_bound;
+  float lower_bound;
 } kda_chunk_args;
 
 /* Upper bound on the number of chunks: every sequence adds at most one partial chunk. */

@@ -42,6 +42,8 @@ class ChunkArgs(C.Structure):
         ("io_dtype", C.c_int32), ("use_qk_l2norm", C.c_int32), ("save_for_backward", C.c_int32),
         ("scale", C.c_float), ("HQ", C.c_int32), ("scan_slices", C.c_int32), ("safe_gate", C.c_int32),
         ("k_cols", C.c_int32), ("v_cols", C.c_int32),
+        ("g_raw", C.c_void_p), ("beta_raw", C.c_void_p), ("A_log", C.c_void_p), ("dt_bias", C.c_void_p),
+        ("g_raw_dtype", C.c_int32), ("beta_raw_dtype", C.c_int32), ("use_lower_bound", C.c_int32), ("lower_bound", C.c_float),
     ]
 
 

@@ -270,21 +270,23 @@ std::pair<Tensor, Tensor> chunk_forward(ChunkSaved& s, const Tensor& q, const Te
   const cudaStream_t st = stream_of(dev);
   const int64_t B = q.size(0), T = q.size(1), H = v.size(2), K = q.size(3), V = v.size(3), tokens = B * T;
   s.q = dense(q); s.k = dense(k); s.v = dense(v); s.h0 = dense(h0);
+  // bf16: the forward kernel activates g and beta itself, and the activated values exist only for a backward
+  const bool fused = q.scalar_type() == at::kBFloat16, keep = need_grad || !fused;
   if (o.gate) {
     s.g_raw = dense(g);
     s.A32 = f32(A_log);
     s.b32 = f32(dt_bias);
-    s.g = empty(g.sizes(), at::kFloat, dev);
+    if (keep) s.g = empty(g.sizes(), at::kFloat, dev);
   } else {
     s.g = f32(g);
   }
   if (o.beta_sigmoid) {
     s.beta_raw = dense(beta);
-    s.beta = empty(beta.sizes(), at::kFloat, dev);
+    if (keep) s.beta = empty(beta.sizes(), at::kFloat, dev);
   } else {
     s.beta = f32(beta);
   }
-  if (o.gate || o.beta_sigmoid) {
+  if ((o.gate || o.beta_sigmoid) && !fused) {
     kda_gate_args a = gate_args(s, o, tokens, H, K);
     a.g = o.gate ? ptr<float>(s.g) : nullptr;
     a.beta = o.beta_sigmoid ? ptr<float>(s.beta) : nullptr;
@@ -300,6 +302,13 @@ std::pair<Tensor, Tensor> chunk_forward(ChunkSaved& s, const Tensor& q, const Te
   kda_chunk_args a = chunk_args(s, o, save);
   a.o = ptr(out);
   a.ht = ptr<float>(ht);
+  if (fused && o.gate) {
+    a.g_raw = ptr(s.g_raw); a.g_raw_dtype = dtype_code(s.g_raw); a.A_log = ptr<float>(s.A32); a.dt_bias = ptr<float>(s.b32);
+    a.use_lower_bound = o.has_lower_bound; a.lower_bound = static_cast<float>(o.lower_bound);
+  }
+  if (fused && o.beta_sigmoid) {
+    a.beta_raw = ptr(s.beta_raw); a.beta_raw_dtype = dtype_code(s.beta_raw);
+  }
   check_rc(kda_chunk_fwd(&a, st), "kda_chunk_fwd");
   if (checked_mode()) check_chunk_status(s.ws, "kda_chunk_fwd");
   return {out, ht};

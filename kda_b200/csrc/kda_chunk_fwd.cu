@@ -120,12 +120,17 @@ int validate_chunk_args(const kda_chunk_args& a, bool backward) {
   if (a.io_dtype != KDA_BF16 && a.io_dtype != KDA_FP32) return KDA_E_DTYPE;
   if (a.tokens / C + a.N > 0x3fffffffLL) return KDA_E_SHAPE;
   if (a.tokens == 0 || a.N == 0) return KDA_OK;
-  if (!a.q || !a.k || !a.v || !a.g || !a.beta || !a.workspace) return KDA_E_NULL;
+  const bool raw_g = !backward && a.g_raw, raw_b = !backward && a.beta_raw;
+  if (!a.q || !a.k || !a.v || (!a.g && !raw_g) || (!a.beta && !raw_b) || !a.workspace) return KDA_E_NULL;
+  if (raw_g && !a.A_log) return KDA_E_NULL;
+  if ((raw_g || raw_b) && a.io_dtype != KDA_BF16) return KDA_E_DTYPE;
+  if ((raw_g && a.g_raw_dtype != KDA_BF16 && a.g_raw_dtype != KDA_FP32) || (raw_b && a.beta_raw_dtype != KDA_BF16 && a.beta_raw_dtype != KDA_FP32))
+    return KDA_E_DTYPE;
   if (!a.cu_seqlens && a.tokens % a.N != 0) return KDA_E_SHAPE;
   if (!backward && !a.o) return KDA_E_NULL;
   uintptr_t bits = reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v) |
                    reinterpret_cast<uintptr_t>(a.g) | reinterpret_cast<uintptr_t>(a.o) | reinterpret_cast<uintptr_t>(a.h0) |
-                   reinterpret_cast<uintptr_t>(a.ht);
+                   reinterpret_cast<uintptr_t>(a.ht) | reinterpret_cast<uintptr_t>(a.g_raw) | reinterpret_cast<uintptr_t>(a.dt_bias);
   if (backward) {
     if (!a.d_o || !a.dq || !a.dk || !a.dv || !a.dg || !a.dbeta || !a.bwd_workspace) return KDA_E_NULL;
     bits |= reinterpret_cast<uintptr_t>(a.d_o) | reinterpret_cast<uintptr_t>(a.dq) | reinterpret_cast<uintptr_t>(a.dk) |
@@ -218,7 +223,11 @@ extern "C" int kda_chunk_fwd(const kda_chunk_args* args, void* stream) {
   pp.q = static_cast<const __nv_bfloat16*>(a.q);
   pp.k = static_cast<const __nv_bfloat16*>(a.k);
   pp.v = static_cast<const __nv_bfloat16*>(a.v);
-  pp.g = a.g; pp.beta = a.beta; pp.map = map; pp.status = w.status; pp.clear_status = a.cu_seqlens == nullptr;
+  pp.g = a.g; pp.beta = a.beta; pp.map = map;
+  pp.g_raw = a.g_raw; pp.beta_raw = a.beta_raw; pp.A_log = a.A_log; pp.dt_bias = a.dt_bias;
+  pp.g_out = a.g_raw ? const_cast<float*>(a.g) : nullptr; pp.beta_out = a.beta_raw ? const_cast<float*>(a.beta) : nullptr;
+  pp.g_fp32 = a.g_raw_dtype == KDA_FP32; pp.beta_fp32 = a.beta_raw_dtype == KDA_FP32; pp.use_lb = a.use_lower_bound; pp.lb = a.lower_bound;
+  pp.status = w.status; pp.clear_status = a.cu_seqlens == nullptr;
   pp.W = w.W; pp.UT = w.UT; pp.KG = w.KG; pp.QG = w.QG; pp.AQK = w.AQK; pp.GL = w.GL; pp.TI = save ? w.TI : nullptr; pp.RKK = save ? w.RKK : nullptr;
   pp.dbg = g_dbg_clocks; pp.H = a.H; pp.kc = kc; pp.vc = vc; pp.use_l2norm = a.use_qk_l2norm; pp.scale = a.scale;
   pp.HQ = a.HQ > 0 ? a.HQ : a.H; pp.grp = a.H / pp.HQ;

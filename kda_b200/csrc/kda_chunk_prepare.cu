@@ -16,6 +16,7 @@
 // Operands are written to shared memory once as bf16 and read by ldmatrix; level 8 / 4 products stack q and k rows into one m16
 // tile.  The same pass writes QG = scale q Gam, KG = k Gam_last / Gam and k Gam.
 #include "kda_device.cuh"
+#include "kda_gate.cuh"
 #include "kda_prepare.cuh"
 
 namespace kda {
@@ -190,15 +191,21 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
   F4 lam[4];
   uint2 q[4], k[4];
   {
-    const float* gp = p.g + (static_cast<size_t>(ci.tok0 + t0) * p.H + h) * p.kc + kk;
+    const size_t goff = (static_cast<size_t>(ci.tok0 + t0) * p.H + h) * p.kc + kk;
     const size_t qoff = (static_cast<size_t>(ci.tok0 + t0) * p.HQ + h / p.grp) * p.kc + kk;
     const __nv_bfloat16 *qp = p.q + qoff, *kp = p.k + qoff;
     const size_t gs = static_cast<size_t>(p.H) * p.kc, qs = static_cast<size_t>(p.HQ) * p.kc;
+    const bool bf16_gate = p.g_raw && !p.g_fp32;
+    const float* gp = p.g_raw ? static_cast<const float*>(p.g_raw) + goff : p.g + goff;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const bool ok = t0 + i < len && kk < p.kc;
-      const float4 g4 = ok ? ldg_f4(gp + i * gs) : make_float4(0.f, 0.f, 0.f, 0.f);
-      lam[i] = {pair(g4.x, g4.y), pair(g4.z, g4.w)};
+      if (bf16_gate) {
+        lam[i] = widen(ok ? ldg_u2(static_cast<const __nv_bfloat16*>(p.g_raw) + goff + i * gs) : make_uint2(0u, 0u));
+      } else {
+        const float4 g4 = ok ? ldg_f4(gp + i * gs) : make_float4(0.f, 0.f, 0.f, 0.f);
+        lam[i] = {pair(g4.x, g4.y), pair(g4.z, g4.w)};
+      }
       q[i] = ok ? ldg_u2(qp + i * qs) : make_uint2(0u, 0u);
       k[i] = ok ? ldg_u2(kp + i * qs) : make_uint2(0u, 0u);
     }
@@ -218,7 +225,34 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
     }
     static_assert(TILE_TT == 16 * PREP_THREADS, "one piece per thread");
     reinterpret_cast<uint4*>(s.Aqk)[tid] = make_uint4(0u, 0u, 0u, 0u);
-    if (tid < C) s.beta[tid] = tid < len ? __ldg(p.beta + static_cast<size_t>(ci.tok0 + tid) * p.H + h) : 0.f;
+    if (tid < C) {
+      float b = 0.f;
+      if (tid < len) {
+        const size_t i = static_cast<size_t>(ci.tok0 + tid) * p.H + h;
+        if (p.beta_raw) {
+          b = sigmoidf_(p.beta_fp32 ? __ldg(static_cast<const float*>(p.beta_raw) + i) : __bfloat162float(static_cast<const __nv_bfloat16*>(p.beta_raw)[i]));
+          if (p.beta_out) p.beta_out[i] = b;
+        } else {
+          b = __ldg(p.beta + i);
+        }
+      }
+      s.beta[tid] = b;
+    }
+    // the gate's activation here instead of in a kernel of its own: one launch less, and the fp32 g is never read back (forward only: never written)
+    if (p.g_raw) {
+      const float al = __expf(__ldg(p.A_log + h));
+      float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (p.dt_bias && kk < p.kc) bias = __ldg(reinterpret_cast<const float4*>(p.dt_bias + static_cast<size_t>(h) * p.kc + kk));
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (t0 + i >= len || kk >= p.kc) continue;
+        const float2 x = halves(lam[i].a), y = halves(lam[i].b);
+        const float4 g4 = make_float4(gate_value(x.x + bias.x, al, p.use_lb, p.lb), gate_value(x.y + bias.y, al, p.use_lb, p.lb),
+                                      gate_value(y.x + bias.z, al, p.use_lb, p.lb), gate_value(y.y + bias.w, al, p.use_lb, p.lb));
+        lam[i] = {pair(g4.x, g4.y), pair(g4.z, g4.w)};
+        if (p.g_out) *reinterpret_cast<float4*>(p.g_out + goff + i * gs) = g4;
+      }
+    }
   }
   KDA_DBG_CLOCK(p.dbg, 17);
   // ---- P2: lam, the decay over these four rows -------------------------------------------------------------------------
@@ -771,7 +805,7 @@ int launch_prepare(PrepParams& p, long long tiles, long long tokens, bool keep_q
   if (make_rows_tmap(&p.tm_v, p.v, false, tokens, p.H, p.vc, 64, C, true)) return KDA_E_TMAP;
   if (tiles > p.ahead &&
       (make_rows_tmap(&p.tm_q, p.q, false, tokens, p.HQ, p.kc, KD, C, false) || make_rows_tmap(&p.tm_k, p.k, false, tokens, p.HQ, p.kc, KD, C, false) ||
-       make_rows_tmap(&p.tm_g, p.g, true, tokens, p.H, p.kc, KD, C, false)))
+       make_rows_tmap(&p.tm_g, p.g_raw ? p.g_raw : p.g, !p.g_raw || p.g_fp32, tokens, p.H, p.kc, KD, C, false)))
     return KDA_E_TMAP;
   const unsigned grid = static_cast<unsigned>(tiles);
   if (safe_gate) {

@@ -8,25 +8,12 @@
 //   g = lower_bound * sigmoid(exp(A_log[h]) * x)           (when a lower bound is given)
 //   beta = sigmoid(beta_raw)
 #include "kda_chunk.cuh"
+#include "kda_gate.cuh"
 
 namespace kda {
 
 constexpr int GATE_THREADS = 256;
 constexpr int GATE_BWD_THREADS = 256;
-
-__device__ __forceinline__ float sigmoidf_(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
-// softplus and its derivative (the sigmoid) from one exponential: log(1 + e^x), e^x / (1 + e^x); identity / 1 above 20.
-// Below -15 the sum 1 + e^x would round the small term away: log(1 + e) = e there to fp32 accuracy.
-__device__ __forceinline__ float softplusf_(float x, float& sig) {
-  const float e = __expf(fminf(x, 20.f));
-  const float t = 1.f + e;
-  sig = x > 20.f ? 1.f : __fdividef(e, t);
-  return x > 20.f ? x : (x < -15.f ? e : __logf(t));
-}
-__device__ __forceinline__ float softplusf_(float x) {
-  const float e = __expf(fminf(x, 20.f));
-  return x > 20.f ? x : (x < -15.f ? e : __logf(1.f + e));
-}
 
 template <typename T>
 __device__ __forceinline__ void load8(const T* p, float (&v)[8]);

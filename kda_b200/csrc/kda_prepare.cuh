@@ -9,6 +9,12 @@ namespace kda {
 struct PrepParams {
   const __nv_bfloat16 *q, *k, *v;
   const float *g, *beta;
+  // gate front end (g_raw / beta_raw not NULL): g, beta are computed here, and written to g_out / beta_out unless those are NULL
+  const void *g_raw, *beta_raw;
+  const float *A_log, *dt_bias;
+  float *g_out, *beta_out;
+  int g_fp32, beta_fp32, use_lb;      // dtype of the raw tensors: float32 or bf16
+  float lb;
   ChunkMap map;
   unsigned* status;
   bool clear_status;  // there is no tables kernel in front (equal lengths): prepare clears the status word
