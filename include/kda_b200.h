@@ -102,7 +102,7 @@ typedef struct kda_recurrent_args {
 
 int kda_recurrent_fwd(const kda_recurrent_args* args, void* stream);
 
-/* Large decode batches (one token per sequence, K = V = 128, at least four (sequence, head) units per SM) run on a
+/* Large decode batches (one token per sequence, K = V = 128, at least 32 (sequence, head) units per SM) and several tokens with a slot each run on a
  * kernel that moves the states with the bulk-copy engine and waits for them on barriers with a bounded number of
  * polls.  This call copies the device status word of that kernel to *host_out and clears it (it synchronises with
  * the device: a diagnostic, not part of the step).  0: every wait completed; bit 0: a wait gave up and the outputs

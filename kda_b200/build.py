@@ -49,7 +49,7 @@ def _host_command() -> list[str]:
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
     cmd += [f"-I{i}" for i in inc if i.startswith(ROOT)] + [a for i in inc if not i.startswith(ROOT) for a in ("-isystem", i)]
     cmd += [os.path.join(CSRC, "host", "kda_torch.cpp"), "-o", HOST_LIB, f"-L{PKG}", "-l:libkda_b200.so", "-Wl,-rpath,$ORIGIN"]
-    return cmd + [f"-L{d}" for d in library_paths()] + ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+    return cmd + [f"-L{d}" for d in library_paths()] + ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
 
 
 def _stale(target: str, deps: list[str]) -> bool:

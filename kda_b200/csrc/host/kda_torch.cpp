@@ -5,6 +5,7 @@
 // look-ups, a ctypes structure, torch.empty, the device context manager) took 23 us of host time, and a training call 300 to
 // 500 us through three Python autograd functions.  Here a decode call costs about 6 us and a whole forward + backward about 50 us.
 #include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -104,7 +105,7 @@ Tensor i32(const Tensor& t, const at::Device& dev) {
   return t.to(at::TensorOptions().device(dev).dtype(at::kInt)).contiguous();
 }
 Tensor empty(at::IntArrayRef shape, at::ScalarType dt, const at::Device& dev) {
-  return at::empty(shape, at::TensorOptions().device(dev).dtype(dt));
+  return at::detail::empty_cuda(shape, dt, dev, std::nullopt);      // straight to the allocator: 0.5 us less than through the dispatcher
 }
 Tensor bytes(size_t n, const at::Device& dev) { return empty({static_cast<int64_t>(n)}, at::kByte, dev); }
 cudaStream_t stream_of(const at::Device& dev) { return c10::cuda::getCurrentCUDAStream(dev.index()).stream(); }

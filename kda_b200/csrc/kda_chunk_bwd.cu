@@ -77,8 +77,7 @@ __global__ void __launch_bounds__(256) kda_l2norm_bwd_kernel(const __nv_bfloat16
 
 // one persistent CTA per SM (the kernel needs a whole SM's shared memory), never more CTAs than tiles
 static int main_grid(int max_chunks, int H) {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const long long tiles = static_cast<long long>(max_chunks) * H;
   return static_cast<int>(tiles < sms ? (tiles > 0 ? tiles : 1) : sms);
 }

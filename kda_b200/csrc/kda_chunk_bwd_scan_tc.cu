@@ -48,6 +48,7 @@ __device__ __forceinline__ unsigned char* swq(unsigned char* tile, int row, int 
 }  // namespace
 
 __global__ void __launch_bounds__(RNT, 1) kda_chunk_bwd_scan_tc_kernel(const __grid_constant__ RScanParams p) {
+  chain_point();
   extern __shared__ unsigned char smem_raw[];
   TcRScanSmem& s = *reinterpret_cast<TcRScanSmem*>(smem_raw + pad_to_1024(smem_raw));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;

@@ -72,6 +72,7 @@ __device__ __forceinline__ void rwarp_arrive(uint64_t* bar, int lane) {
 
 template <int VS>
 __global__ void __launch_bounds__(RVS_THREADS, 1) kda_chunk_bwd_scan_vs_kernel(const __grid_constant__ RScanParams p) {
+  chain_point();
   constexpr int NS = VD / VS;
   constexpr int HC = VS / 2;
   constexpr int C_H = 0, C_VN = VS;      // TMEM columns

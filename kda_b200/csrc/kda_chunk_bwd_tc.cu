@@ -92,6 +92,7 @@ __device__ __forceinline__ unsigned char* sw_piece(unsigned char* tile, int row,
 // L2: q, k are L2-normalised rows and dq, dk leave through the normalisation's backward (fla/modules/l2norm.py:190-240).
 template <bool L2>
 __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __grid_constant__ MainParams p) {
+  chain_point();
   extern __shared__ unsigned char smem_raw[];
   TcSmem& s = *reinterpret_cast<TcSmem*>(smem_raw + pad_to_1024(smem_raw));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -836,9 +837,8 @@ int launch_bwd_main_tc(const MainParams& p, int grid, cudaStream_t st) {
     return e;
   });
   if (rc != KDA_OK) return rc;
-  if (p.rstd != nullptr && p.grp == 1) kda_chunk_bwd_main_tc_kernel<true><<<grid, NT, smem, st>>>(p);
-  else kda_chunk_bwd_main_tc_kernel<false><<<grid, NT, smem, st>>>(p);
-  return static_cast<int>(cudaGetLastError());
+  const auto kernel = p.rstd != nullptr && p.grp == 1 ? kda_chunk_bwd_main_tc_kernel<true> : kda_chunk_bwd_main_tc_kernel<false>;
+  return static_cast<int>(launch_chained(kernel, grid, NT, smem, st, p));
 }
 
 }  // namespace kda

@@ -44,6 +44,7 @@ __device__ __forceinline__ float4 lds4v(const float* p) { return *reinterpret_ca
 }  // namespace
 
 __global__ void __launch_bounds__(NT, 1) kda_f32_prepare_kernel(const F32Params p) {
+  chain_point();
   extern __shared__ unsigned char smem_raw[];
   PrepSmem32& s = *reinterpret_cast<PrepSmem32*>(smem_raw + pad_to_1024(smem_raw));
   const int tid = threadIdx.x, lane = tid & 31;
@@ -406,6 +407,7 @@ constexpr int TC_H = 0, TC_VN = 128, TC_O = 192;
 }  // namespace
 
 __global__ void __launch_bounds__(NT, 1) kda_f32_scan_kernel(const F32Params p) {
+  chain_point();
   extern __shared__ unsigned char smem_raw[];
   ScanSmem32& s = *reinterpret_cast<ScanSmem32*>(smem_raw + pad_to_1024(smem_raw));
   const int tid = threadIdx.x, lane = tid & 31;
@@ -563,8 +565,9 @@ int launch_f32_fwd(const F32Params& p, long long tiles, cudaStream_t st) {
   if (rc != KDA_OK) return rc;
   if (tiles > 0x7fffffffLL) return KDA_E_SHAPE;
   kda_f32_prepare_kernel<<<static_cast<unsigned>(tiles), NT, PREP32_SMEM, st>>>(p);
-  kda_f32_scan_kernel<<<static_cast<unsigned>(p.map.N * p.H), NT, SCAN32_SMEM, st>>>(p);
-  return static_cast<int>(cudaGetLastError());
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return static_cast<int>(e);
+  return static_cast<int>(launch_chained(kda_f32_scan_kernel, static_cast<unsigned>(p.map.N * p.H), NT, SCAN32_SMEM, st, p));
 }
 
 }  // namespace kda

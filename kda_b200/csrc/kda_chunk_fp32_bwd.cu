@@ -41,6 +41,7 @@ __device__ __forceinline__ void load_rows_t(float4 (&x)[4], const float* base, s
 }  // namespace
 
 __global__ void __launch_bounds__(NT, 1) kda_f32_bwd_scan_kernel(const F32Params p) {
+  chain_point();
   extern __shared__ unsigned char smem_raw[];
   RScanSmem32& s = *reinterpret_cast<RScanSmem32*>(smem_raw + pad_to_1024(smem_raw));
   const int tid = threadIdx.x, lane = tid & 31;
@@ -197,6 +198,7 @@ constexpr int M_DQG = 0, M_DW = 64, M_DKG = 128, M_DAQ = 192, M_DTM = 256, M_DBV
 }  // namespace
 
 __global__ void __launch_bounds__(NT, 1) kda_f32_bwd_main_kernel(const F32Params p) {
+  chain_point();
   extern __shared__ unsigned char smem_raw[];
   MainSmem32& s = *reinterpret_cast<MainSmem32*>(smem_raw + pad_to_1024(smem_raw));
   const int tid = threadIdx.x, lane = tid & 31;
@@ -563,6 +565,7 @@ __global__ void __launch_bounds__(NT, 1) kda_f32_bwd_main_kernel(const F32Params
 // dq, dk from the gradients w.r.t. the rows the chunk kernels saw, per value head: sum over the heads of a group, then the backward of
 // x^ = x rsqrt(sum x^2 + eps).  One warp per row of q and k.
 __global__ void __launch_bounds__(256) kda_f32_bwd_finish_kernel(const F32Params p, long long rows) {
+  chain_point();
   const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31, kk = 4 * lane;
   if (row >= rows) return;
@@ -596,12 +599,12 @@ int launch_f32_bwd(const F32Params& p, long long tiles, cudaStream_t st) {
   if (rc != KDA_OK) return rc;
   if (tiles > 0x7fffffffLL) return KDA_E_SHAPE;
   kda_f32_bwd_scan_kernel<<<static_cast<unsigned>(p.map.N * p.H), NT, RSCAN32_SMEM, st>>>(p);
-  kda_f32_bwd_main_kernel<<<static_cast<unsigned>(tiles), NT, MAIN32_SMEM, st>>>(p);
-  return static_cast<int>(cudaGetLastError());
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return static_cast<int>(e);
+  return static_cast<int>(launch_chained(kda_f32_bwd_main_kernel, static_cast<unsigned>(tiles), NT, MAIN32_SMEM, st, p));
 }
 int launch_f32_finish(const F32Params& p, long long rows, cudaStream_t st) {
-  kda_f32_bwd_finish_kernel<<<static_cast<unsigned>((rows + 7) / 8), 256, 0, st>>>(p, rows);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_chained(kda_f32_bwd_finish_kernel, static_cast<unsigned>((rows + 7) / 8), 256, 0, st, p, rows));
 }
 
 }  // namespace kda

@@ -28,6 +28,7 @@ namespace kda {
 __global__ void __launch_bounds__(1024) kda_chunk_tables_kernel(const int* __restrict__ cu, int N, long long tokens, int max_chunks,
                                                                 int* __restrict__ seq_chunk_off, int* __restrict__ chunk_seq,
                                                                 int* __restrict__ seq_order, unsigned* __restrict__ status) {
+  chain_point();
   __shared__ int warp_sum_[32];
   __shared__ int offs[1025];      // chunk offsets of the first 1,024 sequences (all of them in ordinary calls)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;

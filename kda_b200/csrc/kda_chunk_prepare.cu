@@ -173,6 +173,7 @@ __device__ __forceinline__ void prep_mma(float (&acc)[NB][4], const __nv_bfloat1
 // SAFE: the caller promises bounded gates (safe_gate: at least -5 per token), see above.
 template <bool KEEP_QN, bool SAFE>
 __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(const __grid_constant__ PrepParams p) {
+  chain_point();
   extern __shared__ unsigned char smem_raw[];
   PrepSmem& s = *reinterpret_cast<PrepSmem*>(smem_raw + pad_to_1024(smem_raw));
   const int tid = threadIdx.x, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
@@ -808,13 +809,10 @@ int launch_prepare(PrepParams& p, long long tiles, long long tokens, bool keep_q
        make_rows_tmap(&p.tm_g, p.g_raw ? p.g_raw : p.g, !p.g_raw || p.g_fp32, tokens, p.H, p.kc, KD, C, false)))
     return KDA_E_TMAP;
   const unsigned grid = static_cast<unsigned>(tiles);
-  if (safe_gate) {
-    if (keep_qn) kda_chunk_prepare_kernel<true, true><<<grid, PREP_THREADS, smem, st>>>(p);
-    else kda_chunk_prepare_kernel<false, true><<<grid, PREP_THREADS, smem, st>>>(p);
-  } else {
-    if (keep_qn) kda_chunk_prepare_kernel<true, false><<<grid, PREP_THREADS, smem, st>>>(p);
-    else kda_chunk_prepare_kernel<false, false><<<grid, PREP_THREADS, smem, st>>>(p);
-  }
+  const auto kernel = safe_gate ? (keep_qn ? kda_chunk_prepare_kernel<true, true> : kda_chunk_prepare_kernel<false, true>)
+                                : (keep_qn ? kda_chunk_prepare_kernel<true, false> : kda_chunk_prepare_kernel<false, false>);
+  if (!p.clear_status) return static_cast<int>(launch_chained(kernel, grid, PREP_THREADS, smem, st, p));      // behind the tables kernel
+  kernel<<<grid, PREP_THREADS, smem, st>>>(p);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -53,6 +53,7 @@ __device__ __forceinline__ unsigned char* swp(unsigned char* tile, int row, int 
 }  // namespace
 
 __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanParams p) {
+  chain_point();
   extern __shared__ unsigned char smem_raw[];
   TcScanSmem& s = *reinterpret_cast<TcScanSmem*>(smem_raw + pad_to_1024(smem_raw));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -303,8 +304,7 @@ int launch_scan_tc(const ScanParams& p, int blocks, cudaStream_t st) {
   const int smem = static_cast<int>(sizeof(TcScanSmem)) + 1024;
   const int rc = once.run([&] { return cudaFuncSetAttribute(kda_chunk_scan_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
   if (rc != KDA_OK) return rc;
-  kda_chunk_scan_tc_kernel<<<blocks, SNT, smem, st>>>(p);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_chained(kda_chunk_scan_tc_kernel, blocks, SNT, smem, st, p));
 }
 
 }  // namespace kda

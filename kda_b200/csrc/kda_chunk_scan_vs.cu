@@ -86,6 +86,7 @@ __device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
 
 template <int VS>
 __global__ void __launch_bounds__(VS_THREADS, 1) kda_chunk_scan_vs_kernel(const ScanParams p) {
+  chain_point();
   constexpr int NS = VD / VS;            // slices (CTAs) per unit
   constexpr int HC = VS / 2;             // columns per compute thread (two column halves)
   constexpr int C_H = 0, C_VN = VS, C_O = 2 * VS;      // TMEM columns; o double buffered: C_O + VS * (chunk & 1)
@@ -387,8 +388,7 @@ static int launch_vs(const ScanParams& p, int units, cudaStream_t st) {
   const int smem = static_cast<int>(sizeof(VsSmem<VS>)) + 1024;
   const int rc = once.run([&] { return cudaFuncSetAttribute(kda_chunk_scan_vs_kernel<VS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
   if (rc != KDA_OK) return rc;
-  kda_chunk_scan_vs_kernel<VS><<<units * (VD / VS), VS_THREADS, smem, st>>>(p);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_chained(kda_chunk_scan_vs_kernel<VS>, units * (VD / VS), VS_THREADS, smem, st, p));
 }
 
 int launch_scan_vs(const ScanParams& p, int units, cudaStream_t st) { return launch_vs<32>(p, units, st); }

@@ -13,6 +13,13 @@ constexpr int C = KDA_CHUNK;              // tokens per chunk
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float L2NORM_EPS = 1e-6f;
 
+// First statement of every kernel that takes part in a chain of launches (launch_chained): waits until the kernels in front have finished
+// and their writes are visible, then lets the next kernel of the chain come up.
+__device__ __forceinline__ void chain_point() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---- small numeric helpers ---------------------------------------------------------------------
 __device__ __forceinline__ float ex2(float x) {  // 2^x, ex2.approx (flushes tiny results to 0, never overflows for x<=0)
   float y;

@@ -9,6 +9,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "kda_b200.h"
@@ -47,10 +48,33 @@ struct DeviceOnce {
   }
 };
 
-// SMs of the current device
+// Launches a kernel of a call behind the previous kernel of the same call: its CTAs may be brought up while that one's last CTAs still
+// run (programmatic dependent launch), which hides the launch latency and the drain.  Such a kernel starts with chain_point(), before
+// it touches memory or asks for tensor memory: that is where it waits for everything in front of it.
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &attr;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
+// SMs of the current device (asked once per device)
 inline int sm_count() {
+  static std::atomic<int> known[kMaxDeviceOrdinals];
   int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (cudaGetDevice(&dev) != cudaSuccess) return sms;
+  const bool keep = dev >= 0 && dev < kMaxDeviceOrdinals;
+  if (keep && known[dev].load(std::memory_order_relaxed) > 0) return known[dev].load(std::memory_order_relaxed);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (keep) known[dev].store(sms, std::memory_order_relaxed);
   return sms;
 }
 

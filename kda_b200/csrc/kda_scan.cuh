@@ -2,6 +2,7 @@
 #pragma once
 
 #include "kda_chunk.cuh"
+#include "kda_device.cuh"
 
 namespace kda {
 
@@ -30,9 +31,7 @@ int launch_scan_vs(const ScanParams& p, int units, cudaStream_t st);
 // than one CTA per unit at every size, because the chain's cost is latency, not the width of its products.)
 inline int scan_slices_for(int units, int requested) {
   if (requested == 1 || requested == 4) return requested;
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return units * 4 <= sms ? 4 : 1;
+  return units * 4 <= sm_count() ? 4 : 1;
 }
 
 }  // namespace kda

@@ -51,6 +51,36 @@ inline int make_rows_tmap(CUtensorMap* m, const void* base, bool fp32, long long
   return r == CUDA_SUCCESS ? 0 : 2;
 }
 
+// Map of fp32 rows of `cols` columns (states as [slots * heads * K][V]) with boxes of box_rows rows x box_cols columns.  The number of
+// rows is not known to the callers (slot numbers are device data): the map has no useful upper bound.
+inline int make_states_tmap(CUtensorMap* m, const void* base, int cols, int box_cols, int box_rows) {
+  TmapEncodeFn fn = tmap_encode_fn();
+  if (!fn) return 1;
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), 0x7fffffffull};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 4};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows)}, estr[2] = {1u, 1u};
+  auto encode = [&] {
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {      // see make_rows_tmap
+    cudaFree(nullptr);
+    r = encode();
+  }
+  return r == CUDA_SUCCESS ? 0 : 2;
+}
+
+// the box at (column c0, row c1) of a two-dimensional map: global -> shared, completing its bytes on `bar`, and shared -> global
+__device__ __forceinline__ void tma_load_2d(void* dst_smem, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst_smem)),
+               "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
+               : "memory");
+}
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int c0, int c1, const void* src_smem) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(c0), "r"(c1), "r"(smem_u32(src_smem)) : "memory");
+}
+
 // global -> shared tiled load of the box at (column c0, head c1, token c2); completes `box bytes` on `bar`.
 // c0 * element size must be a multiple of 16 bytes.
 __device__ __forceinline__ void tma_load_rows(void* dst_smem, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {

@@ -248,3 +248,57 @@ def test_empty_and_errors():
     e = _cuda(make_inputs(2, 0, 2, 64, 64, torch.float32, seed=1, h0_std=0.1))
     o, ht = fused_recurrent_kda(e["q"], e["k"], e["v"], e["g"], e["beta"], initial_state=e["h0"], output_final_state=True)
     assert o.shape == (2, 0, 2, 64) and torch.equal(ht, e["h0"])
+
+
+@pytest.mark.parametrize("case", ["plain", "gate_slots_gva", "transposed_slots"])
+def test_whole_state_decode_kernel(case):
+    """37 sequences x 128 heads = 4,736 states, one token each: whole states on the bulk-copy kernel (from 32 per SM on).  o and states
+    against the float64 oracle on the GPU."""
+    from kda_b200 import _lib, fused_recurrent_kda_fwd
+    N, H = 37, 128
+    d = make_inputs(N, 1, H, 128, 128, torch.bfloat16, seed=77, h0_std=0.05, device="cuda", generate_on_device=True)
+    HQ = 32 if "gva" in case else H
+    q, k = d["q"][:, :, :HQ].contiguous(), d["k"][:, :, :HQ].contiguous()
+    rep = H // HQ
+    g, beta, kw = d["g"], d["beta"], {}
+    if "gate" in case:
+        from oracle.kda_oracle import beta_sigmoid, kda_gate
+        g_raw, beta_raw = torch.randn_like(g).bfloat16(), torch.randn_like(beta).bfloat16()
+        A_log, dt_bias = torch.rand(H, device="cuda"), torch.randn(H * 128, device="cuda") * 0.5
+        g, beta = kda_gate(g_raw, A_log, dt_bias), beta_sigmoid(beta_raw)
+        kw = dict(A_log=A_log, dt_bias=dt_bias, use_gate_in_kernel=True, use_beta_sigmoid_in_kernel=True)
+    o_ref, h_ref = recurrent_kda(q.repeat_interleave(rep, 2), k.repeat_interleave(rep, 2), d["v"], g, beta, initial_state=d["h0"], output_final_state=True)
+    tr = case.startswith("transposed")
+    h0 = d["h0"].transpose(-1, -2).contiguous() if tr else d["h0"]
+    pool, idx = h0.clone(), None
+    if "slots" in case:
+        idx = torch.randperm(N + 3, device="cuda")[:N].to(torch.int32)
+        pool = torch.full((N + 3, *h0.shape[1:]), 7.0, device="cuda")
+        pool[idx.long()] = h0
+    gin, bin_ = (g_raw, beta_raw) if "gate" in case else (g, beta)
+    o, _ = fused_recurrent_kda_fwd(q, k, d["v"], gin, bin_, initial_state=pool, ssm_state_indices=idx, transpose_state_layout=tr, **kw)
+    ht = pool if idx is None else pool[idx.long()]
+    assert _lib.recurrent_status() == 0
+    assert max_norm_err(o, o_ref) <= 2e-2 and cosine(o, o_ref) >= 0.9999
+    assert max_norm_err(ht.transpose(-1, -2) if tr else ht, h_ref) <= 1e-4
+
+
+@pytest.mark.parametrize("N,T,H,tr", [(5, 2, 16, False), (5, 5, 16, True), (70, 3, 16, False), (70, 3, 16, True)])
+def test_draft_tokens_on_half_states(N, T, H, tr):
+    """Several tokens per sequence with a slot for every state: fewer units than CTAs, an odd number of tokens, several rounds."""
+    from kda_b200 import _lib, fused_recurrent_kda_fwd
+    d = make_inputs(N, T, H, 128, 128, torch.bfloat16, seed=78 + N + T, h0_std=0.05, device="cuda", generate_on_device=True)
+    slots = torch.randperm(N * T + 2, device="cuda")[:N * T].to(torch.int32).view(N, T)
+    accepted = torch.randint(1, T + 1, (N,), device="cuda").to(torch.int32)
+    start = slots.gather(1, (accepted.long() - 1).unsqueeze(1)).squeeze(1).long()
+    pool = torch.full((N * T + 2, H, 128, 128), 7.0, device="cuda")
+    pool[start] = d["h0"].transpose(-1, -2) if tr else d["h0"]
+    o, _ = fused_recurrent_kda_fwd(d["q"], d["k"], d["v"], d["g"], d["beta"], initial_state=pool, ssm_state_indices=slots, num_accepted_tokens=accepted,
+                                   transpose_state_layout=tr)
+    assert _lib.recurrent_status() == 0
+    for t in range(T):
+        o_ref, h_ref = recurrent_kda(*(d[n][:, :t + 1] for n in ("q", "k", "v", "g", "beta")), initial_state=d["h0"], output_final_state=True)
+        got = pool[slots[:, t].long()]
+        assert max_norm_err(got.transpose(-1, -2) if tr else got, h_ref) <= 1e-4, t
+    assert max_norm_err(o, o_ref) <= 2e-2 and cosine(o, o_ref) >= 0.9999
+    assert int((pool == 7.0).all(-1).all(-1).all(-1).sum()) == 2      # the two slots nobody owns
