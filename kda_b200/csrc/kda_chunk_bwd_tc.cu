@@ -23,6 +23,8 @@
 #include "kda_device.cuh"
 #include "kda_umma.cuh"
 
+#include <type_traits>
+
 namespace kda {
 
 namespace {
@@ -41,10 +43,10 @@ struct TcSmem {
   unsigned char TI[TILE_TT];    // B1..B3.  D (with RKK): dk staging [64][128]
   unsigned char RKK[TILE_TT];   // post-B3
   // ---- plain arrays -----------------------------------------------------------------------------------------------
-  __nv_bfloat16 q[C * KD];      // [64][128]   (q, k, g of the NEXT tile arrive here during phase D)
+  __nv_bfloat16 q[C * KD];      // [64][128]
   __nv_bfloat16 k[C * KD];
-  float G[C * KD];              // log2-domain cumsum of g
-  float2 Ad[4][16][17];         // diagonal blocks: (a1, a2) = (scale dAqk, beta dAkk); rows padded against bank conflicts
+  float G[C * KD];              // log2-domain cumsum of g (g of the NEXT tile arrives here during phase D)
+  float2 Ad[4][16][18];         // diagonal blocks: (a1, a2) = (scale dAqk, beta dAkk); rows 16-byte aligned
   float beta[C];
   float hdh[KD];                // sum over v of h dh'
   union {
@@ -55,7 +57,7 @@ struct TcSmem {
     };
   };
   float carry[4][KD];           // block totals of the reverse cumsum
-  uint64_t barS, barQ, barB, barM;
+  uint64_t barS, barG, barQ, barB, barM;
   long long ci_tok0[2];         // first token and length of the chunk of the current / next tile (written by thread 0)
   int ci_len[2];
   uint32_t tmem_slot;
@@ -96,8 +98,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
   extern __shared__ unsigned char smem_raw[];
   TcSmem& s = *reinterpret_cast<TcSmem*>(smem_raw + pad_to_1024(smem_raw));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int q4 = warp & 3, part = warp >> 2;          // TMEM lane quadrant of this warp; which 16 of the 64 columns
-  const long long total_tiles = static_cast<long long>(p.map.total()) * p.H;
+  const int total_tiles = p.map.total() * p.H;      // the launch checks that it fits
 
   // aliases inside the tile regions
   unsigned char* const sKG = s.HS;
@@ -118,47 +119,55 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
   // thread 0: the phase-A operands of tile idx -- state tiles by bulk copy, dO by two tiled loads (64 value columns each)
   // thread 0: first token and length of tile idx's chunk into slot (two dependent global loads: done early, off the
   // critical path, while phase B2 executes and the other warps build operands)
-  auto stash_chunk = [&](long long idx, int slot) {
-    const ChunkInfo cn = p.map.info(static_cast<int>(idx / p.H));
+  auto stash_chunk = [&](int idx, int slot) {
+    const ChunkInfo cn = p.map.info(idx / p.H);
     s.ci_tok0[slot] = cn.tok0;
     s.ci_len[slot] = cn.len;
   };
-  auto fetch_state = [&](long long idx, int slot) {      // after stash_chunk(idx, slot)
+  // copy `which` of the seven that bring tile idx's state tiles and dO (barS) and g (barG); after stash_chunk(idx, slot).  One warp issues
+  // one each: a copy costs its thread 200 cycles.
+  auto fetch = [&](int idx, int slot, int which) {
     const size_t tl = static_cast<size_t>(idx);
-    const int hh = static_cast<int>(idx % p.H);
-    struct { long long tok0; } cn;
-    cn.tok0 = s.ci_tok0[slot];
-    mbar_expect_tx(&s.barS, 2 * TILE_VK + 2 * TILE_VT + TILE_TK);
-    bulk_g2s(s.HS, p.HS + tl * TILE_VK, TILE_VK, &s.barS);
-    bulk_g2s(s.DH, p.DH + tl * TILE_VK, TILE_VK, &s.barS);
-    bulk_g2s(s.VN, p.VNEWT + tl * TILE_VT, TILE_VT, &s.barS);
-    bulk_g2s(s.DVN, p.DVNEWT + tl * TILE_VT, TILE_VT, &s.barS);
-    tma_load_rows(s.dO, &p.tm_do, 0, hh, static_cast<int>(cn.tok0), &s.barS);
-    tma_load_rows(s.dO + 8192, &p.tm_do, 64, hh, static_cast<int>(cn.tok0), &s.barS);
+    const int hh = idx % p.H, tk = static_cast<int>(s.ci_tok0[slot]);
+    mbar_expect_tx(which < 6 ? &s.barS : &s.barG, which < 2 ? TILE_VK : (which < 4 ? TILE_VT : (which < 6 ? TILE_TK / 2 : C * KD * 4)));
+    switch (which) {
+      case 0: bulk_g2s(s.HS, p.HS + tl * TILE_VK, TILE_VK, &s.barS); break;
+      case 1: bulk_g2s(s.DH, p.DH + tl * TILE_VK, TILE_VK, &s.barS); break;
+      case 2: bulk_g2s(s.VN, p.VNEWT + tl * TILE_VT, TILE_VT, &s.barS); break;
+      case 3: bulk_g2s(s.DVN, p.DVNEWT + tl * TILE_VT, TILE_VT, &s.barS); break;
+      case 4: tma_load_rows(s.dO, &p.tm_do, 0, hh, tk, &s.barS); break;
+      case 5: tma_load_rows(s.dO + 8192, &p.tm_do, 64, hh, tk, &s.barS); break;
+      default: tma_load_rows(s.G, &p.tm_g, 0, hh, tk, &s.barG); break;
+    }
   };
-  // thread 0: q, k, g of tile idx
-  auto fetch_qkg = [&](long long idx, int slot) {      // after fetch_state(idx, slot)
-    const int hh = static_cast<int>(idx % p.H);
-    const int tk = static_cast<int>(s.ci_tok0[slot]);
-    mbar_expect_tx(&s.barQ, 2 * TILE_TK + C * KD * 4);
-    tma_load_rows(s.q, &p.tm_q, 0, hh / p.grp, tk, &s.barQ);
-    tma_load_rows(s.k, &p.tm_k, 0, hh / p.grp, tk, &s.barQ);
-    tma_load_rows(s.G, &p.tm_g, 0, hh, tk, &s.barQ);
+  // copy `which` of the six that this tile itself starts with: q, k (barQ, needed behind phase A), Tm, raw kk, v (barB, from phase B1 on)
+  auto fetch_late = [&](int idx, int h, int tk, int which) {
+    const size_t tl = static_cast<size_t>(idx);
+    fence_proxy_async();        // the previous tile read q, k and its dq / dk staging out of this memory
+    mbar_expect_tx(which < 2 ? &s.barQ : &s.barB, which < 2 ? TILE_TK : TILE_TT);
+    switch (which) {
+      case 0: tma_load_rows(s.k, &p.tm_k, 0, h / p.grp, tk, &s.barQ); break;
+      case 1: tma_load_rows(s.q, &p.tm_q, 0, h / p.grp, tk, &s.barQ); break;
+      case 2: bulk_g2s(s.TI, p.TI + tl * TILE_TT, TILE_TT, &s.barB); break;
+      case 3: bulk_g2s(s.RKK, p.RKK + tl * TILE_TT, TILE_TT, &s.barB); break;
+      case 4: tma_load_rows(s.V, &p.tm_v, 0, h, tk, &s.barB); break;
+      default: tma_load_rows(s.V + 8192, &p.tm_v, 64, h, tk, &s.barB); break;
+    }
   };
   // rows of a partial chunk beyond its length hold the next sequence's tokens after a tiled load: clear them
   auto zero_rows_sw = [&](unsigned char* tile, int len) {          // [64][64] bf16 sub-tile, 128-byte rows
     for (int i = len * 8 + tid; i < C * 8; i += NT) *reinterpret_cast<uint4*>(tile + i * 16) = make_uint4(0u, 0u, 0u, 0u);
   };
   if (tid == 0) {
-    mbar_init(&s.barS, 1);
-    mbar_init(&s.barQ, 1);
-    mbar_init(&s.barB, 1);
+    mbar_init(&s.barS, 6);      // one arrival per copy
+    mbar_init(&s.barG, 1);
+    mbar_init(&s.barQ, 2);
+    mbar_init(&s.barB, 4);
     mbar_init(&s.barM, 1);
     fence_mbar_init();
-    if (static_cast<long long>(blockIdx.x) < total_tiles) {
+    if (static_cast<int>(blockIdx.x) < total_tiles) {
       stash_chunk(blockIdx.x, 0);
-      fetch_state(blockIdx.x, 0);
-      fetch_qkg(blockIdx.x, 0);
+      for (int i = 0; i < 7; ++i) fetch(blockIdx.x, 0, i);
     }
   }
   __syncwarp();
@@ -169,7 +178,8 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
   const uint32_t tb = __shfl_sync(0xffffffffu, s.tmem_slot, 0);          // warp-uniform for the compiler
   const int warp_u = __shfl_sync(0xffffffffu, warp, 0);
   const uint32_t lead = lane == 0;                                      // the lane of warp 0 that issues the MMAs
-  const uint32_t tq = tb + (static_cast<uint32_t>(32 * q4) << 16);     // this warp's lanes
+  // TMEM lane quadrant of a warp: warp & 3; which 16 of the 64 columns: warp >> 2
+  const uint32_t tq = tb + (static_cast<uint32_t>(32 * (warp_u & 3)) << 16);     // this warp's lanes
 
   // Operands of phase C, built while the phase-B products run (rows R of the stacked tiles, 16-byte pieces pc):
   // kR_I[j][kk] = k_j 2^(G_r - G_j),  r = 16 I,  j < 16 I            rows stacked: I=1 -> 0..15, I=2 -> 16..47, I=3 -> 48..95
@@ -213,27 +223,28 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
   uint32_t mph = 0;      // phase counter of barM
   bool alive = true;
   int it = 0;
-  for (long long idx = blockIdx.x; idx < total_tiles && alive; idx += gridDim.x, ++it) {
-    const int h = static_cast<int>(idx % p.H);
-    struct { long long tok0; int len; } ci;
-    ci.tok0 = s.ci_tok0[it & 1];
+  // An opaque copy of the thread number, taken afresh in the phases: what is derived from it (shared-memory addresses above all) then
+  // lives for that phase alone.  Kept across a tile it all together left the last phase 40 registers short, and its spills miss
+  // the little L1 that is left beside 224 KB of shared memory.
+  auto fresh_tid = [&] {
+    int t = threadIdx.x;
+    asm volatile("" : "+r"(t));
+    return t;
+  };
+  for (int idx = blockIdx.x; idx < total_tiles && alive; idx += gridDim.x, ++it) {
+    const int tid = fresh_tid(), lane = tid & 31, q4 = warp_u & 3, part = warp_u >> 2;
+    const int h = idx % p.H;
+    struct { int tok0; int len; } ci;
+    ci.tok0 = static_cast<int>(s.ci_tok0[it & 1]);
     ci.len = s.ci_len[it & 1];
     const int len = ci.len;
     const size_t tile = static_cast<size_t>(idx);
-    const long long next_idx = idx + gridDim.x;
+    const int next_idx = idx + gridDim.x;
     long long* const dbg = (it == 2) ? p.dbg : nullptr;   // development aid: clocks of a steady-state tile
 
     KDA_DBG_CLOCK(dbg, 0);
-    // ---- third load group: Tm, raw kk (bulk), v (tiled), beta (async copies); needed from phase B1 on ---------------
-    if (tid == 0) {
-      fence_proxy_async();        // the previous tile read its dq / dk staging out of this memory
-      mbar_expect_tx(&s.barB, 2 * TILE_TT + TILE_TK);
-      bulk_g2s(s.TI, p.TI + tile * TILE_TT, TILE_TT, &s.barB);
-      bulk_g2s(s.RKK, p.RKK + tile * TILE_TT, TILE_TT, &s.barB);
-      const int tk = static_cast<int>(ci.tok0);
-      tma_load_rows(s.V, &p.tm_v, 0, h, tk, &s.barB);
-      tma_load_rows(s.V + 8192, &p.tm_v, 64, h, tk, &s.barB);
-    }
+    // ---- second load group: q, k, Tm, raw kk, v; beta by async copies
+    if (lane == 0 && warp_u >= 1 && warp_u < 7) fetch_late(idx, h, ci.tok0, warp_u - 1);
     if (tid < C) cp_async4(&s.beta[tid], p.beta + static_cast<size_t>(ci.tok0 + (tid < len ? tid : 0)) * p.H + h, tid < len);
     cp_async_commit();
     if (!mbar_wait(&s.barS, it & 1)) {
@@ -287,13 +298,11 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     KDA_DBG_CLOCK(dbg, 2);
     // ---- meanwhile, on warps 1..15 (warp 0 is held up by the issue loop; a barrier that includes it would make
     // everybody wait for the loop's end, so these warps meet at named barrier 1 and warp 1 takes warp 0's columns):
-    // G = cumsum(g) log2(e)  (q, k, g arrived during the previous tile's phase D) ------------------------------------
+    // G = cumsum(g) log2(e)  (g arrived during the previous tile's phase D) ------------------------------------
     if (warp_u != 0) {
-      if (alive && !mbar_wait(&s.barQ, it & 1)) alive = false;
+      if (alive && !mbar_wait(&s.barG, it & 1)) alive = false;
       if (len < C) {
         for (int i = len * 16 + tid - 32; i < C * 16; i += NT - 32) {
-          reinterpret_cast<uint4*>(s.q)[i] = make_uint4(0u, 0u, 0u, 0u);
-          reinterpret_cast<uint4*>(s.k)[i] = make_uint4(0u, 0u, 0u, 0u);
           reinterpret_cast<uint4*>(s.G)[2 * i] = make_uint4(0u, 0u, 0u, 0u);
           reinterpret_cast<uint4*>(s.G)[2 * i + 1] = make_uint4(0u, 0u, 0u, 0u);
         }
@@ -365,6 +374,14 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
           for (int cc = 0; cc < 16; ++cc) s.Ad[q4][lane][cc].x = p.scale * v[cc];
         }
       }
+    }
+    if (!mbar_wait(&s.barQ, it & 1)) alive = false;
+    if (len < C) {                 // uniform over the CTA
+      for (int i = len * 16 + tid; i < C * 16; i += NT) {
+        reinterpret_cast<uint4*>(s.q)[i] = make_uint4(0u, 0u, 0u, 0u);
+        reinterpret_cast<uint4*>(s.k)[i] = make_uint4(0u, 0u, 0u, 0u);
+      }
+      __syncthreads();
     }
     for (int i = tid; i < C * 32; i += NT) {          // k Gam as two K-major sub-tiles [64 j][64 kk]
       const int j = i >> 5, g4 = i & 31;
@@ -597,14 +614,14 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     }
     // =========================== phase D: one thread per key column and 16-row block ================================
     // Part 1 needs only accumulators of phases A and B1 and runs while phase C executes.
-    const int kk = 32 * q4 + lane, blk = part, t0 = 16 * blk;
-    float cq[16], cp[16], cn[16], lam[16], qv[16], kv[16];
-    float gam_last;
+    const int kk = fresh_tid() & 127, blk = warp_u >> 2, t0 = 16 * blk;
+    float cq[16], cp[16], lam[16];
+    float gam_last, e_last;
     {
       // Decay inside the block as running products of lam_i = 2^(G_i - G_{i-1}) (every factor <= 1):
       //   2^(G_i - G_first) = fl_i,  2^(G_i) = 2^(G_first) fl_i,  2^(G_e - G_i) = fr_i,  2^(G_last - G_i) = 2^(G_last - G_e) fr_i
       float a[16], a2[16];
-      float g_first, e_last;
+      float g_first;
       {
         float prev = s.G[t0 * KD + kk];
         g_first = ex2(prev);
@@ -627,9 +644,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
         float dglp = 0.f, fr = 1.f;
 #pragma unroll
         for (int i = 15; i >= 0; --i) {
-          const float dke = a[i] * (e_last * fr);
-          dglp = fmaf(__bfloat162float(s.k[(t0 + i) * KD + kk]), dke, dglp);
-          cn[i] = dke;
+          dglp = fmaf(__bfloat162float(s.k[(t0 + i) * KD + kk]), a[i] * (e_last * fr), dglp);
           fr *= lam[i];
         }
         s.dglp[blk][kk] = dglp;
@@ -654,26 +669,18 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
           cp[i] = fl * s.beta[t0 + i] * a[i];
         }
       }
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        qv[i] = __bfloat162float(s.q[(t0 + i) * KD + kk]);
-        kv[i] = __bfloat162float(s.k[(t0 + i) * KD + kk]);
-      }
     }
     if (!mbar_wait(&s.barM, mph & 1)) alive = false;
     ++mph;
-    alive = __syncthreads_and(alive);      // phase C complete; q, k, G have been read by everybody; dglp is complete
+    alive = __syncthreads_and(alive);      // phase C complete; G has been read by everybody; dglp is complete
     if (!alive) {
       if (tid == 0) atomicOr(p.status, 64u);
       break;
     }
     umma::fence_after_sync();
     KDA_DBG_CLOCK(dbg, 10);
-    // every shared-memory operand tile is dead now and q, k, g are in registers: fetch the next tile behind the rest
-    if (next_idx < total_tiles && tid == 0) {
-      fetch_state(next_idx, (it + 1) & 1);
-      fetch_qkg(next_idx, (it + 1) & 1);
-    }
+    // every shared-memory operand tile is dead now and g is in registers (lam): fetch the next tile behind the rest
+    if (next_idx < total_tiles && warp_u < 7 && lane == 0) fetch(next_idx, (it + 1) & 1, warp_u);
     if (tid < len)
       p.dbeta[static_cast<size_t>(ci.tok0 + tid) * p.H + h] = s.dbp[0][tid] + s.dbp[1][tid] + s.dbp[2][tid] + s.dbp[3][tid] +
                                                              s.dbp[4][tid] + s.dbp[5][tid] + s.dbp[6][tid] + s.dbp[7][tid];
@@ -683,16 +690,6 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
       {
         // part 2: the off-diagonal blocks of phase C, scaled back from their reference rows
         float b[16];
-        if (blk < 3) {                          // dk-: + 2^(G_e - G) Cn
-          umma::tmem_ld16(tq + C_CN + t0, b);
-          umma::tmem_ld_wait();
-          float fr = 1.f;
-#pragma unroll
-          for (int i = 15; i >= 0; --i) {
-            cn[i] = fmaf(fr, b[i], cn[i]);
-            fr *= lam[i];
-          }
-        }
         if (blk > 0) {                          // dq: + scale L Cq;  dk+: + L Cp
           umma::tmem_ld16(tq + C_CQ + t0, b);
           umma::tmem_ld_wait();
@@ -713,37 +710,132 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
         }
       }
       KDA_DBG_CLOCK(dbg, 12);
-      // diagonal block, pairwise; D = running product of lam (range-safe)
+      // Diagonal block.  Rows 8..15 against columns 0..7, then 4..7 against 0..3 and 12..15 against 8..11, with the decay cut at the
+      // border between them: L_t = prod(border .. t) on the row side, R_j = prod(j+1 .. border-1) on the column side, both running products
+      // of lam (range-safe).  Factored this way an entry costs four multiply-adds instead of the eight operations of a pair with its
+      // own decay; only the 4 x 4 blocks on the diagonal stay pairwise.
+      // Four columns at a time, in rising order: behind its own columns a row is final (it only sees earlier ones), so dk- lives for four
+      // rows only (its other terms wait in tensor memory) and dq, dk leave for their staging tiles at once.  With dk- of all sixteen
+      // rows in registers the phase spilled, and spills miss the little L1 that is left: it took 6.4 k of a tile's 30 k cycles.
+      auto qof = [&](int i) { return __bfloat162float(s.q[(t0 + i) * KD + kk]); };
+      auto kof = [&](int i) { return __bfloat162float(s.k[(t0 + i) * KD + kk]); };
+      // keeps the compiler from carrying q, k (read from shared memory where they are used) or products of lam, and (a warp barrier orders memory accesses) from starting later
+      // loads early: sixteen loads of four registers in front of a part would not fit
+      auto step = [&] {
 #pragma unroll
-      for (int t = 0; t < 16; ++t) {
-        float D = 1.f;
+        for (int i = 0; i < 16; ++i) asm volatile("" : "+f"(lam[i])::"memory");
+        __syncwarp();
+      };
+      float cn[4];
+      // rows r0 .. r0 + W - 1 against the four columns c0 .. c0 + 3, the border in front of row r0
+      auto part4 = [&](auto width, const int r0, const int c0) {
+        constexpr int W = decltype(width)::value;
+        float kR[4], sn[4];
+        float Rc = 1.f;
 #pragma unroll
-        for (int j = t; j >= 0; --j) {
-          const float2 a = s.Ad[blk][t][j];
-          const float kd = kv[j] * D;
-          cq[t] = fmaf(a.x, kd, cq[t]);
-          cp[t] = fmaf(a.y, kd, cp[t]);
-          cn[j] = fmaf(D, fmaf(a.y, kv[t], a.x * qv[t]), cn[j]);
-          D *= lam[j];
+        for (int j = c0 + 4; j < r0; ++j) Rc *= lam[j];
+        {
+          float R = Rc;
+#pragma unroll
+          for (int j = 3; j >= 0; --j) {
+            kR[j] = kof(c0 + j) * R;
+            sn[j] = 0.f;
+            R *= lam[c0 + j];
+          }
         }
-      }
-      KDA_DBG_CLOCK(dbg, 13);
-      // dG; dq, dk into their staging tiles
-      float dGv[16];
+        float L = 1.f;
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        dGv[i] = qv[i] * cq[i] + kv[i] * (cp[i] - cn[i]);
-        stq[(t0 + i) * KD + kk] = __float2bfloat16_rn(cq[i]);
-        stk[(t0 + i) * KD + kk] = __float2bfloat16_rn(cp[i] + cn[i]);
-      }
+        for (int t = 0; t < W; ++t) {
+          if (t && t % 4 == 0) __syncwarp();
+          L *= lam[r0 + t];
+          const float ql = qof(r0 + t) * L, kl = kof(r0 + t) * L;
+          float sq = 0.f, sp = 0.f;
+#pragma unroll
+          for (int j = 0; j < 4; j += 2) {
+            const float4 a = *reinterpret_cast<const float4*>(&s.Ad[blk][r0 + t][c0 + j]);
+            sq = fmaf(a.x, kR[j], sq);
+            sp = fmaf(a.y, kR[j], sp);
+            sn[j] = fmaf(a.x, ql, fmaf(a.y, kl, sn[j]));
+            sq = fmaf(a.z, kR[j + 1], sq);
+            sp = fmaf(a.w, kR[j + 1], sp);
+            sn[j + 1] = fmaf(a.z, ql, fmaf(a.w, kl, sn[j + 1]));
+          }
+          cq[r0 + t] = fmaf(L, sq, cq[r0 + t]);
+          cp[r0 + t] = fmaf(L, sp, cp[r0 + t]);
+        }
+#pragma unroll
+        for (int j = 3; j >= 0; --j) {
+          cn[j] = fmaf(Rc, sn[j], cn[j]);
+          Rc *= lam[c0 + j];
+        }
+      };
+      auto columns = [&](auto first) {
+        constexpr int c0 = decltype(first)::value;
+        {      // dk-: 2^(G_e - G) (2^(G_last - G_e) dkg + Cn)
+          float d4[4];
+          umma::tmem_ld4(tq + C_DKG + t0 + c0, d4);
+          if (blk < 3) umma::tmem_ld4(tq + C_CN + t0 + c0, cn);
+          umma::tmem_ld_wait();
+          float fr = 1.f;
+#pragma unroll
+          for (int j = c0 + 4; j < 16; ++j) fr *= lam[j];
+#pragma unroll
+          for (int j = 3; j >= 0; --j) {
+            cn[j] = fr * (blk < 3 ? fmaf(e_last, d4[j], cn[j]) : e_last * d4[j]);
+            fr *= lam[c0 + j];
+          }
+        }
+        step();
+        if constexpr (c0 < 8) {
+          part4(std::integral_constant<int, 8>{}, 8, c0);
+          step();
+        }
+        if constexpr (c0 % 8 == 0) {
+          part4(std::integral_constant<int, 4>{}, c0 + 4, c0);
+          step();
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const float qt = qof(c0 + t), kt = kof(c0 + t);
+          {
+            const float ax = s.Ad[blk][c0 + t][c0 + t].x;      // dAkk has no diagonal
+            cq[c0 + t] = fmaf(ax, kt, cq[c0 + t]);
+            cn[t] = fmaf(ax, qt, cn[t]);
+          }
+          float D = 1.f;
+#pragma unroll
+          for (int j = t - 1; j >= 0; --j) {
+            D *= lam[c0 + j + 1];
+            const float2 a = s.Ad[blk][c0 + t][c0 + j];
+            const float kd = kof(c0 + j) * D;
+            cq[c0 + t] = fmaf(a.x, kd, cq[c0 + t]);
+            cp[c0 + t] = fmaf(a.y, kd, cp[c0 + t]);
+            cn[j] = fmaf(D, fmaf(a.y, kt, a.x * qt), cn[j]);
+          }
+        }
+        // dq, dk into their staging tiles; cq becomes dG
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const int i = c0 + t;
+          stq[(t0 + i) * KD + kk] = __float2bfloat16_rn(cq[i]);
+          stk[(t0 + i) * KD + kk] = __float2bfloat16_rn(cp[i] + cn[t]);
+          cq[i] = qof(i) * cq[i] + kof(i) * (cp[i] - cn[t]);
+        }
+        step();
+      };
+      columns(std::integral_constant<int, 0>{});
+      columns(std::integral_constant<int, 4>{});
+      columns(std::integral_constant<int, 8>{});
+      columns(std::integral_constant<int, 12>{});
+      KDA_DBG_CLOCK(dbg, 13);
       if (blk == 3)          // the chunk's last row carries the chunk-end terms
-        dGv[15] += s.dglp[0][kk] + s.dglp[1][kk] + s.dglp[2][kk] + s.dglp[3][kk] + gam_last * s.hdh[kk];
+        cq[15] += s.dglp[0][kk] + s.dglp[1][kk] + s.dglp[2][kk] + s.dglp[3][kk] + gam_last * s.hdh[kk];
       {
         float run = 0.f;
 #pragma unroll
         for (int i = 15; i >= 0; --i) {
-          run += dGv[i];
-          dGv[i] = run;
+          run += cq[i];
+          cq[i] = run;
         }
         s.carry[blk][kk] = run;
       }
@@ -771,7 +863,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
         float* const dgp = p.dg + (static_cast<size_t>(ci.tok0 + t0) * p.H + h) * p.kc + kk;      // a warp stores 128 contiguous bytes
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          if (t0 + i < len && kk < p.kc) dgp[static_cast<size_t>(i) * p.H * p.kc] = dGv[i] + add;
+          if (t0 + i < len && kk < p.kc) dgp[static_cast<size_t>(i) * p.H * p.kc] = cq[i] + add;
       }
 #pragma unroll
       for (int u = 0; u < C * 16 / NT; ++u) {
