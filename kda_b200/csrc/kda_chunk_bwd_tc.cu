@@ -115,6 +115,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
   unsigned char* const sKL1 = s.HS + SPAN;
   __nv_bfloat16* const stq = reinterpret_cast<__nv_bfloat16*>(s.V);      // phase D: dq, dk before their coalesced stores
   __nv_bfloat16* const stk = reinterpret_cast<__nv_bfloat16*>(s.TI);
+  float* const stg = reinterpret_cast<float*>(s.q);                            // and dg, over q and k
 
   // thread 0: the phase-A operands of tile idx -- state tiles by bulk copy, dO by two tiled loads (64 value columns each)
   // thread 0: first token and length of tile idx's chunk into slot (two dependent global loads: done early, off the
@@ -140,10 +141,10 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
       default: tma_load_rows(s.G, &p.tm_g, 0, hh, tk, &s.barG); break;
     }
   };
-  // copy `which` of the six that this tile itself starts with: q, k (barQ, needed behind phase A), Tm, raw kk, v (barB, from phase B1 on)
+  // copy `which` of the six that this tile itself starts with: q, k (barQ, needed behind phase A), Tm, raw kk, v (barB, from phase B1 on).
+  // They land where the previous tile staged its results; the warps 1..3 that stored those bring them.
   auto fetch_late = [&](int idx, int h, int tk, int which) {
     const size_t tl = static_cast<size_t>(idx);
-    fence_proxy_async();        // the previous tile read q, k and its dq / dk staging out of this memory
     mbar_expect_tx(which < 2 ? &s.barQ : &s.barB, which < 2 ? TILE_TK : TILE_TT);
     switch (which) {
       case 0: tma_load_rows(s.k, &p.tm_k, 0, h / p.grp, tk, &s.barQ); break;
@@ -154,6 +155,8 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
       default: tma_load_rows(s.V + 8192, &p.tm_v, 64, h, tk, &s.barB); break;
     }
   };
+  // [64 t][32 v] of dv: behind the 96 rows of four phase-C operand tiles
+  auto dv_stage = [&](int i) { return (i == 0 ? sKR0 : (i == 1 ? sKR1 : (i == 2 ? sQL0 : sKL0))) + 96 * 128; };
   // rows of a partial chunk beyond its length hold the next sequence's tokens after a tiled load: clear them
   auto zero_rows_sw = [&](unsigned char* tile, int len) {          // [64][64] bf16 sub-tile, 128-byte rows
     for (int i = len * 8 + tid; i < C * 8; i += NT) *reinterpret_cast<uint4*>(tile + i * 16) = make_uint4(0u, 0u, 0u, 0u);
@@ -243,8 +246,6 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     long long* const dbg = (it == 2) ? p.dbg : nullptr;   // development aid: clocks of a steady-state tile
 
     KDA_DBG_CLOCK(dbg, 0);
-    // ---- second load group: q, k, Tm, raw kk, v; beta by async copies
-    if (lane == 0 && warp_u >= 1 && warp_u < 7) fetch_late(idx, h, ci.tok0, warp_u - 1);
     if (tid < C) cp_async4(&s.beta[tid], p.beta + static_cast<size_t>(ci.tok0 + (tid < len ? tid : 0)) * p.H + h, tid < len);
     cp_async_commit();
     if (!mbar_wait(&s.barS, it & 1)) {
@@ -273,6 +274,13 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
       }
       s.hdh_part[vq][2 * kp] = ax;
       s.hdh_part[vq][2 * kp + 1] = ay;
+    }
+    // ---- second load group: q, k, Tm, raw kk, v (not earlier: the stores of the previous tile's results have to have read this memory)
+    if (lane == 0 && warp_u >= 1 && warp_u < 4) {
+      fence_proxy_async();
+      bulk_wait_read<0>();
+      fetch_late(idx, h, ci.tok0, 2 * (warp_u - 1));
+      fetch_late(idx, h, ci.tok0, 2 * (warp_u - 1) + 1);
     }
     // =========================== phase A: state-dependent products ==================================================
     if (warp_u == 0 && alive) {
@@ -465,7 +473,11 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
         }
         s.dbp[part][j] = acc;
       }
-      {
+      if (len == C) {      // staged in the ends of four operand regions (rows 96.. of the tiles to come) and stored by the copy engine
+        __nv_bfloat16* const st = reinterpret_cast<__nv_bfloat16*>(dv_stage(q4)) + 16 * part * 32 + lane;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) st[32 * i] = __float2bfloat16_rn(s.beta[16 * part + i] * v3[i]);
+      } else {
         const int vcol = 32 * q4 + lane;
         __nv_bfloat16* const dvp = p.dv + (static_cast<size_t>(ci.tok0 + 16 * part) * p.H + h) * p.vc + vcol;
         const size_t tstride = static_cast<size_t>(p.H) * p.vc;
@@ -484,6 +496,11 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     umma::fence_after_sync();
 
     KDA_DBG_CLOCK(dbg, 6);
+    if (warp_u == 4 && lane == 0 && len == C) {
+#pragma unroll 1
+      for (int i = 0; i < 4 && 32 * i < p.vc; ++i) tma_store_rows(&p.tm_dv, 32 * i, h, ci.tok0, dv_stage(i));
+      bulk_commit();
+    }
     // =========================== phase B2: X = dTm Tm^T ============================================================
     if (warp_u == 0) {
       const uint32_t aDT = smem_u32(sDT), aTI = smem_u32(s.TI);
@@ -577,6 +594,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     }
     umma::fence_after_sync();
     KDA_DBG_CLOCK(dbg, 8);
+    if (warp_u == 4 && lane == 0) bulk_wait_read<0>();      // dv has left before the next tile's state tiles arrive there (phase D)
 
     KDA_DBG_CLOCK(dbg, 9);
     // =========================== phase C: off-diagonal blocks of the intra-chunk terms ==============================
@@ -860,11 +878,17 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
         float add = 0.f;             // totals of the later blocks
 #pragma unroll
         for (int bb = 1; bb < 4; ++bb) add += (bb > blk) ? s.carry[bb][kk] : 0.f;
+        if (len == C) {      // into the q, k tiles, which everybody has read
+#pragma unroll
+          for (int i = 0; i < 16; ++i) stg[(t0 + i) * KD + kk] = cq[i] + add;
+        } else {
         float* const dgp = p.dg + (static_cast<size_t>(ci.tok0 + t0) * p.H + h) * p.kc + kk;      // a warp stores 128 contiguous bytes
 #pragma unroll
         for (int i = 0; i < 16; ++i)
           if (t0 + i < len && kk < p.kc) dgp[static_cast<size_t>(i) * p.H * p.kc] = cq[i] + add;
+        }
       }
+      if (L2 || len < C)
 #pragma unroll
       for (int u = 0; u < C * 16 / NT; ++u) {
         const int i = tid + u * NT, r = i >> 4, pc = i & 15;
@@ -909,11 +933,19 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
       }
     }
     KDA_DBG_CLOCK(dbg, 14);
+    fence_proxy_async();
     umma::fence_before_sync();
     __syncthreads();   // beta, Ad, the staging tiles, TMEM ... may be overwritten by the next tile
+    if (lane == 0 && len == C) {      // full chunks leave by the copy engine (partial ones: the rows behind them are another sequence's)
+      if (warp_u == 1) tma_store_rows(&p.tm_dg, 0, h, ci.tok0, stg);
+      if (!L2 && warp_u == 2) tma_store_rows(&p.tm_dk, 0, h, ci.tok0, stk);
+      if (!L2 && warp_u == 3) tma_store_rows(&p.tm_dq, 0, h, ci.tok0, stq);
+      if (warp_u >= 1 && warp_u <= 3) bulk_commit();
+    }
   }
 
   // drain: a copy that is still in flight must not outlive the CTA's shared memory
+  bulk_wait<0>();      // stores
   cp_async_wait<0>();
   umma::fence_before_sync();
   __syncthreads();

@@ -90,6 +90,12 @@ __device__ __forceinline__ void tma_load_rows(void* dst_smem, const CUtensorMap*
                : "memory");
 }
 
+// shared -> global store of a box (bulk group of the issuing thread); columns beyond the tensor's are not written
+__device__ __forceinline__ void tma_store_rows(const CUtensorMap* map, int c0, int c1, int c2, const void* src_smem) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(map), "r"(c0), "r"(c1), "r"(c2),
+               "r"(smem_u32(src_smem))
+               : "memory");
+}
 // the same box into L2 only
 __device__ __forceinline__ void tma_prefetch_rows(const CUtensorMap* map, int c0, int c1, int c2) {
   asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(map), "r"(c0), "r"(c1), "r"(c2) : "memory");
