@@ -132,6 +132,11 @@ __device__ __forceinline__ uint2 ldg_u2(const void* p) {
   asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
   return r;
 }
+__device__ __forceinline__ unsigned long long ldg_u64(const void* p) {
+  unsigned long long r;
+  asm volatile("ld.global.nc.L1::no_allocate.u64 %0, [%1];" : "=l"(r) : "l"(p));
+  return r;
+}
 __device__ __forceinline__ float4 ldg_f4(const float* p) {
   float4 r;
   asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(p));
@@ -191,53 +196,62 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
   // ---- P1: q, k, g of this thread's columns and rows; rows >= len and columns >= kc: q = k = 0, no decay ---------------------------------
   F4 lam[4];
   uint2 q[4], k[4];
+  uint32_t beta_bits = 0u;
   {
     const size_t goff = (static_cast<size_t>(ci.tok0 + t0) * p.H + h) * p.kc + kk;
     const size_t qoff = (static_cast<size_t>(ci.tok0 + t0) * p.HQ + h / p.grp) * p.kc + kk;
     const __nv_bfloat16 *qp = p.q + qoff, *kp = p.k + qoff;
     const size_t gs = static_cast<size_t>(p.H) * p.kc, qs = static_cast<size_t>(p.HQ) * p.kc;
+    // every load is issued before anything waits for one
     const bool bf16_gate = p.g_raw && !p.g_fp32;
-    const float* gp = p.g_raw ? static_cast<const float*>(p.g_raw) + goff : p.g + goff;
+    if (bf16_gate) {
+      const __nv_bfloat16* gp = static_cast<const __nv_bfloat16*>(p.g_raw) + goff;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) lam[i].a = t0 + i < len && kk < p.kc ? ldg_u64(gp + i * gs) : 0ull;      // four bf16 for now
+    } else {
+      const float* gp = p.g_raw ? static_cast<const float*>(p.g_raw) + goff : p.g + goff;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 g4 = t0 + i < len && kk < p.kc ? ldg_f4(gp + i * gs) : make_float4(0.f, 0.f, 0.f, 0.f);
+        lam[i] = {pair(g4.x, g4.y), pair(g4.z, g4.w)};
+      }
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const bool ok = t0 + i < len && kk < p.kc;
-      if (bf16_gate) {
-        lam[i] = widen(ok ? ldg_u2(static_cast<const __nv_bfloat16*>(p.g_raw) + goff + i * gs) : make_uint2(0u, 0u));
-      } else {
-        const float4 g4 = ok ? ldg_f4(gp + i * gs) : make_float4(0.f, 0.f, 0.f, 0.f);
-        lam[i] = {pair(g4.x, g4.y), pair(g4.z, g4.w)};
-      }
       q[i] = ok ? ldg_u2(qp + i * qs) : make_uint2(0u, 0u);
       k[i] = ok ? ldg_u2(kp + i * qs) : make_uint2(0u, 0u);
     }
-    // the tile that will run here next: its inputs into L2 (tiled prefetches by one thread)
+    if (tid < len) {      // (only threads below C keep a value)
+      const size_t i = static_cast<size_t>(ci.tok0 + tid) * p.H + h;
+      if (!p.beta_raw) beta_bits = __float_as_uint(__ldg(p.beta + i));
+      else if (p.beta_fp32) beta_bits = __ldg(static_cast<const uint32_t*>(p.beta_raw) + i);
+      else beta_bits = static_cast<uint32_t>(__ldg(static_cast<const unsigned short*>(p.beta_raw) + i)) << 16;
+    }
     if (tid == 0) {
       mbar_init(&s.barV, 1);
       fence_mbar_init();
+    }
+    // the inputs of the tile that will take this CTA's place into L2, one tiled prefetch by each of five warps (500 cycles a piece: by one
+    // thread, as it was, the whole CTA waited for them at the next barrier)
+    if (lane == 0 && warp >= 8 && warp < 13) {
       const long long nt = static_cast<long long>(blockIdx.x) + p.ahead;
       if (nt < static_cast<long long>(p.map.total()) * p.H) {
         const int tok = static_cast<int>(p.map.info(static_cast<int>(nt / p.H)).tok0), hn = static_cast<int>(nt % p.H);
-        tma_prefetch_rows(&p.tm_g, 0, hn, tok);
-        tma_prefetch_rows(&p.tm_q, 0, hn / p.grp, tok);
-        tma_prefetch_rows(&p.tm_k, 0, hn / p.grp, tok);
-        tma_prefetch_rows(&p.tm_v, 0, hn, tok);
-        tma_prefetch_rows(&p.tm_v, 64, hn, tok);
+        switch (warp) {
+          case 8: tma_prefetch_rows(&p.tm_g, 0, hn, tok); break;
+          case 9: tma_prefetch_rows(&p.tm_q, 0, hn / p.grp, tok); break;
+          case 10: tma_prefetch_rows(&p.tm_k, 0, hn / p.grp, tok); break;
+          case 11: tma_prefetch_rows(&p.tm_v, 0, hn, tok); break;
+          default: tma_prefetch_rows(&p.tm_v, 64, hn, tok); break;
+        }
       }
     }
     static_assert(TILE_TT == 16 * PREP_THREADS, "one piece per thread");
     reinterpret_cast<uint4*>(s.Aqk)[tid] = make_uint4(0u, 0u, 0u, 0u);
-    if (tid < C) {
-      float b = 0.f;
-      if (tid < len) {
-        const size_t i = static_cast<size_t>(ci.tok0 + tid) * p.H + h;
-        if (p.beta_raw) {
-          b = sigmoidf_(p.beta_fp32 ? __ldg(static_cast<const float*>(p.beta_raw) + i) : __bfloat162float(static_cast<const __nv_bfloat16*>(p.beta_raw)[i]));
-          if (p.beta_out) p.beta_out[i] = b;
-        } else {
-          b = __ldg(p.beta + i);
-        }
-      }
-      s.beta[tid] = b;
+    if (bf16_gate) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) lam[i] = widen(make_uint2(static_cast<uint32_t>(lam[i].a), static_cast<uint32_t>(lam[i].a >> 32)));
     }
     // the gate's activation here instead of in a kernel of its own: one launch less, and the fp32 g is never read back (forward only: never written)
     if (p.g_raw) {
@@ -301,7 +315,15 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
     for (int i = 0; i < 4; ++i)
       asm volatile("" : "+r"(q[i].x), "+r"(q[i].y), "+l"(lam[i].a), "+l"(lam[i].b));
   };
-  __syncthreads();      // T; Aqk is cleared
+  if (tid < C) {
+    float b = __uint_as_float(beta_bits);
+    if (p.beta_raw && tid < len) {
+      b = sigmoidf_(b);
+      if (p.beta_out) p.beta_out[static_cast<size_t>(ci.tok0 + tid) * p.H + h] = b;
+    }
+    s.beta[tid] = b;
+  }
+  __syncthreads();      // T; beta; Aqk is cleared
   KDA_DBG_CLOCK(p.dbg, 18);
 
   if constexpr (!SAFE) {
