@@ -4,8 +4,8 @@
 //                            so that variable-length calls need no device->host copy.
 //  kda_chunk_prepare_kernel  (kda_chunk_prepare.cu) one CTA per (chunk, head): everything that does not depend on the state:
 //                            G = cumsum(g), Aqk, Akk, Tm = (I+Akk)^-1, w, u, qg, kg  -> tiles in the workspace.
-//  kda_chunk_scan_tc_kernel  (kda_chunk_scan_tc.cu) one CTA per (sequence, head): walks the chunks in order with
-//                            the fp32 state in tensor memory, products on tcgen05.
+//  kda_chunk_scan_kernel     (kda_chunk_scan.cu; many units: kda_chunk_scan_tc.cu) walks the chunks of a (sequence, head) in order with
+//                            the fp32 state in registers or tensor memory.
 //                            v_new = u - w h;  o = qg h + Aqk v_new;  h = Diag(Gam_last) h + kg^T v_new.
 #include <mutex>
 
@@ -244,8 +244,7 @@ extern "C" int kda_chunk_fwd(const kda_chunk_args* args, void* stream) {
   sp.HS = save ? w.HS : nullptr; sp.VNEWT = save ? w.VNEWT : nullptr;
   sp.h0 = a.h0; sp.ht = a.ht; sp.o = static_cast<__nv_bfloat16*>(a.o); sp.status = w.status; sp.dbg = g_dbg_clocks;
   sp.H = a.H; sp.kc = kc; sp.vc = vc;
-  const int slices = scan_slices_for(a.N * a.H, a.scan_slices);
-  if ((rc = slices > 1 ? launch_scan_vs(sp, a.N * a.H, st) : launch_scan_tc(sp, a.N * a.H, st)) != KDA_OK) return rc;
+  if ((rc = launch_scan(sp, a.N * a.H, a.scan_slices, st)) != KDA_OK) return rc;
   prof_mark(prof, KDA_STAGE_SCAN, st);
   return KDA_OK;
 }

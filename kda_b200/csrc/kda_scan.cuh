@@ -19,12 +19,10 @@ struct ScanParams {
   int kc, vc;           // key and value columns of the tensors (<= 128; tiles and state are 128 wide, zero beyond)
 };
 
-// tcgen05 / TMEM version (kda_chunk_scan_tc.cu); returns KDA_OK, a negative KDA_E_* or a positive cudaError_t
+// kda_chunk_scan.cu; `requested` CTAs per (sequence, head) unit (1 or 4), 0: chosen from the number of units and of SMs.  Returns KDA_OK, a
+// negative KDA_E_* or a positive cudaError_t.
+int launch_scan(const ScanParams& p, int units, int requested, cudaStream_t st);
 int launch_scan_tc(const ScanParams& p, int blocks, cudaStream_t st);
-
-// The same scan with four CTAs per (sequence, head) unit, one per slice of 32 value columns (kda_chunk_scan_vs.cu): for
-// calls with so few units that one CTA's chunk-to-chunk chain sets the time.
-int launch_scan_vs(const ScanParams& p, int units, cudaStream_t st);
 
 // How many CTAs per unit the two state scans use: `requested` (1 or 4) if the caller chose, otherwise four while the
 // grid stays within one CTA per SM of the current device.  (Two slices of 64 columns were built and measured: slower
