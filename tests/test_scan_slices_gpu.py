@@ -68,3 +68,14 @@ def test_automatic_choice_and_argument_check():
         assert torch.equal(auto[n], one[n]), n
     a = _lib.ChunkArgs(tokens=64, N=1, H=2, K=128, V=128, io_dtype=0, scan_slices=2)
     assert _lib.load().kda_chunk_fwd(C.byref(a), None) == -2
+
+
+@pytest.mark.parametrize("lens", [[1], [64, 65], [130, 63, 257]])
+def test_two_ctas_per_unit_give_the_same_bits(lens):
+    """Between a quarter and half as many units as SMs the forward scan takes two CTAs of 64 value columns per unit."""
+    N, H = len(lens), -(-(torch.cuda.get_device_properties(0).multi_processor_count // 4 + 1) // len(lens))
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32) if N > 1 else None
+    d = make_inputs(1, sum(lens), H, 128, 128, torch.bfloat16, seed=970 + sum(lens), h0_std=0.02, n_states=N, backward=True)
+    one, two = _run(d, cu, 1), _run(d, cu, 0)
+    for n in NAMES:
+        assert torch.equal(two[n], one[n]), n
