@@ -201,8 +201,8 @@ typedef struct kda_chunk_args {
                                   ([tokens, HQ, K]) while v, g, beta, o, the states and their gradients have H; value head h reads
                                   q/k head h / (H / HQ), and dq, dk are summed over each group.  0 or H: no grouping. */
   int32_t scan_slices;         /* CTAs per (sequence, head) of the two state scans: 0 = chosen from N * H and the SM count (a call with
-                                  at most a quarter as many units as SMs cuts every unit into 4 slices of 32 value columns, which
-                                  shortens the chunk-to-chunk chain); 1 or 4 force a layout.  The results do not depend on it. */
+                                  at most a quarter as many units as SMs cuts every unit into 4 slices of 32 value columns, the forward
+                                  one with at most half as many into 2 of 64, which shortens the chunk-to-chunk chain); 1 or 4 force a layout.  The results do not depend on it. */
   int32_t safe_gate;           /* nonzero: the caller promises g >= -5 for every token and channel (fla's safe_gate,
                                   fla/ops/kda/chunk.py:235-246, chunk_intra.py:659-761).  The forward then computes the diagonal 16 x 16
                                   blocks of the intra-chunk products on tensor cores too, factored around each block's middle row,

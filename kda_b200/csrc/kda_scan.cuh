@@ -24,7 +24,7 @@ struct ScanParams {
 int launch_scan(const ScanParams& p, int units, int requested, cudaStream_t st);
 int launch_scan_tc(const ScanParams& p, int blocks, cudaStream_t st);
 
-// How many CTAs per unit the two state scans use: `requested` (1 or 4) if the caller chose, otherwise four while the
+// How many CTAs per unit the reverse scan uses: `requested` (1 or 4) if the caller chose, otherwise four while the
 // grid stays within one CTA per SM of the current device.  (Two slices of 64 columns were built and measured: slower
 // than one CTA per unit at every size, because the chain's cost is latency, not the width of its products.)
 inline int scan_slices_for(int units, int requested) {
