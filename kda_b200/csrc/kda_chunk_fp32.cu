@@ -3,7 +3,7 @@
 // Replaces the token-recurrent pair of kernels for calls with gradients and for long forward-only calls: those walk a (sequence,
 // head) token by token on CUDA cores (1.8 us a token forward, 11 us backward), this one 64 tokens at a time.  8 x 2048 tokens x 32
 // heads: preparation 1.24 ms, scan 0.7; forward and backward 26.0 -> 5.2.  What bounds it is the operands' way into shared
-// memory (split in two TF32 parts, swizzled stores), one CTA per SM with its phases in a row; the products take less than a third.
+// memory (split in two TF32 parts, swizzled stores), one CTA per SM with its phases in a row.
 #include "kda_device.cuh"
 #include "kda_fp32.cuh"
 

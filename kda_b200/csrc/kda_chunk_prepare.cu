@@ -16,7 +16,7 @@
 // Operands are written to shared memory once as bf16 and read by ldmatrix; level 8 / 4 products stack q and k rows into one m16
 // tile.  The same pass writes QG = scale q Gam, KG = k Gam_last / Gam and k Gam.
 //
-// What bounds it: instruction issue and shared-memory wavefronts, about 24 k cycles per CTA with two CTAs per SM; its bytes take 0.75 ms
+// What bounds it: instruction issue and shared-memory wavefronts, about 24 k cycles per CTA with two CTAs per SM; its bytes take 0.81 ms
 // at 8 x 8192 tokens x 32 heads, where it takes 1.50 ms.  (A thread per key column and row, decays as exp2 of cumulative sums and row
 // references, 256 threads: 1.98.)  Bounded gates at 1 x 32768 x 32: 0.77 ms with the gate's activation, 0.97 with a kernel before it.  Without the
 // L2 prefetch of the next wave's rows 1.65, two waves ahead 1.59.

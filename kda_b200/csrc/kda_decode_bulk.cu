@@ -5,7 +5,8 @@
 // waits for slot numbers, so that the loads of the next unit and the stores of the last tokens are in flight beside the arithmetic.
 // HV = 64, two persistent CTAs per SM, for several tokens per sequence: the two CTAs of an SM fill each other's waits and the last round of
 // units is shorter (24 sequences x 4 tokens x 32 heads: 47.7 us, whole states 59.9).  HV = 128, one CTA per SM, for one token: contiguous
-// 64 KiB copies, which DRAM likes better (1,024 sequences x 32 heads: 672 us = 0.98 of the measured copy rate, half states 692).
+// 64 KiB copies, which DRAM likes better (1,024 sequences x 32 heads: 670 us = 0.98 of the measured copy rate, half states 692).
+// Whatever a warp does between a unit's arrival and its store adds to every unit: o leaves behind the hand-over (in front of it: 674).
 // Per token (order as in fla/ops/kda/fused_recurrent.py:146-192): S *= exp(g); v' = beta (v - S^T k);
 // S += k v'^T; o = scale S^T q.
 #include <algorithm>
@@ -348,7 +349,6 @@ __global__ void __launch_bounds__(HV * 2 + 32, 128 / HV) kda_decode_bulk_kernel(
     if (nxt.u < p.total) stash(buf1, rx);
     rx = ry;
     meet();
-    if (!TR && step > 0 && warp == (step % NW)) write_o(prev, par ^ 1);
     if (keep && c > 0 && ((any >> dst) & 1u)) wait(s.gone, ~sp, dst);      // the copy engine has read the buffer's last store
     if constexpr (TR) {
       const float4 e4 = lds4f(&s.eg[buf][4 * lane]);
@@ -411,6 +411,7 @@ __global__ void __launch_bounds__(HV * 2 + 32, 128 / HV) kda_decode_bulk_kernel(
       any |= 1u << dst;
       ++c;
     }
+    if (!TR && step > 0 && warp == (step % NW)) write_o(prev, par ^ 1);      // behind the hand-over: in front of it this warp held up the unit's store
     prev = cur;
     if (cur.t == a.T - 1) {         // the buffers take the roles the copying warp gives them
       const int last = (c & 1) ? x : y, other = last == x ? y : x;

@@ -93,3 +93,29 @@ def test_fp32_backward_is_deterministic():
     a, b = _run(d), _run(d)
     for n in NAMES:
         assert torch.equal(a[n], b[n]), n
+
+
+# 256 tokens and more take the chunked kernels: edges of 16-token blocks and 64-token chunks, heads that end inside a tile, an empty sequence
+@pytest.mark.parametrize("lens,K,V,l2,transpose", [([256], 128, 128, False, False), ([257], 128, 128, True, False), ([303], 64, 128, False, True),
+                                                   ([320], 40, 24, True, False), ([64, 0, 1, 63, 145], 128, 128, True, True),
+                                                   ([300, 17], 96, 64, False, False)])
+def test_fp32_chunked_training(lens, K, V, l2, transpose):
+    N = len(lens)
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32) if N > 1 else None
+    d = make_inputs(1, sum(lens), 3, K, V, torch.float32, seed=500 + sum(lens), h0_std=0.1, n_states=N, backward=True)
+    if l2:
+        d["q"], d["k"] = d["q"] * 2.5, d["k"] * 0.4
+    ref = recurrent_kda_grads(d["q"], d["k"], d["v"], d["g"], d["beta"], d["do"], d["dht"], initial_state=d["h0"], cu_seqlens=cu,
+                              use_qk_l2norm=l2)
+    _check(_run(d, cu=cu, l2=l2, transpose=transpose), ref)
+
+
+def test_fp32_chunked_training_grouped_value_heads():
+    from oracle.kda_oracle import recurrent_kda
+    d = make_inputs(2, 150, 4, 128, 128, torch.float32, seed=47, h0_std=0.1, backward=True)
+    d["q"], d["k"] = d["q"][:, :, :2].contiguous(), d["k"][:, :, :2].contiguous()
+    lv = [d[n].double().requires_grad_(True) for n in ("q", "k", "v", "g", "beta", "h0")]
+    two = lambda t: t.repeat_interleave(2, dim=2)      # noqa: E731
+    o, ht = recurrent_kda(two(lv[0]), two(lv[1]), *lv[2:5], initial_state=lv[5], output_final_state=True)
+    gr = torch.autograd.grad([o, ht], lv, [d["do"].double(), d["dht"].double()])
+    _check(_run(d), dict(o=o.detach(), ht=ht.detach(), dq=gr[0], dk=gr[1], dv=gr[2], dg=gr[3], dbeta=gr[4], dh0=gr[5]))
