@@ -1,5 +1,5 @@
 // Reverse state scan of chunked KDA for FEW (sequence, head) units: several CTAs per unit, one per slice of the value
-// columns (sm_100a, tcgen05 + TMEM).  The counterpart of kda_chunk_scan_vs.cu for the backward.
+// columns (sm_100a, tcgen05 + TMEM).  The counterpart of kda_chunk_scan.cu for the backward.
 //
 // A unit is cut into 128 / VS slices of VS value columns (VS = 32: four slices); each CTA walks the unit's chunks from the last
 // to the first with its slice of the state gradient in tensor memory, TMEM lane = KEY row k: dh[k][v].  Per chunk:

@@ -96,7 +96,8 @@ __global__ void __launch_bounds__(ScanCfg<NP>::THREADS, 1) kda_chunk_scan_kernel
   if (warp == 2 * NP + 4) {
     // ================= copies =================
     if (lane == 0) {
-      for (int i = 0; i < nchunks; ++i) {
+      int i = 0;
+      for (; i < nchunks; ++i) {
         if (i >= ST && !mbar_wait(&s.empty[i % ST], (i / ST + 1) & 1)) {
           atomicOr(p.status, KDA_STATUS_SCAN_LOAD_WAIT);
           break;
@@ -112,6 +113,7 @@ __global__ void __launch_bounds__(ScanCfg<NP>::THREADS, 1) kda_chunk_scan_kernel
         bulk_g2s(d.QG, p.QG + tile * TILE_TK, TILE_TK, bar);
         bulk_g2s(d.AQK, p.AQK + tile * TILE_TT, TILE_TT, bar);
       }
+      for (int j = i > ST ? i - ST : 0; j < i; ++j) mbar_wait(&s.full[j % ST], (j / ST) & 1);      // no copy in flight outlives the CTA, also where others gave up
     }
     return;      // (nothing waits for this warp; the CTA's memory lives until the others leave)
   }
