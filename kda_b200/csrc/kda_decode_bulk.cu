@@ -200,7 +200,10 @@ __global__ void __launch_bounds__(HV * 2 + 32, 128 / HV) kda_decode_bulk_kernel(
   // A thread fetches its elements of a step's vectors (HV = 64: one of each; 128: of q and k, or of g and v) two steps ahead of its use and keeps the untouched bits in registers until
   // stash(): an instruction that depends on a load makes the thread wait for it right there, and a small load takes longer than
   // a unit's update when the memory system is saturated.
-  struct Raw { uint32_t q, k, g, v, b, al, bias; };
+  // Four registers a step, not seven: with gates the rest made the compiler touch loads still in flight (1,000 x 32, the layer's call: 682 -> 649 us)
+  // (HV = 128: the threads of q, k and those of g, v use the same registers; beta waits in thread 0's slot for A_log, which it has no use for)
+  constexpr int RQ = 0, RK = 1, RG = HV == 64 ? 2 : 0, RV = HV == 64 ? 3 : 1, RA = HV == 64 ? 4 : 2, RBIAS = HV == 64 ? 5 : 3, RB = HV == 64 ? 6 : 2;
+  struct Raw { uint32_t x[HV == 64 ? 7 : 4]; };
   constexpr bool IO16 = sizeof(IO) == 2;
   auto ld_bits = [&](const void* ptr, size_t i, bool bf16) -> uint32_t {
     if (bf16) return static_cast<const unsigned short*>(ptr)[i];
@@ -213,29 +216,29 @@ __global__ void __launch_bounds__(HV * 2 + 32, 128 / HV) kda_decode_bulk_kernel(
     const size_t tok = static_cast<size_t>(q.n) * a.T + q.t, row = tok * a.H + q.h;
     const size_t rowq = (tok * HQ + q.h / grp) * DK + e;
     if (has_qk) {
-      r.q = ld_bits(a.q, rowq, IO16);
-      r.k = ld_bits(a.k, rowq, IO16);
+      r.x[RQ] = ld_bits(a.q, rowq, IO16);
+      r.x[RK] = ld_bits(a.k, rowq, IO16);
     }
     if (has_gv) {
       if constexpr (GATE) {
-        r.g = ld_bits(a.g, row * DK + e, a.A_log && a.g_raw_dtype == KDA_BF16);
+        r.x[RG] = ld_bits(a.g, row * DK + e, a.A_log && a.g_raw_dtype == KDA_BF16);
         if (a.A_log) {
-          r.al = __float_as_uint(__ldg(a.A_log + q.h));
-          r.bias = a.dt_bias ? __float_as_uint(__ldg(a.dt_bias + static_cast<size_t>(q.h) * DK + e)) : 0u;
+          r.x[RA] = __float_as_uint(__ldg(a.A_log + q.h));
+          r.x[RBIAS] = a.dt_bias ? __float_as_uint(__ldg(a.dt_bias + static_cast<size_t>(q.h) * DK + e)) : 0u;
         }
       } else {
-        r.g = __float_as_uint(__ldg(a.g + row * DK + e));
+        r.x[RG] = __float_as_uint(__ldg(a.g + row * DK + e));
       }
-      if (e < HV) r.v = ld_bits(a.v, row * DV + half * HV + e, IO16);
+      if (e < HV) r.x[RV] = ld_bits(a.v, row * DV + half * HV + e, IO16);
     }
     if (tid == 0) {
-      if constexpr (GATE) r.b = ld_bits(a.beta, row, a.beta_sigmoid && a.beta_raw_dtype == KDA_BF16);
-      else r.b = __float_as_uint(__ldg(a.beta + row));
+      if constexpr (GATE) r.x[RB] = ld_bits(a.beta, row, a.beta_sigmoid && a.beta_raw_dtype == KDA_BF16);
+      else r.x[RB] = __float_as_uint(__ldg(a.beta + row));
     }
   };
   auto stash = [&](int buf, const Raw& r) {
     if (has_qk) {
-      const float q = to_float(r.q, IO16), k = to_float(r.k, IO16);
+      const float q = to_float(r.x[RQ], IO16), k = to_float(r.x[RK], IO16);
       s.qv[buf][e] = q;
       s.kv[buf][e] = k;
       if (a.use_qk_l2norm) {
@@ -247,21 +250,21 @@ __global__ void __launch_bounds__(HV * 2 + 32, 128 / HV) kda_decode_bulk_kernel(
       }
     }
     if (has_gv) {
-      float g = __uint_as_float(r.g);
+      float g = __uint_as_float(r.x[RG]);
       if constexpr (GATE) {
         if (a.A_log) {
-          const float x = to_float(r.g, a.g_raw_dtype == KDA_BF16) + __uint_as_float(r.bias);
-          const float al = __expf(__uint_as_float(r.al));
+          const float x = to_float(r.x[RG], a.g_raw_dtype == KDA_BF16) + __uint_as_float(r.x[RBIAS]);
+          const float al = __expf(__uint_as_float(r.x[RA]));
           g = a.use_lower_bound ? a.lower_bound * sigmoid_fast(al * x) : -al * softplus_fast(x);
         }
       }
       s.eg[buf][e] = __expf(g);
-      if (e < HV) s.vv[buf][e] = to_float(r.v, IO16);
+      if (e < HV) s.vv[buf][e] = to_float(r.x[RV], IO16);
     }
     if (tid == 0) {
-      float b = __uint_as_float(r.b);
+      float b = __uint_as_float(r.x[RB]);
       if constexpr (GATE) {
-        if (a.beta_sigmoid) b = sigmoid_fast(to_float(r.b, a.beta_raw_dtype == KDA_BF16));
+        if (a.beta_sigmoid) b = sigmoid_fast(to_float(r.x[RB], a.beta_raw_dtype == KDA_BF16));
       }
       s.beta[buf] = b;
     }
@@ -271,7 +274,7 @@ __global__ void __launch_bounds__(HV * 2 + 32, 128 / HV) kda_decode_bulk_kernel(
   // !TR: this thread's four value columns and sixteen key rows
   const int col = HV == 64 ? 4 * (lane & 15) : 4 * lane, row0 = HV == 64 ? 32 * warp + 16 * (lane >> 4) : 16 * warp;
   const bool lead = HV == 128 || lane < 16;      // HV = 64: the two halves of a warp share columns
-  auto write_o = [&](const Pos& q, int par) {                               // !TR: o of a finished step (one warp)
+  auto write_o = [&](size_t row, int par) {                               // !TR: o of a finished step (one warp)
     if (lead) {
       float4 o = lds4f(&s.red2[par][0][col]);
 #pragma unroll
@@ -279,11 +282,12 @@ __global__ void __launch_bounds__(HV * 2 + 32, 128 / HV) kda_decode_bulk_kernel(
         const float4 x = lds4f(&s.red2[par][w][col]);
         o.x += x.x; o.y += x.y; o.z += x.z; o.w += x.w;
       }
-      st4o(op + ((static_cast<size_t>(q.n) * a.T + q.t) * a.H + q.h) * DV + half * HV + col, o);
+      st4o(op + row * DV + half * HV + col, o);
     }
   };
 
-  Pos cur = first, nxt = first, ahead = first, prev = first;
+  Pos cur = first, nxt = first, ahead = first;
+  size_t prev = 0;
   Raw rx = {}, ry;
   {
     Raw r0 = {};
@@ -412,7 +416,7 @@ __global__ void __launch_bounds__(HV * 2 + 32, 128 / HV) kda_decode_bulk_kernel(
       ++c;
     }
     if (!TR && step > 0 && warp == (step % NW)) write_o(prev, par ^ 1);      // behind the hand-over: in front of it this warp held up the unit's store
-    prev = cur;
+    if (!TR) prev = (static_cast<size_t>(cur.n) * a.T + cur.t) * a.H + cur.h;
     if (cur.t == a.T - 1) {         // the buffers take the roles the copying warp gives them
       const int last = (c & 1) ? x : y, other = last == x ? y : x;
       x = z;
