@@ -218,6 +218,8 @@ def make_step(workload: str, x: dict, cu, gate: bool = False, l2: bool = False, 
                               output_final_state=True, cu_seqlens=cu, use_qk_l2norm_in_kernel=l2, safe_gate=safe, **kw)
             grads = torch.autograd.grad([o, ht], leaves, [x["do"], x["dht"]])
             return (o, ht) + tuple(grads)
+        if x["q"].dtype == torch.float32:
+            return step, 3, grad_names                    # token-recurrent forward, backward, its finishing kernel
         # prepare, scan, reverse scan, main; packed sequences: + the tables; gate: + its backward and the reduction
         return step, 4 + (cu is not None) + (2 if gate else 0), grad_names
 
@@ -605,11 +607,11 @@ def main():
         staged = [s for s in kernels if s in KERNEL_WORK]
         dom = max(staged, key=lambda s: kernels[s]["ms_per_launch"] * kernels[s]["launches"]) if staged else None
         if dom is None:
-            # float32 tensors: kernels the library does not time one by one; the whole
+            # float32 tensors: the token-recurrent kernels, which the library does not time one by one; the whole
             # step against the operator-boundary bytes (all tensors float32)
             io = 4 * (3 * 128 + 2 * 128 + 1) + (4 * (4 * 128 + 2 * 128 + 1) if w.backward else 0)
             ach = io * th / (ms_step * 1e-3) / 1e9
-            roof = {"kernel": "kda_f32 prepare, scan, bwd_scan, bwd_main" if w.backward else "kda_recurrent_kernel", "bound": "hbm",
+            roof = {"kernel": "kda_recurrent_kernel" + (" + kda_recurrent_bwd_kernel" if w.backward else ""), "bound": "hbm",
                     "achieved": ach, "peak": peaks["hbm"], "unit": "GB/s", "frac": ach / peaks["hbm"], "traffic": None,
                     "peak_source": peaks["src"], "algorithmic_bytes_per_launch": io * th,
                     "note": "exact fp32 path: one warp (forward) or CTA (backward) per (sequence, head), token-serial; not HBM-bound"}

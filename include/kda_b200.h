@@ -31,7 +31,7 @@ extern "C" {
 #pragma GCC visibility push(default) /* the entry points below are the library's only exports */
 #endif
 
-#define KDA_B200_ABI_VERSION 10
+#define KDA_B200_ABI_VERSION 11
 #define KDA_CHUNK 64 /* tokens per chunk of the chunked kernels */
 
 /* io_dtype of q, k, v, o and of their gradients */
@@ -149,9 +149,7 @@ size_t kda_recurrent_bwd_workspace_bytes(int64_t tokens, int32_t N, int32_t H, i
 int kda_recurrent_bwd(const kda_recurrent_bwd_args* args, void* stream);
 
 /* ------------------------------------------------------------------------------------------------
- * Chunked forward / backward (chunk = 64 tokens) on tensor cores, K = V = 128 (narrower rows: k_cols, v_cols).  io_dtype
- * KDA_BF16: bf16 operands.  KDA_FP32: q, k, v, o, d_o, dq, dk, dv are float32 and so is every product's accuracy (each fp32 operand
- * is split into two TF32 parts); safe_gate and scan_slices have no effect there.
+ * Chunked forward / backward (chunk = 64 tokens), bf16 tensor-core path, K = V = 128 (narrower rows: k_cols, v_cols).
  * Stand behind chunk_kda and its autograd function (fla/ops/kda/chunk.py:167-411, :22-162).
  *
  * The caller passes one scratch buffer ("workspace") of at least kda_chunk_workspace_bytes(...).
@@ -190,12 +188,11 @@ typedef struct kda_chunk_args {
   /* sizes */
   int64_t tokens;
   int32_t N, H, K, V;
-  int32_t io_dtype;            /* KDA_BF16 or KDA_FP32 */
+  int32_t io_dtype;            /* KDA_BF16 */
   int32_t use_qk_l2norm;
   int32_t save_for_backward;   /* bit 0: keep what kda_chunk_bwd reads in the workspace; bit 1 (with use_qk_l2norm): also keep
                                   the normalised q, k there, so that the backward does not recompute them.  Pass the same
-                                  value to kda_chunk_workspace_bytes, kda_chunk_fwd and kda_chunk_bwd.  KDA_FP32: bit 1 is
-                                  required with use_qk_l2norm, and kda_chunk_workspace_bytes takes bit 2 (value 4) as well. */
+                                  value to kda_chunk_workspace_bytes, kda_chunk_fwd and kda_chunk_bwd. */
   float scale;
   int32_t HQ;                  /* grouped value heads (GVA, fla/ops/kda/chunk.py:194-196,379-386): q, k, dq, dk have HQ heads
                                   ([tokens, HQ, K]) while v, g, beta, o, the states and their gradients have H; value head h reads
@@ -212,7 +209,7 @@ typedef struct kda_chunk_args {
                                   gradients when they are narrower than the kernels' K = V = 128: multiples of 8, 0 = 128.  The
                                   missing columns count as zero (k = q = v = 0, g = 0), which leaves every result unchanged.  Backward
                                   with narrow rows: no grouped heads; with use_qk_l2norm only with save_for_backward bit 1. */
-  /* Gate front end inside the forward (KDA_BF16), all zero / NULL: g and beta are the activated fp32 values.  With g_raw (beta_raw)
+  /* Gate front end inside the forward, all zero / NULL: g and beta are the activated fp32 values.  With g_raw (beta_raw)
    * the forward activates them itself, with the formulas of kda_gate_fwd, and `g` (`beta`) is an OUTPUT: it receives the activated
    * values, which kda_chunk_bwd reads; NULL in a forward-only call.  kda_gate_bwd turns dg, dbeta into the raw tensors' gradients. */
   const void* g_raw;           /* [tokens, H, K] of g_raw_dtype, or NULL */
@@ -231,7 +228,7 @@ size_t kda_chunk_workspace_bytes(int64_t tokens, int32_t N, int32_t H, int32_t K
 /* Bytes of the backward's own scratch (args->bwd_workspace); it need not outlive the backward call.
  * use_qk_l2norm is a flag word here: bit 0 = q/k are L2-normalised in the kernels, bit 1 = grouped value heads
  * (HQ < H), which needs room for the per-value-head dq, dk before they are summed, bit 2 = the forward kept the
- * normalised q, k (save_for_backward bit 1), so the backward needs no room for them; bit 3 = io_dtype KDA_FP32. */
+ * normalised q, k (save_for_backward bit 1), so the backward needs no room for them. */
 size_t kda_chunk_bwd_workspace_bytes(int64_t tokens, int32_t N, int32_t H, int32_t K, int32_t V, int32_t use_qk_l2norm);
 
 int kda_chunk_fwd(const kda_chunk_args* args, void* stream);

@@ -271,43 +271,35 @@ std::pair<Tensor, Tensor> chunk_forward(ChunkSaved& s, const Tensor& q, const Te
   const cudaStream_t st = stream_of(dev);
   const int64_t B = q.size(0), T = q.size(1), H = v.size(2), K = q.size(3), V = v.size(3), tokens = B * T;
   s.q = dense(q); s.k = dense(k); s.v = dense(v); s.h0 = dense(h0);
-  // bf16: the forward kernel activates g and beta itself, and the activated values exist only for a backward
-  const bool fused = q.scalar_type() == at::kBFloat16, keep = need_grad || !fused;
+  // the forward kernel activates g and beta itself; the activated values are written only for a backward
   if (o.gate) {
     s.g_raw = dense(g);
     s.A32 = f32(A_log);
     s.b32 = f32(dt_bias);
-    if (keep) s.g = empty(g.sizes(), at::kFloat, dev);
+    if (need_grad) s.g = empty(g.sizes(), at::kFloat, dev);
   } else {
     s.g = f32(g);
   }
   if (o.beta_sigmoid) {
     s.beta_raw = dense(beta);
-    if (keep) s.beta = empty(beta.sizes(), at::kFloat, dev);
+    if (need_grad) s.beta = empty(beta.sizes(), at::kFloat, dev);
   } else {
     s.beta = f32(beta);
-  }
-  if ((o.gate || o.beta_sigmoid) && !fused) {
-    kda_gate_args a = gate_args(s, o, tokens, H, K);
-    a.g = o.gate ? ptr<float>(s.g) : nullptr;
-    a.beta = o.beta_sigmoid ? ptr<float>(s.beta) : nullptr;
-    check_rc(kda_gate_fwd(&a, st), "kda_gate_fwd");
   }
   s.cu = cu;
   const int64_t N = sequences(s);
   const int save = need_grad ? save_bits(o) : 0;
-  const int fp32 = dtype_code(q) == KDA_FP32 ? 4 : 0;
-  s.ws = bytes(kda_chunk_workspace_bytes(tokens, static_cast<int32_t>(N), static_cast<int32_t>(H), static_cast<int32_t>(K), static_cast<int32_t>(V), save | fp32), dev);
+  s.ws = bytes(kda_chunk_workspace_bytes(tokens, static_cast<int32_t>(N), static_cast<int32_t>(H), static_cast<int32_t>(K), static_cast<int32_t>(V), save), dev);
   const Tensor out = empty(v.sizes(), v.scalar_type(), dev);
   const Tensor ht = o.output_final ? empty({N, H, K, V}, at::kFloat, dev) : Tensor();
   kda_chunk_args a = chunk_args(s, o, save);
   a.o = ptr(out);
   a.ht = ptr<float>(ht);
-  if (fused && o.gate) {
+  if (o.gate) {
     a.g_raw = ptr(s.g_raw); a.g_raw_dtype = dtype_code(s.g_raw); a.A_log = ptr<float>(s.A32); a.dt_bias = ptr<float>(s.b32);
     a.use_lower_bound = o.has_lower_bound; a.lower_bound = static_cast<float>(o.lower_bound);
   }
-  if (fused && o.beta_sigmoid) {
+  if (o.beta_sigmoid) {
     a.beta_raw = ptr(s.beta_raw); a.beta_raw_dtype = dtype_code(s.beta_raw);
   }
   check_rc(kda_chunk_fwd(&a, st), "kda_chunk_fwd");
@@ -354,7 +346,7 @@ class ChunkFunction : public torch::autograd::Function<ChunkFunction> {
     const Tensor dq = empty(s.q.sizes(), s.q.scalar_type(), dev), dk = empty(s.k.sizes(), s.k.scalar_type(), dev), dv = empty(s.v.sizes(), s.v.scalar_type(), dev);
     Tensor dg = empty(s.g.sizes(), at::kFloat, dev), dbeta = empty(s.beta.sizes(), at::kFloat, dev);
     const Tensor dh0 = s.h0.defined() ? empty(s.h0.sizes(), at::kFloat, dev) : Tensor();
-    const int flags = (o.l2norm ? 1 | 4 : 0) | (s.q.size(2) != H ? 2 : 0) | (dtype_code(s.q) == KDA_FP32 ? 8 : 0);
+    const int flags = (o.l2norm ? 1 | 4 : 0) | (s.q.size(2) != H ? 2 : 0);
     const Tensor bws = bytes(
         kda_chunk_bwd_workspace_bytes(tokens, static_cast<int32_t>(N), static_cast<int32_t>(H), static_cast<int32_t>(K), static_cast<int32_t>(V), flags), dev);
     kda_chunk_args a = chunk_args(s, o, save_bits(o));
@@ -406,23 +398,13 @@ bool wants_grad(std::initializer_list<const Tensor*> ts) {
   return false;
 }
 
-// float32 gradients of a handful of tokens (fewer than four chunks in all: gradient checks) stay with the token-recurrent kernels, which
-// take the recurrence's own steps; anything longer takes the chunked ones (8 x 2048 tokens x 32 heads: 26 ms there).
-bool recurrent_backward(const Sizes& s) {
-  auto built = [](int64_t d) { return d == 32 || d == 64 || d == 128; };
-  return s.B * s.T < 256 && built(s.K) && built(s.V);
-}
-
-// Heads up to 128, bf16, and float32 with gradients.  Returns false for a call that takes another path: float32 without gradients
-// (token-recurrent kernel), larger heads, and the narrow ones that the kernels do not read in place (no multiple of eight columns; bf16
-// gradients with grouped value heads).
+// bf16, heads up to 128.  Returns false for a call that takes another path: float32 (token-recurrent kernels), larger heads, and the narrow
+// ones that the kernels do not read in place (no multiple of eight columns; gradients with grouped value heads).
 bool chunk_kda(ChunkCall& c, Tensor& o, Tensor& ht) {
   const Sizes s = check_common(c.q, c.k, c.v, c.g, c.beta, c.h0, c.cu);
   const bool grads = wants_grad({&c.q, &c.k, &c.v, &c.g, &c.beta, &c.h0, &c.A_log, &c.dt_bias});
-  const bool fp32 = c.q.scalar_type() == at::kFloat;
-  if (s.K > 128 || s.V > 128 || s.K % 8 || s.V % 8) return false;
-  if (!fp32 && (s.K < 128 || s.V < 128) && grads && s.HQ != s.H) return false;
-  if (fp32 && (!grads || recurrent_backward(s))) return false;
+  if (c.q.scalar_type() != at::kBFloat16 || s.K > 128 || s.V > 128 || s.K % 8 || s.V % 8) return false;
+  if ((s.K < 128 || s.V < 128) && grads && s.HQ != s.H) return false;
   ChunkOpts opt;
   opt.scale = c.scale ? *c.scale : 1.0 / std::sqrt(static_cast<double>(s.K));
   opt.output_final = c.output_final; opt.l2norm = c.l2norm; opt.gate = c.gate; opt.beta_sigmoid = c.beta_sigmoid; opt.safe_gate = c.safe_gate;

@@ -20,7 +20,6 @@
 //   dg = reverse cumsum of dG inside the chunk.
 #include "kda_chunk.cuh"
 #include "kda_chunk_bwd.cuh"
-#include "kda_fp32.cuh"
 #include "kda_scan.cuh"
 
 namespace kda {
@@ -108,30 +107,8 @@ __global__ void __launch_bounds__(256) kda_group_sum_kernel(const __nv_bfloat16*
 }
 }  // namespace kda
 
-namespace kda {
-F32Params f32_params(const kda_chunk_args& a, const F32Ws& w, int kc, int vc);      // kda_chunk_fwd.cu
-
-static int chunk_bwd_f32(const kda_chunk_args& a, cudaStream_t st) {
-  const F32Ws w = carve_f32(static_cast<unsigned char*>(a.workspace), static_cast<unsigned char*>(a.bwd_workspace), a.tokens, a.N, a.H, true,
-                            (a.save_for_backward & 2) != 0);
-  if (a.workspace_bytes < w.fwd_bytes || a.bwd_workspace_bytes < w.bwd_bytes) return KDA_E_WORKSPACE;
-  if (a.use_qk_l2norm && !(a.save_for_backward & 2)) return KDA_E_SHAPE;
-  F32Params p = f32_params(a, w, a.k_cols > 0 ? a.k_cols : KD, a.v_cols > 0 ? a.v_cols : VD);
-  p.d_o = static_cast<const float*>(a.d_o); p.d_ht = a.d_ht;
-  p.dq = static_cast<float*>(a.dq); p.dk = static_cast<float*>(a.dk); p.dv = static_cast<float*>(a.dv);
-  p.dg = a.dg; p.dbeta = a.dbeta; p.dh0 = a.dh0;
-  const long long chunks = p.map.T > 0 ? static_cast<long long>(a.N) * p.map.per_seq : a.tokens / C + a.N;
-  ProfCall* prof = prof_begin(st);
-  int rc = launch_f32_bwd(p, chunks * a.H, st);
-  if (rc == KDA_OK && (p.grp > 1 || p.use_l2)) rc = launch_f32_finish(p, static_cast<long long>(a.tokens) * p.HQ, st);
-  prof_mark(prof, KDA_STAGE_BWD_MAIN, st);
-  return rc;
-}
-}  // namespace kda
-
 extern "C" size_t kda_chunk_bwd_workspace_bytes(int64_t tokens, int32_t N, int32_t H, int32_t K, int32_t V, int32_t use_qk_l2norm) {
   (void)K; (void)V;
-  if (use_qk_l2norm & 8) return kda::carve_f32(nullptr, nullptr, tokens, N, H, true, false).bwd_bytes;
   return kda::carve_ws(nullptr, nullptr, tokens, N, H, true, (use_qk_l2norm & 1) != 0, (use_qk_l2norm & 2) != 0, (use_qk_l2norm & 4) != 0).bwd_bytes;
 }
 
@@ -151,7 +128,6 @@ extern "C" int kda_chunk_bwd(const kda_chunk_args* args, void* stream) {
     }
     return KDA_OK;
   }
-  if (a.io_dtype == KDA_FP32) return chunk_bwd_f32(a, st);
   const bool l2 = a.use_qk_l2norm != 0;
   const int HQ = a.HQ > 0 ? a.HQ : a.H, grp = a.H / HQ;
   const int kc = a.k_cols > 0 ? a.k_cols : KD, vc = a.v_cols > 0 ? a.v_cols : VD;

@@ -11,7 +11,6 @@
 
 #include "kda_chunk.cuh"
 #include "kda_device.cuh"
-#include "kda_fp32.cuh"
 #include "kda_prepare.cuh"
 #include "kda_scan.cuh"
 
@@ -118,13 +117,12 @@ int validate_chunk_args(const kda_chunk_args& a, bool backward) {
   if (a.K != KD || a.V != VD) return KDA_E_SHAPE;
   if (a.k_cols < 0 || a.k_cols > KD || a.k_cols % 8 || a.v_cols < 0 || a.v_cols > VD || a.v_cols % 8) return KDA_E_SHAPE;
   if (a.scan_slices != 0 && a.scan_slices != 1 && a.scan_slices != 4) return KDA_E_SHAPE;
-  if (a.io_dtype != KDA_BF16 && a.io_dtype != KDA_FP32) return KDA_E_DTYPE;
+  if (a.io_dtype != KDA_BF16) return KDA_E_DTYPE;      // float32: the token-recurrent entry points
   if (a.tokens / C + a.N > 0x3fffffffLL) return KDA_E_SHAPE;
   if (a.tokens == 0 || a.N == 0) return KDA_OK;
   const bool raw_g = !backward && a.g_raw, raw_b = !backward && a.beta_raw;
   if (!a.q || !a.k || !a.v || (!a.g && !raw_g) || (!a.beta && !raw_b) || !a.workspace) return KDA_E_NULL;
   if (raw_g && !a.A_log) return KDA_E_NULL;
-  if ((raw_g || raw_b) && a.io_dtype != KDA_BF16) return KDA_E_DTYPE;
   if ((raw_g && a.g_raw_dtype != KDA_BF16 && a.g_raw_dtype != KDA_FP32) || (raw_b && a.beta_raw_dtype != KDA_BF16 && a.beta_raw_dtype != KDA_FP32))
     return KDA_E_DTYPE;
   if (!a.cu_seqlens && a.tokens % a.N != 0) return KDA_E_SHAPE;
@@ -147,42 +145,12 @@ static void launch_tables(const kda_chunk_args& a, int max_chunks, int* off, int
   kda_chunk_tables_kernel<<<1, 1024, 0, st>>>(a.cu_seqlens, a.N, a.tokens, max_chunks, off, seq, order, status);
 }
 
-// what both directions of the float32 path share
-F32Params f32_params(const kda_chunk_args& a, const F32Ws& w, int kc, int vc);
-F32Params f32_params(const kda_chunk_args& a, const F32Ws& w, int kc, int vc) {
-  F32Params p{};
-  p.q = static_cast<const float*>(a.q); p.k = static_cast<const float*>(a.k); p.v = static_cast<const float*>(a.v);
-  p.g = a.g; p.beta = a.beta; p.h0 = a.h0; p.w = w;
-  p.map = chunk_map(w, a.cu_seqlens, a.tokens, a.N);
-  p.H = a.H; p.HQ = a.HQ > 0 ? a.HQ : a.H; p.grp = a.H / p.HQ; p.kc = kc; p.vc = vc; p.use_l2 = a.use_qk_l2norm != 0; p.scale = a.scale;
-  p.save = (a.save_for_backward & 1) != 0;
-  return p;
-}
-
-static int chunk_fwd_f32(const kda_chunk_args& a, int kc, int vc, cudaStream_t st) {
-  const bool save = (a.save_for_backward & 1) != 0, keep = (a.save_for_backward & 2) != 0;
-  if (save && a.use_qk_l2norm && !keep) return KDA_E_SHAPE;
-  const F32Ws w = carve_f32(static_cast<unsigned char*>(a.workspace), nullptr, a.tokens, a.N, a.H, save, keep);
-  if (a.workspace_bytes < w.fwd_bytes) return KDA_E_WORKSPACE;
-  const int NTmax = static_cast<int>(a.tokens / C + a.N);
-  ProfCall* prof = prof_begin(st);
-  if (a.cu_seqlens) launch_tables(a, NTmax, w.seq_chunk_off, w.chunk_seq, w.seq_order, w.status, st);
-  F32Params p = f32_params(a, w, kc, vc);
-  p.clear_status = !a.cu_seqlens;
-  p.o = static_cast<float*>(a.o); p.ht = a.ht;
-  const long long chunks = p.map.T > 0 ? static_cast<long long>(a.N) * p.map.per_seq : NTmax;
-  const int rc = launch_f32_fwd(p, chunks * a.H, st);
-  prof_mark(prof, KDA_STAGE_SCAN, st);
-  return rc;
-}
-
 }  // namespace kda
 
 extern "C" int64_t kda_chunk_max_chunks(int64_t tokens, int32_t N) { return tokens / kda::C + N; }
 
 extern "C" size_t kda_chunk_workspace_bytes(int64_t tokens, int32_t N, int32_t H, int32_t K, int32_t V, int32_t save) {
   (void)K; (void)V;
-  if (save & 4) return kda::carve_f32(nullptr, nullptr, tokens, N, H, (save & 1) != 0, (save & 2) != 0).fwd_bytes;
   return kda::carve_ws(nullptr, nullptr, tokens, N, H, (save & 1) != 0, true, false, (save & 2) != 0).fwd_bytes;
 }
 
@@ -203,7 +171,6 @@ extern "C" int kda_chunk_fwd(const kda_chunk_args* args, void* stream) {
     }
     return KDA_OK;
   }
-  if (a.io_dtype == KDA_FP32) return chunk_fwd_f32(a, kc, vc, st);
   const bool save = (a.save_for_backward & 1) != 0;
   const bool keep_qn = save && (a.save_for_backward & 2) != 0 && a.use_qk_l2norm != 0;
   ChunkWs w = carve_ws(static_cast<unsigned char*>(a.workspace), nullptr, a.tokens, a.N, a.H, save, true, false,
@@ -271,7 +238,6 @@ unsigned char* g_noalloc_addr[kMaxDevices] = {};   // device address of g_noallo
 extern "C" int kda_chunk_fwd_noalloc(const kda_chunk_args* args, void* stream) {
   if (!args) return KDA_E_NULL;
   if (args->save_for_backward != 0) return KDA_E_SHAPE;
-  if (args->io_dtype != KDA_BF16) return KDA_E_DTYPE;
   if (args->tokens < 0 || args->N < 0 || args->H <= 0) return KDA_E_SHAPE;
   const size_t need = kda::carve_ws(nullptr, nullptr, args->tokens, args->N, args->H, false).fwd_bytes;
   if (need > static_cast<size_t>(KDA_NOALLOC_SCRATCH_BYTES)) return KDA_E_LIMIT;

@@ -475,9 +475,9 @@ def chunk_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_sta
     [B, NT, H, K, V] bf16 holds the state at the start of every chunk.  `transpose_state_layout`: every state
     tensor is [.., V, K] instead of [.., K, V].
 
-    bf16 inputs with K, V <= 128 take the chunked tensor-core kernels (built for K = V = 128; smaller heads are
-    zero-padded to 128 channels, which leaves every result unchanged; K = 256 runs forward-only through the
-    token-recurrent kernel).  float32 inputs take the exact
+    bf16 inputs with K, V <= 128 take the chunked tensor-core kernels (built for K = V = 128; heads of fewer columns are read and
+    written in place where K and V are multiples of 8, zero-padded otherwise: either leaves every result unchanged; K = 256 runs
+    forward-only through the token-recurrent kernel).  float32 inputs take the exact
     token-recurrent fp32 kernels: forward for K in {32, 64, 128, 256}, with gradients for K, V in {32, 64, 128}.  `safe_gate=True` is the caller's promise that every gate value is at least
     -5 (fla/ops/kda/chunk.py:235-246); the forward then computes the diagonal 16 x 16 blocks of the intra-chunk products on
     tensor cores as well (factored around each block's middle row) instead of pairwise, which is faster and only safe under

@@ -95,11 +95,10 @@ def test_fp32_backward_is_deterministic():
         assert torch.equal(a[n], b[n]), n
 
 
-# 256 tokens and more take the chunked kernels: edges of 16-token blocks and 64-token chunks, heads that end inside a tile, an empty sequence
+# longer calls: several hundred tokens, an empty sequence between others
 @pytest.mark.parametrize("lens,K,V,l2,transpose", [([256], 128, 128, False, False), ([257], 128, 128, True, False), ([303], 64, 128, False, True),
-                                                   ([320], 40, 24, True, False), ([64, 0, 1, 63, 145], 128, 128, True, True),
-                                                   ([300, 17], 96, 64, False, False)])
-def test_fp32_chunked_training(lens, K, V, l2, transpose):
+                                                   ([64, 0, 1, 63, 145], 128, 128, True, True)])
+def test_fp32_training_of_longer_calls(lens, K, V, l2, transpose):
     N = len(lens)
     cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32) if N > 1 else None
     d = make_inputs(1, sum(lens), 3, K, V, torch.float32, seed=500 + sum(lens), h0_std=0.1, n_states=N, backward=True)
@@ -110,7 +109,7 @@ def test_fp32_chunked_training(lens, K, V, l2, transpose):
     _check(_run(d, cu=cu, l2=l2, transpose=transpose), ref)
 
 
-def test_fp32_chunked_training_grouped_value_heads():
+def test_fp32_training_grouped_value_heads_longer():
     from oracle.kda_oracle import recurrent_kda
     d = make_inputs(2, 150, 4, 128, 128, torch.float32, seed=47, h0_std=0.1, backward=True)
     d["q"], d["k"] = d["q"][:, :, :2].contiguous(), d["k"][:, :, :2].contiguous()
@@ -119,3 +118,37 @@ def test_fp32_chunked_training_grouped_value_heads():
     o, ht = recurrent_kda(two(lv[0]), two(lv[1]), *lv[2:5], initial_state=lv[5], output_final_state=True)
     gr = torch.autograd.grad([o, ht], lv, [d["do"].double(), d["dht"].double()])
     _check(_run(d), dict(o=o.detach(), ht=ht.detach(), dq=gr[0], dk=gr[1], dv=gr[2], dg=gr[3], dbeta=gr[4], dh0=gr[5]))
+
+
+@pytest.mark.parametrize("K,V", [(40, 24), (96, 64), (128, 256)])
+def test_fp32_gradients_of_other_head_sizes_are_refused(K, V):
+    from kda_b200 import chunk_kda
+    d = make_inputs(1, 300, 2, K, V, torch.float32, seed=48)
+    lv = [d[n].cuda().requires_grad_(True) for n in ("q", "k", "v", "g", "beta")]
+    with pytest.raises(NotImplementedError, match="float32 gradients need K, V"):
+        chunk_kda(*lv)
+
+
+@pytest.mark.parametrize("B,T,H,D", [(2, 512, 4, 64), (1, 512, 4, 128)])
+def test_fp32_layer_gradients_are_float32_accurate(B, T, H, D):
+    """The layer's call (raw gate, beta logits, L2 norm) in float32.  The gradients of A_log and dt_bias sum the gate gradients of all tokens, large
+    terms of either sign: whatever a backward loses in dg shows there many times over.  Against float64 autograd through the token-by-token
+    oracle, 2-norm: 1e-5 (products and sums in float32, a few hundred terms: 2^-24 sqrt(B T) = 2e-6, gate functions 1e-6; measured 1e-6)."""
+    import torch.nn.functional as F
+    from kda_b200 import chunk_kda
+    from oracle.kda_oracle import recurrent_kda
+    gen = torch.Generator().manual_seed(49)
+    rn = lambda *s: torch.randn(*s, generator=gen)      # noqa: E731
+    x = dict(q=rn(B, T, H, D), k=rn(B, T, H, D), v=rn(B, T, H, D), g=rn(B, T, H, D), beta=rn(B, T, H),
+             A_log=torch.log(1.0 + 15.0 * torch.rand(H, generator=gen)), dt_bias=rn(H * D))
+    up = rn(B, T, H, D)
+    lv = {n: t.cuda().requires_grad_(True) for n, t in x.items()}
+    o, _ = chunk_kda(**lv, use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True, use_beta_sigmoid_in_kernel=True)
+    got = dict(zip(lv, torch.autograd.grad(o, list(lv.values()), up.cuda())))
+    r = {n: t.cuda().double().requires_grad_(True) for n, t in x.items()}
+    g = -torch.exp(r["A_log"]).view(1, 1, H, 1) * F.softplus(r["g"] + r["dt_bias"].view(1, 1, H, D), threshold=1e9)
+    ro, _ = recurrent_kda(r["q"], r["k"], r["v"], g, torch.sigmoid(r["beta"]), use_qk_l2norm=True)
+    ref = dict(zip(r, torch.autograd.grad(ro, list(r.values()), up.cuda().double())))
+    for n in x:
+        e = float((got[n].double() - ref[n]).norm() / ref[n].norm())
+        assert e <= 1e-5, f"d_{n}: relative error {e:.2e}"
