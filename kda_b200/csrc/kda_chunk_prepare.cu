@@ -11,14 +11,16 @@
 //   16   blocks I > J of 16 x 16:   rows x_t prod(16 I .. t),   columns k_j prod(j+1 .. 16 J + 15) times the blocks in between
 //    8   rows 8..15 against 0..7 of a 16-row block, cut at row 8
 //    4   rows 4..7 against 0..3 and 12..15 against 8..11, cut at rows 4 and 12
-//   the 4 x 4 diagonal blocks pairwise, summed over the lanes 16 values at a time.
+//   the 4 x 4 diagonal blocks pairwise.
+// Levels 16 and 8 are products of bf16 rows on tensor cores; level 4 and the diagonal blocks, which hold the largest entries, stay float32
+// sums over the lanes (level 4 as a bf16 product, as it was: o 1.7 % further from 64 bits with slowly decaying gates).
 // With the caller's promise of bounded gates (SAFE) the 16 x 16 diagonal blocks go whole, cut at their row 8 from both sides.
-// Operands are written to shared memory once as bf16 and read by ldmatrix; level 8 / 4 products stack q and k rows into one m16
+// Product operands are written to shared memory once as bf16 and read by ldmatrix; the level 8 product stacks q and k rows into one m16
 // tile.  The same pass writes QG = scale q Gam, KG = k Gam_last / Gam and k Gam.
 //
-// What bounds it: instruction issue and shared-memory wavefronts, about 24 k cycles per CTA with two CTAs per SM; its bytes take 0.81 ms
-// at 8 x 8192 tokens x 32 heads, where it takes 1.50 ms.  (A thread per key column and row, decays as exp2 of cumulative sums and row
-// references, 256 threads: 1.98.)  Bounded gates at 1 x 32768 x 32: 0.77 ms with the gate's activation, 0.97 with a kernel before it.  Without the
+// What bounds it: instruction issue and shared-memory wavefronts, about 23 k cycles per CTA with two CTAs per SM; its bytes take 0.81 ms
+// at 8 x 8192 tokens x 32 heads, where it takes 1.55 ms (with level 4 as a bf16 product 1.50; a thread per key column and row, decays as exp2
+// of cumulative sums and row references, 256 threads: 1.98).  Bounded gates at 1 x 32768 x 32: 0.74 ms with the gate's activation.  Without the
 // L2 prefetch of the next wave's rows 1.65, two waves ahead 1.59.
 #include "kda_device.cuh"
 #include "kda_gate.cuh"
@@ -36,13 +38,14 @@ constexpr int DS = 20;    // floats per row of a 16 x 16 fp32 block
 
 // Operand rows of the region `op`: every 16-row block has its own part, written and (levels 8, 4) read by its four warps alone, so that
 // they meet at a barrier of 128 threads instead of the whole CTA.  Inside a part:
-//   levels 8 and 4:  A8 16 rows (q 8..15, k 8..15) | B8 8 | A4 16 (q 4..7, k 4..7, q 12..15, k 12..15) | B4 8
+//   levels 8 and 4:  A8 16 rows (q 8..15, k 8..15) | B8 8 | C4: columns 0..3 and 8..11 of level 4 in fp32 (eight rows of 512 bytes)
 //   SAFE diagonal:   q 16 | k 16 (row side) | k 16 (column side)
 //   level 16:        blocks 1..3: q 16 | k 16; then columns for the blocks at distance 1, 2, 3 (16 rows each)
 // Afterwards the region holds v (two 64-column tiles in the 128-byte swizzle), the staged UT tile and Tm as bf16 (times beta: TB;
 // plain: TI, in its tile image).
 constexpr int OP_ROWS = 208;
-constexpr int OP_B8 = 16, OP_A4 = 24, OP_B4 = 40;
+constexpr int OP_B8 = 16, OP_C4 = 24;
+static_assert(8 * KD * 4 <= (48 - OP_C4) * QS * 2, "the columns of level 4 must fit behind the level 8 operands");
 __device__ __forceinline__ int op_base(int blk) { return blk == 0 ? 0 : 48 * blk + (blk > 1 ? 16 : 0); }      // 48, 64, 48, 48 rows
 __device__ __forceinline__ int op_cols(int blk, int dist) { return op_base(blk) + (blk > 0 ? 32 : 0) + 16 * (dist - 1); }
 
@@ -401,22 +404,14 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
       }
     }
     forget();
-    const int u = quad >> 1;
-    if (quad & 1) {                                     // rows 4..7, 12..15: prod from row 4, 12
-      F4 f = lam[0];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (i > 0) f = mul4c(f, lam[i]);
-        put(OP_A4 + 8 * u + i, mul4c(widen(q[i]), f));
-        put(OP_A4 + 8 * u + 4 + i, mul4c(key(i), f));
-      }
-    } else {                                            // columns 0..3, 8..11: prod up to row 3, 11
-      put(OP_B4 + 4 * u + 3, key(3));
+    if (!(quad & 1)) {                                  // level 4, columns 0..3, 8..11: prod up to row 3, 11
+      float* const c4 = reinterpret_cast<float*>(s.op + (op_base(blk) + OP_C4) * QS) + 2 * quad * KD + kk;
+      sts4(c4 + 3 * KD, key(3));
       F4 f = lam[3];
 #pragma unroll
       for (int j = 2; j >= 0; --j) {
         if (j < 2) f = mul4c(f, lam[j + 1]);
-        put(OP_B4 + 4 * u + j, mul4c(key(j), f));
+        sts4(c4 + j * KD, mul4c(key(j), f));
       }
     }
   } else {
@@ -458,12 +453,45 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
       const int row = b0 + 8 + gid, col = b0 + 2 * tig;
       *reinterpret_cast<uint32_t*>(s.Aqk + swz<128>(row, col)) = pack_bf16(p.scale * a[0][0], p.scale * a[0][1]);
       *reinterpret_cast<float2*>(&s.Akk[row * AS + col]) = make_float2(a[0][2], a[0][3]);
-    } else if (quad == 1) {      // level 4: accumulator rows 0..7 (q 4..7, k 4..7) go with columns 0..3, rows 8..15 (q, k 12..15) with columns 4..7
-      prep_mma<1>(a, part + OP_A4 * QS, part + OP_B4 * QS, lane);
-      const int u = tig >> 1, row = b0 + 8 * u + 4 + (gid & 3), col = b0 + 8 * u + 2 * (tig & 1);
-      const float x = u ? a[0][2] : a[0][0], y = u ? a[0][3] : a[0][1];
-      if (gid < 4) *reinterpret_cast<uint32_t*>(s.Aqk + swz<128>(row, col)) = pack_bf16(p.scale * x, p.scale * y);
-      else *reinterpret_cast<float2*>(&s.Akk[row * AS + col]) = make_float2(x, y);
+    } else if (quad & 1) {
+      // level 4: these rows, prod from row 4 or 12, against the four columns in front, float32 sums over the lanes.  A lane takes the columns in
+      // an order of its own, j = i ^ (lane & 3): the first two steps of the sums then pass values on without choosing any.
+      const float* const c4 = reinterpret_cast<const float*>(part + OP_C4 * QS) + 2 * (quad - 1) * KD + kk;
+      float w[8];      // q and k of the four rows, column lane & 3, summed over four lanes
+      F4 f = lam[0];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        if (t > 0) f = mul4c(f, lam[t]);
+        const F4 qt = mul4c(widen(q[t]), f), kt = mul4c(key(t), f);
+        float vq[4], vk[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const F4 c = lds4(c4 + (i ^ (lane & 3)) * KD);
+          vq[i] = dot(qt, c);
+          vk[i] = dot(kt, c);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          vq[i] += __shfl_xor_sync(0xffffffffu, vq[i + 2], 2);
+          vk[i] += __shfl_xor_sync(0xffffffffu, vk[i + 2], 2);
+        }
+        w[2 * t] = vq[0] + __shfl_xor_sync(0xffffffffu, vq[1], 1);
+        w[2 * t + 1] = vk[0] + __shfl_xor_sync(0xffffffffu, vk[1], 1);
+        forget();
+      }
+#pragma unroll
+      for (int o = 4; o >= 1; o >>= 1) {      // lanes 4, 8, 16 apart
+        const bool up = (lane & (16 / o)) != 0;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+          const float mine = up ? w[i + o] : w[i];
+          const float other = up ? w[i] : w[i + o];
+          w[i] = mine + __shfl_xor_sync(0xffffffffu, other, 16 / o);
+        }
+      }
+      const int row = t0 + ((lane >> 1) & 2) + ((lane >> 3) & 1), col = t0 - 4 + (lane & 3);
+      if (lane & 16) s.Akk[row * AS + col] = w[0];
+      else *reinterpret_cast<__nv_bfloat16*>(s.Aqk + swz<128>(row, col)) = __float2bfloat16_rn(p.scale * w[0]);
     }
   } else {
     // one product per warp: q or k rows of the block against one half of its columns; Aqk keeps j <= t, Akk j < t
@@ -481,8 +509,8 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
       *reinterpret_cast<uint32_t*>(s.Aqk + swz<128>((b0 + rb), b0 + col)) = pack_bf16(p.scale * v2, p.scale * v3);
     }
   }
-  if (quad == 3) {               // the decay over the whole block, for the next phase
-    sts4(&s.TB[blk][kk], mul4c(mul4c(lds4(&s.T[warp - 3][kk]), lds4(&s.T[warp - 2][kk])), mul4c(lds4(&s.T[warp - 1][kk]), lds4(&s.T[warp][kk]))));
+  if (quad == 2) {               // the decay over the whole block, for the next phase
+    sts4(&s.TB[blk][kk], mul4c(mul4c(lds4(&s.T[warp - 2][kk]), lds4(&s.T[warp - 1][kk])), mul4c(lds4(&s.T[warp][kk]), lds4(&s.T[warp + 1][kk]))));
   }
   __syncthreads();      // the level 8 / 4 operands have been read; TB is there
   KDA_DBG_CLOCK(p.dbg, 20);
@@ -499,25 +527,23 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
     if (quad < 2) f = mul4c(f, lds4(&s.T[4 * blk + 2][kk]));
     if (quad < 1) f = mul4c(f, lds4(&s.T[4 * blk + 1][kk]));
     {
-      F4 post = splat(1.f), m2 = splat(1.f), m3 = splat(1.f);
+      F4 post = splat(1.f);
       if (blk < 3) post = lds4(&s.TB[blk + 1][kk]);
-      if (blk < 2) {
-        m2 = post;
-        post = mul4c(post, lds4(&s.TB[blk + 2][kk]));
-      }
-      if (blk < 1) {
-        m3 = post;
-        post = mul4c(post, lds4(&s.TB[3][kk]));
-      }
+      if (blk < 2) post = mul4c(post, lds4(&s.TB[blk + 2][kk]));
+      if (blk < 1) post = mul4c(post, lds4(&s.TB[3][kk]));
       const int cb = (blk > 0 ? 32 : 0) + 4 * quad;
+      // (the block decays between are read again for every row: kept in registers they spilled; bounded gates 1,370 -> 1,336 us at 1 x 32768)
 #pragma unroll
       for (int i = 3; i >= 0; --i) {                    // f = prod(i+1 .. last row of the block)
         if (i < 3) f = mul4c(f, lam[i + 1]);
-        const F4 kf = mul4c(key(i), f);
+        F4 kf = mul4c(key(i), f);
         *reinterpret_cast<uint2*>(gKG + i * 128 + ((piece ^ ((t0 + i) & 7)) << 4)) = narrow(mul4c(kf, post));
         if (blk < 3) put(cb + i, kf);
-        if (blk < 2) put(cb + 16 + i, mul4c(kf, m2));
-        if (blk < 1) put(cb + 32 + i, mul4c(kf, m3));
+        if (blk < 2) {
+          kf = mul4c(kf, lds4(&s.TB[blk + 1][kk]));
+          put(cb + 16 + i, kf);
+        }
+        if (blk < 1) put(cb + 32 + i, mul4c(kf, lds4(&s.TB[blk + 2][kk])));
       }
     }
     // decay over the rows of the block in front of these; over the blocks in front

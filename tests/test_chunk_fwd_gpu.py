@@ -58,6 +58,34 @@ def test_chunk_fwd_mild_gates():
     _check(o, ht, ref_o, ref_h)
 
 
+@pytest.mark.parametrize("K,tokens", [(128, 64), (64, 64), (128, 190)])
+def test_diagonal_8x8_blocks_are_float32_sums(K, tokens):
+    """Entries of the intra-chunk products inside the 8 x 8 diagonal blocks, read out one by one: row j's key lives on a channel of its own and
+    its value is one unit vector, so o[t, column j] = q_t k_j prod(decay).  The entry is a float32 sum that is rounded to bf16 as the product's
+    operand and as o: 2 x 2^-9; operands rounded to bf16 before the product would add two more."""
+    from kda_b200 import chunk_kda
+    gen = torch.Generator().manual_seed(70 + K)
+    H = 8
+    q = torch.randn(1, tokens, H, K, generator=gen).bfloat16()
+    ch = torch.arange(tokens) % 64
+    k = torch.zeros(1, tokens, H, K)
+    k[0, torch.arange(tokens), :, ch] = 0.5 + torch.rand(tokens, H, generator=gen)
+    k = k.bfloat16()
+    v = torch.zeros(1, tokens, H, 64)
+    v[0, torch.arange(tokens), :, ch] = 1.0
+    g = -0.5 * torch.rand(1, tokens, H, K, generator=gen)
+    with torch.no_grad():
+        o, _ = chunk_kda(q.cuda(), k.cuda(), v.bfloat16().cuda(), g.cuda(), torch.ones(1, tokens, H).cuda(), scale=1.0)
+    G = g.double()[0].cumsum(0)
+    worst = 0.0
+    for t in range(tokens):
+        for j in range(t - t % 8, t + 1):
+            c = int(ch[j])
+            ref = q[0, t, :, c].double() * k[0, j, :, c].double() * torch.exp(G[t, :, c] - G[j, :, c])
+            worst = max(worst, float(((o[0, t, :, c].cpu().double() - ref).abs() / ref.abs()).max()))
+    assert worst <= 2.0 ** -8 + 1e-4, worst
+
+
 def test_chunk_fwd_varlen_bit_exact_segmentation():
     """Packed variable-length result == each sequence run alone, bit for bit; and both match the oracle."""
     from kda_b200 import chunk_kda
