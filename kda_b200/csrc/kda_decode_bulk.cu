@@ -157,9 +157,13 @@ __global__ void __launch_bounds__(HV * 2 + 32, 128 / HV) kda_decode_bulk_kernel(
         const bool more = ahead.u < p.total;
         const long long lslot = more ? start_slot(ahead) : 0;
         const int nst = slotted ? a.T : 1;
+        // Two tokens of a sequence may name the same slot, whose last state counts.  Stores of the copy engine are not ordered among each
+        // other: at most four are in flight, and one to a slot among theirs waits until those have been written.
+        long long recent[4] = {-1, -1, -1, -1};
         for (int c = 0; c < nst; ++c) {
           const int b = (c & 1) ? y : x;
           const long long st = (slotted ? static_cast<long long>(a.state_indices[static_cast<size_t>(cur.n) * a.state_indices_stride + c]) : cur.n) * a.H + cur.h;
+          if (HV != DV && (st == recent[0] || st == recent[1] || st == recent[2] || st == recent[3])) bulk_wait<0>();
           wait(s.ready, ready, b);
           ready ^= 1u << b;
           if (s.dead) break;
@@ -167,6 +171,10 @@ __global__ void __launch_bounds__(HV * 2 + 32, 128 / HV) kda_decode_bulk_kernel(
           else tma_store_2d(&p.tm_out, HV * half, static_cast<int>(st * DK), s.S[b]);
           bulk_commit();
           bulk_wait_read<1>();
+          if constexpr (HV != DV) {
+            bulk_wait<4>();
+            recent[3] = recent[2]; recent[2] = recent[1]; recent[1] = recent[0]; recent[0] = st;
+          }
           if (last >= 0) mbar_arrive(&s.gone[last]);
           last = b;
         }

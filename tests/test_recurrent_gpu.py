@@ -302,3 +302,25 @@ def test_draft_tokens_on_half_states(N, T, H, tr):
         assert max_norm_err(got.transpose(-1, -2) if tr else got, h_ref) <= 1e-4, t
     assert max_norm_err(o, o_ref) <= 2e-2 and cosine(o, o_ref) >= 0.9999
     assert int((pool == 7.0).all(-1).all(-1).all(-1).sum()) == 2      # the two slots nobody owns
+
+
+@pytest.mark.parametrize("N,T,H,tr,pattern", [(24, 4, 16, False, "same"), (24, 7, 16, False, "alternate"), (24, 4, 16, True, "same"),
+                                              (24, 9, 16, False, "far"), (2, 4, 8, False, "same")])
+def test_a_slot_named_by_several_tokens_keeps_the_last_state(N, T, H, tr, pattern):
+    """A caller that only wants the state behind the last token names one slot for all tokens (or a few in turn): every slot holds the state of
+    the last token that names it.  Half states on the bulk-copy kernel (N = 24) and per-warp kernel (N = 2), many sequences at once."""
+    from kda_b200 import _lib, fused_recurrent_kda_fwd
+    d = make_inputs(N, T, H, 128, 128, torch.bfloat16, seed=80 + T, h0_std=0.05, device="cuda", generate_on_device=True)
+    which = {"same": [0] * T, "alternate": [t % 2 for t in range(T)], "far": [0] + list(range(1, T - 1)) + [0]}[pattern]
+    slots = torch.randperm(N * T, device="cuda").view(N, T)[:, which].to(torch.int32)
+    h0 = d["h0"].transpose(-1, -2).contiguous() if tr else d["h0"]
+    for _ in range(5):
+        pool = torch.full((N * T, H, 128, 128), 7.0, device="cuda")
+        pool[slots[:, 0].long()] = h0
+        o, _ = fused_recurrent_kda_fwd(d["q"], d["k"], d["v"], d["g"], d["beta"], initial_state=pool, ssm_state_indices=slots, transpose_state_layout=tr)
+        assert _lib.recurrent_status() == 0
+        for w in set(which):
+            last = max(t for t in range(T) if which[t] == w)
+            _, h_ref = recurrent_kda(*(d[n][:, :last + 1] for n in ("q", "k", "v", "g", "beta")), initial_state=d["h0"], output_final_state=True)
+            got = pool[slots[:, last].long()]
+            assert max_norm_err(got.transpose(-1, -2) if tr else got, h_ref) <= 1e-4, (w, last)
