@@ -391,6 +391,13 @@ struct ChunkCall {
   int slices = 0;
 };
 
+// Forward-mode tangents: there is no forward-mode derivative, and a call without gradients passes autograd by, which would drop them.
+bool has_tangent(std::initializer_list<const Tensor*> ts) {
+  for (const Tensor* t : ts)
+    if (t->defined() && t->_fw_grad(0).defined()) return true;
+  return false;
+}
+
 bool wants_grad(std::initializer_list<const Tensor*> ts) {
   if (!at::GradMode::is_enabled()) return false;
   for (const Tensor* t : ts)
@@ -405,6 +412,8 @@ bool chunk_kda(ChunkCall& c, Tensor& o, Tensor& ht) {
   const bool grads = wants_grad({&c.q, &c.k, &c.v, &c.g, &c.beta, &c.h0, &c.A_log, &c.dt_bias});
   if (c.q.scalar_type() != at::kBFloat16 || s.K > 128 || s.V > 128 || s.K % 8 || s.V % 8) return false;
   if ((s.K < 128 || s.V < 128) && grads && s.HQ != s.H) return false;
+  KDA_REQUIRE(!has_tangent({&c.q, &c.k, &c.v, &c.g, &c.beta, &c.h0, &c.A_log, &c.dt_bias}), PyExc_NotImplementedError,
+              "kda_b200: chunk_kda has no forward-mode derivative (jvp)");
   ChunkOpts opt;
   opt.scale = c.scale ? *c.scale : 1.0 / std::sqrt(static_cast<double>(s.K));
   opt.output_final = c.output_final; opt.l2norm = c.l2norm; opt.gate = c.gate; opt.beta_sigmoid = c.beta_sigmoid; opt.safe_gate = c.safe_gate;
