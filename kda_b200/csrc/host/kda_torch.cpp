@@ -99,6 +99,11 @@ Tensor f32(const Tensor& t) {
   const Tensor c = t.contiguous();
   return c.scalar_type() == at::kFloat ? c : c.to(at::kFloat);
 }
+// The kernels need 16-byte aligned rows.  Heads narrower than theirs are read in place but may start anywhere (they used to be padded into new
+// tensors); full-width tensors at odd addresses are refused by the library.
+Tensor aligned(const Tensor& t, bool narrow) {
+  return narrow && t.defined() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 ? t.clone() : t;
+}
 Tensor i32(const Tensor& t, const at::Device& dev) {
   if (!t.defined()) return t;
   if (t.scalar_type() == at::kInt && t.device() == dev) return t.contiguous();
@@ -270,7 +275,8 @@ std::pair<Tensor, Tensor> chunk_forward(ChunkSaved& s, const Tensor& q, const Te
   const c10::cuda::CUDAGuard guard(dev);
   const cudaStream_t st = stream_of(dev);
   const int64_t B = q.size(0), T = q.size(1), H = v.size(2), K = q.size(3), V = v.size(3), tokens = B * T;
-  s.q = dense(q); s.k = dense(k); s.v = dense(v); s.h0 = dense(h0);
+  const bool narrow = K < 128 || V < 128;
+  s.q = aligned(dense(q), narrow); s.k = aligned(dense(k), narrow); s.v = aligned(dense(v), narrow); s.h0 = aligned(dense(h0), narrow);
   // the forward kernel activates g and beta itself; the activated values are written only for a backward
   if (o.gate) {
     s.g_raw = dense(g);
@@ -278,7 +284,7 @@ std::pair<Tensor, Tensor> chunk_forward(ChunkSaved& s, const Tensor& q, const Te
     s.b32 = f32(dt_bias);
     if (need_grad) s.g = empty(g.sizes(), at::kFloat, dev);
   } else {
-    s.g = f32(g);
+    s.g = aligned(f32(g), narrow);
   }
   if (o.beta_sigmoid) {
     s.beta_raw = dense(beta);
@@ -341,8 +347,9 @@ class ChunkFunction : public torch::autograd::Function<ChunkFunction> {
     const c10::cuda::CUDAGuard guard(dev);
     const cudaStream_t st = stream_of(dev);
     const int64_t tokens = s.q.size(0) * s.q.size(1), H = s.v.size(2), K = s.q.size(3), V = s.v.size(3), N = sequences(s);
-    Tensor d_o = grads[0].defined() ? dense(grads[0].scalar_type() == s.v.scalar_type() ? grads[0] : grads[0].to(s.v.scalar_type())) : at::zeros_like(s.v);
-    const Tensor d_ht = grads.size() > 1 ? f32(grads[1]) : Tensor();
+    const bool narrow = K < 128 || V < 128;
+    const Tensor d_o = grads[0].defined() ? aligned(dense(grads[0].scalar_type() == s.v.scalar_type() ? grads[0] : grads[0].to(s.v.scalar_type())), narrow) : at::zeros_like(s.v);
+    const Tensor d_ht = grads.size() > 1 ? aligned(f32(grads[1]), narrow) : Tensor();
     const Tensor dq = empty(s.q.sizes(), s.q.scalar_type(), dev), dk = empty(s.k.sizes(), s.k.scalar_type(), dev), dv = empty(s.v.sizes(), s.v.scalar_type(), dev);
     Tensor dg = empty(s.g.sizes(), at::kFloat, dev), dbeta = empty(s.beta.sizes(), at::kFloat, dev);
     const Tensor dh0 = s.h0.defined() ? empty(s.h0.sizes(), at::kFloat, dev) : Tensor();

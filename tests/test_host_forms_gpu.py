@@ -30,3 +30,37 @@ def test_forward_mode_tangents_are_refused_not_dropped(which, grads):
         with pytest.raises(RuntimeError, match="jvp"):
             chunk_kda(**x, **kw)
     assert torch.isfinite(chunk_kda(d["q"], d["k"], d["v"], d["g"], d["beta"])[0].float()).all()
+
+
+def _shifted(t, by):
+    """The same values in a dense tensor that starts `by` elements into its buffer."""
+    buf = torch.empty(t.numel() + by, dtype=t.dtype, device=t.device)
+    out = buf[by:].view(t.shape)
+    out.copy_(t)
+    assert out.is_contiguous() and out.data_ptr() % 16 != 0
+    return out
+
+
+@pytest.mark.parametrize("K,V", [(64, 64), (128, 64), (96, 32)])
+@pytest.mark.parametrize("grads", [False, True])
+def test_narrow_heads_at_odd_addresses(K, V, grads):
+    """Heads of fewer than 128 columns: dense tensors that do not start on a 16-byte boundary are taken (they were padded into new ones
+    once), with the results of aligned ones, gradients from odd addresses included."""
+    from kda_b200 import chunk_kda
+    d = {n: t.cuda() for n, t in make_inputs(1, 130, 2, K, V, torch.bfloat16, seed=3, h0_std=0.02, backward=True).items()}
+
+    def run(shift):
+        x = {n: (_shifted(d[n], by) if shift else d[n].clone()) for n, by in (("q", 1), ("k", 3), ("v", 4), ("g", 1), ("h0", 2), ("do", 5), ("dht", 1))}
+        lv = [x[n].requires_grad_(grads) for n in ("q", "k", "v", "g")] + [d["beta"].clone().requires_grad_(grads), x["h0"].requires_grad_(grads)]
+        o, ht = chunk_kda(*lv[:5], initial_state=lv[5], output_final_state=True)
+        return [o, ht] + (list(torch.autograd.grad([o, ht], lv, [x["do"], x["dht"]])) if grads else [])
+
+    for i, (a, b) in enumerate(zip(run(True), run(False))):
+        assert torch.equal(a, b), i
+
+
+def test_full_width_heads_at_odd_addresses_are_refused():
+    from kda_b200 import _lib, chunk_kda
+    d = _inputs(1, 70, 2, 128, 4)
+    with pytest.raises(_lib.KdaError, match="align"):
+        chunk_kda(_shifted(d["q"], 1), d["k"], d["v"], d["g"], d["beta"])
