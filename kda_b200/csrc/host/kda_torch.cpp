@@ -322,7 +322,13 @@ class ChunkFunction : public torch::autograd::Function<ChunkFunction> {
     auto [out, ht] = chunk_forward(s, q, k, v, g, beta, h0.value_or(Tensor()), A_log.value_or(Tensor()), dt_bias.value_or(Tensor()),
                                    cu.value_or(Tensor()), o, true);
     ctx->set_materialize_grads(false);
-    ctx->save_for_backward({s.q, s.k, s.v, s.g, s.beta, s.h0, s.cu, s.ws, s.g_raw, s.A32, s.b32, s.beta_raw, A_log.value_or(Tensor()), dt_bias.value_or(Tensor())});
+    ctx->save_for_backward({s.q, s.k, s.v, s.g, s.beta, s.h0, s.cu, s.ws, s.g_raw, s.A32, s.b32, s.beta_raw});
+    // of the parameters themselves only shape and type: they may be updated before the backward (which reads the float32 copies)
+    for (const auto& [name, t] : {std::pair{"A_log", A_log}, std::pair{"dt_bias", dt_bias}}) {
+      if (!t) continue;
+      ctx->saved_data[std::string(name) + "_sizes"] = t->sizes().vec();
+      ctx->saved_data[std::string(name) + "_dtype"] = static_cast<int64_t>(t->scalar_type());
+    }
     ctx->saved_data["flags"] = static_cast<int64_t>(o.has_lower_bound | o.output_final << 1 | o.l2norm << 2 | o.gate << 3 | o.beta_sigmoid << 4 | o.safe_gate << 5 |
                                                     static_cast<int64_t>(o.slices) << 8);
     ctx->saved_data["scale"] = o.scale;
@@ -336,7 +342,6 @@ class ChunkFunction : public torch::autograd::Function<ChunkFunction> {
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const variable_list t = ctx->get_saved_variables();
     ChunkSaved s{t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], t[9], t[10], t[11]};
-    const Tensor &A_log = t[12], &dt_bias = t[13];
     ChunkOpts o;
     const int64_t f = ctx->saved_data["flags"].toInt();
     o.has_lower_bound = f & 1; o.output_final = f & 2; o.l2norm = f & 4; o.gate = f & 8; o.beta_sigmoid = f & 16; o.safe_gate = f & 32;
@@ -385,8 +390,11 @@ class ChunkFunction : public torch::autograd::Function<ChunkFunction> {
     const auto beta_dtype = static_cast<at::ScalarType>(ctx->saved_data["beta_dtype"].toInt());
     if (dg.scalar_type() != g_dtype) dg = dg.to(g_dtype);
     if (dbeta.scalar_type() != beta_dtype) dbeta = dbeta.to(beta_dtype);
-    if (dA.defined()) dA = dA.view(A_log.sizes()).to(A_log.scalar_type());
-    if (db.defined()) db = db.view(dt_bias.sizes()).to(dt_bias.scalar_type());
+    auto as = [&](const Tensor& d, const std::string& name) {
+      return d.view(ctx->saved_data[name + "_sizes"].toIntVector()).to(static_cast<at::ScalarType>(ctx->saved_data[name + "_dtype"].toInt()));
+    };
+    if (dA.defined()) dA = as(dA, "A_log");
+    if (db.defined()) db = as(db, "dt_bias");
     return {dq, dk, dv, dg, dbeta, dh0, dA, db, Tensor(), Tensor()};
   }
 };

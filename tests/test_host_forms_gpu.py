@@ -64,3 +64,19 @@ def test_full_width_heads_at_odd_addresses_are_refused():
     d = _inputs(1, 70, 2, 128, 4)
     with pytest.raises(_lib.KdaError, match="align"):
         chunk_kda(_shifted(d["q"], 1), d["k"], d["v"], d["g"], d["beta"])
+
+
+def test_bf16_gate_parameters_may_change_between_forward_and_backward():
+    """The backward needs the float32 copies of A_log and dt_bias that the forward made; bf16 parameters may be updated in between."""
+    from kda_b200 import chunk_kda
+    d = _inputs(1, 100, 2, 128, 5)
+    out = []
+    for touch in (False, True):
+        A, b = (torch.full((2,), 0.3, device="cuda").bfloat16().requires_grad_(True), torch.zeros(256, device="cuda").bfloat16().requires_grad_(True))
+        o, _ = chunk_kda(d["q"], d["k"], d["v"], torch.sin(d["g"]), d["beta"], A_log=A, dt_bias=b, use_gate_in_kernel=True)
+        if touch:
+            with torch.no_grad():
+                A.add_(1.0)
+                b.sub_(1.0)
+        out.append(torch.autograd.grad(o, [A, b], d["do"]))
+    assert all(torch.equal(x, y) for x, y in zip(*out))
