@@ -355,6 +355,9 @@ extern "C" int kda_recurrent_bwd(const kda_recurrent_bwd_args* a, void* stream) 
   const RecBwdLayout l = rec_bwd_layout(a->tokens, a->N, a->H, a->K, a->V);
   if (a->workspace_bytes < l.total) return KDA_E_WORKSPACE;
   if (reinterpret_cast<uintptr_t>(a->workspace) & 255) return KDA_E_ALIGN;
+  const void* wide[] = {a->v, a->h0, a->d_o, a->d_ht, a->dv, a->dh0};      // 16-byte loads and stores
+  for (const void* p : wide)
+    if (reinterpret_cast<uintptr_t>(p) & 15) return KDA_E_ALIGN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (a->N == 0) return KDA_OK;
   if (a->tokens == 0) {      // empty sequences: the initial state is the final state

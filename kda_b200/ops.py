@@ -294,8 +294,9 @@ class RecurrentKDAFunction(torch.autograd.Function):
         N = B if cu is None else cu.numel() - 1
         dev = q.device
         lib = _lib.load()
-        do = do.contiguous().float()
-        dht = dht.contiguous().float() if dht is not None else None
+        aligned = lambda t: t if t.data_ptr() % 16 == 0 else t.clone()      # noqa: E731  the kernel loads 16 bytes at a time
+        do = aligned(do.contiguous().float())
+        dht = aligned(dht.contiguous().float()) if dht is not None else None
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         dg, dbeta = torch.empty_like(g32), torch.empty_like(beta32)
         dh0 = torch.empty(N, H, K, V, dtype=torch.float32, device=dev) if h0 is not None else None

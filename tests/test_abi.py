@@ -79,6 +79,17 @@ def test_argument_errors_without_gpu(lib):
     assert lib.kda_chunk_fwd(C.byref(a), None) == -5              # workspace too small
 
 
+def test_recurrent_backward_refuses_unaligned_pointers(lib):
+    """Loads and stores that are 16 bytes wide: an odd address is an argument error on the host, never a launch."""
+    from kda_b200 import _lib
+    size = lib.kda_recurrent_bwd_workspace_bytes(64, 1, 2, 64, 64)
+    names = ("q", "k", "v", "g", "h0", "d_o", "d_ht", "dq", "dk", "dv", "dg", "dh0")
+    for odd in ("v", "h0", "d_o", "d_ht", "dv", "dh0"):
+        r = _lib.RecurrentBwdArgs(N=1, T=64, tokens=64, H=2, K=64, V=64, HQ=2, io_dtype=_lib.KDA_FP32, beta=256, dbeta=256, workspace=512, workspace_bytes=size,
+                                  **{n: 256 + (4 if n == odd else 0) for n in names})
+        assert lib.kda_recurrent_bwd(C.byref(r), None) == -4, odd
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     from kda_b200 import _lib
     monkeypatch.setattr(_lib, "_lib", None)

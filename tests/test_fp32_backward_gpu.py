@@ -152,3 +152,19 @@ def test_fp32_layer_gradients_are_float32_accurate(B, T, H, D):
     for n in x:
         e = float((got[n].double() - ref[n]).norm() / ref[n].norm())
         assert e <= 1e-5, f"d_{n}: relative error {e:.2e}"
+
+
+def test_fp32_gradients_at_odd_addresses():
+    """Incoming gradients that do not start on a 16-byte boundary (views into a larger buffer) give the results of aligned ones."""
+    from kda_b200 import chunk_kda
+    d = {n: t.cuda() for n, t in make_inputs(1, 70, 2, 64, 64, torch.float32, seed=50, h0_std=0.1, backward=True).items()}
+    lv = [d[n].requires_grad_(True) for n in ("q", "k", "v", "g", "beta", "h0")]
+    out = []
+    for shift in (0, 1):
+        ups = []
+        for n in ("do", "dht"):
+            buf = torch.zeros(d[n].numel() + shift, device="cuda")
+            ups.append(buf[shift:].view(d[n].shape).copy_(d[n]))
+        o, ht = chunk_kda(*lv[:5], initial_state=lv[5], output_final_state=True)
+        out.append(torch.autograd.grad([o, ht], lv, ups))
+    assert all(torch.equal(a, b) for a, b in zip(*out))
