@@ -192,7 +192,10 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
   const int tid = threadIdx.x, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);      // warp-uniform for the compiler: role branches need no reconvergence code
   const int c = blockIdx.x / p.H, h = blockIdx.x % p.H;        // neighbouring CTAs take neighbouring heads: contiguous rows and tiles
-  if (p.clear_status && blockIdx.x == 0 && tid < 4) p.status[tid] = 0u;
+  if (p.clear_status && blockIdx.x == 0 && tid < 5) {      // no tables kernel has run: its share of the workspace that others read
+    if (tid < 4) p.status[tid] = 0u;
+    else const_cast<int*>(p.map.seq_chunk_off)[p.map.N] = p.map.total();      // kda_chunk_export_states
+  }
   if (c >= p.map.total()) return;
   const ChunkInfo ci = p.map.info(c);
   const int len = ci.len;

@@ -253,3 +253,29 @@ def test_prefill_forward_replays_from_a_cuda_graph():
         o_e, ht_e = run()
         torch.cuda.synchronize()
         assert torch.equal(o_g, o_e) and torch.equal(ht_g, ht_e)
+
+
+@pytest.mark.parametrize("N,T", [(1, 64), (2, 100), (3, 64), (1, 1)])
+def test_export_states_after_an_equal_length_forward(N, T):
+    """cu_seqlens == NULL: the forward builds no tables, and the states are exported all the same: those of the call with cu_seqlens."""
+    import ctypes as C
+    from kda_b200 import _lib
+    lib = _lib.load()
+    H, tokens = 2, N * T
+    d = {n: t.cuda().contiguous() for n, t in make_inputs(N, T, H, 128, 128, torch.bfloat16, seed=6, h0_std=0.02).items() if t is not None}
+    cu = torch.arange(0, tokens + 1, T, dtype=torch.int32, device="cuda")
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    got = []
+    for c in (None, cu):
+        ws = torch.full((lib.kda_chunk_workspace_bytes(tokens, N, H, 128, 128, 1),), 0 if c is None else 0xA5, dtype=torch.uint8, device="cuda")
+        o = torch.empty_like(d["v"])
+        a = _lib.ChunkArgs(q=d["q"].data_ptr(), k=d["k"].data_ptr(), v=d["v"].data_ptr(), g=d["g"].data_ptr(), beta=d["beta"].data_ptr(), h0=d["h0"].data_ptr(),
+                           cu_seqlens=c.data_ptr() if c is not None else None, o=o.data_ptr(), workspace=ws.data_ptr(), workspace_bytes=ws.numel(), tokens=tokens,
+                           N=N, H=H, K=128, V=128, io_dtype=_lib.KDA_BF16, scale=0.1, save_for_backward=1)
+        _lib.check(lib.kda_chunk_fwd(C.byref(a), st), "kda_chunk_fwd")
+        h = torch.full((lib.kda_chunk_max_chunks(tokens, N), H, 128, 128), 7.0, dtype=torch.bfloat16, device="cuda")
+        _lib.check(lib.kda_chunk_export_states(C.c_void_p(ws.data_ptr()), ws.numel(), tokens, N, H, C.c_void_p(h.data_ptr()), st), "kda_chunk_export_states")
+        got.append(h)
+    torch.cuda.synchronize()
+    chunks = N * ((T + 63) // 64)
+    assert torch.equal(got[0], got[1]) and bool((got[0][chunks:] == 7.0).all()) and not bool((got[0][:chunks] == 7.0).all())
