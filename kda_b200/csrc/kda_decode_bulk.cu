@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(HV * 2 + 32, 128 / HV) kda_decode_bulk_kernel(
   // ================= the compute warps =================
   // A thread fetches its elements of a step's vectors (HV = 64: one of each; 128: of q and k, or of g and v) two steps ahead of its use and keeps the untouched bits in registers until
   // stash(): an instruction that depends on a load makes the thread wait for it right there, and a small load takes longer than
-  // a unit's update when the memory system is saturated.
+  // a unit's update when the memory system is saturated.  Plain loads, no read-only ones (__ldg): see kda_recurrent.cu.
   // Four registers a step, not seven: with gates the rest made the compiler touch loads still in flight (1,000 x 32, the layer's call: 682 -> 649 us)
   // (HV = 128: the threads of q, k and those of g, v use the same registers; beta waits in thread 0's slot for A_log, which it has no use for)
   constexpr int RQ = 0, RK = 1, RG = HV == 64 ? 2 : 0, RV = HV == 64 ? 3 : 1, RA = HV == 64 ? 4 : 2, RBIAS = HV == 64 ? 5 : 3, RB = HV == 64 ? 6 : 2;
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(HV * 2 + 32, 128 / HV) kda_decode_bulk_kernel(
   constexpr bool IO16 = sizeof(IO) == 2;
   auto ld_bits = [&](const void* ptr, size_t i, bool bf16) -> uint32_t {
     if (bf16) return static_cast<const unsigned short*>(ptr)[i];
-    return __float_as_uint(__ldg(static_cast<const float*>(ptr) + i));
+    return static_cast<const uint32_t*>(ptr)[i];
   };
   auto to_float = [&](uint32_t bits, bool bf16) -> float { return __uint_as_float(bf16 ? bits << 16 : bits); };
   const int e = tid & 127;
@@ -231,17 +231,17 @@ __global__ void __launch_bounds__(HV * 2 + 32, 128 / HV) kda_decode_bulk_kernel(
       if constexpr (GATE) {
         r.x[RG] = ld_bits(a.g, row * DK + e, a.A_log && a.g_raw_dtype == KDA_BF16);
         if (a.A_log) {
-          r.x[RA] = __float_as_uint(__ldg(a.A_log + q.h));
-          r.x[RBIAS] = a.dt_bias ? __float_as_uint(__ldg(a.dt_bias + static_cast<size_t>(q.h) * DK + e)) : 0u;
+          r.x[RA] = __float_as_uint(a.A_log[q.h]);
+          r.x[RBIAS] = a.dt_bias ? __float_as_uint(a.dt_bias[static_cast<size_t>(q.h) * DK + e]) : 0u;
         }
       } else {
-        r.x[RG] = __float_as_uint(__ldg(a.g + row * DK + e));
+        r.x[RG] = __float_as_uint(a.g[row * DK + e]);
       }
       if (e < HV) r.x[RV] = ld_bits(a.v, row * DV + half * HV + e, IO16);
     }
     if (tid == 0) {
       if constexpr (GATE) r.x[RB] = ld_bits(a.beta, row, a.beta_sigmoid && a.beta_raw_dtype == KDA_BF16);
-      else r.x[RB] = __float_as_uint(__ldg(a.beta + row));
+      else r.x[RB] = __float_as_uint(a.beta[row]);
     }
   };
   auto stash = [&](int buf, const Raw& r) {

@@ -15,9 +15,9 @@ namespace kda {
 
 template <typename IO> struct IoTraits;
 template <> struct IoTraits<float> {
-  static __device__ __forceinline__ float ld(const float* p) { return __ldg(p); }
+  static __device__ __forceinline__ float ld(const float* p) { return *p; }
   static __device__ __forceinline__ void st4(float* p, float4 x) { *reinterpret_cast<float4*>(p) = x; }
-  static __device__ __forceinline__ float4 ld4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+  static __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 };
 template <> struct IoTraits<__nv_bfloat16> {
   static __device__ __forceinline__ float ld(const __nv_bfloat16* p) { return __bfloat162float(*p); }
@@ -26,7 +26,7 @@ template <> struct IoTraits<__nv_bfloat16> {
     *reinterpret_cast<uint2*>(p) = u;
   }
   static __device__ __forceinline__ float4 ld4(const __nv_bfloat16* p) {
-    uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
+    uint2 u = *reinterpret_cast<const uint2*>(p);
     float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y);
     return make_float4(a.x, a.y, b.x, b.y);
   }
@@ -50,28 +50,30 @@ __device__ __forceinline__ float butterfly_sum32(float (&v)[32], int lane) {
 }
 
 // E consecutive elements of a row as untouched bits: a conversion right behind the load would make the warp wait for it there.
+// Plain loads, no read-only ones (__ldg) in this file: a chained kernel's lifetime overlaps that of the kernel in front, which may be writing
+// these tensors, and read-only loads are defined only for data that nobody writes meanwhile (nor are they held behind chain_point()).
 template <int E>
 struct RowBits {
   uint32_t w[E];
   __device__ __forceinline__ void load(const void* base, size_t i, bool bf16) {
     if (bf16) {
       const __nv_bfloat16* p = static_cast<const __nv_bfloat16*>(base) + i;
-      if constexpr (E == 1) w[0] = __ldg(reinterpret_cast<const unsigned short*>(p));
-      else if constexpr (E == 2) w[0] = __ldg(reinterpret_cast<const uint32_t*>(p));
+      if constexpr (E == 1) w[0] = *reinterpret_cast<const unsigned short*>(p);
+      else if constexpr (E == 2) w[0] = *reinterpret_cast<const uint32_t*>(p);
       else {
 #pragma unroll
         for (int e = 0; e < E / 4; ++e) {
-          const uint2 u = __ldg(reinterpret_cast<const uint2*>(p) + e);
+          const uint2 u = reinterpret_cast<const uint2*>(p)[e];
           w[2 * e] = u.x; w[2 * e + 1] = u.y;
         }
       }
     } else {
       const uint32_t* p = static_cast<const uint32_t*>(base) + i;
-      if constexpr (E == 1) w[0] = __ldg(p);
+      if constexpr (E == 1) w[0] = *p;
       else {
 #pragma unroll
         for (int e = 0; e < E / 2; ++e) {
-          const uint2 u = __ldg(reinterpret_cast<const uint2*>(p) + e);
+          const uint2 u = reinterpret_cast<const uint2*>(p)[e];
           w[2 * e] = u.x; w[2 * e + 1] = u.y;
         }
       }
@@ -140,8 +142,8 @@ __global__ void __launch_bounds__(REC_WARPS * 32) kda_recurrent_kernel(const kda
   if (bos < eos) fetch(bos, cur);
   float bias[E], al = 0.f;
 #pragma unroll
-  for (int e = 0; e < E; ++e) bias[e] = a.dt_bias ? __ldg(a.dt_bias + static_cast<size_t>(h) * K + lane * E + e) : 0.f;
-  if (a.A_log) al = __expf(__ldg(a.A_log + h));
+  for (int e = 0; e < E; ++e) bias[e] = a.dt_bias ? a.dt_bias[static_cast<size_t>(h) * K + lane * E + e] : 0.f;
+  if (a.A_log) al = __expf(a.A_log[h]);
   const size_t sbase = (static_cast<size_t>(slot) * a.H + h) * K * a.V + col;
 
   float4 S[R];

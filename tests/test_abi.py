@@ -90,6 +90,21 @@ def test_recurrent_backward_refuses_unaligned_pointers(lib):
         assert lib.kda_recurrent_bwd(C.byref(r), None) == -4, odd
 
 
+def test_kernels_chained_to_the_callers_use_no_read_only_loads():
+    """A decode kernel is launched as a programmatic dependent of whatever the caller ran before: it may be brought up while that kernel still
+    writes q, k, v, g, beta.  Read-only loads (__ldg, ld.global.nc, const __restrict__ parameters) are undefined for such data."""
+    import re
+    csrc = os.path.join(ROOT, "kda_b200", "csrc")
+    for name in ("kda_decode_bulk.cu", "kda_recurrent.cu"):
+        text = open(os.path.join(csrc, name)).read()
+        assert "launch_chained" in text and "chain_point();" in text, name
+        code = re.sub(r"//[^\n]*", "", text)
+        for word in ("__ldg", "ld.global.nc", "__restrict__"):
+            assert word not in code, (name, word)
+    loaders = open(os.path.join(csrc, "kda_common.cuh")).read()
+    assert "__ldg" not in re.sub(r"//[^\n]*", "", loaders)
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     from kda_b200 import _lib
     monkeypatch.setattr(_lib, "_lib", None)
