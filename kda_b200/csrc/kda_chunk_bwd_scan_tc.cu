@@ -233,6 +233,11 @@ __global__ void __launch_bounds__(RNT, 1) kda_chunk_bwd_scan_tc_kernel(const __g
       }
     }
   }
+  if (!alive && tid == 0) {              // a wait gave up: loads and products may still be under way
+    mbar_drain(&s.full[0]);
+    mbar_drain(&s.full[1]);
+    mbar_drain(&s.barM);
+  }
   if (tid == 0) bulk_wait<0>();
   umma::fence_before_sync();
   __syncthreads();

@@ -292,7 +292,8 @@ __global__ void __launch_bounds__(RVS_THREADS, 1) kda_chunk_bwd_scan_vs_kernel(c
     __syncwarp();
   } else if (warp == RW_STORE) {
     if (lane == 0) {
-      for (int i = 0; i < nchunks; ++i) {
+      int i = 0;
+      for (; i < nchunks; ++i) {
         const size_t tile = static_cast<size_t>(c_end - 1 - i) * p.H + h;
         if (s.dead) break;
         if (!mbar_wait(&s.sgReady, i & 1)) {
@@ -305,6 +306,11 @@ __global__ void __launch_bounds__(RVS_THREADS, 1) kda_chunk_bwd_scan_vs_kernel(c
         bulk_commit();
         bulk_wait_read<0>();                             // the staging tiles may be rewritten
         mbar_arrive(&s.sgFree);
+      }
+      if (i < nchunks) {      // somebody gave up: loads and products may still be under way
+        mbar_drain(&s.full[0]);
+        mbar_drain(&s.full[1]);
+        mbar_drain(&s.barM);
       }
       bulk_wait<0>();                                    // the stores read shared memory that dies with the CTA
     }

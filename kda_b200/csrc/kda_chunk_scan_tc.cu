@@ -293,6 +293,11 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
       }
     }
   }
+  if (!alive && tid == 0) {              // a wait gave up: loads and products may still be under way
+    mbar_drain(&s.full[0]);
+    mbar_drain(&s.full[1]);
+    mbar_drain(&s.barM);
+  }
   if (lead) bulk_wait<0>();              // outstanding bulk stores read shared memory that dies with the CTA
   umma::fence_before_sync();
   __syncthreads();

@@ -136,6 +136,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
   }
   return false;
 }
+// Give-up path, one thread: waits (bounded, some ten milliseconds a phase) for what may still complete on `bar`, because copies and products in
+// flight must not outlive the CTA's shared memory.  Which phase is open does not matter: the wait for a completed one returns at once.
+// Out of line, so that the loops around it stay as they are.
+static __device__ __noinline__ void mbar_drain(uint64_t* bar) {
+  for (unsigned parity = 0; parity < 2; ++parity)
+    for (int i = 0; i < 4096 && !mbar_try_wait(bar, parity); ++i) __nanosleep(64);
+}
 // global -> shared, `bytes` a multiple of 16, both addresses 16-byte aligned; completion on `bar`.
 __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, unsigned bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(

@@ -192,11 +192,7 @@ __global__ void __launch_bounds__(HV * 2 + 32, 128 / HV) kda_decode_bulk_kernel(
         y = last;
       }
       if (s.dead) {      // give the loads that may still be in flight into this CTA's memory a bounded time
-        for (int i = 0; i < DEC_BUFS; ++i) {
-          for (unsigned j = 0; j < 2; ++j) {
-            for (int k = 0; k < 4096 && !mbar_try_wait(&s.full[i], j); ++k) __nanosleep(64);
-          }
-        }
+        for (int i = 0; i < DEC_BUFS; ++i) mbar_drain(&s.full[i]);
       }
       bulk_wait<0>();      // the stores read shared memory and write the states: both complete before the CTA leaves
     }

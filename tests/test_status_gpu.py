@@ -37,6 +37,20 @@ def test_a_wait_that_runs_out_is_reported_and_the_gpu_stays_usable():
     assert torch.isfinite(o.float()).all()
 
 
+@pytest.mark.parametrize("nbytes", [16, 4096, 32768])
+def test_what_is_in_flight_has_landed_behind_the_give_up_drain(nbytes):
+    """The chunked kernels drain their barriers before they leave after a wait that gave up: copies in flight must not outlive the CTA's shared
+    memory.  The helper itself, on a barrier with a copy in flight in its first and in its second phase."""
+    lib = _debug_lib()
+    lib.kda_b200_debug_wait_drain.restype = C.c_int
+    lib.kda_b200_debug_wait_drain.argtypes = [C.c_void_p, C.c_void_p, C.c_uint, C.c_void_p]
+    src = torch.randint(0, 256, (2 * nbytes,), dtype=torch.uint8, device="cuda")
+    dst = torch.zeros_like(src)
+    assert lib.kda_b200_debug_wait_drain(src.data_ptr(), dst.data_ptr(), nbytes, torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(src, dst)
+
+
 @pytest.mark.parametrize("cu_list", [[0, 300], [0, 150, 100, 200], [-64, 200]])
 def test_inconsistent_cu_seqlens_is_reported_not_executed(cu_list):
     """cu_seqlens beyond the tensors, not monotone, or negative: the tables kernel sets KDA_STATUS_BAD_CU_SEQLENS and
