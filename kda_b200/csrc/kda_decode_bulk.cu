@@ -461,7 +461,10 @@ int launch_hv(const kda_recurrent_args& a, cudaStream_t st) {
 
 template <typename IO, bool TR, bool GATE>
 int launch(const kda_recurrent_args& a, cudaStream_t st) {
-  return a.T > 1 ? launch_hv<IO, TR, GATE, 64>(a, st) : launch_hv<IO, TR, GATE, 128>(a, st);
+  if constexpr (TR || GATE) {
+    if (a.T == 1) return launch_hv<IO, TR, GATE, 128>(a, st);
+  }
+  return launch_hv<IO, TR, GATE, 64>(a, st);
 }
 
 }  // namespace
@@ -480,7 +483,10 @@ bool decode_bulk_covers(const kda_recurrent_args& a) {
 }
 
 int decode_bulk_launch(const kda_recurrent_args& a, cudaStream_t st) {
-  const bool gate = a.A_log != nullptr || a.beta_sigmoid != 0;
+  // One token, states [K, V]: the variant with gates also serves the calls without.  At the copy rate it is when the loads and stores of the SMs
+  // meet in DRAM that decides, and that variant's steps fall better (without gates, us, its own variant | this one: 148 sequences x 32 heads
+  // 102.0 | 100.5, 512: 340 | 334, 1,024: 666 | 657, 1,500: 978 | 962).  States [V, K]: its own is better (1,024: 655 | 680).
+  const bool gate = a.A_log != nullptr || a.beta_sigmoid != 0 || (a.T == 1 && !a.transpose_state);
   const int which = (a.io_dtype == KDA_BF16 ? 0 : 4) + (a.transpose_state ? 2 : 0) + (gate ? 1 : 0);
   switch (which) {
     case 0: return launch<__nv_bfloat16, false, false>(a, st);
