@@ -105,6 +105,37 @@ def test_kernels_chained_to_the_callers_use_no_read_only_loads():
     assert "__ldg" not in re.sub(r"//[^\n]*", "", loaders)
 
 
+def _header_fields(struct):
+    """(name, ctype) of a struct of the public header, in order."""
+    import re
+    text = open(os.path.join(ROOT, "include", "kda_b200.h")).read()
+    text = re.sub(r"/\*.*?\*/", "", text, flags=re.S)
+    body = re.search(r"typedef struct %s \{(.*?)\} %s;" % (struct, struct), text, flags=re.S).group(1)
+    kinds = {"int32_t": C.c_int32, "int64_t": C.c_int64, "size_t": C.c_size_t, "float": C.c_float}
+    out = []
+    for decl in filter(None, (d.strip() for d in body.split(";"))):
+        kind, names = re.match(r"(?:const\s+)?(\w+)\s*(.*)", decl, flags=re.S).groups()
+        for n in names.split(","):
+            out.append((n.strip(" *\n"), C.c_void_p if "*" in n else kinds[kind]))
+    return out
+
+
+def test_bindings_have_the_headers_fields(lib):
+    """The ctypes structs of the package, and the binding that the integration document gives a maintainer to copy, list the header's fields in
+    the header's order: a struct that ends early makes the library read whatever lies behind it."""
+    import re
+    from kda_b200 import _lib
+    for struct, cls in (("kda_recurrent_args", _lib.RecurrentArgs), ("kda_recurrent_bwd_args", _lib.RecurrentBwdArgs), ("kda_chunk_args", _lib.ChunkArgs),
+                        ("kda_gate_args", _lib.GateArgs)):
+        assert list(cls._fields_) == _header_fields(struct), struct
+    doc = open(os.path.join(ROOT, "INTEGRATION.md")).read()
+    code = re.search(r"class ChunkArgs\(C\.Structure\):.*?(?=\n\n)", doc, flags=re.S).group(0)
+    scope = {"C": C}
+    exec(code, scope)      # the class statement of the document
+    assert list(scope["ChunkArgs"]._fields_) == _header_fields("kda_chunk_args")
+    assert "kda_b200_abi_version() == %d" % _lib.ABI_VERSION in doc
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     from kda_b200 import _lib
     monkeypatch.setattr(_lib, "_lib", None)
