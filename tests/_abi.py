@@ -29,6 +29,13 @@ class Guarded:
         return bool((lo == SENTINEL).all()) and bool((hi == SENTINEL).all())
 
 
+def bulk_decode_batch():
+    """(sequences, heads) of the smallest one-token batch that takes the whole-state decode kernel: 32 states per SM."""
+    heads = 128
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    return -(-32 * sms // heads), heads
+
+
 def guarded_like(shape, dtype, device="cuda"):
     n = 1
     for s in shape:
@@ -60,7 +67,7 @@ def chunk_fwd_bwd_guarded(d, cu, noalloc=False, l2=False):
     save = 0 if noalloc else (1 | (2 if l2 else 0))
     a = _lib.ChunkArgs(q=d["q"].data_ptr(), k=d["k"].data_ptr(), v=d["v"].data_ptr(), g=d["g"].data_ptr(),
                        beta=d["beta"].data_ptr(), h0=d["h0"].data_ptr(), cu_seqlens=cu.data_ptr(), o=o.data_ptr(),
-                       ht=ht.data_ptr(), tokens=tokens, N=N, H=H, K=K, V=V, io_dtype=_lib.KDA_BF16, use_qk_l2norm=int(l2),
+                       ht=ht.data_ptr(), tokens=tokens, N=N, H=H, K=128, V=128, k_cols=K % 128, v_cols=V % 128, io_dtype=_lib.KDA_BF16, use_qk_l2norm=int(l2),
                        save_for_backward=save, scale=K ** -0.5, HQ=d["q"].shape[-2])
     if noalloc:
         rc = lib.kda_chunk_fwd_noalloc(C.byref(a), st)

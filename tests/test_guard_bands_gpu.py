@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from kda_b200.inputs import make_inputs
-from _abi import Guarded, chunk_fwd_bwd_guarded
+from _abi import Guarded, bulk_decode_batch, chunk_fwd_bwd_guarded
 
 pytestmark = pytest.mark.gpu
 
@@ -38,6 +38,23 @@ def test_chunk_fwd_bwd_stays_inside_its_buffers(lens, l2):
         assert torch.equal(got[n].view(ref[n].shape), ref[n]), n
 
 
+@pytest.mark.parametrize("lens,K,V,l2", [([64], 64, 64, False), ([130, 1, 64, 77], 96, 32, True), ([65], 8, 8, False), ([5, 200, 64], 128, 72, True),
+                                          ([192, 70], 40, 128, False)])
+def test_narrow_heads_stay_inside_their_buffers(lens, K, V, l2):
+    """Rows of fewer than 128 columns are read and written in place: a tile is wider than the row, and the columns of the neighbouring heads and
+    the margins of every buffer must stay as they are."""
+    tokens, N = sum(lens), len(lens)
+    d = make_inputs(1, tokens, 3, K, V, torch.bfloat16, seed=550 + tokens, h0_std=0.02, n_states=N, backward=True)
+    d = {n: t.cuda().contiguous() for n, t in d.items()}
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device="cuda")
+    got, guards = chunk_fwd_bwd_guarded(d, cu, l2=l2)
+    for name, g in guards:
+        assert g.margins_intact(), name
+    ref = _ordinary(d, cu, l2=l2)
+    for n in ref:
+        assert torch.equal(got[n].view(ref[n].shape), ref[n]), n
+
+
 @pytest.mark.parametrize("lens", [[1], [65], [70, 3, 129]])
 def test_noalloc_forward_stays_inside_its_buffers(lens):
     tokens, N = sum(lens), len(lens)
@@ -51,13 +68,14 @@ def test_noalloc_forward_stays_inside_its_buffers(lens):
     assert torch.equal(got["o"].view(ref["o"].shape), ref["o"]) and torch.equal(got["ht"], ref["ht"])
 
 
-@pytest.mark.parametrize("N,H,slots", [(3, 2, False), (40, 16, False), (40, 16, True), (5, 3, True)])
+@pytest.mark.parametrize("N,H,slots", [(3, 2, False), (40, 16, False), (40, 16, True), (5, 3, True), (0, 0, False), (0, 0, True)])
 def test_decode_stays_inside_its_buffers(N, H, slots):
-    """One decode step with the output and the state pool between sentinel margins: the per-warp kernel (few units)
-    and the bulk-copy kernel (640 units), with and without a state-slot table."""
+    """One decode step with the output and the state pool between sentinel margins: the per-warp kernel (up to 640 states)
+    and the whole-state bulk-copy kernel (0, 0: its smallest batch), with and without a state-slot table."""
     from kda_b200 import _lib, fused_recurrent_kda_fwd
-    d = make_inputs(N, 1, H, 128, 128, torch.bfloat16, seed=700 + N, h0_std=0.05)
-    c = {n: t.cuda() for n, t in d.items() if t is not None}
+    if N == 0:
+        N, H = bulk_decode_batch()
+    c = make_inputs(N, 1, H, 128, 128, torch.bfloat16, seed=700 + N, h0_std=0.05, device="cuda", generate_on_device=True)
     extra = 4 if slots else 0
     gpool = Guarded((N + extra) * H * 128 * 128 * 4)
     pool = gpool.view(torch.float32, (N + extra, H, 128, 128))
@@ -123,3 +141,26 @@ def test_fp32_recurrent_backward_stays_inside_its_buffers(lens, K, V):
     assert lib.kda_recurrent_bwd(C.byref(a), None) == -2
     a.K, a.workspace_bytes = K, 16
     assert lib.kda_recurrent_bwd(C.byref(a), None) == -5
+
+
+@pytest.mark.parametrize("tr", [False, True])
+def test_draft_tokens_stay_inside_their_buffers(tr):
+    """Several tokens with a slot each on half states: the pool's margins, the slots nobody owns and the output's margins stay as they are."""
+    from kda_b200 import _lib, fused_recurrent_kda_fwd
+    N, T, H = 24, 3, 16
+    c = make_inputs(N, T, H, 128, 128, torch.bfloat16, seed=731, h0_std=0.05, device="cuda", generate_on_device=True)
+    gpool, go = Guarded((N * T + 3) * H * 128 * 128 * 4), Guarded(N * T * H * 128 * 2)
+    pool, out = gpool.view(torch.float32, (N * T + 3, H, 128, 128)), go.view(torch.bfloat16, (N, T, H, 128))
+    slots = torch.randperm(N * T + 3, device="cuda")[:N * T].to(torch.int32).view(N, T)
+    pool.fill_(3.0)
+    pool[slots[:, 0].long()] = c["h0"]
+    plain = pool.clone()
+    args = (c["q"], c["k"], c["v"], c["g"], c["beta"])
+    fused_recurrent_kda_fwd(*args, initial_state=pool, ssm_state_indices=slots, out=out, transpose_state_layout=tr)
+    o_ref, _ = fused_recurrent_kda_fwd(*args, initial_state=plain, ssm_state_indices=slots, transpose_state_layout=tr)
+    torch.cuda.synchronize()
+    assert _lib.recurrent_status() == 0
+    assert gpool.margins_intact() and go.margins_intact()
+    assert torch.equal(out, o_ref) and torch.equal(pool, plain)
+    rest = sorted(set(range(N * T + 3)) - set(slots.flatten().tolist()))
+    assert all(bool((pool[i] == 3.0).all()) for i in rest)

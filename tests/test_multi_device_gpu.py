@@ -4,9 +4,15 @@ peer access, no collective."""
 import pytest
 import torch
 
+from _abi import bulk_decode_batch
 from kda_b200.inputs import make_inputs
 
 pytestmark = pytest.mark.gpu
+
+
+def _decode_batch():
+    N, H = bulk_decode_batch()
+    return N, 1, H
 
 
 def _step(d, dev):
@@ -17,10 +23,14 @@ def _step(d, dev):
                       use_qk_l2norm_in_kernel=True)
     torch.autograd.backward([o, ht], [c["do"], c["dht"]])
     outs = [o.detach(), ht.detach()] + [lv[n].grad for n in ("q", "k", "v", "g", "beta", "h0")]
-    # a bulk decode step: 640 (sequence, head) units, one token each
-    e = {n: t.to(dev) for n, t in make_inputs(40, 1, 16, 128, 128, torch.bfloat16, seed=9, h0_std=0.05).items() if t is not None}
+    # decode steps: whole states (32 per SM, one token each) and half states (several tokens with a slot each) on the bulk-copy kernel
+    e = {n: t.to(dev) for n, t in make_inputs(*_decode_batch(), 128, 128, torch.bfloat16, seed=9, h0_std=0.05).items() if t is not None}
     state = e["h0"].clone()
     od, _ = fused_recurrent_kda_fwd(e["q"], e["k"], e["v"], e["g"], e["beta"], scale=0.1, initial_state=state, inplace_final_state=True)
+    e = {n: t.to(dev) for n, t in make_inputs(12, 3, 16, 128, 128, torch.bfloat16, seed=11, h0_std=0.05).items() if t is not None}
+    pool = e["h0"].repeat_interleave(3, 0)
+    of, _ = fused_recurrent_kda_fwd(e["q"], e["k"], e["v"], e["g"], e["beta"], initial_state=pool,
+                                    ssm_state_indices=torch.arange(36, dtype=torch.int32, device=dev).view(12, 3))
     # the bounded-gate variant of the forward and the float32 training path have kernels (and attributes) of their own
     with torch.no_grad():
         gs = -5.0 * torch.sigmoid(c["g"])
@@ -31,7 +41,7 @@ def _step(d, dev):
     torch.autograd.backward([o32, ht32], [f["do"], f["dht"]])
     outs += [o_safe, o32.detach(), lf["q"].grad, lf["g"].grad, lf["h0"].grad]
     torch.cuda.synchronize(dev)
-    return [t.cpu() for t in outs + [od, state]]
+    return [t.cpu() for t in outs + [od, state, of, pool]]
 
 
 def test_same_bits_on_a_second_device():

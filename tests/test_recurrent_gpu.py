@@ -3,6 +3,7 @@ import numpy as np
 import pytest
 import torch
 
+from _abi import bulk_decode_batch
 from kda_b200.inputs import make_inputs, make_workload
 from oracle.kda_oracle import cosine, max_norm_err, recurrent_kda
 
@@ -79,17 +80,18 @@ def test_decode_inplace_steps_match_scan():
     assert torch.count_nonzero(pool[1]) == 0 and torch.count_nonzero(pool[3]) == 0
 
 
-@pytest.mark.parametrize("case", ["plain", "l2norm_slots_gva", "fp32", "transposed", "transposed_l2norm_slots_gva"])
-def test_large_decode_batch_bulk_copy_kernel(case):
-    """640 (sequence, head) units with one token each: the step runs on the kernel that moves whole state tiles with the
-    bulk-copy engine (at least four units per SM).  o and the new states against the float64 oracle: bf16 o 2e-2,
+@pytest.mark.parametrize("bulk", [False, True])
+@pytest.mark.parametrize("case", ["plain", "l2norm_slots_gva", "fp32", "transposed", "transposed_l2norm_slots_gva", "fp32_transposed"])
+def test_large_decode_batch_bulk_copy_kernel(case, bulk):
+    """One token each: 640 (sequence, head) units on the per-warp kernels, and the smallest batch that runs on the kernel that moves whole states
+    with the bulk-copy engine (32 units per SM).  o and the new states against the float64 oracle: bf16 o 2e-2,
     fp32 o and the fp32 states 1e-4 (max-normalised); untouched slots stay untouched; the status word stays 0."""
     from kda_b200 import _lib, fused_recurrent_kda_fwd
-    N, H = 40, 16
-    dtype = torch.float32 if case == "fp32" else torch.bfloat16
-    d = make_inputs(N, 1, H, 128, 128, dtype, seed=21, h0_std=0.05)
+    N, H = bulk_decode_batch() if bulk else (40, 16)
+    dtype = torch.float32 if case.startswith("fp32") else torch.bfloat16
+    d = make_inputs(N, 1, H, 128, 128, dtype, seed=21, h0_std=0.05, device="cuda", generate_on_device=True)
     l2 = case.endswith("l2norm_slots_gva")
-    tr = case.startswith("transposed")          # states [.., V, K]
+    tr = "transposed" in case          # states [.., V, K]
     HQ = 4 if l2 else H
     q, k = d["q"][:, :, :HQ].contiguous(), d["k"][:, :, :HQ].contiguous()
     if l2:
@@ -119,19 +121,19 @@ def test_large_decode_batch_bulk_copy_kernel(case):
     if tr:
         ht = ht.transpose(-1, -2)
     assert _lib.recurrent_status() == 0
-    assert max_norm_err(o, o_ref) <= (1e-4 if case == "fp32" else 2e-2) and cosine(o, o_ref) >= 0.9999
+    assert max_norm_err(o, o_ref) <= (1e-4 if case.startswith("fp32") else 2e-2) and cosine(o, o_ref) >= 0.9999
     assert max_norm_err(ht, h_ref) <= 1e-4
 
 
 @pytest.mark.captures_graph
-@pytest.mark.parametrize("N", [4, 40])
+@pytest.mark.parametrize("N", [4, 40, "bulk"])
 def test_decode_step_replays_from_a_cuda_graph(N):
     """Serving loops capture the decode step in a CUDA graph: the C entry point makes no synchronising call and takes the
-    capturing stream, so a captured in-place step (per-warp kernel for N = 4, bulk-copy kernel for N = 40) replays to the
+    capturing stream, so a captured in-place step (per-warp kernel for N = 4 and 40, bulk-copy kernel for its smallest batch) replays to the
     same states and outputs as eager calls, bit for bit."""
     from kda_b200 import fused_recurrent_kda_fwd
-    H = 16
-    c = _cuda(make_inputs(N, 1, H, 128, 128, torch.bfloat16, seed=31, h0_std=0.05))
+    N, H = bulk_decode_batch() if N == "bulk" else (N, 16)
+    c = make_inputs(N, 1, H, 128, 128, torch.bfloat16, seed=31, h0_std=0.05, device="cuda", generate_on_device=True)
     args = (c["q"], c["k"], c["v"], c["g"], c["beta"])
     eager_state, graph_state, scratch = c["h0"].clone(), c["h0"].clone(), c["h0"].clone()
     side = torch.cuda.Stream()
@@ -150,20 +152,21 @@ def test_decode_step_replays_from_a_cuda_graph(N):
         assert torch.equal(graph_state, eager_state), step
 
 
-@pytest.mark.parametrize("N,tr,lb", [(3, False, None), (3, True, -5.0), (40, False, -5.0), (40, True, None)])
+@pytest.mark.parametrize("N,tr,lb", [(3, False, None), (3, True, -5.0), (40, False, -5.0), (40, True, None), ("bulk", False, -5.0), ("bulk", False, None),
+                                     ("bulk", True, -5.0), ("bulk", True, None)])
 def test_decode_with_the_gate_front_end_in_kernel(N, tr, lb):
     """The layer's decode call (fla/layers/kda.py:282-296): raw bf16 gate input with A_log, dt_bias (optionally the
     lower-bound form), beta logits, l2norm -- all inside the recurrent kernel, no pass over g and beta in front of it.
-    Per-warp kernels (N = 3) and bulk-copy kernel (N = 40), both state layouts; o 2e-2, states 1e-4 against the oracle."""
+    Per-warp kernels (N = 3, 40) and bulk-copy kernel (its smallest batch), both state layouts; o 2e-2, states 1e-4 against the oracle."""
     from kda_b200 import fused_recurrent_kda
     from oracle.kda_oracle import beta_sigmoid, kda_gate
-    H = 16
-    d = make_inputs(N, 1, H, 128, 128, torch.bfloat16, seed=33, h0_std=0.05)
-    gen = torch.Generator().manual_seed(34)
-    g_raw = torch.randn(N, 1, H, 128, generator=gen).bfloat16()
-    beta_raw = torch.randn(N, 1, H, generator=gen).bfloat16()
-    A_log = torch.log(torch.empty(H).uniform_(1, 16, generator=gen))
-    dt_bias = torch.randn(H * 128, generator=gen) * 0.5
+    N, H = bulk_decode_batch() if N == "bulk" else (N, 16)
+    d = make_inputs(N, 1, H, 128, 128, torch.bfloat16, seed=33, h0_std=0.05, device="cuda", generate_on_device=True)
+    gen = torch.Generator(device="cuda").manual_seed(34)
+    g_raw = torch.randn(N, 1, H, 128, generator=gen, device="cuda").bfloat16()
+    beta_raw = torch.randn(N, 1, H, generator=gen, device="cuda").bfloat16()
+    A_log = torch.log(torch.empty(H, device="cuda").uniform_(1, 16, generator=gen))
+    dt_bias = torch.randn(H * 128, generator=gen, device="cuda") * 0.5
     o_ref, h_ref = recurrent_kda(d["q"], d["k"], d["v"], kda_gate(g_raw, A_log, dt_bias, lower_bound=lb), beta_sigmoid(beta_raw),
                                  initial_state=d["h0"], output_final_state=True, use_qk_l2norm=True)
     h0 = d["h0"].cuda()
@@ -324,3 +327,32 @@ def test_a_slot_named_by_several_tokens_keeps_the_last_state(N, T, H, tr, patter
             _, h_ref = recurrent_kda(*(d[n][:, :last + 1] for n in ("q", "k", "v", "g", "beta")), initial_state=d["h0"], output_final_state=True)
             got = pool[slots[:, last].long()]
             assert max_norm_err(got.transpose(-1, -2) if tr else got, h_ref) <= 1e-4, (w, last)
+
+
+@pytest.mark.parametrize("dtype,tr,lb,HQ", [(torch.bfloat16, False, None, 16), (torch.bfloat16, False, -5.0, 4), (torch.bfloat16, True, None, 4),
+                                            (torch.float32, False, -5.0, 16), (torch.float32, True, None, 16)])
+def test_draft_tokens_with_the_gate_front_end(dtype, tr, lb, HQ):
+    """The layer's draft-token call on half states: raw gate, beta logits, L2 norm, grouped value heads, bounded gates, both layouts and types.  o and
+    the state behind every token against the float64 oracle."""
+    from kda_b200 import _lib, fused_recurrent_kda_fwd
+    from oracle.kda_oracle import beta_sigmoid, kda_gate
+    N, T, H = 12, 3, 16
+    d = make_inputs(N, T, H, 128, 128, dtype, seed=90, h0_std=0.05, device="cuda", generate_on_device=True)
+    q, k = d["q"][:, :, :HQ].contiguous() * 2, d["k"][:, :, :HQ].contiguous()
+    g_raw, beta_raw = torch.randn_like(d["g"]).to(dtype), torch.randn_like(d["beta"]).to(dtype)
+    A_log, dt_bias = torch.rand(H, device="cuda"), torch.randn(H * 128, device="cuda") * 0.5
+    slots = torch.randperm(N * T, device="cuda").to(torch.int32).view(N, T)
+    pool = torch.zeros(N * T, H, 128, 128, device="cuda")
+    pool[slots[:, 0].long()] = d["h0"].transpose(-1, -2) if tr else d["h0"]
+    o, _ = fused_recurrent_kda_fwd(q, k, d["v"], g_raw, beta_raw, A_log=A_log, dt_bias=dt_bias, initial_state=pool, ssm_state_indices=slots,
+                                   use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True, use_beta_sigmoid_in_kernel=True, lower_bound=lb,
+                                   transpose_state_layout=tr)
+    assert _lib.recurrent_status() == 0
+    wide = lambda t: t.repeat_interleave(H // HQ, 2)      # noqa: E731
+    g, beta = kda_gate(g_raw, A_log, dt_bias, lower_bound=lb), beta_sigmoid(beta_raw)
+    for t in range(T):
+        o_ref, h_ref = recurrent_kda(*(x[:, :t + 1] for x in (wide(q), wide(k), d["v"], g, beta)), initial_state=d["h0"], output_final_state=True,
+                                     use_qk_l2norm=True)
+        got = pool[slots[:, t].long()]
+        assert max_norm_err(got.transpose(-1, -2) if tr else got, h_ref) <= 1e-4, t
+    assert max_norm_err(o, o_ref) <= (1e-4 if dtype == torch.float32 else 2e-2) and cosine(o, o_ref) >= 0.9999
