@@ -138,8 +138,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
 }
 // Give-up path, one thread: waits (bounded, some ten milliseconds a phase) for what may still complete on `bar`, because copies and products in
 // flight must not outlive the CTA's shared memory.  Which phase is open does not matter: the wait for a completed one returns at once.
-// Out of line, so that the loops around it stay as they are.
-static __device__ __noinline__ void mbar_drain(uint64_t* bar) {
+__device__ __forceinline__ void mbar_drain(uint64_t* bar) {
   for (unsigned parity = 0; parity < 2; ++parity)
     for (int i = 0; i < 4096 && !mbar_try_wait(bar, parity); ++i) __nanosleep(64);
 }
