@@ -69,17 +69,6 @@ constexpr int C_DQG = 0, C_DKG = 64, C_DW = 128 /* later dbk^T */, C_DAQ = 192 /
               C_XY = 320, C_DBV = 384 /* later Cq */, C_CP = 448;
 constexpr int C_CQ = C_DBV, C_CN = C_DAQ, C_DBK = C_DW;
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-  float a[16], b[16];
-  umma::tmem_ld16(taddr, a);
-  umma::tmem_ld16(taddr + 16, b);
-  umma::tmem_ld_wait();
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    v[i] = a[i];
-    v[16 + i] = b[i];
-  }
-}
 // eight floats -> one 16-byte piece of bf16
 __device__ __forceinline__ uint4 pack8(const float* v) {
   return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
@@ -241,7 +230,6 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     ci.tok0 = static_cast<int>(s.ci_tok0[it & 1]);
     ci.len = s.ci_len[it & 1];
     const int len = ci.len;
-    const size_t tile = static_cast<size_t>(idx);
     const int next_idx = idx + gridDim.x;
     long long* const dbg = (it == 2) ? p.dbg : nullptr;   // development aid: clocks of a steady-state tile
 

@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
   if (tid < C) {
     float b = __uint_as_float(beta_bits);
     if (p.beta_raw && tid < len) {
-      b = sigmoidf_(b);
+      b = sigmoid_fast(b);
       if (p.beta_out) p.beta_out[static_cast<size_t>(ci.tok0 + tid) * p.H + h] = b;
     }
     s.beta[tid] = b;
@@ -587,7 +587,7 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
       float s0 = 0.f, s1 = 0.f;
 #pragma unroll
       for (int m = 0; m < i; m += 4) {
-        const float4 a = *reinterpret_cast<const float4*>(&A[i * AS + m]);      // entries at and above the diagonal are zero
+        const float4 a = *reinterpret_cast<const float4*>(&A[i * AS + m]);      // entries at and above the diagonal are undefined (nothing writes them) and not used
         s0 = fmaf(a.x, x[m], s0);
         if (m + 1 < i) s1 = fmaf(a.y, x[m + 1], s1);
         if (m + 2 < i) s0 = fmaf(a.z, x[m + 2], s0);

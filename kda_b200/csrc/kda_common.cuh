@@ -43,13 +43,14 @@ __device__ __forceinline__ float warp_sum(float x) {
   return x;
 }
 
-// ---- gate front end of the recurrent kernels: activated log-decay and beta from the raw layer outputs -------------
+// ---- the gate's activations (gate kernels, preparation, recurrent kernels: the same values from each) --------------
 __device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 // softplus(x) = log(1 + e^x); identity above 20; below -15 the sum would round e^x away and log(1 + e) = e to fp32 accuracy
 __device__ __forceinline__ float softplus_fast(float x) {
   const float e = __expf(fminf(x, 20.f));
   return x > 20.f ? x : (x < -15.f ? e : __logf(1.f + e));
 }
+// ---- gate front end of the recurrent kernels: activated log-decay and beta from the raw layer outputs -------------
 __device__ __forceinline__ float load_raw(const void* p, size_t i, int dtype) {      // dtype: KDA_BF16 or KDA_FP32
   return dtype == KDA_BF16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]) : static_cast<const float*>(p)[i];
 }
@@ -165,12 +166,7 @@ __device__ __forceinline__ void bulk_wait() {
   asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// ---- Ampere-style 16-byte async copies for strided rows ------------------------------------------
-__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src_gmem, bool valid) {
-  const unsigned sz = valid ? 16u : 0u;   // src-size 0 -> destination is zero-filled
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst_smem)), "l"(src_gmem), "r"(sz)
-               : "memory");
-}
+// ---- Ampere-style async copies for strided elements ----------------------------------------------
 __device__ __forceinline__ void cp_async4(void* dst_smem, const void* src_gmem, bool valid) {
   const unsigned sz = valid ? 4u : 0u;
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst_smem)), "l"(src_gmem), "r"(sz) : "memory");

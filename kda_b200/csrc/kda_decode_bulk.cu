@@ -5,8 +5,8 @@
 // waits for slot numbers, so that the loads of the next unit and the stores of the last tokens are in flight beside the arithmetic.
 // HV = 64, two persistent CTAs per SM, for several tokens per sequence: the two CTAs of an SM fill each other's waits and the last round of
 // units is shorter (24 sequences x 4 tokens x 32 heads: 47.7 us, whole states 59.9).  HV = 128, one CTA per SM, for one token: contiguous
-// 64 KiB copies, which DRAM likes better (1,024 sequences x 32 heads: 670 us = 0.98 of the measured copy rate, half states 692).
-// Whatever a warp does between a unit's arrival and its store adds to every unit: o leaves behind the hand-over (in front of it: 674).
+// 64 KiB copies, which DRAM likes better (1,024 sequences x 32 heads: 657 to 662 us = the measured copy rate, half states 692).
+// Whatever a warp does between a unit's arrival and its store adds to every unit: o leaves behind the hand-over (in front of it 4 us more).
 // Per token (order as in fla/ops/kda/fused_recurrent.py:146-192): S *= exp(g); v' = beta (v - S^T k);
 // S += k v'^T; o = scale S^T q.
 #include <algorithm>
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(HV * 2 + 32, 128 / HV) kda_decode_bulk_kernel(
         const int other = last == x ? y : x;      // its store, if any, has been read: every store but the last one has
         if (more) {
           // whole states: the load waits until the store has left shared memory.  Loads issued earlier mix with the stores in DRAM
-          // (1,024 sequences x 32 heads: 692 us issued in front of the store, 663..667 right behind it, 661 so)
+          // (1,024 sequences x 32 heads, the variant without gates: 692 us issued in front of the store, 663..668 right behind it or so)
           if constexpr (HV == DV) bulk_wait_read<0>();
           load(lslot, ahead.h, other);
         }

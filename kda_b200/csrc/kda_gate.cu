@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(GATE_THREADS) kda_gate_fwd_kernel(const T* __r
         for (int e = 0; e < 8; ++e) x[u][e] += b[e];
       }
 #pragma unroll
-      for (int e = 0; e < 8; ++e) x[u][e] = use_lb ? lb * sigmoidf_(a * x[u][e]) : -a * softplusf_(x[u][e]);
+      for (int e = 0; e < 8; ++e) x[u][e] = use_lb ? lb * sigmoid_fast(a * x[u][e]) : -a * softplus_fast(x[u][e]);
       store8(g + i * 8, x[u]);
     }
   }
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(GATE_THREADS) kda_beta_sigmoid_fwd_kernel(cons
                                                                             long long n) {
   for (long long i = static_cast<long long>(blockIdx.x) * GATE_THREADS + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * GATE_THREADS)
-    beta[i] = sigmoidf_(load1(beta_raw + i));
+    beta[i] = sigmoid_fast(load1(beta_raw + i));
 }
 
 // ---- backward: CTA (cb, rb) owns 256 groups of eight columns and the token rows rb, rb + nblk, ...; two rows per
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(GATE_BWD_THREADS, 3) kda_gate_bwd_kernel(const
         const float xe = x[u][e] + b[e];
         float dx;
         if (use_lb) {
-          const float sg = sigmoidf_(a * xe);
+          const float sg = sigmoid_fast(a * xe);
           dx = d[u][e] * lb * sg * (1.f - sg) * a;    // d/dx of lb sigmoid(a x);  d/dA_log = dx * x
           sA = fmaf(dx, xe, sA);
         } else {
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(GATE_THREADS) kda_gate_bwd_finish_kernel(const
   }
   const int rest = gridDim.x - cols - heads;
   for (long long i = static_cast<long long>(blockIdx.x - cols - heads) * GATE_THREADS + threadIdx.x; i < nb; i += static_cast<long long>(rest) * GATE_THREADS) {
-    const float b = sigmoidf_(load1(beta_raw + i));
+    const float b = sigmoid_fast(load1(beta_raw + i));
     store1(dbeta_raw + i, dbeta[i] * b * (1.f - b));
   }
 }

@@ -1,5 +1,5 @@
 """GPU parity of the bf16 chunked path for head sizes below 128 (fla allows any K <= 256,
-fla/ops/kda/chunk.py:376-384): the operator pads key and value channels to the kernels' 128 with zeros, which must leave
+fla/ops/kda/chunk.py:376-384): the kernels' tiles are 128 columns wide and the missing columns count as zeros, which must leave
 o, the states and every gradient those of the unpadded problem -- checked against float64 autograd through the
 token-by-token oracle at the real head sizes."""
 import numpy as np
