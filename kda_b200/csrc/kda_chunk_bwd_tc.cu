@@ -57,7 +57,7 @@ struct TcSmem {
     };
   };
   float carry[4][KD];           // block totals of the reverse cumsum
-  uint64_t barS, barG, barQ, barB, barM;
+  uint64_t barS, barG, barQ, barB, barM;      // (in this order: drained together)
   long long ci_tok0[2];         // first token and length of the chunk of the current / next tile (written by thread 0)
   int ci_len[2];
   uint32_t tmem_slot;
@@ -933,13 +933,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
   }
 
   // drain: a copy that is still in flight must not outlive the CTA's shared memory
-  if (!alive && lane == 0) {      // a wait gave up: loads and products may be under way on any of the barriers
-    if (warp_u == 0) mbar_drain(&s.barM);
-    if (warp_u == 1) mbar_drain(&s.barS);
-    if (warp_u == 2) mbar_drain(&s.barG);
-    if (warp_u == 3) mbar_drain(&s.barQ);
-    if (warp_u == 4) mbar_drain(&s.barB);
-  }
+  if (!alive && lane == 0 && warp_u < 5) mbar_drain(&s.barS + warp_u);      // a wait gave up: loads and products may be under way on any of the five barriers
   bulk_wait<0>();      // stores
   cp_async_wait<0>();
   umma::fence_before_sync();
