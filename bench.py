@@ -219,7 +219,7 @@ def make_step(workload: str, x: dict, cu, gate: bool = False, l2: bool = False, 
             grads = torch.autograd.grad([o, ht], leaves, [x["do"], x["dht"]])
             return (o, ht) + tuple(grads)
         if x["q"].dtype == torch.float32:
-            return step, 3, grad_names                    # token-recurrent forward, backward, its finishing kernel
+            return step, 3 + bool(l2), grad_names           # forward walk; backward walk, middle, the normalisation's backward
         # prepare, scan, reverse scan, main; packed sequences: + the tables; gate: + its backward and the reduction
         return step, 4 + (cu is not None) + (2 if gate else 0), grad_names
 
@@ -611,10 +611,10 @@ def main():
             # step against the operator-boundary bytes (all tensors float32)
             io = 4 * (3 * 128 + 2 * 128 + 1) + (4 * (4 * 128 + 2 * 128 + 1) if w.backward else 0)
             ach = io * th / (ms_step * 1e-3) / 1e9
-            roof = {"kernel": "kda_recurrent_kernel" + (" + kda_recurrent_bwd_kernel" if w.backward else ""), "bound": "hbm",
+            roof = {"kernel": "kda_recurrent_walk_kernel x 2 + kda_recurrent_mid_kernel" if w.backward else "kda_recurrent_kernel", "bound": "hbm",
                     "achieved": ach, "peak": peaks["hbm"], "unit": "GB/s", "frac": ach / peaks["hbm"], "traffic": None,
                     "peak_source": peaks["src"], "algorithmic_bytes_per_launch": io * th,
-                    "note": "exact fp32 path: one warp (forward) or CTA (backward) per (sequence, head), token-serial; not HBM-bound"}
+                    "note": "exact fp32 path: token-serial walks over independent state columns, 32-token pieces between them; FP32 pipe, not HBM"}
     if roof is None:
         fl, by, design = KERNEL_WORK[dom]
         sec = kernels[dom]["ms_per_launch"] * 1e-3

@@ -143,10 +143,19 @@ typedef struct kda_recurrent_bwd_args {
   float scale;
 } kda_recurrent_bwd_args;
 
-/* Scratch for kda_recurrent_bwd: per-value-head dq, dk, the state at the start of every 64-token chunk
- * ((tokens / 64 + N + 1) x H x K x V x 4 bytes) and the per-token states of the chunks in flight. */
+/* Scratch for kda_recurrent_bwd: per-value-head dq, dk, the state and its gradient every 32 tokens
+ * (2 x (tokens / 32 + N) x H x K x V x 4 bytes), and one row per token. */
 size_t kda_recurrent_bwd_workspace_bytes(int64_t tokens, int32_t N, int32_t H, int32_t K, int32_t V);
 int kda_recurrent_bwd(const kda_recurrent_bwd_args* args, void* stream);
+
+/* The same pair for a caller that runs the forward anyway: kda_recurrent_train_fwd is kda_recurrent_fwd for fp32, K, V in {32, 64, 128},
+ * whole sequences, activated g and beta, [K, V] states and ht != h0 (KDA_E_SHAPE otherwise), and leaves in `saved` (256-byte
+ * aligned, kda_recurrent_saved_bytes(..)) what kda_recurrent_train_bwd, called with the same tensors, then need not compute
+ * again.  `saved` is only read by the backward; its results are those of kda_recurrent_bwd, bit for bit, and its workspace
+ * needs only kda_recurrent_bwd_workspace_bytes(..) - kda_recurrent_saved_bytes(..). */
+size_t kda_recurrent_saved_bytes(int64_t tokens, int32_t N, int32_t H, int32_t K, int32_t V);
+int kda_recurrent_train_fwd(const kda_recurrent_args* args, void* saved, size_t saved_bytes, void* stream);
+int kda_recurrent_train_bwd(const kda_recurrent_bwd_args* args, const void* saved, size_t saved_bytes, void* stream);
 
 /* ------------------------------------------------------------------------------------------------
  * Chunked forward / backward (chunk = 64 tokens), bf16 tensor-core path, K = V = 128 (narrower rows: k_cols, v_cols).

@@ -23,6 +23,7 @@
 // of cumulative sums and row references, 256 threads: 1.98).  Bounded gates at 1 x 32768 x 32: 0.74 ms with the gate's activation.  Without the
 // L2 prefetch of the next wave's rows 1.65, two waves ahead 1.59.
 #include "kda_device.cuh"
+#include "kda_f32x2.cuh"
 #include "kda_gate.cuh"
 #include "kda_prepare.cuh"
 
@@ -89,29 +90,7 @@ __device__ __forceinline__ float butterfly(float (&v)[N], int lane) {
   return v[0];
 }
 
-// Four adjacent key columns in fp32, as two packed pairs (sm_100 multiplies a pair in one instruction).
-using f32x2 = unsigned long long;
-struct F4 { f32x2 a, b; };
-__device__ __forceinline__ f32x2 pair(float x, float y) {
-  f32x2 d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
-  return d;
-}
-__device__ __forceinline__ float2 halves(f32x2 v) {
-  float2 d;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(v));
-  return d;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
+// Four adjacent key columns in fp32: F4.
 __device__ __forceinline__ F4 mul4c(const F4& x, const F4& y) { return {mul2(x.a, y.a), mul2(x.b, y.b)}; }
 __device__ __forceinline__ f32x2 widen2(uint32_t u) {      // two bf16 -> two fp32
   f32x2 d;
@@ -124,11 +103,6 @@ __device__ __forceinline__ uint32_t narrow2(f32x2 v) {
 }
 __device__ __forceinline__ F4 widen(const uint2 u) { return {widen2(u.x), widen2(u.y)}; }
 __device__ __forceinline__ uint2 narrow(const F4& x) { return make_uint2(narrow2(x.a), narrow2(x.b)); }
-__device__ __forceinline__ F4 lds4(const float* p) {
-  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
-  return {v.x, v.y};
-}
-__device__ __forceinline__ void sts4(float* p, const F4& x) { *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(x.a, x.b); }
 __device__ __forceinline__ F4 splat(float x) { return {pair(x, x), pair(x, x)}; }
 __device__ __forceinline__ float dot(const F4& x, const F4& y) {
   const float2 v = halves(fma2(x.b, y.b, mul2(x.a, y.a)));

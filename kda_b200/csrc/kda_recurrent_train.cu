@@ -1,0 +1,893 @@
+// Token-recurrent KDA training in fp32 (K, V in {32, 64, 128}): forward that keeps what the backward needs, and its exact reverse mode.
+// The recurrence of fla/ops/kda/naive.py:12-66,
+//
+//   S' = Diag(exp g_t) S_{t-1};   r = v - S'^T k;   w = beta_t r;   S_t = S' + k w^T;   o_t = scale S_t^T q_t,
+//
+// differentiated step by step, with no chunk formula in between (those lose dg to cancellation: 3e-6 against 1.4e-7):
+//
+//   dS += scale q do^T;  dq^ = scale S_t do;  dw = dS^T k;  dk^ = dS w - S' (beta dw);  dbeta = <dw, r>;
+//   dv = beta dw;  dS' = dS - k (beta dw)^T;  dg = rowsum(dS' . S');  dS <- Diag(exp g) dS'.
+//
+// Only two chains run through a whole sequence, and both fall apart into the state's columns: S forward (its sums run over k) and dS
+// backward (needs q, k, g, beta, do, but no S).  So three kernels:
+//   walk forward    S alone.  Leaves the state at the start of every 32 tokens and r of every token.
+//   walk backward   dS alone.  Leaves dS at the end of every 32 tokens, dv, and dbeta summed over 16 columns.
+//   middle          every (32 tokens, 32 rows of the state) on its own.  With r and beta dw known a step needs no sum over k: S and dS of
+//                   a row follow from that row's q, k, g, and its dq^, dk^, dg are sums along the row.
+// Walks: a warp holds 16 or 32 columns of all K rows (a lane 16 rows x 4 or 8 columns, packed two rows to a register pair), and nothing is
+// shared between warps but the staged q, k, exp g.
+// Middle: a thread holds 8 columns of 4 rows of S and dS.  S' of four tokens lives in registers; states in between are replayed from the
+// state at every eighth token in shared memory: 11.5 multiply-adds per element and token instead of 9, and no per-token state through memory
+// (128 KB per token: what a CTA per sequence waited for).  The tile's shape is set by shared-memory bandwidth, which is 128 bytes per cycle
+// delivered to registers, broadcast or not: with 16 columns of one row a thread read 90 floats per 16 elements and token (92 % of the LSU's rate,
+// 7.5 ms), with 4 x 8 it reads 36 (5.9 ms).
+// What bounds them: the FP32 pipe (60 % busy; one CTA's load of its rows and states under the other's arithmetic) and, in the walks,
+// the 256 units' uneven share of 148 SMs.  8 x 2048 tokens x 32 heads of 128: forward walk 2.14, backward walk 2.11, middle 5.0 ms; 25.7 ms for
+// the whole step as a CTA per sequence -> 9.3.  One sequence x 32 heads: 12.8 -> 2.4 ms; 2 x 200 tokens x 8 heads: 1.23 -> 0.24.
+// dq^, dk^ (gradients w.r.t. the possibly L2-normalised rows, per VALUE head) go to the workspace; a last kernel sums grouped value
+// heads, applies the normalisation's backward (fla/modules/l2norm.py:190-240) and writes dq, dk; with neither they are dq, dk.  Every sum has a
+// fixed order.
+#include <algorithm>
+
+#include "kda_common.cuh"
+#include "kda_device.cuh"
+#include "kda_f32x2.cuh"
+
+namespace kda {
+
+namespace {
+
+constexpr int TC = 32;      // tokens between two kept states
+constexpr int TS = 8;       // tokens staged at a time in the walks (TC is a multiple)
+
+struct TrainParams {
+  const float *q, *k, *v, *g, *beta, *h0, *d_o, *d_ht;
+  const int32_t* cu;
+  float *o, *ht;
+  float *dqh, *dkh;            // [tokens, H, K] per value head, w.r.t. the normalised rows
+  float *dv, *dg, *dbeta, *dh0;
+  float *ckpt;                 // [tokens / 32 + N][H][K][V] states at the start of every 32 tokens
+  float *resid;                // [tokens, H, V] r
+  float *norms;                // [tokens, H, 2] reciprocal norms of q, k (only with use_l2)
+  float *dckpt;                // like ckpt: dS at the end of every 32 tokens
+  float *dbp;                  // [tokens, H, V / 16] dbeta over 16 columns
+  long long T, slots;
+  int N, H, HQ, V;
+  int use_l2, wide;            // wide: q, k, g start on 16-byte boundaries
+  float scale, dq_scale;       // dq_scale: what dqh still gets (without grouped heads and norms dqh, dkh are dq, dk themselves)
+};
+
+// first token and length of sequence n; the states of its 32-token pieces start at slot bos / 32 + n (disjoint for any lengths)
+struct Seq { long long bos, len; };
+__device__ __forceinline__ long long seq_start(const TrainParams& p, long long n) { return p.cu ? p.cu[n] : n * p.T; }
+__device__ __forceinline__ Seq sequence(const TrainParams& p, int n) {
+  const long long b = seq_start(p, n);
+  return {b, seq_start(p, n + 1) - b};
+}
+
+__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src_gmem, bool valid) {
+  const unsigned sz = valid ? 16u : 0u;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst_smem)), "l"(src_gmem), "r"(sz) : "memory");
+}
+// 16 bytes of q, k or g, which a caller of the backward may hand over at any 4-byte boundary
+__device__ __forceinline__ void cp_row16(float* dst_smem, const float* src_gmem, int wide) {
+  if (wide) {
+    cp_async16(dst_smem, src_gmem, true);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) cp_async4(dst_smem + e, src_gmem + e, true);
+  }
+}
+// E consecutive floats of a row in shared memory
+template <int E>
+__device__ __forceinline__ void row_get(float (&x)[E], const float* p) {
+  if constexpr (E == 4) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+  } else if constexpr (E == 2) {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    x[0] = v.x; x[1] = v.y;
+  } else {
+    x[0] = *p;
+  }
+}
+template <int E>
+__device__ __forceinline__ void row_put(float* p, const float (&x)[E]) {
+  if constexpr (E == 4) *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
+  else if constexpr (E == 2) *reinterpret_cast<float2*>(p) = make_float2(x[0], x[1]);
+  else *p = x[0];
+}
+__device__ __forceinline__ float dot4(const float4 a, const float4 b) { return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
+
+// ---------------------------------------------------------------------------------------------------------------------
+// the walks
+// ---------------------------------------------------------------------------------------------------------------------
+template <int K, int CPL>
+struct WalkSmem {
+  static constexpr int COLS = CPL * 16;      // a CTA's columns, at most
+  float q[2][TS][K];          // scale * q^
+  float k[2][TS][K];          // k^
+  float a[2][TS][K];          // exp g
+  float x[2][TS][COLS];       // this CTA's columns of v (forward), do (backward)
+  float y[2][TS][COLS];       // of r (backward)
+  float beta[2][TS];
+};
+
+// A warp's share of a [K, V] state, 4 CPL columns: a lane has columns col + 16 m + (0..3), m < CPL / 4, of rows 32 i + 4 rg + (0..3);
+// pairs are two neighbouring rows.
+template <int K, int CPL>
+struct Slice {
+  f32x2 v[K / 32][2][CPL];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int i = 0; i < K / 32; ++i)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) v[i][e][c] = 0ull;
+  }
+  __device__ __forceinline__ void load(const float* base, int rg, int V) {      // base: row 0, column col
+#pragma unroll
+    for (int i = 0; i < K / 32; ++i)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int m = 0; m < CPL / 4; ++m) {
+          const float4 x = *reinterpret_cast<const float4*>(base + static_cast<size_t>(32 * i + 4 * rg + 2 * e) * V + 16 * m);
+          const float4 y = *reinterpret_cast<const float4*>(base + static_cast<size_t>(32 * i + 4 * rg + 2 * e + 1) * V + 16 * m);
+          v[i][e][4 * m] = pair(x.x, y.x); v[i][e][4 * m + 1] = pair(x.y, y.y);
+          v[i][e][4 * m + 2] = pair(x.z, y.z); v[i][e][4 * m + 3] = pair(x.w, y.w);
+        }
+  }
+  __device__ __forceinline__ void store(float* base, int rg, int V) const {
+#pragma unroll
+    for (int i = 0; i < K / 32; ++i)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int m = 0; m < CPL / 4; ++m) {
+          const float2 c0 = halves(v[i][e][4 * m]), c1 = halves(v[i][e][4 * m + 1]), c2 = halves(v[i][e][4 * m + 2]), c3 = halves(v[i][e][4 * m + 3]);
+          *reinterpret_cast<float4*>(base + static_cast<size_t>(32 * i + 4 * rg + 2 * e) * V + 16 * m) = make_float4(c0.x, c1.x, c2.x, c3.x);
+          *reinterpret_cast<float4*>(base + static_cast<size_t>(32 * i + 4 * rg + 2 * e + 1) * V + 16 * m) = make_float4(c0.y, c1.y, c2.y, c3.y);
+        }
+  }
+};
+// sums over the rows of a lane's columns: the pairs' halves, then the eight row groups of the warp (lane bits 2..4); every lane gets all
+template <int CPL, int P>
+__device__ __forceinline__ float row_sum(const f32x2 (&h)[P][CPL], int c) {
+  const float2 x = halves(h[0][c]), y = halves(h[P - 1][c]);
+  return P == 1 ? x.x + x.y : (x.x + x.y) + (y.x + y.y);
+}
+template <int CPL, int P>
+__device__ __forceinline__ void column_sums(const f32x2 (&h)[P][CPL], float (&s)[CPL]) {
+#pragma unroll
+  for (int c = 0; c < CPL; ++c) s[c] = row_sum<CPL, P>(h, c);
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1)
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
+}
+// one of two values with the other lane's share of it added: the lane whose bit `o` is set keeps `hi`
+__device__ __forceinline__ float fold(float lo, float hi, int o, int lane) {
+  const bool up = (lane & o) != 0;
+  return (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, o);
+}
+
+// FWD: v comes in, o (when wanted), r and the states leave; otherwise do and r come in, dv, dbeta's parts and the dS leave.
+template <int K, int CPL, bool FWD>
+__global__ void __launch_bounds__(128, CPL == 8 ? 2 : 4) kda_recurrent_walk_kernel(const TrainParams p) {
+  chain_point();
+  constexpr int I = K / 32, E = K / 32;
+  constexpr int P = CPL == 8 ? 1 : 2;      // sums in flight per column: eight chains a lane
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  WalkSmem<K, CPL>& s = *reinterpret_cast<WalkSmem<K, CPL>*>(smem_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5, nt = blockDim.x;
+  const int ncols = 4 * CPL * nw, parts = p.V / ncols;
+  const int unit = blockIdx.x / parts, part = blockIdx.x % parts;
+  const int n = unit / p.H, h = unit % p.H, hq = h / (p.H / p.HQ);
+  const int V = p.V, cg = lane & 3, rg = lane >> 2, lcol = 4 * CPL * warp + 4 * cg, col = part * ncols + lcol;
+  const Seq sq = sequence(p, n);
+  const int stages = static_cast<int>((sq.len + TS - 1) / TS);
+  float* const kept = (FWD ? p.ckpt : p.dckpt) + ((sq.bos / TC + n) * p.H + h) * static_cast<size_t>(K) * V + col;
+  const size_t sbase = (static_cast<size_t>(n) * p.H + h) * K * V + col;
+
+  const long long out_step = (FWD ? 1LL : -1LL) * p.H * V, aux_step = FWD ? out_step : -1LL * p.H * (V / 16);
+  const int oc = CPL == 8 ? rg : rg >> 1, ocol = col + 16 * (oc >> 2) + (oc & 3);      // the column whose o this lane ends with
+
+  auto tokens_of = [&](int st) { return static_cast<int>(min(static_cast<long long>(TS), sq.len - static_cast<long long>(st) * TS)); };
+  auto issue = [&](int st) {      // raw rows of stage st on their way
+    const int b = st & 1, cnt = tokens_of(st);
+    const size_t tok0 = static_cast<size_t>(sq.bos + static_cast<long long>(st) * TS);
+    for (int i = tid; i < cnt * (K / 4); i += nt) {
+      const int j = i / (K / 4), c = 4 * (i % (K / 4));
+      const size_t rowq = ((tok0 + j) * p.HQ + hq) * K + c;
+      cp_row16(&s.k[b][j][c], p.k + rowq, p.wide);
+      if (!FWD || p.o) cp_row16(&s.q[b][j][c], p.q + rowq, p.wide);
+      cp_row16(&s.a[b][j][c], p.g + ((tok0 + j) * p.H + h) * K + c, p.wide);
+    }
+    for (int i = tid; i < cnt * (ncols / 4); i += nt) {
+      const int j = i / (ncols / 4), c = 4 * (i % (ncols / 4));
+      const size_t row = ((tok0 + j) * p.H + h) * V + part * ncols + c;
+      cp_async16(&s.x[b][j][c], (FWD ? p.v : p.d_o) + row, true);
+      if (!FWD) cp_async16(&s.y[b][j][c], p.resid + row, true);
+    }
+    if (tid < cnt) cp_async4(&s.beta[b][tid], p.beta + (tok0 + tid) * p.H + h, true);
+    cp_async_commit();
+  };
+  auto activate = [&](int st) {      // in place: exp g, normalised rows, scale; a warp per token
+    const int b = st & 1, cnt = tokens_of(st);
+    for (int j = warp; j < cnt; j += nw) {
+      float kf[E], qf[E], gf[E];
+      row_get<E>(kf, &s.k[b][j][lane * E]);
+      row_get<E>(gf, &s.a[b][j][lane * E]);
+      const bool with_q = !FWD || p.o || p.use_l2;
+      if (!FWD || p.o) row_get<E>(qf, &s.q[b][j][lane * E]);
+      float qs = p.scale, ks = 1.f;
+      if (p.use_l2) {
+        const size_t tok = static_cast<size_t>(sq.bos + static_cast<long long>(st) * TS + j), row = tok * p.H + h;
+        if (FWD) {
+          if (!p.o) {      // (replay in front of a backward: q is only here for its norm)
+#pragma unroll
+            for (int e = 0; e < E; ++e) qf[e] = p.q[(tok * p.HQ + hq) * K + lane * E + e];
+          }
+          float ssq = 0.f, ssk = 0.f;
+#pragma unroll
+          for (int e = 0; e < E; ++e) {
+            ssq += qf[e] * qf[e];
+            ssk += kf[e] * kf[e];
+          }
+          const float rq = rsqrtf(warp_sum(ssq) + L2NORM_EPS), rk = rsqrtf(warp_sum(ssk) + L2NORM_EPS);
+          if (lane == 0 && part == 0) *reinterpret_cast<float2*>(p.norms + 2 * row) = make_float2(rq, rk);
+          qs *= rq;
+          ks = rk;
+        } else {
+          const float2 r = *reinterpret_cast<const float2*>(p.norms + 2 * row);
+          qs *= r.x;
+          ks = r.y;
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        if (with_q) qf[e] *= qs;
+        kf[e] *= ks;
+        gf[e] = expf(gf[e]);
+      }
+      row_put<E>(&s.k[b][j][lane * E], kf);
+      row_put<E>(&s.a[b][j][lane * E], gf);
+      if (!FWD || p.o) row_put<E>(&s.q[b][j][lane * E], qf);
+    }
+  };
+
+  Slice<K, CPL> S;
+  const float* const start = FWD ? p.h0 : p.d_ht;
+  if (start) S.load(start + sbase, rg, V);
+  else S.zero();
+  if (stages > 0) issue(FWD ? 0 : stages - 1);
+  for (int it = 0; it < stages; ++it) {
+    const int st = FWD ? it : stages - 1 - it, b = st & 1, cnt = tokens_of(st);
+    cp_async_wait<0>();
+    __syncthreads();      // stage st has arrived; everybody is done with the other buffer
+    if (it + 1 < stages) issue(FWD ? st + 1 : st - 1);
+    activate(st);
+    if (FWD ? st % (TC / TS) == 0 : (it == 0 || st % (TC / TS) == TC / TS - 1))
+      S.store(kept + static_cast<size_t>(st / (TC / TS)) * p.H * K * V, rg, V);
+    __syncthreads();
+    // (running pointers: the products of 64-bit indices cost more than a tenth of a token's instructions)
+    const size_t row0 = (static_cast<size_t>(sq.bos + static_cast<long long>(st) * TS + (FWD ? 0 : cnt - 1))) * p.H + h;
+    float* out = (FWD ? p.resid : p.dv) + row0 * V + col + 16 * rg;                    // r, dv: row groups 0 (and 1) store
+    float* aux = FWD ? p.o + row0 * V + ocol : p.dbp + row0 * (V / 16) + col / 16;      // o, dbeta's parts
+    for (int jj = 0; jj < cnt; ++jj, out += out_step, aux += aux_step) {
+      const int j = FWD ? jj : cnt - 1 - jj;
+      const float* const kr = &s.k[b][j][4 * rg];
+      const float* const ar = &s.a[b][j][4 * rg];
+      const float* const qr = &s.q[b][j][4 * rg];
+      float x[CPL];
+#pragma unroll
+      for (int m = 0; m < CPL / 4; ++m) {
+        const float4 y = *reinterpret_cast<const float4*>(&s.x[b][j][lcol + 16 * m]);
+        x[4 * m] = y.x; x[4 * m + 1] = y.y; x[4 * m + 2] = y.z; x[4 * m + 3] = y.w;
+      }
+      const float beta = s.beta[b][j];
+      f32x2 acc[P][CPL];
+      F4 k[I];
+#pragma unroll
+      for (int i = 0; i < I; ++i) k[i] = lds4(kr + 32 * i);
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) acc[0][c] = acc[P - 1][c] = 0ull;
+      if constexpr (FWD) {
+#pragma unroll
+        for (int i = 0; i < I; ++i) {
+          const F4 a = lds4(ar + 32 * i);
+#pragma unroll
+          for (int c = 0; c < CPL; ++c) {
+            S.v[i][0][c] = mul2(S.v[i][0][c], a.a);
+            S.v[i][1][c] = mul2(S.v[i][1][c], a.b);
+            acc[0][c] = fma2(S.v[i][0][c], k[i].a, acc[0][c]);
+            acc[P - 1][c] = fma2(S.v[i][1][c], k[i].b, acc[P - 1][c]);
+          }
+        }
+        float hk[CPL];
+        column_sums<CPL, P>(acc, hk);
+        f32x2 w2[CPL];
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) {
+          x[c] -= hk[c];      // r
+          w2[c] = pair(beta * x[c], beta * x[c]);
+          acc[0][c] = acc[P - 1][c] = 0ull;
+        }
+        if (rg < CPL / 4)
+          *reinterpret_cast<float4*>(out) =
+              CPL == 8 && rg ? make_float4(x[CPL - 4], x[CPL - 3], x[CPL - 2], x[CPL - 1]) : make_float4(x[0], x[1], x[2], x[3]);
+#pragma unroll
+        for (int i = 0; i < I; ++i) {
+          const F4 q = lds4(qr + 32 * i);
+#pragma unroll
+          for (int c = 0; c < CPL; ++c) {
+            S.v[i][0][c] = fma2(k[i].a, w2[c], S.v[i][0][c]);
+            S.v[i][1][c] = fma2(k[i].b, w2[c], S.v[i][1][c]);
+            acc[0][c] = fma2(S.v[i][0][c], q.a, acc[0][c]);
+            acc[P - 1][c] = fma2(S.v[i][1][c], q.b, acc[P - 1][c]);
+          }
+        }
+        if (p.o) {      // summed off the chain: a lane ends with one column
+          float y[CPL];
+#pragma unroll
+          for (int c = 0; c < CPL; ++c) y[c] = row_sum<CPL, P>(acc, c);
+          int o = 16;
+#pragma unroll
+          for (int half = CPL / 2; half >= 1; half >>= 1, o >>= 1)
+#pragma unroll
+            for (int c = 0; c < half; ++c) y[c] = fold(y[c], y[c + half], o, lane);
+          if (CPL == 4) y[0] += __shfl_xor_sync(0xffffffffu, y[0], 4);
+          if (CPL == 8 || !(lane & 4)) *aux = y[0];
+        }
+      } else {
+        f32x2 d2[CPL];
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) d2[c] = pair(x[c], x[c]);
+#pragma unroll
+        for (int i = 0; i < I; ++i) {
+          const F4 q = lds4(qr + 32 * i);
+#pragma unroll
+          for (int c = 0; c < CPL; ++c) {
+            S.v[i][0][c] = fma2(q.a, d2[c], S.v[i][0][c]);
+            S.v[i][1][c] = fma2(q.b, d2[c], S.v[i][1][c]);
+            acc[0][c] = fma2(S.v[i][0][c], k[i].a, acc[0][c]);
+            acc[P - 1][c] = fma2(S.v[i][1][c], k[i].b, acc[P - 1][c]);
+          }
+        }
+        float dw[CPL], dr[CPL];
+        column_sums<CPL, P>(acc, dw);
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) {
+          dr[c] = beta * dw[c];
+          d2[c] = pair(-dr[c], -dr[c]);
+        }
+        if (rg < CPL / 4)
+          *reinterpret_cast<float4*>(out) =
+              CPL == 8 && rg ? make_float4(dr[CPL - 4], dr[CPL - 3], dr[CPL - 2], dr[CPL - 1]) : make_float4(dr[0], dr[1], dr[2], dr[3]);
+#pragma unroll
+        for (int i = 0; i < I; ++i) {
+          const F4 a = lds4(ar + 32 * i);
+#pragma unroll
+          for (int c = 0; c < CPL; ++c) {
+            S.v[i][0][c] = mul2(fma2(k[i].a, d2[c], S.v[i][0][c]), a.a);
+            S.v[i][1][c] = mul2(fma2(k[i].b, d2[c], S.v[i][1][c]), a.b);
+          }
+        }
+        // dbeta over 16 columns: four lanes, and with eight columns a lane two groups of them
+#pragma unroll
+        for (int m = 0; m < CPL / 4; ++m) {
+          float pb = dot4(make_float4(dw[4 * m], dw[4 * m + 1], dw[4 * m + 2], dw[4 * m + 3]), *reinterpret_cast<const float4*>(&s.y[b][j][lcol + 16 * m]));
+          pb += __shfl_xor_sync(0xffffffffu, pb, 1);
+          pb += __shfl_xor_sync(0xffffffffu, pb, 2);
+          if (lane == 0) aux[m] = pb;
+        }
+      }
+    }
+  }
+  float* const end = FWD ? p.ht : p.dh0;
+  if (end) S.store(end + sbase, rg, V);
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// the middle: 32 tokens of ROWS rows of a state
+// ---------------------------------------------------------------------------------------------------------------------
+template <int K, int V>
+struct Mid {
+  static constexpr int LPR = V / 8;                          // lanes along a row, 8 columns each: 4 l + 4 LPR m + (0..3), m < 2
+  static constexpr int RPW = 4 * (32 / LPR);                 // rows per warp, four per lane
+  static constexpr int NW = K / RPW < 4 ? K / RPW : 4;       // warps
+  static constexpr int ROWS = NW * RPW, SLICES = K / ROWS, NT = 32 * NW;
+  static constexpr int RP = ROWS + 8;                        // padded row of a token's values: the sums of four tokens go to different banks
+  struct Smem {
+    float w[TC][V];              // r, then beta r
+    float d_o[TC][V];
+    float dr[TC][V];             // beta dw, then -beta dw
+    float q[TC][RP];             // scale q^, then dq^
+    float k[TC][RP];             // k^, then dk^
+    float a[TC][RP];             // exp g, then dg
+    float4 state[3][8][NT];      // this thread's part of the state in front of tokens 8, 16, 24
+    float wdo[TC];               // <w, do>
+    float beta[TC];
+    int n;
+  };
+};
+
+template <int K, int V>
+__global__ void __launch_bounds__(Mid<K, V>::NT, 2) kda_recurrent_mid_kernel(const TrainParams p) {
+  chain_point();
+  using M = Mid<K, V>;
+  constexpr int NT = M::NT, ROWS = M::ROWS, LPR = M::LPR;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  typename M::Smem& s = *reinterpret_cast<typename M::Smem*>(smem_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int slice = blockIdx.x % M::SLICES, h = blockIdx.x / M::SLICES % p.H, hq = h / (p.H / p.HQ);
+  const long long slot = blockIdx.x / M::SLICES / p.H;
+  if (tid == 0) {      // the last sequence whose first slot is not behind this one
+    int lo = 0, hi = p.N - 1;
+    while (lo < hi) {
+      const int m = (lo + hi + 1) >> 1;
+      if (seq_start(p, m) / TC + m <= slot) lo = m;
+      else hi = m - 1;
+    }
+    s.n = lo;
+  }
+  __syncthreads();
+  const int n = s.n;
+  const Seq sq = sequence(p, n);
+  const long long c = slot - (sq.bos / TC + n);
+  if (c < 0 || c * TC >= sq.len) return;
+  const int cnt = static_cast<int>(min(static_cast<long long>(TC), sq.len - c * TC));
+  const size_t tok0 = static_cast<size_t>(sq.bos + c * TC);
+
+  // ---- this thread's eight columns of four rows of S and dS; the tokens' rows -------------------------------------------------------
+  const int l = lane % LPR, lrow = warp * M::RPW + 4 * (lane / LPR);
+  const size_t sbase = ((static_cast<size_t>(slot) * p.H + h) * K + slice * ROWS + lrow) * V + 4 * l;
+  using Tile = f32x2[4][4];      // [row][pair of columns]
+  auto load_state = [&](Tile& x, const float* base) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const F4 y = lds4(base + sbase + i * V + 4 * LPR * m);
+        x[i][2 * m] = y.a;
+        x[i][2 * m + 1] = y.b;
+      }
+  };
+  for (int i = tid; i < TC * (V / 4); i += NT) {
+    const int t = i / (V / 4), cc = 4 * (i % (V / 4));
+    const bool ok = t < cnt;
+    const size_t row = ((tok0 + (ok ? t : 0)) * p.H + h) * V + cc;
+    cp_async16(&s.w[t][cc], p.resid + row, ok);
+    cp_async16(&s.d_o[t][cc], p.d_o + row, ok);
+    cp_async16(&s.dr[t][cc], p.dv + row, ok);
+  }
+  cp_async_commit();
+  if (tid < TC) s.beta[tid] = tid < cnt ? p.beta[(tok0 + tid) * p.H + h] : 0.f;
+  Tile dS, S;
+  load_state(S, p.ckpt);
+  load_state(dS, p.dckpt);
+  for (int i = tid; i < TC * ROWS; i += NT) {      // tokens beyond the sequence leave S and dS as they are
+    const int t = i / ROWS, row = i % ROWS;
+    const bool ok = t < cnt;
+    const size_t tok = tok0 + (ok ? t : 0), rq = (tok * p.HQ + hq) * K + slice * ROWS + row, rv = tok * p.H + h;
+    float2 r = make_float2(1.f, 1.f);
+    if (p.use_l2) r = *reinterpret_cast<const float2*>(p.norms + 2 * rv);
+    s.q[t][row] = ok ? p.q[rq] * (p.scale * r.x) : 0.f;
+    s.k[t][row] = ok ? p.k[rq] * r.y : 0.f;
+    s.a[t][row] = ok ? expf(p.g[rv * K + slice * ROWS + row]) : 1.f;
+  }
+  if (slice == 0 && tid < cnt) {
+    const float* const part = p.dbp + ((tok0 + tid) * p.H + h) * (V / 16);
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < V / 16; ++i) sum += part[i];
+    p.dbeta[(tok0 + tid) * p.H + h] = sum;
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  for (int t = warp; t < TC; t += M::NW) {
+    constexpr int E = V / 32;
+    float w[E], d[E], dot = 0.f;
+    row_get<E>(w, &s.w[t][lane * E]);
+    row_get<E>(d, &s.d_o[t][lane * E]);
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      w[e] *= s.beta[t];
+      dot += w[e] * d[e];
+    }
+    row_put<E>(&s.w[t][lane * E], w);
+    row_get<E>(w, &s.dr[t][lane * E]);
+#pragma unroll
+    for (int e = 0; e < E; ++e) w[e] = -w[e];
+    row_put<E>(&s.dr[t][lane * E], w);
+    dot = warp_sum(dot);
+    if (lane == 0) s.wdo[t] = dot;
+  }
+  __syncthreads();
+
+  auto rows4 = [&](const float (&x)[TC][M::RP], int t, float (&y)[4]) {      // a token's values of this thread's rows
+    const float4 z = *reinterpret_cast<const float4*>(&x[t][lrow]);
+    y[0] = z.x; y[1] = z.y; y[2] = z.z; y[3] = z.w;
+  };
+  auto step = [&](Tile& to, const Tile& from, int t) {      // `from` is S' of token t: S' + k w^T
+    float k[4];
+    rows4(s.k, t, k);
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const F4 w = lds4(&s.w[t][4 * l + 4 * LPR * m]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const f32x2 k2 = pair(k[i], k[i]);
+        to[i][2 * m] = fma2(k2, w.a, from[i][2 * m]);
+        to[i][2 * m + 1] = fma2(k2, w.b, from[i][2 * m + 1]);
+      }
+    }
+  };
+  auto decay = [&](Tile& to, const Tile& from, int t) {
+    float a[4];
+    rows4(s.a, t, a);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const f32x2 a2 = pair(a[i], a[i]);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) to[i][m] = mul2(from[i][m], a2);
+    }
+  };
+  auto step4 = [&](int t) {      // S over four tokens
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      decay(S, S, t + j);
+      step(S, S, t + j);
+    }
+  };
+#pragma unroll 1
+  for (int i = 0; i < 3; ++i) {
+    step4(8 * i);
+    step4(8 * i + 4);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) sts4(reinterpret_cast<float*>(&s.state[i][m][tid]), F4{S[m >> 1][2 * (m & 1)], S[m >> 1][2 * (m & 1) + 1]});
+  }
+#pragma unroll 1
+  for (int half = 7; half >= 0; --half) {      // four tokens each, the last first
+    const int t0 = 4 * half;
+    if (half < 2) {
+      load_state(S, p.ckpt);
+    } else {
+#pragma unroll
+      for (int m = 0; m < 8; ++m) {
+        const F4 x = lds4(reinterpret_cast<const float*>(&s.state[(half >> 1) - 1][m][tid]));
+        S[m >> 1][2 * (m & 1)] = x.a;
+        S[m >> 1][2 * (m & 1) + 1] = x.b;
+      }
+    }
+    if (half & 1) step4(t0 - 4);
+    Tile Sp[4];      // S' of the four tokens
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      decay(Sp[j], S, t0 + j);
+      if (j < 3) step(S, Sp[j], t0 + j);
+    }
+    // sums of the lane's 8 columns, folded over the lanes of a row: first the four rows (one per lane pair), then the tokens
+    float part[4][3];
+    constexpr int R1 = LPR / 2, R2 = LPR / 4;      // lane bits that pick the row
+#pragma unroll
+    for (int j = 3; j >= 0; --j) {
+      const int t = t0 + j;
+      float q[4], k[4], a[4];
+      rows4(s.q, t, q);
+      rows4(s.k, t, k);
+      rows4(s.a, t, a);
+      f32x2 pq[4], pk[4], pg[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) pq[i] = pk[i] = pg[i] = 0ull;
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const int cc = 4 * l + 4 * LPR * m;
+        const F4 d = lds4(&s.d_o[t][cc]), w = lds4(&s.w[t][cc]), r = lds4(&s.dr[t][cc]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const f32x2 q2 = pair(q[i], q[i]), k2 = pair(k[i], k[i]), a2 = pair(a[i], a[i]);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const f32x2 x = Sp[j][i][2 * m + e], dd = e ? d.b : d.a, ww = e ? w.b : w.a, rr = e ? r.b : r.a;
+            f32x2 y = fma2(q2, dd, dS[i][2 * m + e]);      // dS_t
+            pq[i] = fma2(x, dd, pq[i]);
+            pk[i] = fma2(y, ww, pk[i]);
+            pk[i] = fma2(x, rr, pk[i]);
+            y = fma2(k2, rr, y);                            // dS'
+            pg[i] = fma2(x, y, pg[i]);
+            dS[i][2 * m + e] = mul2(y, a2);
+          }
+        }
+      }
+      float sum[4][3];
+      const float wdo = s.wdo[t];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 hq2 = halves(pq[i]), hk2 = halves(pk[i]), hg2 = halves(pg[i]);
+        sum[i][0] = hq2.x + hq2.y;
+        sum[i][1] = hk2.x + hk2.y;
+        sum[i][2] = hg2.x + hg2.y;
+        if (l == 0) sum[i][0] = fmaf(k[i], wdo, sum[i][0]);      // S_t do = S' do + k <w, do>
+      }
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        part[j][i] = fold(fold(sum[0][i], sum[2][i], R1, lane), fold(sum[1][i], sum[3][i], R1, lane), R2, lane);
+    }
+    const int row = lrow + 2 * ((lane & R1) != 0) + ((lane & R2) != 0);
+    auto put = [&](int t, float x, float y, float z) {      // over the tokens' q, k, exp g of these rows, which the whole warp is done with
+      s.q[t][row] = x;
+      s.k[t][row] = y;
+      s.a[t][row] = z;
+    };
+    if constexpr (LPR == 16) {
+      float x[3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        x[i] = fold(fold(part[0][i], part[2][i], 2, lane), fold(part[1][i], part[3][i], 2, lane), 1, lane);
+      put(t0 + (lane & 3), x[0], x[1], x[2]);
+    } else if constexpr (LPR == 8) {
+      float x[2][3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        x[0][i] = fold(part[0][i], part[2][i], 1, lane);
+        x[1][i] = fold(part[1][i], part[3][i], 1, lane);
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) put(t0 + 2 * (lane & 1) + j, x[j][0], x[j][1], x[j][2]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) put(t0 + j, part[j][0], part[j][1], part[j][2]);
+    }
+    __syncwarp();
+  }
+  __syncthreads();
+  for (int i = tid; i < cnt * ROWS; i += NT) {
+    const int t = i / ROWS, row = i % ROWS;
+    const size_t o = ((tok0 + t) * p.H + h) * K + slice * ROWS + row;
+    p.dqh[o] = s.q[t][row] * p.dq_scale;
+    p.dkh[o] = s.k[t][row];
+    p.dg[o] = s.a[t][row];
+  }
+}
+
+// dq, dk from the per-value-head gradients w.r.t. the rows the recurrence saw: sum over the value heads of a group,
+// scale (q only), then the backward of x^ = x rsqrt(sum x^2 + eps) when the rows were normalised.  One warp per row.
+template <int K>
+__global__ void __launch_bounds__(256) kda_recurrent_bwd_finish_kernel(const TrainParams p, float* __restrict__ dq, float* __restrict__ dk,
+                                                                       long long rows) {
+  chain_point();
+  constexpr int E = K / 32;
+  const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);      // token * HQ + q head
+  const int lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const int grp = p.H / p.HQ;
+  const long long tok = row / p.HQ;
+  const int hq = static_cast<int>(row % p.HQ);
+#pragma unroll
+  for (int which = 0; which < 2; ++which) {
+    const float* x = (which ? p.k : p.q) + row * K + lane * E;
+    const float* src = (which ? p.dkh : p.dqh) + (tok * p.H + static_cast<long long>(hq) * grp) * K + lane * E;
+    float d[E], xf[E];
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      float acc = 0.f;
+      for (int j = 0; j < grp; ++j) acc += src[static_cast<size_t>(j) * K + e];
+      d[e] = which ? acc : acc * p.scale;
+      xf[e] = x[e];
+      ss += xf[e] * xf[e];
+    }
+    if (p.use_l2) {
+      const float rs = rsqrtf(warp_sum(ss) + L2NORM_EPS);
+      float dot = 0.f;
+#pragma unroll
+      for (int e = 0; e < E; ++e) dot += xf[e] * rs * d[e];
+      dot = warp_sum(dot);
+#pragma unroll
+      for (int e = 0; e < E; ++e) d[e] = rs * (d[e] - xf[e] * rs * dot);
+    }
+    float* out = (which ? dk : dq) + row * K + lane * E;
+#pragma unroll
+    for (int e = 0; e < E; ++e) out[e] = d[e];
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// buffers and launches
+// ---------------------------------------------------------------------------------------------------------------------
+size_t up256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
+size_t kept_states(int64_t tokens, int N) { return static_cast<size_t>(tokens) / TC + static_cast<size_t>(N); }
+
+struct SavedLayout {      // what the forward leaves for the backward
+  size_t ckpt, resid, norms, total;
+};
+SavedLayout saved_layout(int64_t tokens, int N, int H, int K, int V) {
+  SavedLayout l{};
+  size_t off = 0;
+  l.ckpt = off; off = up256(off + kept_states(tokens, N) * H * K * V * 4);
+  l.resid = off; off = up256(off + static_cast<size_t>(tokens) * H * V * 4);
+  l.norms = off; off = up256(off + static_cast<size_t>(tokens) * H * 2 * 4);
+  l.total = off;
+  return l;
+}
+struct WorkLayout {      // the backward's own scratch; kda_recurrent_bwd's workspace continues with a SavedLayout
+  size_t dqh, dkh, dckpt, dbp, total;
+};
+WorkLayout work_layout(int64_t tokens, int N, int H, int K, int V) {
+  WorkLayout l{};
+  size_t off = 0;
+  l.dqh = off; off = up256(off + static_cast<size_t>(tokens) * H * K * 4);
+  l.dkh = off; off = up256(off + static_cast<size_t>(tokens) * H * K * 4);
+  l.dckpt = off; off = up256(off + kept_states(tokens, N) * H * K * V * 4);
+  l.dbp = off; off = up256(off + static_cast<size_t>(tokens) * H * (V / 16) * 4);
+  l.total = off;
+  return l;
+}
+bool head_size_ok(int d) { return d == 32 || d == 64 || d == 128; }
+void use_saved(TrainParams& p, void* saved, const SavedLayout& l) {
+  unsigned char* const b = static_cast<unsigned char*>(saved);
+  p.ckpt = reinterpret_cast<float*>(b + l.ckpt);
+  p.resid = reinterpret_cast<float*>(b + l.resid);
+  p.norms = reinterpret_cast<float*>(b + l.norms);
+}
+int wide(const void* q, const void* k, const void* g) {
+  return ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(g)) & 15) == 0;
+}
+
+template <int K, int CPL, bool FWD>
+int launch_walk(const TrainParams& p, bool first, cudaStream_t st) {
+  static DeviceOnce once;
+  const auto kernel = kda_recurrent_walk_kernel<K, CPL, FWD>;
+  const int smem = static_cast<int>(sizeof(WalkSmem<K, CPL>));
+  const int rc = once.run([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
+  if (rc != KDA_OK) return rc;
+  const int cols = std::min(p.V, WalkSmem<K, CPL>::COLS);
+  const long long grid = static_cast<long long>(p.N) * p.H * (p.V / cols);
+  if (grid > 0x7fffffffLL) return KDA_E_SHAPE;
+  const unsigned threads = static_cast<unsigned>(cols / (4 * CPL) * 32);
+  if (!first) return static_cast<int>(launch_chained(kernel, static_cast<unsigned>(grid), threads, smem, st, p));
+  kernel<<<static_cast<unsigned>(grid), threads, smem, st>>>(p);
+  return static_cast<int>(cudaGetLastError());
+}
+// 32 columns a warp read a row of q, k, exp g for 128 state values instead of 64, and two warps a scheduler are enough to keep the FP32
+// pipe fed; while there are fewer than that, more and narrower warps shorten the chain
+bool wide_slices(const TrainParams& p) { return static_cast<long long>(p.N) * p.H * p.V > 32LL * 4 * sm_count(); }
+template <bool FWD>
+int launch_walk(const TrainParams& p, int K, bool first, cudaStream_t st) {
+  const bool w = wide_slices(p);
+  switch (K) {
+    case 32: return w ? launch_walk<32, 8, FWD>(p, first, st) : launch_walk<32, 4, FWD>(p, first, st);
+    case 64: return w ? launch_walk<64, 8, FWD>(p, first, st) : launch_walk<64, 4, FWD>(p, first, st);
+    default: return w ? launch_walk<128, 8, FWD>(p, first, st) : launch_walk<128, 4, FWD>(p, first, st);
+  }
+}
+template <int K, int V>
+int launch_mid(const TrainParams& p, cudaStream_t st) {
+  static DeviceOnce once;
+  const auto kernel = kda_recurrent_mid_kernel<K, V>;
+  const int smem = static_cast<int>(sizeof(typename Mid<K, V>::Smem));
+  const int rc = once.run([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
+  if (rc != KDA_OK) return rc;
+  const long long grid = p.slots * p.H * Mid<K, V>::SLICES;
+  if (grid > 0x7fffffffLL) return KDA_E_SHAPE;
+  return static_cast<int>(launch_chained(kernel, static_cast<unsigned>(grid), Mid<K, V>::NT, smem, st, p));
+}
+template <int K>
+int launch_mid(const TrainParams& p, cudaStream_t st) {
+  switch (p.V) {
+    case 32: return launch_mid<K, 32>(p, st);
+    case 64: return launch_mid<K, 64>(p, st);
+    default: return launch_mid<K, 128>(p, st);
+  }
+}
+template <int K>
+int launch_finish(const TrainParams& p, float* dq, float* dk, long long rows, cudaStream_t st) {
+  return static_cast<int>(launch_chained(kda_recurrent_bwd_finish_kernel<K>, static_cast<unsigned>((rows + 7) / 8), 256, 0, st, p, dq, dk, rows));
+}
+
+// saved == NULL: the forward walk runs here first, into the end of the workspace
+int backward(const kda_recurrent_bwd_args* a, const void* saved, size_t saved_bytes, bool with_saved, void* stream) {
+  if (!a) return KDA_E_NULL;
+  if (!a->q || !a->k || !a->v || !a->g || !a->beta || !a->d_o || !a->dq || !a->dk || !a->dv || !a->dg || !a->dbeta || !a->workspace)
+    return KDA_E_NULL;
+  if (with_saved && !saved) return KDA_E_NULL;
+  if (a->io_dtype != KDA_FP32) return KDA_E_DTYPE;
+  if (a->N < 0 || a->H <= 0 || a->tokens < 0 || (!a->cu_seqlens && a->T < 0)) return KDA_E_SHAPE;
+  if (!head_size_ok(a->K) || !head_size_ok(a->V)) return KDA_E_SHAPE;
+  const int HQ = a->HQ > 0 ? a->HQ : a->H;
+  if (a->H % HQ) return KDA_E_SHAPE;
+  const WorkLayout l = work_layout(a->tokens, a->N, a->H, a->K, a->V);
+  const SavedLayout sl = saved_layout(a->tokens, a->N, a->H, a->K, a->V);
+  if (a->workspace_bytes < l.total + (with_saved ? 0 : sl.total)) return KDA_E_WORKSPACE;
+  if (with_saved && saved_bytes < sl.total) return KDA_E_WORKSPACE;
+  if ((reinterpret_cast<uintptr_t>(a->workspace) | reinterpret_cast<uintptr_t>(saved)) & 255) return KDA_E_ALIGN;
+  const void* sixteen[] = {a->v, a->h0, a->d_o, a->d_ht, a->dv, a->dh0};      // 16-byte loads and stores
+  for (const void* p : sixteen)
+    if (reinterpret_cast<uintptr_t>(p) & 15) return KDA_E_ALIGN;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (a->N == 0) return KDA_OK;
+  if (a->tokens == 0) {      // empty sequences: the initial state is the final state
+    if (!a->dh0) return KDA_OK;
+    const size_t bytes = static_cast<size_t>(a->N) * a->H * a->K * a->V * sizeof(float);
+    return static_cast<int>(a->d_ht ? cudaMemcpyAsync(a->dh0, a->d_ht, bytes, cudaMemcpyDeviceToDevice, st) : cudaMemsetAsync(a->dh0, 0, bytes, st));
+  }
+  if (!a->cu_seqlens && static_cast<int64_t>(a->N) * a->T != a->tokens) return KDA_E_SHAPE;
+  unsigned char* const ws = static_cast<unsigned char*>(a->workspace);
+  TrainParams p{};
+  p.q = static_cast<const float*>(a->q); p.k = static_cast<const float*>(a->k); p.v = static_cast<const float*>(a->v);
+  p.g = a->g; p.beta = a->beta; p.h0 = a->h0; p.d_o = static_cast<const float*>(a->d_o); p.d_ht = a->d_ht;
+  p.cu = a->cu_seqlens;
+  p.dqh = reinterpret_cast<float*>(ws + l.dqh); p.dkh = reinterpret_cast<float*>(ws + l.dkh);
+  p.dckpt = reinterpret_cast<float*>(ws + l.dckpt); p.dbp = reinterpret_cast<float*>(ws + l.dbp);
+  p.dv = static_cast<float*>(a->dv); p.dg = a->dg; p.dbeta = a->dbeta; p.dh0 = a->dh0;
+  p.T = a->T; p.slots = static_cast<long long>(kept_states(a->tokens, a->N));
+  p.N = a->N; p.H = a->H; p.HQ = HQ; p.V = a->V; p.use_l2 = a->use_qk_l2norm; p.scale = a->scale;
+  p.wide = wide(a->q, a->k, a->g);
+  const bool direct = HQ == a->H && !p.use_l2;      // nothing to sum or to take back: no pass of its own (0.27 ms at 8 x 2048 x 32)
+  float *const dq = static_cast<float*>(a->dq), *const dk = static_cast<float*>(a->dk);
+  if (direct) p.dqh = dq, p.dkh = dk;
+  p.dq_scale = direct ? p.scale : 1.f;
+  use_saved(p, with_saved ? const_cast<void*>(saved) : ws + l.total, sl);
+  int rc = KDA_OK;
+  if (!with_saved) rc = launch_walk<true>(p, a->K, true, st);
+  if (rc == KDA_OK) rc = launch_walk<false>(p, a->K, with_saved, st);
+  const long long rows = a->tokens * HQ;
+  if (rc == KDA_OK) rc = a->K == 32 ? launch_mid<32>(p, st) : (a->K == 64 ? launch_mid<64>(p, st) : launch_mid<128>(p, st));
+  if (rc == KDA_OK && !direct)
+    rc = a->K == 32 ? launch_finish<32>(p, dq, dk, rows, st) : (a->K == 64 ? launch_finish<64>(p, dq, dk, rows, st) : launch_finish<128>(p, dq, dk, rows, st));
+  return rc;
+}
+
+}  // namespace
+
+}  // namespace kda
+
+using namespace kda;
+
+extern "C" size_t kda_recurrent_saved_bytes(int64_t tokens, int32_t N, int32_t H, int32_t K, int32_t V) {
+  if (tokens < 0 || N < 0 || H <= 0 || K <= 0 || V <= 0) return 0;
+  return saved_layout(tokens, N, H, K, V).total;
+}
+
+extern "C" size_t kda_recurrent_bwd_workspace_bytes(int64_t tokens, int32_t N, int32_t H, int32_t K, int32_t V) {
+  if (tokens < 0 || N < 0 || H <= 0 || K <= 0 || V <= 0) return 0;
+  return work_layout(tokens, N, H, K, V).total + saved_layout(tokens, N, H, K, V).total;
+}
+
+extern "C" int kda_recurrent_train_fwd(const kda_recurrent_args* a, void* saved, size_t saved_bytes, void* stream) {
+  if (!a) return KDA_E_NULL;
+  if (a->N < 0 || a->H <= 0 || a->tokens < 0 || (!a->cu_seqlens && a->T < 0)) return KDA_E_SHAPE;
+  if (!head_size_ok(a->K) || !head_size_ok(a->V)) return KDA_E_SHAPE;
+  const int HQ = a->HQ > 0 ? a->HQ : a->H;
+  if (a->HQ < 0 || a->H % HQ) return KDA_E_SHAPE;
+  // whole sequences, activated gates, [K, V] states
+  if (a->state_indices || a->num_accepted_tokens || a->transpose_state || a->A_log || a->beta_sigmoid || (a->ht && a->ht == a->h0)) return KDA_E_SHAPE;
+  if (a->N == 0 || a->tokens == 0) return kda_recurrent_fwd(a, stream);      // nothing to walk: the final state is the initial one
+  if (!a->q || !a->k || !a->v || !a->g || !a->beta || !a->o || !saved) return KDA_E_NULL;
+  if (a->io_dtype != KDA_FP32) return KDA_E_DTYPE;
+  if (!a->cu_seqlens && static_cast<int64_t>(a->N) * a->T != a->tokens) return KDA_E_SHAPE;
+  const SavedLayout sl = saved_layout(a->tokens, a->N, a->H, a->K, a->V);
+  if (saved_bytes < sl.total) return KDA_E_WORKSPACE;
+  if (reinterpret_cast<uintptr_t>(saved) & 255) return KDA_E_ALIGN;
+  const void* sixteen[] = {a->q, a->k, a->v, a->g, a->o, a->h0, a->ht};      // as kda_recurrent_fwd
+  for (const void* p : sixteen)
+    if (reinterpret_cast<uintptr_t>(p) & 15) return KDA_E_ALIGN;
+  TrainParams p{};
+  p.q = static_cast<const float*>(a->q); p.k = static_cast<const float*>(a->k); p.v = static_cast<const float*>(a->v);
+  p.g = a->g; p.beta = a->beta; p.h0 = a->h0; p.ht = a->ht; p.o = static_cast<float*>(a->o);
+  p.cu = a->cu_seqlens;
+  p.T = a->T; p.slots = static_cast<long long>(kept_states(a->tokens, a->N));
+  p.N = a->N; p.H = a->H; p.HQ = HQ; p.V = a->V; p.use_l2 = a->use_qk_l2norm; p.scale = a->scale;
+  p.wide = wide(a->q, a->k, a->g);
+  use_saved(p, saved, sl);
+  return launch_walk<true>(p, a->K, true, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int kda_recurrent_bwd(const kda_recurrent_bwd_args* args, void* stream) { return backward(args, nullptr, 0, false, stream); }
+
+extern "C" int kda_recurrent_train_bwd(const kda_recurrent_bwd_args* args, const void* saved, size_t saved_bytes, void* stream) {
+  return backward(args, saved, saved_bytes, true, stream);
+}

@@ -269,45 +269,56 @@ def fused_recurrent_kda(q, k, v, g, beta, A_log=None, dt_bias=None, scale=None, 
 
 
 class RecurrentKDAFunction(torch.autograd.Function):
-    """float32 path of chunk_kda with gradients: forward by the token-recurrent fp32 kernel, backward by its exact
-    reverse-mode counterpart (`kda_recurrent_bwd`, fla/ops/kda/naive.py:12-66 differentiated).  K, V in {32, 64, 128}."""
+    """float32 path of chunk_kda with gradients: token-recurrent forward that keeps the state of every 32nd token, and its exact
+    reverse mode (`kda_recurrent_train_fwd`, `kda_recurrent_train_bwd`, fla/ops/kda/naive.py:12-66 differentiated).  K, V in
+    {32, 64, 128}."""
 
     @staticmethod
     def forward(ctx, q, k, v, g, beta, scale, initial_state, output_final_state, use_l2norm, cu_seqlens):
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
         g32, beta32 = g.contiguous().float(), beta.contiguous().float()
         h0 = initial_state.contiguous().float() if initial_state is not None else None
-        o, ht = fused_recurrent_kda_fwd(q, k, v, g32, beta32, initial_state=h0, scale=scale,
-                                        output_final_state=output_final_state, inplace_final_state=False,
-                                        use_qk_l2norm_in_kernel=use_l2norm, cu_seqlens=cu_seqlens)
         cu = _as_i32(cu_seqlens, q.device) if cu_seqlens is not None else None
-        ctx.save_for_backward(q, k, v, g32, beta32, h0, cu)
+        B, T, HQ, K = q.shape
+        H, V = v.shape[-2], v.shape[-1]
+        N = B if cu is None else cu.numel() - 1
+        dev = q.device
+        lib = _lib.load()
+        o = torch.empty_like(v)
+        ht = torch.empty(N, H, K, V, dtype=torch.float32, device=dev) if output_final_state else None
+        saved = torch.empty(lib.kda_recurrent_saved_bytes(B * T, N, H, K, V), dtype=torch.uint8, device=dev)
+        args = _lib.RecurrentArgs(
+            q=_ptr(q), k=_ptr(k), v=_ptr(v), g=_ptr(g32), beta=_ptr(beta32), h0=_ptr(h0), ht=_ptr(ht), o=_ptr(o), cu_seqlens=_ptr(cu),
+            tokens=B * T, N=N, T=T, H=H, K=K, V=V, HQ=HQ, io_dtype=_lib.KDA_FP32, use_qk_l2norm=int(use_l2norm), scale=scale)
+        with torch.cuda.device(dev):
+            _lib.check(lib.kda_recurrent_train_fwd(C.byref(args), _ptr(saved), saved.numel(), _stream(dev)), "kda_recurrent_train_fwd")
+        ctx.save_for_backward(q, k, v, g32, beta32, h0, cu, saved)
         ctx.meta = (float(scale), bool(use_l2norm), g.dtype, beta.dtype)
         return o, ht
 
     @staticmethod
     def backward(ctx, do, dht):
-        q, k, v, g32, beta32, h0, cu = ctx.saved_tensors
+        q, k, v, g32, beta32, h0, cu, saved = ctx.saved_tensors
         scale, use_l2norm, g_dtype, beta_dtype = ctx.meta
         B, T, HQ, K = q.shape
         H, V = v.shape[-2], v.shape[-1]
         N = B if cu is None else cu.numel() - 1
         dev = q.device
         lib = _lib.load()
-        aligned = lambda t: t if t.data_ptr() % 16 == 0 else t.clone()      # noqa: E731  the kernel loads 16 bytes at a time
+        aligned = lambda t: t if t.data_ptr() % 16 == 0 else t.clone()      # noqa: E731  the kernels load 16 bytes at a time
         do = aligned(do.contiguous().float())
         dht = aligned(dht.contiguous().float()) if dht is not None else None
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         dg, dbeta = torch.empty_like(g32), torch.empty_like(beta32)
         dh0 = torch.empty(N, H, K, V, dtype=torch.float32, device=dev) if h0 is not None else None
-        ws = torch.empty(lib.kda_recurrent_bwd_workspace_bytes(B * T, N, H, K, V), dtype=torch.uint8, device=dev)
+        ws = torch.empty(lib.kda_recurrent_bwd_workspace_bytes(B * T, N, H, K, V) - saved.numel(), dtype=torch.uint8, device=dev)
         args = _lib.RecurrentBwdArgs(
             q=_ptr(q), k=_ptr(k), v=_ptr(v), g=_ptr(g32), beta=_ptr(beta32), h0=_ptr(h0), cu_seqlens=_ptr(cu),
             d_o=_ptr(do), d_ht=_ptr(dht), dq=_ptr(dq), dk=_ptr(dk), dv=_ptr(dv), dg=_ptr(dg), dbeta=_ptr(dbeta), dh0=_ptr(dh0),
             workspace=_ptr(ws), workspace_bytes=ws.numel(), tokens=B * T, N=N, T=T, H=H, K=K, V=V, HQ=HQ,
             io_dtype=_lib.KDA_FP32, use_qk_l2norm=int(use_l2norm), scale=scale)
         with torch.cuda.device(dev):
-            _lib.check(lib.kda_recurrent_bwd(C.byref(args), _stream(dev)), "kda_recurrent_bwd")
+            _lib.check(lib.kda_recurrent_train_bwd(C.byref(args), _ptr(saved), saved.numel(), _stream(dev)), "kda_recurrent_train_bwd")
         return dq, dk, dv, dg.to(g_dtype), dbeta.to(beta_dtype), None, dh0, None, None, None
 
 

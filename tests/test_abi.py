@@ -142,3 +142,25 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "LIB_PATH", str(tmp_path / "absent.so"))
     with pytest.raises(RuntimeError, match="no CPU or PyTorch fallback"):
         _lib.load()
+
+
+def test_training_pair_refuses_what_it_does_not_take(lib):
+    """kda_recurrent_train_fwd / _bwd: argument errors on the host, nothing launched."""
+    from kda_b200 import _lib
+    size = lib.kda_recurrent_saved_bytes(64, 1, 2, 64, 64)
+    assert 0 < size < lib.kda_recurrent_bwd_workspace_bytes(64, 1, 2, 64, 64)
+    ok = dict(q=256, k=256, v=256, g=256, beta=256, o=256, N=1, T=64, tokens=64, H=2, K=64, V=64, HQ=2, io_dtype=_lib.KDA_FP32)
+    call = lambda saved=256, n=size, **kw: lib.kda_recurrent_train_fwd(C.byref(_lib.RecurrentArgs(**{**ok, **kw})), saved, n, None)      # noqa: E731
+    assert call(K=96) == -2 and call(V=256) == -2 and call(tokens=63) == -2
+    assert call(h0=512, ht=512) == -2 and call(transpose_state=1) == -2 and call(A_log=256) == -2 and call(beta_sigmoid=1) == -2
+    assert call(state_indices=256) == -2
+    assert call(io_dtype=_lib.KDA_BF16) == -3
+    assert call(saved=None) == -1 and call(o=None) == -1
+    assert call(n=size - 1) == -5
+    assert call(saved=264) == -4 and call(v=260) == -4 and call(ht=264) == -4 and call(q=260) == -4
+    bwd = dict(q=256, k=256, v=256, g=256, beta=256, d_o=256, dq=256, dk=256, dv=256, dg=256, dbeta=256, N=1, T=64, tokens=64, H=2, K=64, V=64, HQ=2,
+               io_dtype=_lib.KDA_FP32, workspace=256, workspace_bytes=lib.kda_recurrent_bwd_workspace_bytes(64, 1, 2, 64, 64) - size)
+    back = lambda saved=256, n=size, **kw: lib.kda_recurrent_train_bwd(C.byref(_lib.RecurrentBwdArgs(**{**bwd, **kw})), saved, n, None)      # noqa: E731
+    assert back(saved=None) == -1 and back(n=size - 1) == -5 and back(saved=272) == -4
+    assert back(workspace_bytes=bwd["workspace_bytes"] - 1) == -5 and back(d_o=260) == -4
+    assert lib.kda_recurrent_bwd(C.byref(_lib.RecurrentBwdArgs(**bwd)), None) == -5      # without the saved states the workspace holds them too

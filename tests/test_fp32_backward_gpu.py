@@ -168,3 +168,72 @@ def test_fp32_gradients_at_odd_addresses():
         o, ht = chunk_kda(*lv[:5], initial_state=lv[5], output_final_state=True)
         out.append(torch.autograd.grad([o, ht], lv, ups))
     assert all(torch.equal(a, b) for a, b in zip(*out))
+
+
+def _errors(got, ref, bound):
+    from oracle.kda_oracle import rel_l2_err
+    for n in NAMES:
+        if ref[n] is not None and got[n] is not None:
+            e = rel_l2_err(got[n], ref[n])
+            assert e <= bound, f"{n}: relative error {e:.2e}"
+
+
+# 2-norm bound of the tests below: float32 steps, each rounding independent (2^-24 = 6e-8), over sums of up to 128 products and a few dozen
+# dependent tokens: 6e-8 sqrt(64) = 5e-7; measured 1.2e-7.
+EXACT = 5e-7
+
+
+@pytest.mark.parametrize("T", [7, 8, 9, 31, 32, 33, 40, 61])
+def test_fp32_training_at_the_edges_of_stages_and_kept_states(T):
+    """The walks stage eight tokens at a time and keep a state every 32; the middle works on four tokens at a time, replayed from every eighth."""
+    d = make_inputs(2, T, 2, 128, 128, torch.float32, seed=600 + T, h0_std=0.1, backward=True)
+    ref = recurrent_kda_grads(d["q"], d["k"], d["v"], d["g"], d["beta"], d["do"], d["dht"], initial_state=d["h0"])
+    _errors(_run(d), ref, EXACT)
+
+
+@pytest.mark.parametrize("K,V", [(32, 32), (32, 64), (32, 128), (64, 32), (64, 64), (64, 128), (128, 32), (128, 64)])
+@pytest.mark.parametrize("wide", [False, True])
+def test_fp32_training_of_both_walks(K, V, wide):
+    """Enough (sequence, head) units for the walks with 32 columns a warp (units * V / 32 > 4 warps per SM), and few units."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    H = 4
+    B = 4 * sms * 32 // (V * H) + 1 if wide else 1
+    d = make_inputs(B, 37, H, K, V, torch.float32, seed=700 + K + V, h0_std=0.1, backward=True)
+    ref = recurrent_kda_grads(*(d[n].cuda() for n in ("q", "k", "v", "g", "beta", "do", "dht")), initial_state=d["h0"].cuda(), use_qk_l2norm=True)
+    _errors(_run(d, l2=True), ref, EXACT)
+
+
+def test_recurrent_bwd_takes_q_k_g_at_odd_addresses():
+    """The C entry asks no alignment of q, k and g: views one float into a buffer give the same bits."""
+    import ctypes as C
+    from kda_b200 import _lib
+    lib = _lib.load()
+    T, H, D = 70, 2, 64
+    d = {n: t.cuda() for n, t in make_inputs(1, T, H, D, D, torch.float32, seed=51, backward=True).items() if t is not None}
+    p = lambda t: C.c_void_p(t.data_ptr())      # noqa: E731
+    out = []
+    for shift in (0, 1):
+        x = {}
+        for n in ("q", "k", "g"):
+            buf = torch.zeros(d[n].numel() + shift, device="cuda")
+            x[n] = buf[shift:].view(d[n].shape).copy_(d[n])
+        r = {n: torch.empty_like(d[n[1:]]) for n in ("dq", "dk", "dv", "dg", "dbeta")}
+        ws = torch.empty(lib.kda_recurrent_bwd_workspace_bytes(T, 1, H, D, D), dtype=torch.uint8, device="cuda")
+        a = _lib.RecurrentBwdArgs(q=p(x["q"]), k=p(x["k"]), v=p(d["v"]), g=p(x["g"]), beta=p(d["beta"]), d_o=p(d["do"]), workspace=p(ws),
+                                  workspace_bytes=ws.numel(), tokens=T, N=1, T=T, H=H, K=D, V=D, HQ=H, io_dtype=_lib.KDA_FP32, use_qk_l2norm=1,
+                                  scale=D ** -0.5, **{n: p(t) for n, t in r.items()})
+        _lib.check(lib.kda_recurrent_bwd(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)), "kda_recurrent_bwd")
+        torch.cuda.synchronize()
+        out.append(r)
+    assert all(torch.equal(out[0][n], out[1][n]) for n in out[0])
+
+
+def test_fp32_backward_twice_through_one_forward():
+    """What the forward keeps is only read: a second backward through the same graph gives the same bits."""
+    from kda_b200 import chunk_kda
+    d = {n: t.cuda() for n, t in make_inputs(1, 100, 2, 128, 128, torch.float32, seed=52, backward=True).items() if t is not None}
+    lv = [d[n].requires_grad_(True) for n in ("q", "k", "v", "g", "beta")]
+    o, _ = chunk_kda(*lv)
+    a = torch.autograd.grad(o, lv, d["do"], retain_graph=True)
+    b = torch.autograd.grad(o, lv, d["do"])
+    assert all(torch.equal(x, y) for x, y in zip(a, b))
