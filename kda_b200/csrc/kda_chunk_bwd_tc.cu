@@ -11,16 +11,26 @@
 // Phases per tile (G = in-chunk cumsum of g in the log2 domain, Gam = 2^G, D[t,j] = 2^(G_t - G_j)):
 //   A   dqg^T = h dO^T,  dw^T = -h dv_new^T,  dkg^T = dh' v_new^T      (M=128 kk, N=64 t, K=128 v)
 //       dAqk  = dO v_new^T                                             (M=64 t,  N=64 j)
-//   B1  dTm = du (beta v)^T + dw (beta k Gam)^T, and its transpose     (M=64)
+//   B1  dTm = du (beta v)^T + dw (beta k Gam)^T                        (M=64)
 //       dbv^T = du^T Tm,  dbk^T = dw^T Tm                              (M=128, N=64 t, K=64 t')
 //   B2  X = dTm Tm^T      B3  Y = Tm^T X,  dAkk = -tril(Y, -1)
 //   C   off-diagonal 16x16 blocks of the intra-chunk terms, decay factored around a row that lies between
 //       j and t (both factors <= 1):  Cq^T, Cp^T (reference = first row of t's block),
-//       Cn^T (reference = last row of j's block)                       (M=128 kk, N=16, K=16..48)
+//       Cn^T (reference = last row of j's block)                       (M=128 kk, N=32 (q and p) or 16, K=16..48)
 //   D   per key column: diagonal blocks pairwise with running products of 2^(g), dG = q dq + k (dk+ - dk-),
 //       dg = reverse cumsum, final dq, dk, dg;  dbeta from  <Tm, dTm_raw> + <dAkk, raw kk>.
+//
+// What bounds it: the work around the products, 51 k warp instructions a tile (22 to 25 k cycles), of which the last phase has a third; the
+// waits for products are filled with it: the operands of phase C are built under B1 and B2, the last phase's parts that need only the
+// accumulators of A and B1 run under B2, B3 and C.  q and k are interleaved into one word per element once they have arrived, and the last
+// phase adds up dq and dk+ as register pairs, one instruction for both sides.  Row numbers are left to the uniform registers.
+// 8 x 8192 tokens x 32 heads: 61 -> 51 k instructions a tile, whole step 6.02 -> 5.91 ms; packed documents with the L2 norm 7.13 -> 6.95 ms (its
+// epilogue reads q and k where they are instead of from global memory); 2 x 1000 x 8 heads of 64: 108 -> 95.5 us, of which 9 are the code's size:
+// 135 KB with every issue loop and wait unrolled, 85 now, and a short step fetches all of it anew.  Kept as they were: the points where
+// operands are rounded to bf16 (one scaled copy of each row instead of one per reference row halves the builds and moves dA_log by 4 %).
 #include "kda_chunk_bwd.cuh"
 #include "kda_device.cuh"
+#include "kda_f32x2.cuh"
 #include "kda_umma.cuh"
 
 #include <type_traits>
@@ -34,17 +44,22 @@ constexpr int NT = 512;             // threads per CTA: 16 warps = 4 TMEM lane q
 
 struct TcSmem {
   // ---- SW128 operand tiles; every offset is a multiple of 1024 -------------------------------------------------
-  unsigned char HS[TILE_VK];    // A.  later: KG = k Gam [64 j][128 kk] (16K) | DWT = dw^T [128 kk][64 t] (16K);  C: kL span 0 | kL span 1 (12K each)
-  unsigned char DH[TILE_VK];    // A.  later: DT (8K) | X (8K) | DAQ (8K) | DAK (8K)
-  unsigned char VN[TILE_VT];    // A.  C: kR span 0 (12K)
-  unsigned char DVN[TILE_VT];   // A, B1.  C: qL span 0 (12K)
-  unsigned char dO[TILE_TK];    // A (two [64 t][64 v] sub-tiles).  C: kR span 1
-  unsigned char V[TILE_TK];     // B1 (two [64 j][64 v] sub-tiles).  C: qL span 1.  D: dq staging [64][128]
+  unsigned char HS[TILE_VK];    // A.  later: KG = k Gam [64 j][128 kk] (16K) | DWT = dw^T [128 kk][64 t] (16K);  from B1's end: DT (8K) | X (8K) | qL, J > 0 (12K)
+  unsigned char DH[TILE_VK];    // A.  later: DAK, DAQ (16K, eight rows of one behind eight of the other) |
+  unsigned char VN[TILE_VT];    // A.                                                  | with the rest of DH and dO 48K: kR (24K), qL, kL of J = 0 (12K each)
+  unsigned char dO[TILE_TK];    // A (two [64 t][64 v] sub-tiles).  later: see VN
+  unsigned char DVN[TILE_VT];   // A, B1.  later: dv staging, four parts [64 t][32 v]
+  unsigned char V[TILE_TK];     // B1 (two [64 j][64 v] sub-tiles).  B2, C: kL, J > 0.  D: dq staging [64][128]
   unsigned char TI[TILE_TT];    // B1..B3.  D (with RKK): dk staging [64][128]
   unsigned char RKK[TILE_TT];   // post-B3
   // ---- plain arrays -----------------------------------------------------------------------------------------------
-  __nv_bfloat16 q[C * KD];      // [64][128]
-  __nv_bfloat16 k[C * KD];
+  union {
+    struct {
+      __nv_bfloat16 q[C * KD];      // [64][128], as they arrive
+      __nv_bfloat16 k[C * KD];
+    };
+    uint32_t qk[C * KD];            // from phase B1 on: (q, k) of an element in one word, q in the low half
+  };
   float G[C * KD];              // log2-domain cumsum of g (g of the NEXT tile arrives here during phase D)
   float2 Ad[4][16][18];         // diagonal blocks: (a1, a2) = (scale dAqk, beta dAkk); rows 16-byte aligned
   float beta[C];
@@ -64,10 +79,9 @@ struct TcSmem {
 };
 static_assert(sizeof(TcSmem) + 1024 <= 227 * 1024, "TcSmem too large");
 
-// TMEM columns (512 allocated): 64 each
-constexpr int C_DQG = 0, C_DKG = 64, C_DW = 128 /* later dbk^T */, C_DAQ = 192 /* later dTm, later Cn */, C_DTT = 256,
-              C_XY = 320, C_DBV = 384 /* later Cq */, C_CP = 448;
-constexpr int C_CQ = C_DBV, C_CN = C_DAQ, C_DBK = C_DW;
+// TMEM columns (512 allocated): 64 each; in phase C 32 per row block I = 1..3 for Cq, Cp (eight columns of one behind eight of the other), 48 for Cn
+constexpr int C_DQG = 0, C_DKG = 64, C_DW = 128 /* later dbk^T */, C_DAQ = 192 /* later dTm */, C_XY = 320, C_DBV = 384;
+constexpr int C_CQP = 192, C_CN = 288, C_DBK = C_DW;
 
 // eight floats -> one 16-byte piece of bf16
 __device__ __forceinline__ uint4 pack8(const float* v) {
@@ -77,6 +91,9 @@ __device__ __forceinline__ uint4 pack8(const float* v) {
 __device__ __forceinline__ unsigned char* sw_piece(unsigned char* tile, int row, int chunk) {
   return tile + row * 128 + (((chunk ^ row) & 7) << 4);
 }
+// a word of the interleaved tile
+__device__ __forceinline__ float q_of(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float k_of(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
 }  // namespace
 
@@ -92,16 +109,16 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
   // aliases inside the tile regions
   unsigned char* const sKG = s.HS;
   unsigned char* const sDWT = s.HS + SPAN;
-  unsigned char* const sDT = s.DH;
-  unsigned char* const sX = s.DH + 8192;
-  unsigned char* const sDAQ = s.DH + 16384;
-  unsigned char* const sDAK = s.DH + 24576;
-  unsigned char* const sKR0 = s.VN;
-  unsigned char* const sKR1 = s.dO;
-  unsigned char* const sQL0 = s.DVN;
-  unsigned char* const sQL1 = s.V;
-  unsigned char* const sKL0 = s.HS;
-  unsigned char* const sKL1 = s.HS + SPAN;
+  unsigned char* const sDT = s.HS;
+  unsigned char* const sX = s.HS + 8192;
+  unsigned char* const sDA = s.DH;      // rows t of dAqk at da_row(t), of dAkk eight rows behind: one product takes the same rows of both
+  auto da_row = [](int t) { return 2 * (t & 56) + (t & 7); };
+  unsigned char* const sKR = s.DH + 16384;
+  constexpr uint32_t KR_SPAN = 12288, L_SPAN = 6144;      // between the two 64-column spans of kR; of qL, kL
+  unsigned char* const sQL0 = sKR + 2 * KR_SPAN;           // J = 0
+  unsigned char* const sKL0 = sQL0 + 2 * L_SPAN;
+  unsigned char* const sQL1 = s.HS + 16384;                // J > 0
+  unsigned char* const sKL1 = s.V;
   __nv_bfloat16* const stq = reinterpret_cast<__nv_bfloat16*>(s.V);      // phase D: dq, dk before their coalesced stores
   __nv_bfloat16* const stk = reinterpret_cast<__nv_bfloat16*>(s.TI);
   float* const stg = reinterpret_cast<float*>(s.q);                            // and dg, over q and k
@@ -144,10 +161,10 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
       default: tma_load_rows(s.V + 8192, &p.tm_v, 64, h, tk, &s.barB); break;
     }
   };
-  // [64 t][32 v] of dv: behind the 96 rows of four phase-C operand tiles
-  auto dv_stage = [&](int i) { return (i == 0 ? sKR0 : (i == 1 ? sKR1 : (i == 2 ? sQL0 : sKL0))) + 96 * 128; };
+  auto dv_stage = [&](int i) { return s.DVN + 4096 * i; };      // [64 t][32 v] of dv
   // rows of a partial chunk beyond its length hold the next sequence's tokens after a tiled load: clear them
   auto zero_rows_sw = [&](unsigned char* tile, int len) {          // [64][64] bf16 sub-tile, 128-byte rows
+#pragma unroll 1
     for (int i = len * 8 + tid; i < C * 8; i += NT) *reinterpret_cast<uint4*>(tile + i * 16) = make_uint4(0u, 0u, 0u, 0u);
   };
   if (tid == 0) {
@@ -173,42 +190,52 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
   // TMEM lane quadrant of a warp: warp & 3; which 16 of the 64 columns: warp >> 2
   const uint32_t tq = tb + (static_cast<uint32_t>(32 * (warp_u & 3)) << 16);     // this warp's lanes
 
-  // Operands of phase C, built while the phase-B products run (rows R of the stacked tiles, 16-byte pieces pc):
+  // Operands of phase C, built while the phase-B products run (rows R of the stacked tiles):
   // kR_I[j][kk] = k_j 2^(G_r - G_j),  r = 16 I,  j < 16 I            rows stacked: I=1 -> 0..15, I=2 -> 16..47, I=3 -> 48..95
   // qL_J[t][kk] = scale q_t 2^(G_t - G_e), kL_J = k_t 2^(G_t - G_e), e = 16 J + 15, t >= 16 (J+1)
-  //                                                                   rows stacked: J=0 -> 0..47, J=1 -> 48..79, J=2 -> 80..95
-  // One item = four key columns of one row (a warp covers one row: conflict-free 8- and 16-byte accesses).
-  auto build_kR = [&](int first, int stride) {
-    for (int i = first; i < 96 * 32; i += stride) {
-      const int R = i >> 5, g4 = i & 31;
-      const int I = (R < 16) ? 1 : (R < 48 ? 2 : 3);
-      const int j = R - (I == 1 ? 0 : (I == 2 ? 16 : 48));
-      const int r = 16 * I;
-      const uint2 kr = *reinterpret_cast<const uint2*>(&s.k[j * KD + g4 * 4]);
-      const float4 Ga = *reinterpret_cast<const float4*>(&s.G[j * KD + g4 * 4]);
-      const float4 Ra = *reinterpret_cast<const float4*>(&s.G[r * KD + g4 * 4]);
-      const float2 k0 = unpack_bf16(kr.x), k1 = unpack_bf16(kr.y);
-      *reinterpret_cast<uint2*>(sw_piece((g4 >> 4) ? sKR1 : sKR0, R, (g4 >> 1) & 7) + (g4 & 1) * 8) =
-          make_uint2(pack_bf16(k0.x * ex2(Ra.x - Ga.x), k0.y * ex2(Ra.y - Ga.y)), pack_bf16(k1.x * ex2(Ra.z - Ga.z), k1.y * ex2(Ra.w - Ga.w)));
+  //                                                                   rows: J=0 -> 0..47 of one tile, J=1 -> 0..31, J=2 -> 32..47 of another
+  // A warp takes whole rows, a lane four key columns.  The row number is the same for the whole warp, so that it and the addresses that come of it are
+  // left to the uniform registers: with items counted through per thread, a third of a row's instructions were its indices.
+  auto four = [&](const void* rows, int row, int lane) { return reinterpret_cast<const unsigned char*>(rows) + row * (KD * 4) + lane * 16; };
+  auto minus2 = [](const F4& x, const F4& y) {      // 2^(x - y)
+    const f32x2 m1 = pair(-1.f, -1.f);
+    const float2 a = halves(fma2(y.a, m1, x.a)), b = halves(fma2(y.b, m1, x.b));
+    return F4{pair(ex2(a.x), ex2(a.y)), pair(ex2(b.x), ex2(b.y))};
+  };
+  auto put4 = [](unsigned char* dst, f32x2 a, f32x2 b) {
+    const float2 x = halves(a), y = halves(b);
+    *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(x.x, x.y), pack_bf16(y.x, y.y));
+  };
+  auto betas = [&](int t, float (&b)[16]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float4 x = *reinterpret_cast<const float4*>(&s.beta[t + 4 * i]);
+      b[4 * i] = x.x; b[4 * i + 1] = x.y; b[4 * i + 2] = x.z; b[4 * i + 3] = x.w;
     }
   };
-  auto build_qkL = [&](int R0, int R1, int first, int stride) {
-    for (int i = R0 * 32 + first; i < R1 * 32; i += stride) {
-      const int R = i >> 5, g4 = i & 31;
-      const int J = (R < 48) ? 0 : (R < 80 ? 1 : 2);
-      const int t = 16 * (J + 1) + R - (J == 0 ? 0 : (J == 1 ? 48 : 80));
-      const int e = 16 * J + 15;
-      const uint2 qr = *reinterpret_cast<const uint2*>(&s.q[t * KD + g4 * 4]);
-      const uint2 kr = *reinterpret_cast<const uint2*>(&s.k[t * KD + g4 * 4]);
-      const float4 Ga = *reinterpret_cast<const float4*>(&s.G[t * KD + g4 * 4]);
-      const float4 Ea = *reinterpret_cast<const float4*>(&s.G[e * KD + g4 * 4]);
-      const float f0 = ex2(Ga.x - Ea.x), f1 = ex2(Ga.y - Ea.y), f2 = ex2(Ga.z - Ea.z), f3 = ex2(Ga.w - Ea.w);
-      const float2 q0 = unpack_bf16(qr.x), q1 = unpack_bf16(qr.y), k0 = unpack_bf16(kr.x), k1 = unpack_bf16(kr.y);
-      const int off = (g4 & 1) * 8, pc = (g4 >> 1) & 7;
-      *reinterpret_cast<uint2*>(sw_piece((g4 >> 4) ? sQL1 : sQL0, R, pc) + off) =
-          make_uint2(pack_bf16(p.scale * q0.x * f0, p.scale * q0.y * f1), pack_bf16(p.scale * q1.x * f2, p.scale * q1.y * f3));
-      *reinterpret_cast<uint2*>(sw_piece((g4 >> 4) ? sKL1 : sKL0, R, pc) + off) =
-          make_uint2(pack_bf16(k0.x * f0, k0.y * f1), pack_bf16(k1.x * f2, k1.y * f3));
+  auto build_kR = [&](int first, int stride, int lane) {
+    unsigned char* const dst = sKR + (lane >> 4) * KR_SPAN + (lane & 1) * 8;
+#pragma unroll 1
+    for (int R = first; R < 96; R += stride) {
+      const int I = (R < 16) ? 1 : (R < 48 ? 2 : 3);
+      const int j = R - (I == 1 ? 0 : (I == 2 ? 16 : 48));
+      const uint4 w = *reinterpret_cast<const uint4*>(four(s.qk, j, lane));
+      const F4 f = minus2(lds4(reinterpret_cast<const float*>(four(s.G, 16 * I, lane))), lds4(reinterpret_cast<const float*>(four(s.G, j, lane))));
+      put4(dst + R * 128 + ((((lane >> 1) ^ R) & 7) << 4), mul2(pair(k_of(w.x), k_of(w.y)), f.a), mul2(pair(k_of(w.z), k_of(w.w)), f.b));
+    }
+  };
+  auto build_qkL = [&](unsigned char* const tq_, unsigned char* const tk_, const bool first_J, int first, int stride, int lane) {
+    const uint32_t off = (lane >> 4) * L_SPAN + (lane & 1) * 8;
+    const f32x2 sc = pair(p.scale, p.scale);
+#pragma unroll 1
+    for (int R = first; R < 48; R += stride) {
+      const int t = first_J || R >= 32 ? 16 + R : 32 + R;
+      const int e = first_J ? 15 : (R < 32 ? 31 : 47);
+      const uint4 w = *reinterpret_cast<const uint4*>(four(s.qk, t, lane));
+      const F4 f = minus2(lds4(reinterpret_cast<const float*>(four(s.G, t, lane))), lds4(reinterpret_cast<const float*>(four(s.G, e, lane))));
+      const uint32_t at = off + R * 128 + ((((lane >> 1) ^ R) & 7) << 4);
+      put4(tq_ + at, mul2(mul2(pair(q_of(w.x), q_of(w.y)), sc), f.a), mul2(mul2(pair(q_of(w.z), q_of(w.w)), sc), f.b));
+      put4(tk_ + at, mul2(pair(k_of(w.x), k_of(w.y)), f.a), mul2(pair(k_of(w.z), k_of(w.w)), f.b));
     }
   };
 
@@ -252,14 +279,15 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     // ---- sum_v h dh' (all warps, before warp 0 starts issuing) -------------------------------------------------------
     {
       const int kp = tid & 63, vq = tid >> 6;
-      float ax = 0.f, ay = 0.f;
-#pragma unroll 4
-      for (int vv = vq * 16; vv < vq * 16 + 16; ++vv) {
-        const float2 hh = unpack_bf16(*reinterpret_cast<const uint32_t*>(s.HS + vk_off(vv, 2 * kp)));
-        const float2 dd = unpack_bf16(*reinterpret_cast<const uint32_t*>(s.DH + vk_off(vv, 2 * kp)));
-        ax += hh.x * dd.x;
-        ay += hh.y * dd.y;
+      f32x2 acc = 0ull;
+      const uint32_t lo = vk_off(16 * vq, 2 * kp);      // row 16 vq + i: + 128 i, and i & 7 in the swizzled piece
+      auto wide = [](uint32_t u) { return pair(q_of(u), k_of(u)); };
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const uint32_t at = (lo ^ ((i & 7) << 4)) + 128 * i;
+        acc = fma2(wide(*reinterpret_cast<const uint32_t*>(s.HS + at)), wide(*reinterpret_cast<const uint32_t*>(s.DH + at)), acc);
       }
+      const float ax = halves(acc).x, ay = halves(acc).y;
       s.hdh_part[vq][2 * kp] = ax;
       s.hdh_part[vq][2 * kp + 1] = ay;
     }
@@ -281,7 +309,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
       const uint64_t dHS = umma::desc_mnmajor(aHS, 0, SPAN), dDHm = umma::desc_mnmajor(aDH, 0, SPAN);
       const uint64_t dVNm = umma::desc_mnmajor(aVN, 0, SPAN), dDVNm = umma::desc_mnmajor(aDVN, 0, SPAN);
       const uint64_t dDO0 = umma::desc_kmajor(aDO, 0), dDO1 = umma::desc_kmajor(aDO + 8192, 0);
-#pragma unroll
+#pragma unroll 1
       for (int sK = 0; sK < 8; ++sK) {
         const uint64_t mn = static_cast<uint64_t>(sK) * 128u, dDOk = ((sK >> 2) ? dDO1 : dDO0) + static_cast<uint64_t>(sK & 3) * 2u;
         umma::mma_ss_lead(tb + C_DQG, dHS + mn, dDOk, i1, sK > 0, lead);                 // dqg^T = h dO^T
@@ -298,6 +326,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     if (warp_u != 0) {
       if (alive && !mbar_wait(&s.barG, it & 1)) alive = false;
       if (len < C) {
+#pragma unroll 1
         for (int i = len * 16 + tid - 32; i < C * 16; i += NT - 32) {
           reinterpret_cast<uint4*>(s.G)[2 * i] = make_uint4(0u, 0u, 0u, 0u);
           reinterpret_cast<uint4*>(s.G)[2 * i + 1] = make_uint4(0u, 0u, 0u, 0u);
@@ -363,8 +392,8 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
         const int t = 16 * q4 + lane;
 #pragma unroll
         for (int i = 0; i < 16; ++i) v[i] = (16 * part + i <= t) ? v[i] : 0.f;
-        *reinterpret_cast<uint4*>(sw_piece(sDAQ, t, 2 * part)) = pack8(&v[0]);
-        *reinterpret_cast<uint4*>(sw_piece(sDAQ, t, 2 * part + 1)) = pack8(&v[8]);
+        *reinterpret_cast<uint4*>(sw_piece(sDA, da_row(t), 2 * part)) = pack8(&v[0]);
+        *reinterpret_cast<uint4*>(sw_piece(sDA, da_row(t), 2 * part + 1)) = pack8(&v[8]);
         if (part == q4) {                              // these 16 columns are the diagonal block of row block q4
 #pragma unroll
           for (int cc = 0; cc < 16; ++cc) s.Ad[q4][lane][cc].x = p.scale * v[cc];
@@ -373,19 +402,35 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     }
     if (!mbar_wait(&s.barQ, it & 1)) alive = false;
     if (len < C) {                 // uniform over the CTA
+#pragma unroll 1
       for (int i = len * 16 + tid; i < C * 16; i += NT) {
         reinterpret_cast<uint4*>(s.q)[i] = make_uint4(0u, 0u, 0u, 0u);
         reinterpret_cast<uint4*>(s.k)[i] = make_uint4(0u, 0u, 0u, 0u);
       }
       __syncthreads();
     }
-    for (int i = tid; i < C * 32; i += NT) {          // k Gam as two K-major sub-tiles [64 j][64 kk]
-      const int j = i >> 5, g4 = i & 31;
-      const uint2 kr = *reinterpret_cast<const uint2*>(&s.k[j * KD + g4 * 4]);
-      const float4 Ga = *reinterpret_cast<const float4*>(&s.G[j * KD + g4 * 4]);
-      const float2 k0 = unpack_bf16(kr.x), k1 = unpack_bf16(kr.y);
-      *reinterpret_cast<uint2*>(sw_piece(sKG + (g4 >> 4) * 8192, j, (g4 >> 1) & 7) + (g4 & 1) * 8) =
-          make_uint2(pack_bf16(k0.x * ex2(Ga.x), k0.y * ex2(Ga.y)), pack_bf16(k1.x * ex2(Ga.z), k1.y * ex2(Ga.w)));
+    {      // k Gam as two K-major sub-tiles [64 j][64 kk]; q and k interleaved over themselves
+      static_assert(C * 32 == 4 * NT, "four pieces per thread");
+      uint2 qr[4], kr[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        qr[u] = *reinterpret_cast<const uint2*>(&s.q[4 * (tid + u * NT)]);
+        kr[u] = *reinterpret_cast<const uint2*>(&s.k[4 * (tid + u * NT)]);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int j = warp_u + u * (NT / 32);
+        const F4 Ga = lds4(reinterpret_cast<const float*>(four(s.G, j, lane)));
+        const float2 a = halves(Ga.a), b = halves(Ga.b), k0 = unpack_bf16(kr[u].x), k1 = unpack_bf16(kr[u].y);
+        put4(sKG + (lane >> 4) * 8192 + (lane & 1) * 8 + j * 128 + ((((lane >> 1) ^ j) & 7) << 4), mul2(pair(k0.x, k0.y), pair(ex2(a.x), ex2(a.y))),
+             mul2(pair(k1.x, k1.y), pair(ex2(b.x), ex2(b.y))));
+      }
+      __syncthreads();      // everybody has read q and k
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        *reinterpret_cast<uint4*>(&s.qk[4 * (tid + u * NT)]) =
+            make_uint4(__byte_perm(qr[u].x, kr[u].x, 0x5410), __byte_perm(qr[u].x, kr[u].x, 0x7632), __byte_perm(qr[u].y, kr[u].y, 0x5410),
+                       __byte_perm(qr[u].y, kr[u].y, 0x7632));
     }
     cp_async_wait<0>();
     if (!mbar_wait(&s.barB, it & 1)) alive = false;       // Tm, raw kk, v
@@ -407,25 +452,22 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     if (warp_u == 0) {
       const uint32_t aDVN = smem_u32(s.DVN), aV = smem_u32(s.V), aDWT = smem_u32(sDWT), aKG = smem_u32(sKG), aTI = smem_u32(s.TI);
       constexpr uint32_t iT = umma::instr_desc(64, 64, true, false);
-      constexpr uint32_t iTt = umma::instr_desc(64, 64, false, true);
       constexpr uint32_t iB = umma::instr_desc(128, 64, false, true);
       const uint64_t dDuM = umma::desc_mnmajor(aDVN, 0, SPAN), dDwM = umma::desc_mnmajor(aDWT, 0, SPAN), dTiM = umma::desc_mnmajor(aTI, 0, SPAN);
       const uint64_t dV0 = umma::desc_kmajor(aV, 0), dV1 = umma::desc_kmajor(aV + 8192, 0);
       const uint64_t dKg0 = umma::desc_kmajor(aKG, 0), dKg1 = umma::desc_kmajor(aKG + 8192, 0);
       const uint64_t dDuK = umma::desc_kmajor(aDVN, 0), dDwK = umma::desc_kmajor(aDWT, 0);
-#pragma unroll
+#pragma unroll 1
       for (int sK = 0; sK < 8; ++sK) {
         const uint64_t mn = static_cast<uint64_t>(sK) * 128u, dVk = ((sK >> 2) ? dV1 : dV0) + static_cast<uint64_t>(sK & 3) * 2u;
         umma::mma_ss_lead(tb + C_DAQ, dDuM + mn, dVk, iT, sK > 0, lead);       // dTm[t][j]   += sum_v du[t][v] v[j][v]
-        umma::mma_ss_lead(tb + C_DTT, dVk, dDuM + mn, iTt, sK > 0, lead);      // dTm^T[j][t] += the same
       }
-#pragma unroll
+#pragma unroll 1
       for (int sK = 0; sK < 8; ++sK) {
         const uint64_t mn = static_cast<uint64_t>(sK) * 128u, dKg = ((sK >> 2) ? dKg1 : dKg0) + static_cast<uint64_t>(sK & 3) * 2u;
         umma::mma_ss_lead(tb + C_DAQ, dDwM + mn, dKg, iT, 1, lead);            // += sum_kk dw[t][kk] kGam[j][kk]
-        umma::mma_ss_lead(tb + C_DTT, dKg, dDwM + mn, iTt, 1, lead);
       }
-#pragma unroll
+#pragma unroll 1
       for (int sK = 0; sK < 4; ++sK) {
         const uint64_t dTi = dTiM + static_cast<uint64_t>(sK) * 128u;
         umma::mma_ss_lead(tb + C_DBV, dDuK + static_cast<uint64_t>(sK) * 2u, dTi, iB, sK > 0, lead);     // dbv^T[v][t] = sum_t' du[t'][v] Tm[t'][t]
@@ -433,45 +475,64 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
       }
       if (lead) umma::commit(&s.barM);
     }
-    if (warp_u != 0) build_kR(tid - 32, NT - 32);      // warp 0 is busy issuing; into the v_new and dO tiles, which only phase A read
+    // meanwhile two thirds of phase C's operands (warp 0 is busy issuing), into the v_new, dO and dh tiles, which only phase A read; the next tile's
+    // chunk is looked up by a warp that waits here anyway
+    if (warp_u != 0) {
+      if (warp_u == NT / 32 - 1 && lane == 0 && next_idx < total_tiles) stash_chunk(next_idx, (it + 1) & 1);
+      __syncwarp();
+      build_kR(warp_u - 1, NT / 32 - 1, lane);
+      build_qkL(sQL0, sKL0, true, warp_u - 1, NT / 32 - 1, lane);
+    }
     if (!mbar_wait(&s.barM, mph & 1)) alive = false;
     ++mph;
     umma::fence_after_sync();
     KDA_DBG_CLOCK(dbg, 5);
     if (alive) {
-      float v[16], v2[16], v3[16];                     // the three loads are in flight together
+      float v[16], v3[16];                             // both loads are in flight together
       umma::tmem_ld16(tq + C_DAQ + 16 * part, v);      // dTm rows (M = 64 layout): scale the columns by beta_j
-      umma::tmem_ld16(tq + C_DTT + 16 * part, v2);     // dTm_raw^T rows j: dbeta_j += sum_t' Tm[t'][j] dTm_raw[t'][j]
       umma::tmem_ld16(tq + C_DBV + 16 * part, v3);     // dbv^T rows v: dv[t][v] = beta_t dbv[t][v]
+      float bt[16];
+      betas(16 * part, bt);
       umma::tmem_ld_wait();
+      {      // dbeta_j += sum_t Tm[t][j] dTm_raw[t][j]: rows t are lanes 0..15 (what the others compute is not used); afterwards lane j holds column j
+        float x[16];
+#pragma unroll
+        for (int cix = 0; cix < 2; ++cix) {
+          const uint4 tm = *reinterpret_cast<const uint4*>(sw_piece(s.TI, 16 * q4 + (lane & 15), 2 * part + cix));
+          const uint32_t w[4] = {tm.x, tm.y, tm.z, tm.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 y = unpack_bf16(w[e]);
+            x[8 * cix + 2 * e] = y.x * v[8 * cix + 2 * e];
+            x[8 * cix + 2 * e + 1] = y.y * v[8 * cix + 2 * e + 1];
+          }
+        }
+#pragma unroll
+        for (int o = 8; o >= 1; o >>= 1) {
+          const bool up = (lane & o) != 0;
+#pragma unroll
+          for (int i = 0; i < o; ++i) x[i] = (up ? x[i + o] : x[i]) + __shfl_xor_sync(0xffffffffu, up ? x[i] : x[i + o], o);
+        }
+        if (lane < 16) s.dbp[q4][16 * part + lane] = x[0];
+      }
       if (lane < 16) {
         const int t = 16 * q4 + lane;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] *= s.beta[16 * part + i];
+        for (int i = 0; i < 16; ++i) v[i] *= bt[i];
         *reinterpret_cast<uint4*>(sw_piece(sDT, t, 2 * part)) = pack8(&v[0]);
         *reinterpret_cast<uint4*>(sw_piece(sDT, t, 2 * part + 1)) = pack8(&v[8]);
       }
-      if (lane < 16) {
-        const int j = 16 * q4 + lane;
-        float acc = 0.f;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const int t2 = 16 * part + i;
-          acc += v2[i] * __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(s.TI + umma::sw128(t2, j)));
-        }
-        s.dbp[part][j] = acc;
-      }
-      if (len == C) {      // staged in the ends of four operand regions (rows 96.. of the tiles to come) and stored by the copy engine
+      if (len == C) {      // staged in the dv_new tile, which the products have read, and stored by the copy engine
         __nv_bfloat16* const st = reinterpret_cast<__nv_bfloat16*>(dv_stage(q4)) + 16 * part * 32 + lane;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) st[32 * i] = __float2bfloat16_rn(s.beta[16 * part + i] * v3[i]);
+        for (int i = 0; i < 16; ++i) st[32 * i] = __float2bfloat16_rn(bt[i] * v3[i]);
       } else {
         const int vcol = 32 * q4 + lane;
         __nv_bfloat16* const dvp = p.dv + (static_cast<size_t>(ci.tok0 + 16 * part) * p.H + h) * p.vc + vcol;
         const size_t tstride = static_cast<size_t>(p.H) * p.vc;
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          if (16 * part + i < len && vcol < p.vc) dvp[i * tstride] = __float2bfloat16_rn(s.beta[16 * part + i] * v3[i]);
+          if (16 * part + i < len && vcol < p.vc) dvp[i * tstride] = __float2bfloat16_rn(bt[i] * v3[i]);
       }
     }
     fence_proxy_async();
@@ -493,16 +554,45 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     if (warp_u == 0) {
       const uint32_t aDT = smem_u32(sDT), aTI = smem_u32(s.TI);
       constexpr uint32_t iX = umma::instr_desc(64, 64, false, false);
-#pragma unroll
       const uint64_t dDt = umma::desc_kmajor(aDT, 0), dTiK = umma::desc_kmajor(aTI, 0);
 #pragma unroll
       for (int sK = 0; sK < 4; ++sK) umma::mma_ss_lead(tb + C_XY, dDt + static_cast<uint64_t>(sK) * 2u, dTiK + static_cast<uint64_t>(sK) * 2u, iX, sK > 0, lead);
-      if (lead) {
-        umma::commit(&s.barM);
-        if (next_idx < total_tiles) stash_chunk(next_idx, (it + 1) & 1);      // warp 0 sits this build out: the look-up's latency hides here
-      }
+      if (lead) umma::commit(&s.barM);
     }
-    if (warp_u != 0) build_qkL(0, 48, tid - 32, NT - 32);      // into the dv_new, v, k Gam and dw^T tiles, which phase B1 read last
+    // =========================== phase D: one thread per key column and 16-row block ================================
+    // Its first part needs only accumulators of phases A and B1 and runs in three pieces while the products of B2, B3 and C execute.
+    build_qkL(sQL1, sKL1, false, warp_u, NT / 32, lane);      // the rest of phase C's operands: into the dw^T and v tiles, which phase B1 read last
+    // Decay inside the block as running products of lam_i = 2^(G_i - G_{i-1}) (every factor <= 1):
+    //   2^(G_i - G_first) = lam_1 .. lam_i,  2^(G_i) = g_first lam_1 .. lam_i,  2^(G_e - G_i) = lam_{i+1} .. lam_15,  2^(G_last - G_e) = e_last
+    const int kk = fresh_tid() & 127, blk = warp_u >> 2, t0 = 16 * blk;
+    float cq[16], cp[16], lam[16];
+    float g_first, e_last;
+    {
+      float prev = s.G[t0 * KD + kk];
+      g_first = ex2(prev);
+      lam[0] = 1.f;
+#pragma unroll
+      for (int i = 1; i < 16; ++i) {
+        const float cur = s.G[(t0 + i) * KD + kk];
+        lam[i] = ex2(cur - prev);
+        prev = cur;
+      }
+      const float Gl = s.G[(C - 1) * KD + kk];
+      if (blk == 3) s.hdh[kk] *= ex2(Gl);      // the state's own share of dG at the chunk's last row
+      e_last = ex2(Gl - prev);
+    }
+    {      // sum of k dk_end feeds dG at the chunk's last row (dk_end = dkg 2^(G_last - G))
+      float a[16];
+      umma::tmem_ld16(tq + C_DKG + t0, a);
+      umma::tmem_ld_wait();
+      float dglp = 0.f, fr = e_last;
+#pragma unroll
+      for (int i = 15; i >= 0; --i) {
+        dglp = fmaf(k_of(s.qk[(t0 + i) * KD + kk]), a[i] * fr, dglp);
+        fr *= lam[i];
+      }
+      s.dglp[blk][kk] = dglp;
+    }
     if (!mbar_wait(&s.barM, mph & 1)) alive = false;
     ++mph;
     umma::fence_after_sync();
@@ -530,14 +620,23 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     if (warp_u == 0) {
       const uint32_t aX = smem_u32(sX), aTI = smem_u32(s.TI);
       constexpr uint32_t iY = umma::instr_desc(64, 64, true, true);
-#pragma unroll
       const uint64_t dTiM = umma::desc_mnmajor(aTI, 0, SPAN), dXm = umma::desc_mnmajor(aX, 0, SPAN);
 #pragma unroll
       for (int sK = 0; sK < 4; ++sK)
         umma::mma_ss_lead(tb + C_XY, dTiM + static_cast<uint64_t>(sK) * 128u, dXm + static_cast<uint64_t>(sK) * 128u, iY, sK > 0, lead);
       if (lead) umma::commit(&s.barM);
     }
-    build_qkL(48, 96, tid, NT);
+    {      // dq: scale Gam dqg
+      float a[16];
+      umma::tmem_ld16(tq + C_DQG + t0, a);
+      umma::tmem_ld_wait();
+      float fl = p.scale * g_first;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        fl *= lam[i];
+        cq[i] = fl * a[i];
+      }
+    }
     if (!mbar_wait(&s.barM, mph & 1)) alive = false;
     ++mph;
     umma::fence_after_sync();
@@ -564,8 +663,8 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
             v[8 * cix + 2 * e + 1] = br * x1;
           }
         }
-        *reinterpret_cast<uint4*>(sw_piece(sDAK, i0, 2 * part)) = pack8(&v[0]);
-        *reinterpret_cast<uint4*>(sw_piece(sDAK, i0, 2 * part + 1)) = pack8(&v[8]);
+        *reinterpret_cast<uint4*>(sw_piece(sDA, da_row(i0) + 8, 2 * part)) = pack8(&v[0]);
+        *reinterpret_cast<uint4*>(sw_piece(sDA, da_row(i0) + 8, 2 * part + 1)) = pack8(&v[8]);
         s.dbp[4 + part][i0] = pb;
         if (part == q4) {
 #pragma unroll
@@ -587,95 +686,118 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     KDA_DBG_CLOCK(dbg, 9);
     // =========================== phase C: off-diagonal blocks of the intra-chunk terms ==============================
     if (warp_u == 0) {
-      const uint32_t aKR = smem_u32(sKR0), aQL = smem_u32(sQL0), aKL = smem_u32(sKL0), aDAQ = smem_u32(sDAQ), aDAK = smem_u32(sDAK);
-      const uint32_t lKR = smem_u32(sKR1) - aKR, lQL = smem_u32(sQL1) - aQL, lKL = smem_u32(sKL1) - aKL;
-      constexpr uint32_t iC1 = umma::instr_desc(128, 16, true, false);
+      constexpr uint32_t iC1 = umma::instr_desc(128, 32, true, false);
       constexpr uint32_t iC2 = umma::instr_desc(128, 16, true, true);
-      const uint64_t dKr = umma::smem_desc(aKR, lKR, umma::ATOM_BYTES), dQl = umma::smem_desc(aQL, lQL, umma::ATOM_BYTES);
-      const uint64_t dKl = umma::smem_desc(aKL, lKL, umma::ATOM_BYTES);
-      const uint64_t dAq = umma::smem_desc(aDAQ, 16, umma::ATOM_BYTES), dAk = umma::smem_desc(aDAK, 16, umma::ATOM_BYTES);
+      const uint64_t dKr = umma::smem_desc(smem_u32(sKR), KR_SPAN, umma::ATOM_BYTES), dDa = umma::smem_desc(smem_u32(sDA), 16, umma::ATOM_BYTES);
+      const uint64_t dAq = umma::smem_desc(smem_u32(sDA), 16, 2 * umma::ATOM_BYTES), dAk = dAq + umma::ATOM_BYTES / 16;      // every other atom
 #pragma unroll
       for (int I = 1; I < 4; ++I) {
         const int rb = (I == 1) ? 0 : (I == 2 ? 16 : 48);
 #pragma unroll
-        for (int sK = 0; sK < I; ++sK) {
-          const uint64_t dA = dKr + static_cast<uint64_t>((rb + 16 * sK) * 8);                 // A[kk][j] = kR_I[j][kk]: row offset in 16-byte units
-          const uint64_t bo = static_cast<uint64_t>(16 * I * 8 + sK * 2);                      // B[t][j]: rows 16 I.., k-step sK
-          umma::mma_ss_lead(tb + C_CQ + 16 * I, dA, dAq + bo, iC1, sK > 0, lead);
-          umma::mma_ss_lead(tb + C_CP + 16 * I, dA, dAk + bo, iC1, sK > 0, lead);
-        }
+        for (int sK = 0; sK < I; ++sK)      // A[kk][j] = kR_I[j][kk]: row offset in 16-byte units;  B[t][j]: rows 16 I.. of both, k-step sK
+          umma::mma_ss_lead(tb + C_CQP + 32 * (I - 1), dKr + static_cast<uint64_t>((rb + 16 * sK) * 8), dDa + static_cast<uint64_t>(32 * I * 8 + sK * 2), iC1, sK > 0, lead);
       }
+      const uint64_t dQl0 = umma::smem_desc(smem_u32(sQL0), L_SPAN, umma::ATOM_BYTES), dKl0 = umma::smem_desc(smem_u32(sKL0), L_SPAN, umma::ATOM_BYTES);
+      const uint64_t dQl1 = umma::smem_desc(smem_u32(sQL1), L_SPAN, umma::ATOM_BYTES), dKl1 = umma::smem_desc(smem_u32(sKL1), L_SPAN, umma::ATOM_BYTES);
 #pragma unroll
       for (int J = 0; J < 3; ++J) {
-        const int rb = (J == 0) ? 0 : (J == 1 ? 48 : 80);
+        const int rb = J == 2 ? 32 : 0;
 #pragma unroll
         for (int sK = 0; sK < 3 - J; ++sK) {
           const uint64_t ao = static_cast<uint64_t>((rb + 16 * sK) * 8);
-          const uint64_t bo = static_cast<uint64_t>((16 * (J + 1) + 16 * sK) * 8 + 2 * J);     // B[j][t] = dA[t][j]: rows t, columns 16 J..
-          umma::mma_ss_lead(tb + C_CN + 16 * J, dQl + ao, dAq + bo, iC2, sK > 0, lead);
-          umma::mma_ss_lead(tb + C_CN + 16 * J, dKl + ao, dAk + bo, iC2, 1, lead);
+          const uint64_t bo = static_cast<uint64_t>(32 * (J + 1 + sK) * 8 + 2 * J);            // B[j][t] = dA[t][j]: rows t, columns 16 J..
+          umma::mma_ss_lead(tb + C_CN + 16 * J, (J ? dQl1 : dQl0) + ao, dAq + bo, iC2, sK > 0, lead);
+          umma::mma_ss_lead(tb + C_CN + 16 * J, (J ? dKl1 : dKl0) + ao, dAk + bo, iC2, 1, lead);
         }
       }
       if (lead) umma::commit(&s.barM);
     }
-    // =========================== phase D: one thread per key column and 16-row block ================================
-    // Part 1 needs only accumulators of phases A and B1 and runs while phase C executes.
-    const int kk = fresh_tid() & 127, blk = warp_u >> 2, t0 = 16 * blk;
-    float cq[16], cp[16], lam[16];
-    float gam_last, e_last;
-    {
-      // Decay inside the block as running products of lam_i = 2^(G_i - G_{i-1}) (every factor <= 1):
-      //   2^(G_i - G_first) = fl_i,  2^(G_i) = 2^(G_first) fl_i,  2^(G_e - G_i) = fr_i,  2^(G_last - G_i) = 2^(G_last - G_e) fr_i
-      float a[16], a2[16];
-      float g_first;
-      {
-        float prev = s.G[t0 * KD + kk];
-        g_first = ex2(prev);
-        lam[0] = 1.f;
-#pragma unroll
-        for (int i = 1; i < 16; ++i) {
-          const float cur = s.G[(t0 + i) * KD + kk];
-          lam[i] = ex2(cur - prev);
-          prev = cur;
-        }
-        const float Glast = s.G[(C - 1) * KD + kk];
-        gam_last = ex2(Glast);
-        e_last = ex2(Glast - prev);
-      }
-      // dk-: dkg 2^(G_last - G);  sum of k dk_end feeds dG at the chunk's last row
-      umma::tmem_ld16(tq + C_DKG + t0, a);
-      umma::tmem_ld16(tq + C_DQG + t0, a2);
-      umma::tmem_ld_wait();
-      {
-        float dglp = 0.f, fr = 1.f;
-#pragma unroll
-        for (int i = 15; i >= 0; --i) {
-          dglp = fmaf(__bfloat162float(s.k[(t0 + i) * KD + kk]), a[i] * (e_last * fr), dglp);
-          fr *= lam[i];
-        }
-        s.dglp[blk][kk] = dglp;
-      }
-      // dq: scale Gam dqg
-      {
-        float fl = p.scale * g_first;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          fl *= lam[i];
-          cq[i] = fl * a2[i];
-        }
-      }
-      // dk+: Gam beta dbk
+    {      // dk+: Gam beta dbk
+      float a[16];
       umma::tmem_ld16(tq + C_DBK + t0, a);
+      float bt[16];
+      betas(t0, bt);
       umma::tmem_ld_wait();
-      {
-        float fl = g_first;
+      float fl = g_first;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          fl *= lam[i];
-          cp[i] = fl * s.beta[t0 + i] * a[i];
-        }
+      for (int i = 0; i < 16; ++i) {
+        fl *= lam[i];
+        cp[i] = fl * bt[i] * a[i];
       }
     }
+    // Diagonal block.  Rows 8..15 against columns 0..7, then 4..7 against 0..3 and 12..15 against 8..11, with the decay cut at the
+    // border between them: L_t = prod(border .. t) on the row side, R_j = prod(j+1 .. border-1) on the column side, both running products
+    // of lam (range-safe).  Factored this way an entry costs four multiply-adds instead of the eight operations of a pair with its
+    // own decay; only the 4 x 4 blocks on the diagonal stay pairwise.
+    // Four columns at a time, in rising order: behind its own columns a row is final (it only sees earlier ones), so dk- lives for four
+    // rows only (its other terms wait in tensor memory) and dq, dk leave for their staging tiles at once.  With dk- of all sixteen
+    // rows in registers the phase spilled, and spills miss the little L1 that is left: it took 6.4 k of a tile's 30 k cycles.
+    // dq and dk+ of a row, and the q- and k-side of everything they are made from, travel as a register pair: one instruction for both.
+    auto word = [&](int i) { return s.qk[(t0 + i) * KD + kk]; };
+    auto both = [&](int i) {      // (q, k) of a row
+      const uint32_t w = word(i);
+      return pair(q_of(w), k_of(w));
+    };
+    f32x2 cc[16];      // (dq, dk+)
+#pragma unroll
+    for (int i = 0; i < 16; ++i) cc[i] = pair(cq[i], cp[i]);
+    // keeps the compiler from carrying q, k (read from shared memory where they are used) or products of lam, and (a warp barrier orders memory accesses) from starting later
+    // loads early: sixteen loads of four registers in front of a part would not fit
+    auto step = [&] {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) asm volatile("" : "+f"(lam[i])::"memory");
+      __syncwarp();
+    };
+    float cn[4];
+    // rows r0 .. r0 + W - 1 against the four columns c0 .. c0 + 3, the border in front of row r0
+    auto part4 = [&](auto width, const int r0, const int c0) {
+      constexpr int W = decltype(width)::value;
+      f32x2 kR[4], sn[4];
+      float Rc = 1.f;
+#pragma unroll
+      for (int j = c0 + 4; j < r0; ++j) Rc *= lam[j];
+      {
+        float R = Rc;
+#pragma unroll
+        for (int j = 3; j >= 0; --j) {
+          const float x = k_of(word(c0 + j)) * R;
+          kR[j] = pair(x, x);
+          sn[j] = 0ull;
+          R *= lam[c0 + j];
+        }
+      }
+      float L = 1.f;
+#pragma unroll
+      for (int t = 0; t < W; ++t) {
+        if (t && t % 4 == 0) __syncwarp();
+        L *= lam[r0 + t];
+        const f32x2 LL = pair(L, L), ql = mul2(both(r0 + t), LL);
+        f32x2 sum = 0ull;
+#pragma unroll
+        for (int j = 0; j < 4; j += 2) {
+          const F4 a = lds4(reinterpret_cast<const float*>(&s.Ad[blk][r0 + t][c0 + j]));
+          sum = fma2(a.a, kR[j], sum);
+          sn[j] = fma2(a.a, ql, sn[j]);
+          sum = fma2(a.b, kR[j + 1], sum);
+          sn[j + 1] = fma2(a.b, ql, sn[j + 1]);
+        }
+        cc[r0 + t] = fma2(LL, sum, cc[r0 + t]);
+      }
+#pragma unroll
+      for (int j = 3; j >= 0; --j) {
+        const float2 x = halves(sn[j]);
+        cn[j] = fmaf(Rc, x.x + x.y, cn[j]);
+        Rc *= lam[c0 + j];
+      }
+    };
+    // the first four columns' share of the rows behind them, while the products of phase C execute
+#pragma unroll
+    for (int j = 0; j < 4; ++j) cn[j] = 0.f;
+    step();
+    part4(std::integral_constant<int, 8>{}, 8, 0);
+    step();
+    part4(std::integral_constant<int, 4>{}, 4, 0);
+    step();
     if (!mbar_wait(&s.barM, mph & 1)) alive = false;
     ++mph;
     alive = __syncthreads_and(alive);      // phase C complete; G has been read by everybody; dglp is complete
@@ -694,118 +816,60 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     KDA_DBG_CLOCK(dbg, 11);
     {
       {
-        // part 2: the off-diagonal blocks of phase C, scaled back from their reference rows
-        float b[16];
+        // the off-diagonal blocks of phase C, scaled back from their reference rows
         if (blk > 0) {                          // dq: + scale L Cq;  dk+: + L Cp
-          umma::tmem_ld16(tq + C_CQ + t0, b);
-          umma::tmem_ld_wait();
           float fl = 1.f;
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            fl *= lam[i];
-            cq[i] = fmaf(p.scale * fl, b[i], cq[i]);
-          }
-          umma::tmem_ld16(tq + C_CP + t0, b);
-          umma::tmem_ld_wait();
-          fl = 1.f;
+          for (int hf = 0; hf < 2; ++hf) {
+            float b[16];                        // eight rows of Cq, of Cp
+            umma::tmem_ld16(tq + C_CQP + 32 * (blk - 1) + 16 * hf, b);
+            umma::tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            fl *= lam[i];
-            cp[i] = fmaf(fl, b[i], cp[i]);
+            for (int i = 0; i < 8; ++i) {
+              fl *= lam[8 * hf + i];
+              const float2 c = halves(cc[8 * hf + i]);
+              cc[8 * hf + i] = pair(fmaf(p.scale * fl, b[i], c.x), fmaf(fl, b[8 + i], c.y));
+            }
           }
         }
       }
       KDA_DBG_CLOCK(dbg, 12);
-      // Diagonal block.  Rows 8..15 against columns 0..7, then 4..7 against 0..3 and 12..15 against 8..11, with the decay cut at the
-      // border between them: L_t = prod(border .. t) on the row side, R_j = prod(j+1 .. border-1) on the column side, both running products
-      // of lam (range-safe).  Factored this way an entry costs four multiply-adds instead of the eight operations of a pair with its
-      // own decay; only the 4 x 4 blocks on the diagonal stay pairwise.
-      // Four columns at a time, in rising order: behind its own columns a row is final (it only sees earlier ones), so dk- lives for four
-      // rows only (its other terms wait in tensor memory) and dq, dk leave for their staging tiles at once.  With dk- of all sixteen
-      // rows in registers the phase spilled, and spills miss the little L1 that is left: it took 6.4 k of a tile's 30 k cycles.
-      auto qof = [&](int i) { return __bfloat162float(s.q[(t0 + i) * KD + kk]); };
-      auto kof = [&](int i) { return __bfloat162float(s.k[(t0 + i) * KD + kk]); };
-      // keeps the compiler from carrying q, k (read from shared memory where they are used) or products of lam, and (a warp barrier orders memory accesses) from starting later
-      // loads early: sixteen loads of four registers in front of a part would not fit
-      auto step = [&] {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) asm volatile("" : "+f"(lam[i])::"memory");
-        __syncwarp();
-      };
-      float cn[4];
-      // rows r0 .. r0 + W - 1 against the four columns c0 .. c0 + 3, the border in front of row r0
-      auto part4 = [&](auto width, const int r0, const int c0) {
-        constexpr int W = decltype(width)::value;
-        float kR[4], sn[4];
-        float Rc = 1.f;
-#pragma unroll
-        for (int j = c0 + 4; j < r0; ++j) Rc *= lam[j];
-        {
-          float R = Rc;
-#pragma unroll
-          for (int j = 3; j >= 0; --j) {
-            kR[j] = kof(c0 + j) * R;
-            sn[j] = 0.f;
-            R *= lam[c0 + j];
-          }
-        }
-        float L = 1.f;
-#pragma unroll
-        for (int t = 0; t < W; ++t) {
-          if (t && t % 4 == 0) __syncwarp();
-          L *= lam[r0 + t];
-          const float ql = qof(r0 + t) * L, kl = kof(r0 + t) * L;
-          float sq = 0.f, sp = 0.f;
-#pragma unroll
-          for (int j = 0; j < 4; j += 2) {
-            const float4 a = *reinterpret_cast<const float4*>(&s.Ad[blk][r0 + t][c0 + j]);
-            sq = fmaf(a.x, kR[j], sq);
-            sp = fmaf(a.y, kR[j], sp);
-            sn[j] = fmaf(a.x, ql, fmaf(a.y, kl, sn[j]));
-            sq = fmaf(a.z, kR[j + 1], sq);
-            sp = fmaf(a.w, kR[j + 1], sp);
-            sn[j + 1] = fmaf(a.z, ql, fmaf(a.w, kl, sn[j + 1]));
-          }
-          cq[r0 + t] = fmaf(L, sq, cq[r0 + t]);
-          cp[r0 + t] = fmaf(L, sp, cp[r0 + t]);
-        }
-#pragma unroll
-        for (int j = 3; j >= 0; --j) {
-          cn[j] = fmaf(Rc, sn[j], cn[j]);
-          Rc *= lam[c0 + j];
-        }
-      };
       auto columns = [&](auto first) {
         constexpr int c0 = decltype(first)::value;
         {      // dk-: 2^(G_e - G) (2^(G_last - G_e) dkg + Cn)
-          float d4[4];
+          float d4[4], b4[4];
           umma::tmem_ld4(tq + C_DKG + t0 + c0, d4);
-          if (blk < 3) umma::tmem_ld4(tq + C_CN + t0 + c0, cn);
+          if (blk < 3) umma::tmem_ld4(tq + C_CN + t0 + c0, b4);
           umma::tmem_ld_wait();
           float fr = 1.f;
 #pragma unroll
           for (int j = c0 + 4; j < 16; ++j) fr *= lam[j];
 #pragma unroll
           for (int j = 3; j >= 0; --j) {
-            cn[j] = fr * (blk < 3 ? fmaf(e_last, d4[j], cn[j]) : e_last * d4[j]);
+            const float x = fr * (blk < 3 ? fmaf(e_last, d4[j], b4[j]) : e_last * d4[j]);
+            cn[j] = c0 ? x : cn[j] + x;
             fr *= lam[c0 + j];
           }
         }
         step();
-        if constexpr (c0 < 8) {
+        if constexpr (c0 == 4) {
           part4(std::integral_constant<int, 8>{}, 8, c0);
           step();
         }
-        if constexpr (c0 % 8 == 0) {
+        if constexpr (c0 == 8) {
           part4(std::integral_constant<int, 4>{}, c0 + 4, c0);
           step();
         }
+        uint32_t w[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) w[t] = word(c0 + t);
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-          const float qt = qof(c0 + t), kt = kof(c0 + t);
+          const float qt = q_of(w[t]), kt = k_of(w[t]);
+          float2 c = halves(cc[c0 + t]);
           {
             const float ax = s.Ad[blk][c0 + t][c0 + t].x;      // dAkk has no diagonal
-            cq[c0 + t] = fmaf(ax, kt, cq[c0 + t]);
+            c.x = fmaf(ax, kt, c.x);
             cn[t] = fmaf(ax, qt, cn[t]);
           }
           float D = 1.f;
@@ -813,19 +877,21 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
           for (int j = t - 1; j >= 0; --j) {
             D *= lam[c0 + j + 1];
             const float2 a = s.Ad[blk][c0 + t][c0 + j];
-            const float kd = kof(c0 + j) * D;
-            cq[c0 + t] = fmaf(a.x, kd, cq[c0 + t]);
-            cp[c0 + t] = fmaf(a.y, kd, cp[c0 + t]);
+            const float kd = k_of(w[j]) * D;
+            c.x = fmaf(a.x, kd, c.x);
+            c.y = fmaf(a.y, kd, c.y);
             cn[j] = fmaf(D, fmaf(a.y, kt, a.x * qt), cn[j]);
           }
+          cc[c0 + t] = pair(c.x, c.y);
         }
         // dq, dk into their staging tiles; cq becomes dG
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
           const int i = c0 + t;
-          stq[(t0 + i) * KD + kk] = __float2bfloat16_rn(cq[i]);
-          stk[(t0 + i) * KD + kk] = __float2bfloat16_rn(cp[i] + cn[t]);
-          cq[i] = qof(i) * cq[i] + kof(i) * (cp[i] - cn[t]);
+          const float2 c = halves(cc[i]);
+          stq[(t0 + i) * KD + kk] = __float2bfloat16_rn(c.x);
+          stk[(t0 + i) * KD + kk] = __float2bfloat16_rn(c.y + cn[t]);
+          cq[i] = q_of(w[t]) * c.x + k_of(w[t]) * (c.y - cn[t]);
         }
         step();
       };
@@ -835,7 +901,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
       columns(std::integral_constant<int, 12>{});
       KDA_DBG_CLOCK(dbg, 13);
       if (blk == 3)          // the chunk's last row carries the chunk-end terms
-        cq[15] += s.dglp[0][kk] + s.dglp[1][kk] + s.dglp[2][kk] + s.dglp[3][kk] + gam_last * s.hdh[kk];
+        cq[15] += s.dglp[0][kk] + s.dglp[1][kk] + s.dglp[2][kk] + s.dglp[3][kk] + s.hdh[kk];
       {
         float run = 0.f;
 #pragma unroll
@@ -845,37 +911,19 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
         }
         s.carry[blk][kk] = run;
       }
-      // L2: the normalised q, k pieces and the reciprocal norms this thread needs for its two copy-out pieces, asked
-      // for before the barrier so that they arrive behind it
-      uint4 yq2[2], yk2[2];
+      // L2: the reciprocal norms of this thread's two copy-out pieces, asked for before the barrier so that they arrive behind it
       float rq2[2], rk2[2];
       if constexpr (L2) {
         static_assert(C * 16 == 2 * NT, "two copy-out pieces per thread");
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-          const int i = tid + u * NT, r = i >> 4, pc = i & 15;
+          const int r = (tid + u * NT) >> 4;
           const size_t grow = static_cast<size_t>(ci.tok0 + (r < len ? r : 0)) * p.H + h;
-          yq2[u] = __ldg(reinterpret_cast<const uint4*>(p.q + grow * p.qc + pc * 8));
-          yk2[u] = __ldg(reinterpret_cast<const uint4*>(p.k + grow * p.qc + pc * 8));
           rq2[u] = __ldg(p.rstd + grow);
           rk2[u] = __ldg(p.rstd + p.qrows + grow);
         }
       }
       __syncthreads();       // block totals and the staged dq, dk are complete
-      {
-        float add = 0.f;             // totals of the later blocks
-#pragma unroll
-        for (int bb = 1; bb < 4; ++bb) add += (bb > blk) ? s.carry[bb][kk] : 0.f;
-        if (len == C) {      // into the q, k tiles, which everybody has read
-#pragma unroll
-          for (int i = 0; i < 16; ++i) stg[(t0 + i) * KD + kk] = cq[i] + add;
-        } else {
-        float* const dgp = p.dg + (static_cast<size_t>(ci.tok0 + t0) * p.H + h) * p.kc + kk;      // a warp stores 128 contiguous bytes
-#pragma unroll
-        for (int i = 0; i < 16; ++i)
-          if (t0 + i < len && kk < p.kc) dgp[static_cast<size_t>(i) * p.H * p.kc] = cq[i] + add;
-        }
-      }
       if (L2 || len < C)
 #pragma unroll
       for (int u = 0; u < C * 16 / NT; ++u) {
@@ -884,18 +932,18 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
         uint4 oq = *reinterpret_cast<const uint4*>(&stq[r * KD + pc * 8]);
         uint4 ok = *reinterpret_cast<const uint4*>(&stk[r * KD + pc * 8]);
         if constexpr (L2) {
-          // dx = rstd (dy - y <y, dy>) per row; sixteen consecutive lanes hold one row (y: the normalised q, k, re-read
-          // from global memory -- the tile loaded them a few microseconds ago; dy: the staged bf16 values, as the
-          // separate pass would read them)
-          const uint4 yq = yq2[u], yk = yk2[u];
+          // dx = rstd (dy - y <y, dy>) per row; sixteen consecutive lanes hold one row (y: the normalised q, k; dy: the staged bf16 values, as
+          // the separate pass would read them)
+          uint32_t y[8];
+          *reinterpret_cast<uint4*>(&y[0]) = *reinterpret_cast<const uint4*>(&s.qk[r * KD + pc * 8]);
+          *reinterpret_cast<uint4*>(&y[4]) = *reinterpret_cast<const uint4*>(&s.qk[r * KD + pc * 8 + 4]);
           const uint32_t dqw[4] = {oq.x, oq.y, oq.z, oq.w}, dkw[4] = {ok.x, ok.y, ok.z, ok.w};
-          const uint32_t yqw[4] = {yq.x, yq.y, yq.z, yq.w}, ykw[4] = {yk.x, yk.y, yk.z, yk.w};
           float2 dqf[4], dkf[4], yqf[4], ykf[4];
           float sq = 0.f, sk = 0.f;
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             dqf[e] = unpack_bf16(dqw[e]); dkf[e] = unpack_bf16(dkw[e]);
-            yqf[e] = unpack_bf16(yqw[e]); ykf[e] = unpack_bf16(ykw[e]);
+            yqf[e] = make_float2(q_of(y[2 * e]), q_of(y[2 * e + 1])); ykf[e] = make_float2(k_of(y[2 * e]), k_of(y[2 * e + 1]));
             sq = fmaf(yqf[e].x, dqf[e].x, fmaf(yqf[e].y, dqf[e].y, sq));
             sk = fmaf(ykf[e].x, dkf[e].x, fmaf(ykf[e].y, dkf[e].y, sk));
           }
@@ -917,6 +965,21 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
         if (r < len && pc * 8 < p.dqc) {
           *reinterpret_cast<uint4*>(p.dq + row) = oq;
           *reinterpret_cast<uint4*>(p.dk + row) = ok;
+        }
+      }
+      if constexpr (L2) __syncthreads();      // q and k have been read
+      {
+        float add = 0.f;             // totals of the later blocks
+#pragma unroll
+        for (int bb = 1; bb < 4; ++bb) add += (bb > blk) ? s.carry[bb][kk] : 0.f;
+        if (len == C) {      // into the q, k tiles, which everybody has read
+#pragma unroll
+          for (int i = 0; i < 16; ++i) stg[(t0 + i) * KD + kk] = cq[i] + add;
+        } else {
+        float* const dgp = p.dg + (static_cast<size_t>(ci.tok0 + t0) * p.H + h) * p.kc + kk;      // a warp stores 128 contiguous bytes
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (t0 + i < len && kk < p.kc) dgp[static_cast<size_t>(i) * p.H * p.kc] = cq[i] + add;
         }
       }
     }
