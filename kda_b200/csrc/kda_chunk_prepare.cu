@@ -213,6 +213,13 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
       else if (p.beta_fp32) beta_bits = __ldg(static_cast<const uint32_t*>(p.beta_raw) + i);
       else beta_bits = static_cast<uint32_t>(__ldg(static_cast<const unsigned short*>(p.beta_raw) + i)) << 16;
     }
+    // the gate's parameters with the rest: asked for where they are used, behind the wait for g, they cost a round trip of their own
+    float al = 0.f;
+    float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p.g_raw) {
+      al = __ldg(p.A_log + h);
+      if (p.dt_bias && kk < p.kc) bias = __ldg(reinterpret_cast<const float4*>(p.dt_bias + static_cast<size_t>(h) * p.kc + kk));
+    }
     if (tid == 0) {
       mbar_init(&s.barV, 1);
       fence_mbar_init();
@@ -240,9 +247,7 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
     }
     // the gate's activation here instead of in a kernel of its own: one launch less, and the fp32 g is never read back (forward only: never written)
     if (p.g_raw) {
-      const float al = __expf(__ldg(p.A_log + h));
-      float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (p.dt_bias && kk < p.kc) bias = __ldg(reinterpret_cast<const float4*>(p.dt_bias + static_cast<size_t>(h) * p.kc + kk));
+      al = __expf(al);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         if (t0 + i >= len || kk >= p.kc) continue;
