@@ -16,14 +16,16 @@
 //                   a row follow from that row's q, k, g, and its dq^, dk^, dg are sums along the row.
 // Walks: a warp holds 16 or 32 columns of all K rows (a lane 16 rows x 4 or 8 columns, packed two rows to a register pair), and nothing is
 // shared between warps but the staged q, k, exp g.
-// Middle: a thread holds 8 columns of 4 rows of S and dS.  S' of four tokens lives in registers; states in between are replayed from the
-// state at every eighth token in shared memory: 11.5 multiply-adds per element and token instead of 9, and no per-token state through memory
-// (128 KB per token: what a CTA per sequence waited for).  The tile's shape is set by shared-memory bandwidth, which is 128 bytes per cycle
+// Middle: a thread holds 8 columns of 4 rows of S and dS.  S' of four tokens lives in registers; the states between are replayed once and kept as they
+// are, every fourth token, in tensor memory (256 columns a CTA, which nothing else here uses): 10.5 multiply-adds per element and token, and no
+// per-token state through memory (128 KB per token: what a CTA per sequence waited for).  Every eighth token's in shared memory, replayed
+// further from there: 9.33 -> 9.03 ms for the whole step.  The tile's shape is set by shared-memory bandwidth, which is 128 bytes per cycle
 // delivered to registers, broadcast or not: with 16 columns of one row a thread read 90 floats per 16 elements and token (92 % of the LSU's rate,
-// 7.5 ms), with 4 x 8 it reads 36 (5.9 ms).
+// 7.5 ms), with 4 x 8 it reads 36 (5.0 ms, with the states in tensor memory 4.7).
 // What bounds them: the FP32 pipe (60 % busy; one CTA's load of its rows and states under the other's arithmetic) and, in the walks,
-// the 256 units' uneven share of 148 SMs.  8 x 2048 tokens x 32 heads of 128: forward walk 2.14, backward walk 2.11, middle 5.0 ms; 25.7 ms for
-// the whole step as a CTA per sequence -> 9.3.  One sequence x 32 heads: 12.8 -> 2.4 ms; 2 x 200 tokens x 8 heads: 1.23 -> 0.24.
+// the 256 units' uneven share of 148 SMs.  8 x 2048 tokens x 32 heads of 128: forward walk 2.14, backward walk 2.11, middle 4.7 ms; 25.7 ms for
+// the whole step as a CTA per sequence -> 9.03.  One sequence x 32 heads: 12.8 -> 2.39 ms; 2 x 200 tokens x 8 heads: 1.23 -> 0.23.
+// (Walks of two tokens a step, seven multiply-adds instead of eight and one reduction: 1 % less at 256 units, 5 % more at 32.)
 // dq^, dk^ (gradients w.r.t. the possibly L2-normalised rows, per VALUE head) go to the workspace; a last kernel sums grouped value
 // heads, applies the normalisation's backward (fla/modules/l2norm.py:190-240) and writes dq, dk; with neither they are dq, dk.  Every sum has a
 // fixed order.
@@ -32,6 +34,7 @@
 #include "kda_common.cuh"
 #include "kda_device.cuh"
 #include "kda_f32x2.cuh"
+#include "kda_umma.cuh"
 
 namespace kda {
 
@@ -407,9 +410,9 @@ struct Mid {
     float q[TC][RP];             // scale q^, then dq^
     float k[TC][RP];             // k^, then dk^
     float a[TC][RP];             // exp g, then dg
-    float4 state[3][8][NT];      // this thread's part of the state in front of tokens 8, 16, 24
     float wdo[TC];               // <w, do>
     float beta[TC];
+    uint32_t tmem_slot;
     int n;
   };
 };
@@ -421,7 +424,7 @@ __global__ void __launch_bounds__(Mid<K, V>::NT, 2) kda_recurrent_mid_kernel(con
   constexpr int NT = M::NT, ROWS = M::ROWS, LPR = M::LPR;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   typename M::Smem& s = *reinterpret_cast<typename M::Smem*>(smem_raw);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int slice = blockIdx.x % M::SLICES, h = blockIdx.x / M::SLICES % p.H, hq = h / (p.H / p.HQ);
   const long long slot = blockIdx.x / M::SLICES / p.H;
   if (tid == 0) {      // the last sequence whose first slot is not behind this one
@@ -441,6 +444,8 @@ __global__ void __launch_bounds__(Mid<K, V>::NT, 2) kda_recurrent_mid_kernel(con
   const int cnt = static_cast<int>(min(static_cast<long long>(TC), sq.len - c * TC));
   const size_t tok0 = static_cast<size_t>(sq.bos + c * TC);
 
+  // Tensor memory holds the states between: this thread's part of the state in front of tokens 0, 4, .. 24, 32 words each (the fp32 values themselves)
+  if (warp == 0) umma::tmem_alloc(&s.tmem_slot, 256);
   // ---- this thread's eight columns of four rows of S and dS; the tokens' rows -------------------------------------------------------
   const int l = lane % LPR, lrow = warp * M::RPW + 4 * (lane / LPR);
   const size_t sbase = ((static_cast<size_t>(slot) * p.H + h) * K + slice * ROWS + lrow) * V + 4 * l;
@@ -486,7 +491,10 @@ __global__ void __launch_bounds__(Mid<K, V>::NT, 2) kda_recurrent_mid_kernel(con
     p.dbeta[(tok0 + tid) * p.H + h] = sum;
   }
   cp_async_wait<0>();
+  umma::fence_before_sync();
   __syncthreads();
+  umma::fence_after_sync();
+  const uint32_t tq = __shfl_sync(0xffffffffu, s.tmem_slot, 0) + (static_cast<uint32_t>(32 * warp) << 16);      // this warp's lanes
   for (int t = warp; t < TC; t += M::NW) {
     constexpr int E = V / 32;
     float w[E], d[E], dot = 0.f;
@@ -542,27 +550,37 @@ __global__ void __launch_bounds__(Mid<K, V>::NT, 2) kda_recurrent_mid_kernel(con
       step(S, S, t + j);
     }
   };
-#pragma unroll 1
-  for (int i = 0; i < 3; ++i) {
-    step4(8 * i);
-    step4(8 * i + 4);
+  auto keep = [&](int slot) {
 #pragma unroll
-    for (int m = 0; m < 8; ++m) sts4(reinterpret_cast<float*>(&s.state[i][m][tid]), F4{S[m >> 1][2 * (m & 1)], S[m >> 1][2 * (m & 1) + 1]});
+    for (int m = 0; m < 2; ++m) {
+      float x[16];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float2 y = halves(S[2 * m + (i >> 2)][i & 3]);
+        x[2 * i] = y.x;
+        x[2 * i + 1] = y.y;
+      }
+      umma::tmem_st16(tq + 32 * slot + 16 * m, x);
+    }
+  };
+  auto fetch = [&](int slot) {
+    float x[2][16];
+    umma::tmem_ld16(tq + 32 * slot, x[0]);
+    umma::tmem_ld16(tq + 32 * slot + 16, x[1]);
+    umma::tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) S[i >> 2][i & 3] = pair(x[i >> 3][2 * (i & 7)], x[i >> 3][2 * (i & 7) + 1]);
+  };
+#pragma unroll 1
+  for (int i = 0; i < 7; ++i) {
+    keep(i);
+    step4(4 * i);
   }
+  umma::tmem_st_wait();
 #pragma unroll 1
   for (int half = 7; half >= 0; --half) {      // four tokens each, the last first
     const int t0 = 4 * half;
-    if (half < 2) {
-      load_state(S, p.ckpt);
-    } else {
-#pragma unroll
-      for (int m = 0; m < 8; ++m) {
-        const F4 x = lds4(reinterpret_cast<const float*>(&s.state[(half >> 1) - 1][m][tid]));
-        S[m >> 1][2 * (m & 1)] = x.a;
-        S[m >> 1][2 * (m & 1) + 1] = x.b;
-      }
-    }
-    if (half & 1) step4(t0 - 4);
+    if (half < 7) fetch(half);
     Tile Sp[4];      // S' of the four tokens
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -643,6 +661,7 @@ __global__ void __launch_bounds__(Mid<K, V>::NT, 2) kda_recurrent_mid_kernel(con
     }
     __syncwarp();
   }
+  umma::fence_before_sync();
   __syncthreads();
   for (int i = tid; i < cnt * ROWS; i += NT) {
     const int t = i / ROWS, row = i % ROWS;
@@ -651,6 +670,7 @@ __global__ void __launch_bounds__(Mid<K, V>::NT, 2) kda_recurrent_mid_kernel(con
     p.dkh[o] = s.k[t][row];
     p.dg[o] = s.a[t][row];
   }
+  if (warp == 0) umma::tmem_dealloc(s.tmem_slot, 256);
 }
 
 // dq, dk from the per-value-head gradients w.r.t. the rows the recurrence saw: sum over the value heads of a group,
