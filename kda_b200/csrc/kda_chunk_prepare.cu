@@ -248,14 +248,22 @@ __global__ void __launch_bounds__(PREP_THREADS, 2) kda_chunk_prepare_kernel(cons
     // the gate's activation here instead of in a kernel of its own: one launch less, and the fp32 g is never read back (forward only: never written)
     if (p.g_raw) {
       al = __expf(al);
+      // every element first, then the choice: a branch per row would keep the rows' exponentials apart
+      auto activate = [&](const int use_lb) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 x = halves(lam[i].a), y = halves(lam[i].b);
+          lam[i] = {pair(gate_value(x.x + bias.x, al, use_lb, p.lb), gate_value(x.y + bias.y, al, use_lb, p.lb)),
+                    pair(gate_value(y.x + bias.z, al, use_lb, p.lb), gate_value(y.y + bias.w, al, use_lb, p.lb))};
+        }
+      };
+      if (p.use_lb) activate(1);
+      else activate(0);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        if (t0 + i >= len || kk >= p.kc) continue;
-        const float2 x = halves(lam[i].a), y = halves(lam[i].b);
-        const float4 g4 = make_float4(gate_value(x.x + bias.x, al, p.use_lb, p.lb), gate_value(x.y + bias.y, al, p.use_lb, p.lb),
-                                      gate_value(y.x + bias.z, al, p.use_lb, p.lb), gate_value(y.y + bias.w, al, p.use_lb, p.lb));
-        lam[i] = {pair(g4.x, g4.y), pair(g4.z, g4.w)};
-        if (p.g_out) *reinterpret_cast<float4*>(p.g_out + goff + i * gs) = g4;
+        const bool ok = t0 + i < len && kk < p.kc;
+        if (ok && p.g_out) *reinterpret_cast<ulonglong2*>(p.g_out + goff + i * gs) = make_ulonglong2(lam[i].a, lam[i].b);
+        if (!ok) lam[i] = {0ull, 0ull};
       }
     }
   }
