@@ -239,6 +239,8 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     }
   };
 
+  // heads narrower than the tiles (zeros beyond kc, vc): products stop at the last 16 columns that hold something
+  const int v_steps = (p.vc + 15) >> 4, k_steps = (p.kc + 15) >> 4;
   uint32_t mph = 0;      // phase counter of barM
   bool alive = true;
   int it = 0;
@@ -310,7 +312,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
       const uint64_t dVNm = umma::desc_mnmajor(aVN, 0, SPAN), dDVNm = umma::desc_mnmajor(aDVN, 0, SPAN);
       const uint64_t dDO0 = umma::desc_kmajor(aDO, 0), dDO1 = umma::desc_kmajor(aDO + 8192, 0);
 #pragma unroll 1
-      for (int sK = 0; sK < 8; ++sK) {
+      for (int sK = 0; sK < v_steps; ++sK) {
         const uint64_t mn = static_cast<uint64_t>(sK) * 128u, dDOk = ((sK >> 2) ? dDO1 : dDO0) + static_cast<uint64_t>(sK & 3) * 2u;
         umma::mma_ss_lead(tb + C_DQG, dHS + mn, dDOk, i1, sK > 0, lead);                 // dqg^T = h dO^T
         umma::mma_ss_lead(tb + C_DW, dHS + mn, dDVNm + mn, i2, sK > 0, lead);            // dw^T = -h dv_new^T
@@ -458,12 +460,12 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
       const uint64_t dKg0 = umma::desc_kmajor(aKG, 0), dKg1 = umma::desc_kmajor(aKG + 8192, 0);
       const uint64_t dDuK = umma::desc_kmajor(aDVN, 0), dDwK = umma::desc_kmajor(aDWT, 0);
 #pragma unroll 1
-      for (int sK = 0; sK < 8; ++sK) {
+      for (int sK = 0; sK < v_steps; ++sK) {
         const uint64_t mn = static_cast<uint64_t>(sK) * 128u, dVk = ((sK >> 2) ? dV1 : dV0) + static_cast<uint64_t>(sK & 3) * 2u;
         umma::mma_ss_lead(tb + C_DAQ, dDuM + mn, dVk, iT, sK > 0, lead);       // dTm[t][j]   += sum_v du[t][v] v[j][v]
       }
 #pragma unroll 1
-      for (int sK = 0; sK < 8; ++sK) {
+      for (int sK = 0; sK < k_steps; ++sK) {
         const uint64_t mn = static_cast<uint64_t>(sK) * 128u, dKg = ((sK >> 2) ? dKg1 : dKg0) + static_cast<uint64_t>(sK & 3) * 2u;
         umma::mma_ss_lead(tb + C_DAQ, dDwM + mn, dKg, iT, 1, lead);            // += sum_kk dw[t][kk] kGam[j][kk]
       }
