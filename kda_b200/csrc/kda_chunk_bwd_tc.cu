@@ -73,6 +73,7 @@ struct TcSmem {
   };
   float carry[4][KD];           // block totals of the reverse cumsum
   uint64_t barS, barG, barQ, barB, barM;      // (in this order: drained together)
+  uint64_t barT;                // every warp's share of an operand tile of B2, B3 or C is written
   long long ci_tok0[2];         // first token and length of the chunk of the current / next tile (written by thread 0)
   int ci_len[2];
   uint32_t tmem_slot;
@@ -173,6 +174,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     mbar_init(&s.barQ, 2);
     mbar_init(&s.barB, 4);
     mbar_init(&s.barM, 1);
+    mbar_init(&s.barT, NT / 32);
     fence_mbar_init();
     if (static_cast<int>(blockIdx.x) < total_tiles) {
       stash_chunk(blockIdx.x, 0);
@@ -241,6 +243,21 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
 
   // heads narrower than the tiles (zeros beyond kc, vc): products stop at the last 16 columns that hold something
   const int v_steps = (p.vc + 15) >> 4, k_steps = (p.kc + 15) >> 4;
+  // Operands of B2, B3 and C go to the issuing warp through barT: a warp hands its share over and goes on with what does not depend on the product,
+  // instead of meeting everybody at a barrier first (the products then start while dv, dbeta and the rest are still being written)
+  uint32_t tph = 0;      // phase counter of barT
+  auto hand_over = [&](int lane) {
+    fence_proxy_async();
+    umma::fence_before_sync();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&s.barT);
+    ++tph;
+  };
+  auto handed_over = [&] {
+    const bool ok = mbar_wait(&s.barT, (tph - 1) & 1);
+    umma::fence_after_sync();
+    return ok;
+  };
   uint32_t mph = 0;      // phase counter of barM
   bool alive = true;
   int it = 0;
@@ -489,15 +506,33 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     ++mph;
     umma::fence_after_sync();
     KDA_DBG_CLOCK(dbg, 5);
-    if (alive) {
-      float v[16], v3[16];                             // both loads are in flight together
+    {
+      float v[16], bt[16];
       umma::tmem_ld16(tq + C_DAQ + 16 * part, v);      // dTm rows (M = 64 layout): scale the columns by beta_j
-      umma::tmem_ld16(tq + C_DBV + 16 * part, v3);     // dbv^T rows v: dv[t][v] = beta_t dbv[t][v]
-      float bt[16];
       betas(16 * part, bt);
       umma::tmem_ld_wait();
-      {      // dbeta_j += sum_t Tm[t][j] dTm_raw[t][j]: rows t are lanes 0..15 (what the others compute is not used); afterwards lane j holds column j
+      if (lane < 16) {
+        const int t = 16 * q4 + lane;
         float x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = v[i] * bt[i];
+        *reinterpret_cast<uint4*>(sw_piece(sDT, t, 2 * part)) = pack8(&x[0]);
+        *reinterpret_cast<uint4*>(sw_piece(sDT, t, 2 * part + 1)) = pack8(&x[8]);
+      }
+      hand_over(lane);
+      // =========================== phase B2: X = dTm Tm^T ============================================================
+      if (warp_u == 0) {
+        if (!handed_over()) alive = false;
+        const uint32_t aDT = smem_u32(sDT), aTI = smem_u32(s.TI);
+        constexpr uint32_t iX = umma::instr_desc(64, 64, false, false);
+        const uint64_t dDt = umma::desc_kmajor(aDT, 0), dTiK = umma::desc_kmajor(aTI, 0);
+        if (alive) {
+#pragma unroll
+          for (int sK = 0; sK < 4; ++sK) umma::mma_ss_lead(tb + C_XY, dDt + static_cast<uint64_t>(sK) * 2u, dTiK + static_cast<uint64_t>(sK) * 2u, iX, sK > 0, lead);
+          if (lead) umma::commit(&s.barM);
+        }
+      }
+      {      // dbeta_j += sum_t Tm[t][j] dTm_raw[t][j]: rows t are lanes 0..15 (what the others compute is not used); afterwards lane j holds column j
 #pragma unroll
         for (int cix = 0; cix < 2; ++cix) {
           const uint4 tm = *reinterpret_cast<const uint4*>(sw_piece(s.TI, 16 * q4 + (lane & 15), 2 * part + cix));
@@ -505,62 +540,34 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const float2 y = unpack_bf16(w[e]);
-            x[8 * cix + 2 * e] = y.x * v[8 * cix + 2 * e];
-            x[8 * cix + 2 * e + 1] = y.y * v[8 * cix + 2 * e + 1];
+            v[8 * cix + 2 * e] *= y.x;
+            v[8 * cix + 2 * e + 1] *= y.y;
           }
         }
 #pragma unroll
         for (int o = 8; o >= 1; o >>= 1) {
           const bool up = (lane & o) != 0;
 #pragma unroll
-          for (int i = 0; i < o; ++i) x[i] = (up ? x[i + o] : x[i]) + __shfl_xor_sync(0xffffffffu, up ? x[i] : x[i + o], o);
+          for (int i = 0; i < o; ++i) v[i] = (up ? v[i + o] : v[i]) + __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + o], o);
         }
-        if (lane < 16) s.dbp[q4][16 * part + lane] = x[0];
+        if (lane < 16) s.dbp[q4][16 * part + lane] = v[0];
       }
-      if (lane < 16) {
-        const int t = 16 * q4 + lane;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] *= bt[i];
-        *reinterpret_cast<uint4*>(sw_piece(sDT, t, 2 * part)) = pack8(&v[0]);
-        *reinterpret_cast<uint4*>(sw_piece(sDT, t, 2 * part + 1)) = pack8(&v[8]);
-      }
+      umma::tmem_ld16(tq + C_DBV + 16 * part, v);      // dbv^T rows v: dv[t][v] = beta_t dbv[t][v]
+      umma::tmem_ld_wait();
       if (len == C) {      // staged in the dv_new tile, which the products have read, and stored by the copy engine
         __nv_bfloat16* const st = reinterpret_cast<__nv_bfloat16*>(dv_stage(q4)) + 16 * part * 32 + lane;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) st[32 * i] = __float2bfloat16_rn(bt[i] * v3[i]);
+        for (int i = 0; i < 16; ++i) st[32 * i] = __float2bfloat16_rn(bt[i] * v[i]);
       } else {
         const int vcol = 32 * q4 + lane;
         __nv_bfloat16* const dvp = p.dv + (static_cast<size_t>(ci.tok0 + 16 * part) * p.H + h) * p.vc + vcol;
         const size_t tstride = static_cast<size_t>(p.H) * p.vc;
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          if (16 * part + i < len && vcol < p.vc) dvp[i * tstride] = __float2bfloat16_rn(bt[i] * v3[i]);
+          if (16 * part + i < len && vcol < p.vc) dvp[i * tstride] = __float2bfloat16_rn(bt[i] * v[i]);
       }
     }
-    fence_proxy_async();
-    umma::fence_before_sync();
-    alive = __syncthreads_and(alive);
-    if (!alive) {
-      if (tid == 0) atomicOr(p.status, 64u);
-      break;
-    }
-    umma::fence_after_sync();
-
     KDA_DBG_CLOCK(dbg, 6);
-    if (warp_u == 4 && lane == 0 && len == C) {
-#pragma unroll 1
-      for (int i = 0; i < 4 && 32 * i < p.vc; ++i) tma_store_rows(&p.tm_dv, 32 * i, h, ci.tok0, dv_stage(i));
-      bulk_commit();
-    }
-    // =========================== phase B2: X = dTm Tm^T ============================================================
-    if (warp_u == 0) {
-      const uint32_t aDT = smem_u32(sDT), aTI = smem_u32(s.TI);
-      constexpr uint32_t iX = umma::instr_desc(64, 64, false, false);
-      const uint64_t dDt = umma::desc_kmajor(aDT, 0), dTiK = umma::desc_kmajor(aTI, 0);
-#pragma unroll
-      for (int sK = 0; sK < 4; ++sK) umma::mma_ss_lead(tb + C_XY, dDt + static_cast<uint64_t>(sK) * 2u, dTiK + static_cast<uint64_t>(sK) * 2u, iX, sK > 0, lead);
-      if (lead) umma::commit(&s.barM);
-    }
     // =========================== phase D: one thread per key column and 16-row block ================================
     // Its first part needs only accumulators of phases A and B1 and runs in three pieces while the products of B2, B3 and C execute.
     build_qkL(sQL1, sKL1, false, warp_u, NT / 32, lane);      // the rest of phase C's operands: into the dw^T and v tiles, which phase B1 read last
@@ -598,7 +605,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     if (!mbar_wait(&s.barM, mph & 1)) alive = false;
     ++mph;
     umma::fence_after_sync();
-    if (alive) {
+    {
       float v[16];
       umma::tmem_ld16(tq + C_XY + 16 * part, v);
       umma::tmem_ld_wait();
@@ -608,25 +615,30 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
         *reinterpret_cast<uint4*>(sw_piece(sX, m, 2 * part + 1)) = pack8(&v[8]);
       }
     }
-    fence_proxy_async();
-    umma::fence_before_sync();
-    alive = __syncthreads_and(alive);
-    if (!alive) {
-      if (tid == 0) atomicOr(p.status, 64u);
-      break;
-    }
-    umma::fence_after_sync();
+    hand_over(lane);      // (dv is staged, too)
 
     KDA_DBG_CLOCK(dbg, 7);
     // =========================== phase B3: Y = Tm^T X,  dAkk = -tril(Y, -1) ==========================================
     if (warp_u == 0) {
+      if (!handed_over()) alive = false;
       const uint32_t aX = smem_u32(sX), aTI = smem_u32(s.TI);
       constexpr uint32_t iY = umma::instr_desc(64, 64, true, true);
       const uint64_t dTiM = umma::desc_mnmajor(aTI, 0, SPAN), dXm = umma::desc_mnmajor(aX, 0, SPAN);
+      if (alive) {
 #pragma unroll
-      for (int sK = 0; sK < 4; ++sK)
-        umma::mma_ss_lead(tb + C_XY, dTiM + static_cast<uint64_t>(sK) * 128u, dXm + static_cast<uint64_t>(sK) * 128u, iY, sK > 0, lead);
-      if (lead) umma::commit(&s.barM);
+        for (int sK = 0; sK < 4; ++sK)
+          umma::mma_ss_lead(tb + C_XY, dTiM + static_cast<uint64_t>(sK) * 128u, dXm + static_cast<uint64_t>(sK) * 128u, iY, sK > 0, lead);
+        if (lead) umma::commit(&s.barM);
+      }
+    }
+    if (warp_u == 4 && len == C) {
+      if (!handed_over()) alive = false;
+      if (lane == 0 && alive) {
+#pragma unroll 1
+        for (int i = 0; i < 4 && 32 * i < p.vc; ++i) tma_store_rows(&p.tm_dv, 32 * i, h, ci.tok0, dv_stage(i));
+        bulk_commit();
+      }
+      __syncwarp();
     }
     {      // dq: scale Gam dqg
       float a[16];
@@ -642,7 +654,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     if (!mbar_wait(&s.barM, mph & 1)) alive = false;
     ++mph;
     umma::fence_after_sync();
-    if (alive) {
+    {
       float v[16];
       umma::tmem_ld16(tq + C_XY + 16 * part, v);
       umma::tmem_ld_wait();
@@ -674,20 +686,13 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
         }
       }
     }
-    fence_proxy_async();
-    umma::fence_before_sync();
-    alive = __syncthreads_and(alive);
-    if (!alive) {
-      if (tid == 0) atomicOr(p.status, 64u);
-      break;
-    }
-    umma::fence_after_sync();
+    hand_over(lane);
     KDA_DBG_CLOCK(dbg, 8);
-    if (warp_u == 4 && lane == 0) bulk_wait_read<0>();      // dv has left before the next tile's state tiles arrive there (phase D)
 
     KDA_DBG_CLOCK(dbg, 9);
     // =========================== phase C: off-diagonal blocks of the intra-chunk terms ==============================
     if (warp_u == 0) {
+      if (!handed_over()) alive = false;
       constexpr uint32_t iC1 = umma::instr_desc(128, 32, true, false);
       constexpr uint32_t iC2 = umma::instr_desc(128, 16, true, true);
       const uint64_t dKr = umma::smem_desc(smem_u32(sKR), KR_SPAN, umma::ATOM_BYTES), dDa = umma::smem_desc(smem_u32(sDA), 16, umma::ATOM_BYTES);
@@ -793,6 +798,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
       }
     };
     // the first four columns' share of the rows behind them, while the products of phase C execute
+    if (!handed_over()) alive = false;      // the diagonal blocks of dAkk are there
 #pragma unroll
     for (int j = 0; j < 4; ++j) cn[j] = 0.f;
     step();
@@ -800,6 +806,7 @@ __global__ void __launch_bounds__(512, 1) kda_chunk_bwd_main_tc_kernel(const __g
     step();
     part4(std::integral_constant<int, 4>{}, 4, 0);
     step();
+    if (warp_u == 4 && lane == 0) bulk_wait_read<0>();      // dv has left before the next tile's state tiles arrive there (phase D)
     if (!mbar_wait(&s.barM, mph & 1)) alive = false;
     ++mph;
     alive = __syncthreads_and(alive);      // phase C complete; G has been read by everybody; dglp is complete
