@@ -179,7 +179,7 @@ extern "C" int kda_chunk_bwd(const kda_chunk_args* args, void* stream) {
       make_rows_tmap(&mp.tm_v, a.v, false, a.tokens, a.H, vc, 64, C, true) ||
       make_rows_tmap(&mp.tm_do, a.d_o, false, a.tokens, a.H, vc, 64, C, true) ||
       make_rows_tmap(&mp.tm_dq, mp.dq, false, a.tokens, a.H, mp.dqc, KD, C, false) || make_rows_tmap(&mp.tm_dk, mp.dk, false, a.tokens, a.H, mp.dqc, KD, C, false) ||
-      make_rows_tmap(&mp.tm_dg, a.dg, true, a.tokens, a.H, kc, KD, C, false) || make_rows_tmap(&mp.tm_dv, a.dv, false, a.tokens, a.H, vc, 32, C, false))
+      (reinterpret_cast<uintptr_t>(a.dg) & 15) || make_rows_tmap(&mp.tm_dv, a.dv, false, a.tokens, a.H, vc, 32, C, false))
     return KDA_E_TMAP;
   mp.H = a.H; mp.scale = a.scale; mp.grp = grp;
   // without grouped heads the normalisation's backward is applied by bwd_main's own epilogue

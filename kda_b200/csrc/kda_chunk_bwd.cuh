@@ -26,7 +26,7 @@ struct MainParams {
   // tiled-load maps of the [tokens, H, 128] operator tensors (64-token boxes of one head)
   alignas(64) CUtensorMap tm_q, tm_k, tm_g;   // plain row-major boxes [64][128]
   alignas(64) CUtensorMap tm_v, tm_do;        // 64-column boxes in the 128-byte-swizzled operand layout
-  alignas(64) CUtensorMap tm_dq, tm_dk, tm_dg, tm_dv;      // stores of full chunks: plain boxes [64][128], dv [64][32]
+  alignas(64) CUtensorMap tm_dq, tm_dk, tm_dv;      // stores of full chunks: plain boxes [64][128], dv [64][32]
 };
 
 struct RScanParams {
