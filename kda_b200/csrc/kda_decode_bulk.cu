@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(HV * 2 + 32, 128 / HV) kda_decode_bulk_kernel(
   const bool slotted = a.state_indices != nullptr;
   auto wait = [&](uint64_t* bar, unsigned phases, int b) {
     if (*reinterpret_cast<volatile int*>(&s.dead)) return;
-    if (!mbar_wait<4>(bar + b, (phases >> b) & 1u)) {
+    if (!mbar_wait_unrolled(bar + b, (phases >> b) & 1u)) {
       s.dead = 1;
       atomicOr(&g_decode_status, 1u);
     }
