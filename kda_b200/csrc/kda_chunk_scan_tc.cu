@@ -41,7 +41,8 @@ struct TcScanSmem {
 };
 static_assert(sizeof(TcScanSmem) + 1024 <= 227 * 1024, "TcScanSmem too large");
 
-constexpr int C_H = 0, C_VN = 128, C_O = 192;      // TMEM columns; o is double buffered: C_O + 64 * (chunk & 1)
+// TMEM columns; o is double buffered: C_O + 64 * (chunk & 1); forward only: the bf16 copies of hT and v_new^T, two to a column
+constexpr int C_H = 0, C_VN = 128, C_O = 192, C_HB = 320, C_VB = 384;
 
 __device__ __forceinline__ uint4 pack8f(const float* v) {
   return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
@@ -52,6 +53,9 @@ __device__ __forceinline__ unsigned char* swp(unsigned char* tile, int row, int 
 
 }  // namespace
 
+// TRAIN: the bf16 copies of hT and v_new^T go through shared memory, from where they also leave as the chunk's HS and VNEWT tiles.  Otherwise they
+// stay in tensor memory: the products read their A operand there, and shared memory feeds B alone.
+template <bool TRAIN>
 __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanParams p) {
   chain_point();
   extern __shared__ unsigned char smem_raw[];
@@ -145,14 +149,22 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
         float x[16];
         umma::tmem_ld16(tq + C_H + 64 * half + 16 * g, x);
         umma::tmem_ld_wait();
-        *reinterpret_cast<uint4*>(swp(s.Hb + half * 16384, v, 2 * g)) = pack8f(&x[0]);
-        *reinterpret_cast<uint4*>(swp(s.Hb + half * 16384, v, 2 * g + 1)) = pack8f(&x[8]);
+        const uint4 lo = pack8f(&x[0]), hi = pack8f(&x[8]);
+        if constexpr (TRAIN) {
+          *reinterpret_cast<uint4*>(swp(s.Hb + half * 16384, v, 2 * g)) = lo;
+          *reinterpret_cast<uint4*>(swp(s.Hb + half * 16384, v, 2 * g + 1)) = hi;
+        } else {
+          umma::tmem_st8(tq + C_HB + 32 * half + 8 * g, lo, hi);
+        }
 #pragma unroll
-        for (int e = 0; e < 16; ++e) x[e] *= d.GL[64 * half + 16 * g + e];
+        for (int e = 0; e < 4; ++e) {
+          const float4 gl = *reinterpret_cast<const float4*>(&d.GL[64 * half + 16 * g + 4 * e]);
+          x[4 * e] *= gl.x; x[4 * e + 1] *= gl.y; x[4 * e + 2] *= gl.z; x[4 * e + 3] *= gl.w;
+        }
         umma::tmem_st16(tq + C_H + 64 * half + 16 * g, x);
       }
       umma::tmem_st_wait();
-      fence_proxy_async();
+      if constexpr (TRAIN) fence_proxy_async();
     }
     KDA_DBG_CLOCK(dbg, 34);
     umma::fence_before_sync();
@@ -171,15 +183,17 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
 #pragma unroll
       for (int sK = 0; sK < 8; ++sK) {
         const uint64_t o2 = static_cast<uint64_t>(sK & 3) * 2u;
-        umma::mma_ss(tb + C_VN, ((sK >> 2) ? dH1 : dH0) + o2, ((sK >> 2) ? dW1 : dW0) + o2, id1, sK > 0);      // v_part^T = hT w^T
+        if constexpr (TRAIN) umma::mma_ss(tb + C_VN, ((sK >> 2) ? dH1 : dH0) + o2, ((sK >> 2) ? dW1 : dW0) + o2, id1, sK > 0);      // v_part^T = hT w^T
+        else umma::mma_ts(tb + C_VN, tb + C_HB + 8 * sK, ((sK >> 2) ? dW1 : dW0) + o2, id1, sK > 0);
       }
       umma::commit(&s.barM);
 #pragma unroll
       for (int sK = 0; sK < 8; ++sK) {
         const uint64_t o2 = static_cast<uint64_t>(sK & 3) * 2u;
-        umma::mma_ss(tb + to, ((sK >> 2) ? dH1 : dH0) + o2, ((sK >> 2) ? dQ1 : dQ0) + o2, id1, sK > 0);        // o^T = hT qg^T
+        if constexpr (TRAIN) umma::mma_ss(tb + to, ((sK >> 2) ? dH1 : dH0) + o2, ((sK >> 2) ? dQ1 : dQ0) + o2, id1, sK > 0);        // o^T = hT qg^T
+        else umma::mma_ts(tb + to, tb + C_HB + 8 * sK, ((sK >> 2) ? dQ1 : dQ0) + o2, id1, sK > 0);
       }
-      if (p.HS) {                                       // training: the bf16 state image is the chunk's HS tile
+      if constexpr (TRAIN) {                            // the bf16 state image is the chunk's HS tile
         bulk_s2g(p.HS + tile * TILE_VK, s.Hb, TILE_VK);
         bulk_commit();
       }
@@ -196,6 +210,7 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
         umma::tmem_ld16(tq + C_VN + 32 * half, x);
         umma::tmem_ld16(tq + C_VN + 32 * half + 16, y);
         umma::tmem_ld_wait();
+        uint4 w[4];
 #pragma unroll
         for (int cix = 0; cix < 4; ++cix) {
           const uint4 u4 = *reinterpret_cast<const uint4*>(swp(d.UT, v, 4 * half + cix));
@@ -208,10 +223,16 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
             r[2 * e] = uu.x - src[2 * e];
             r[2 * e + 1] = uu.y - src[2 * e + 1];
           }
-          *reinterpret_cast<uint4*>(swp(s.VNT, v, 4 * half + cix)) = pack8f(r);
+          w[cix] = pack8f(r);
+          if constexpr (TRAIN) *reinterpret_cast<uint4*>(swp(s.VNT, v, 4 * half + cix)) = w[cix];
+        }
+        if constexpr (!TRAIN) {
+          umma::tmem_st8(tq + C_VB + 16 * half, w[0], w[1]);
+          umma::tmem_st8(tq + C_VB + 16 * half + 8, w[2], w[3]);
+          umma::tmem_st_wait();
         }
       }
-      fence_proxy_async();
+      if constexpr (TRAIN) fence_proxy_async();
     }
     ++mph;
     umma::fence_before_sync();
@@ -231,11 +252,16 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
       const uint64_t dV = umma::desc_kmajor(aVN, 0), dK = umma::smem_desc(aKG, 8192, umma::ATOM_BYTES), dA = umma::desc_kmajor(aAQ, 0);
 #pragma unroll
       for (int sK = 0; sK < 4; ++sK) {
-        umma::mma_ss(tb + C_H, dV + static_cast<uint64_t>(sK) * 2u, dK + static_cast<uint64_t>(sK) * 128u, idH, 1);      // hT += v_new^T kg
-        umma::mma_ss(tb + to, dV + static_cast<uint64_t>(sK) * 2u, dA + static_cast<uint64_t>(sK) * 2u, idO, 1);         // o^T += v_new^T Aqk^T
+        if constexpr (TRAIN) {
+          umma::mma_ss(tb + C_H, dV + static_cast<uint64_t>(sK) * 2u, dK + static_cast<uint64_t>(sK) * 128u, idH, 1);      // hT += v_new^T kg
+          umma::mma_ss(tb + to, dV + static_cast<uint64_t>(sK) * 2u, dA + static_cast<uint64_t>(sK) * 2u, idO, 1);         // o^T += v_new^T Aqk^T
+        } else {
+          umma::mma_ts(tb + C_H, tb + C_VB + 8 * sK, dK + static_cast<uint64_t>(sK) * 128u, idH, 1);
+          umma::mma_ts(tb + to, tb + C_VB + 8 * sK, dA + static_cast<uint64_t>(sK) * 2u, idO, 1);
+        }
       }
       umma::commit(&s.barM);
-      if (p.VNEWT) {
+      if constexpr (TRAIN) {
         bulk_s2g(p.VNEWT + tile * TILE_VT, s.VNT, TILE_VT);
         bulk_commit();
       }
@@ -307,9 +333,13 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
 int launch_scan_tc(const ScanParams& p, int blocks, cudaStream_t st) {
   static DeviceOnce once;
   const int smem = static_cast<int>(sizeof(TcScanSmem)) + 1024;
-  const int rc = once.run([&] { return cudaFuncSetAttribute(kda_chunk_scan_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
+  const int rc = once.run([&] {
+    cudaError_t e = cudaFuncSetAttribute(kda_chunk_scan_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kda_chunk_scan_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return e;
+  });
   if (rc != KDA_OK) return rc;
-  return static_cast<int>(launch_chained(kda_chunk_scan_tc_kernel, blocks, SNT, smem, st, p));
+  return static_cast<int>(launch_chained(p.HS ? kda_chunk_scan_tc_kernel<true> : kda_chunk_scan_tc_kernel<false>, blocks, SNT, smem, st, p));
 }
 
 }  // namespace kda
