@@ -117,6 +117,28 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
   __syncthreads();
   umma::fence_after_sync();
 
+  // o of chunk i: out of tensor memory into the staging tile; from there in coalesced rows (compute warps)
+  auto stage_o = [&](int i) {
+    const uint32_t to = C_O + 64 * (i & 1);
+    float x[16], y[16];
+    umma::tmem_ld16(tq + to + 32 * half, x);
+    umma::tmem_ld16(tq + to + 32 * half + 16, y);
+    umma::tmem_ld_wait();
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      s.oS[(32 * half + e) * VD + v] = __float2bfloat16_rn(x[e]);
+      s.oS[(32 * half + 16 + e) * VD + v] = __float2bfloat16_rn(y[e]);
+    }
+  };
+  auto store_o = [&](long long tok0, int len) {
+    asm volatile("bar.sync 1, 256;" ::: "memory");      // the eight compute warps only
+    for (int e = tid; e < C * 16; e += SCT) {
+      const int r = e >> 4, pc = e & 15;
+      if (r < len && pc * 8 < p.vc)
+        *reinterpret_cast<uint4*>(p.o + (static_cast<size_t>(tok0 + r) * p.H + h) * p.vc + pc * 8) = *reinterpret_cast<const uint4*>(&s.oS[r * VD + pc * 8]);
+    }
+  };
+
   uint32_t mph = 0;
   bool alive = true;
   for (int i = 0; i < nchunks; ++i) {       // a failed wait leaves through the uniform vote at the top of the next iteration
@@ -202,6 +224,8 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
 
     // ---- epilogue 1: v_new^T = u^T - v_part^T -> bf16 tile --------------------------------------------------------------
     if (!issuer) {
+      if constexpr (!TRAIN)
+        if (i > 0) stage_o(i - 1);      // the previous chunk's o under these products, its stores under the next ones
       if (!mbar_wait(&s.barM, mph & 1)) alive = false;
       umma::fence_after_sync();
       KDA_DBG_CLOCK(dbg, 36);
@@ -267,6 +291,8 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
       }
     }
     __syncwarp();
+    if constexpr (!TRAIN)
+      if (!issuer && i > 0) store_o(ci.tok0 - C, C);
     if (!mbar_wait(&s.barM, mph & 1)) alive = false;
     ++mph;
     umma::fence_after_sync();
@@ -278,25 +304,12 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
       continue;
     }
 
-    // ---- epilogue 2 (compute warps): o^T -> bf16 -> staged [t][v] -> coalesced rows --------------------------------------
-    if (alive) {
-      float x[16], y[16];
-      umma::tmem_ld16(tq + to + 32 * half, x);
-      umma::tmem_ld16(tq + to + 32 * half + 16, y);
-      umma::tmem_ld_wait();
-#pragma unroll
-      for (int e = 0; e < 16; ++e) {
-        s.oS[(32 * half + e) * VD + v] = __float2bfloat16_rn(x[e]);
-        s.oS[(32 * half + 16 + e) * VD + v] = __float2bfloat16_rn(y[e]);
-      }
-    }
-    umma::fence_before_sync();
-    asm volatile("bar.sync 1, 256;" ::: "memory");      // the eight compute warps only
-    for (int e = tid; e < C * 16; e += SCT) {
-      const int r = e >> 4, pc = e & 15;
-      if (r < ci.len && pc * 8 < p.vc)
-        *reinterpret_cast<uint4*>(p.o + (static_cast<size_t>(ci.tok0 + r) * p.H + h) * p.vc + pc * 8) =
-            *reinterpret_cast<const uint4*>(&s.oS[r * VD + pc * 8]);
+    // ---- epilogue 2 (compute warps): o^T -> bf16 -> staged [t][v] -> coalesced rows; forward only: of the last chunk, for the others see above
+    if (TRAIN || i == nchunks - 1) {
+      if constexpr (!TRAIN) asm volatile("bar.sync 1, 256;" ::: "memory");      // the chunk before has left the staging tile
+      if (alive) stage_o(i);
+      umma::fence_before_sync();
+      store_o(ci.tok0, ci.len);
     }
     // (the next iteration's first barrier orders these reads of oS before it is rewritten)
     KDA_DBG_CLOCK(dbg, 39);
