@@ -139,6 +139,14 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
     }
   };
 
+  auto decay = [](float (&x)[16], const float* gl) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float4 y = *reinterpret_cast<const float4*>(gl + 4 * e);
+      x[4 * e] *= y.x; x[4 * e + 1] *= y.y; x[4 * e + 2] *= y.z; x[4 * e + 3] *= y.w;
+    }
+  };
+
   uint32_t mph = 0;
   bool alive = true;
   for (int i = 0; i < nchunks; ++i) {       // a failed wait leaves through the uniform vote at the top of the next iteration
@@ -164,29 +172,30 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
     }
     KDA_DBG_CLOCK(dbg, 33);
 
-    // ---- state pass: bf16 copy of hT for the products, hT *= Gam_last in TMEM ----------------------------------
+    // ---- state pass: bf16 copy of hT for the products, hT *= Gam_last in TMEM (forward only: behind the barrier, the products do not need it) ----
+    float hx[TRAIN ? 1 : 4][16];
     if (!issuer) {
+      if constexpr (TRAIN) {
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        float x[16];
-        umma::tmem_ld16(tq + C_H + 64 * half + 16 * g, x);
+        for (int g = 0; g < 4; ++g) {
+          float x[16];
+          umma::tmem_ld16(tq + C_H + 64 * half + 16 * g, x);
+          umma::tmem_ld_wait();
+          *reinterpret_cast<uint4*>(swp(s.Hb + half * 16384, v, 2 * g)) = pack8f(&x[0]);
+          *reinterpret_cast<uint4*>(swp(s.Hb + half * 16384, v, 2 * g + 1)) = pack8f(&x[8]);
+          decay(x, &d.GL[64 * half + 16 * g]);
+          umma::tmem_st16(tq + C_H + 64 * half + 16 * g, x);
+        }
+        umma::tmem_st_wait();
+        fence_proxy_async();
+      } else {
+#pragma unroll
+        for (int g = 0; g < 4; ++g) umma::tmem_ld16(tq + C_H + 64 * half + 16 * g, hx[g]);
         umma::tmem_ld_wait();
-        const uint4 lo = pack8f(&x[0]), hi = pack8f(&x[8]);
-        if constexpr (TRAIN) {
-          *reinterpret_cast<uint4*>(swp(s.Hb + half * 16384, v, 2 * g)) = lo;
-          *reinterpret_cast<uint4*>(swp(s.Hb + half * 16384, v, 2 * g + 1)) = hi;
-        } else {
-          umma::tmem_st8(tq + C_HB + 32 * half + 8 * g, lo, hi);
-        }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float4 gl = *reinterpret_cast<const float4*>(&d.GL[64 * half + 16 * g + 4 * e]);
-          x[4 * e] *= gl.x; x[4 * e + 1] *= gl.y; x[4 * e + 2] *= gl.z; x[4 * e + 3] *= gl.w;
-        }
-        umma::tmem_st16(tq + C_H + 64 * half + 16 * g, x);
+        for (int g = 0; g < 4; ++g) umma::tmem_st8(tq + C_HB + 32 * half + 8 * g, pack8f(&hx[g][0]), pack8f(&hx[g][8]));
+        umma::tmem_st_wait();
       }
-      umma::tmem_st_wait();
-      if constexpr (TRAIN) fence_proxy_async();
     }
     KDA_DBG_CLOCK(dbg, 34);
     umma::fence_before_sync();
@@ -224,8 +233,14 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
 
     // ---- epilogue 1: v_new^T = u^T - v_part^T -> bf16 tile --------------------------------------------------------------
     if (!issuer) {
-      if constexpr (!TRAIN)
-        if (i > 0) stage_o(i - 1);      // the previous chunk's o under these products, its stores under the next ones
+      if constexpr (!TRAIN) {
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          decay(hx[g], &d.GL[64 * half + 16 * g]);
+          umma::tmem_st16(tq + C_H + 64 * half + 16 * g, hx[g]);
+        }
+        umma::tmem_st_wait();
+      }
       if (!mbar_wait(&s.barM, mph & 1)) alive = false;
       umma::fence_after_sync();
       KDA_DBG_CLOCK(dbg, 36);
@@ -292,7 +307,10 @@ __global__ void __launch_bounds__(SNT, 1) kda_chunk_scan_tc_kernel(const ScanPar
     }
     __syncwarp();
     if constexpr (!TRAIN)
-      if (!issuer && i > 0) store_o(ci.tok0 - C, C);
+      if (!issuer && i > 0) {      // the previous chunk's o
+        stage_o(i - 1);
+        store_o(ci.tok0 - C, C);
+      }
     if (!mbar_wait(&s.barM, mph & 1)) alive = false;
     ++mph;
     umma::fence_after_sync();
