@@ -20,14 +20,16 @@
 //   D   per key column: diagonal blocks pairwise with running products of 2^(g), dG = q dq + k (dk+ - dk-),
 //       dg = reverse cumsum, final dq, dk, dg;  dbeta from  <Tm, dTm_raw> + <dAkk, raw kk>.
 //
-// What bounds it: the work around the products, 51 k warp instructions a tile (22 to 25 k cycles), of which the last phase has a third; the
+// What bounds it: the work around the products, about 52 k warp instructions a tile (22 to 25 k cycles), of which the last phase has a third; the
 // waits for products are filled with it: the operands of phase C are built under B1 and B2, the last phase's parts that need only the
-// accumulators of A and B1 run under B2, B3 and C.  q and k are interleaved into one word per element once they have arrived, and the last
-// phase adds up dq and dk+ as register pairs, one instruction for both sides.  Row numbers are left to the uniform registers.
-// 8 x 8192 tokens x 32 heads: 61 -> 51 k instructions a tile, whole step 6.02 -> 5.91 ms; packed documents with the L2 norm 7.13 -> 6.95 ms (its
-// epilogue reads q and k where they are instead of from global memory); 2 x 1000 x 8 heads of 64: 108 -> 95.5 us, of which 9 are the code's size:
-// 135 KB with every issue loop and wait unrolled, 85 now, and a short step fetches all of it anew.  Kept as they were: the points where
-// operands are rounded to bf16 (one scaled copy of each row instead of one per reference row halves the builds and moves dA_log by 4 %).
+// accumulators of A and B1 run under B2, B3 and C, and between those a warp hands its share of an operand over instead of meeting everybody.
+// q and k are interleaved into one word per element once they have arrived, and the last phase adds up dq and dk+ as register pairs, one
+// instruction for both sides.  Row numbers are left to the uniform registers.
+// 8 x 8192 tokens x 32 heads, whole step: 6.05 ms with 61 k instructions -> 5.91; operands handed over 5.81; dg from registers and the next q, k early
+// 5.73.  Packed documents with the L2 norm 7.13 -> 6.78 ms (its epilogue reads q and k where they are instead of from global memory); 2 x 1000 x 8
+// heads of 64: 108 -> 94 us, of which 9 are the code's size: 135 KB with every issue loop and wait unrolled, 85 now, and a short step fetches
+// all of it anew.  Kept as they were: the points where operands are rounded to bf16 (one scaled copy of each row instead of one per reference row
+// halves the builds and moves dA_log by 4 %).
 #include "kda_chunk_bwd.cuh"
 #include "kda_device.cuh"
 #include "kda_f32x2.cuh"

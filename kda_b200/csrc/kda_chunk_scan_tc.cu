@@ -2,13 +2,17 @@
 //
 // One CTA per (sequence, head) walks the sequence's chunks in order.  TMEM lane = value column v, so the state
 // is held transposed, hT[v][k] (128 lanes x 128 fp32 columns), for the whole sequence.  Per chunk:
-//   state pass   every thread reads its slice of hT, writes the bf16 copy that the next products use as their A
-//                operand (shared memory, K-major; in training the same image is stored as the chunk's HS tile),
-//                and writes hT * Gam_last back to TMEM;
+//   state pass   every thread reads its slice of hT and leaves the bf16 copy that the next products use as their A operand: forward only in
+//                tensor memory, in training as a K-major tile in shared memory, which is also stored as the chunk's HS tile;
+//                hT * Gam_last goes back to TMEM (forward only: while products 1 execute, which do not need it)
 //   products 1   v_part^T = hT_bf16 w^T,   o^T = hT_bf16 qg^T                          (M=128 v, N=64 t, K=128 k)
-//   epilogue 1   v_new^T = u^T - v_part^T  -> bf16 tile (A operand of products 2; the chunk's VNEWT tile in training)
+//   epilogue 1   v_new^T = u^T - v_part^T  -> bf16, A operand of products 2 (in training the chunk's VNEWT tile)
 //   products 2   hT += v_new^T kg,   o^T += v_new^T Aqk^T                              (K = 64 tokens)
-//   epilogue 2   o^T -> bf16 -> staged in shared memory -> coalesced stores of o[t][v].
+//   epilogue 2   o^T -> bf16 -> staged in shared memory -> coalesced stores of o[t][v]; forward only a chunk later, under products 2.
+// What bounds it: HBM from about 150 units on (0.73 ms, 0.95 of the copy rate at 8 x 8192 x 32 in training), below that the chain of a chunk's
+// phases, in which the products wait for shared memory.  With A there a product reads 6 KB, with A in tensor memory 2: 4 x 4096 x 32 heads (128
+// units), whole call: 535 -> 523 us; with o read out under the next products 520, with the decay behind the hand-over 515.  In training the same costs
+// nothing and gains nothing (604 and 610 us at 6 x 2000 x 16): the tiles have to be written to shared memory in any case.
 // Operand tiles (W, QG, KG, AQK, UT, GL of the chunk) arrive through a 2-stage TMA bulk-copy / mbarrier ring.
 #include "kda_chunk.cuh"
 #include "kda_device.cuh"

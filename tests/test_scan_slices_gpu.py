@@ -79,3 +79,15 @@ def test_two_ctas_per_unit_give_the_same_bits(lens):
     one, two = _run(d, cu, 1), _run(d, cu, 0)
     for n in NAMES:
         assert torch.equal(two[n], one[n]), n
+
+
+@pytest.mark.parametrize("lens", [[1], [64], [65], [128], [129], [3, 0, 64, 200]])
+@pytest.mark.parametrize("D", [64, 128])
+def test_one_cta_scan_forward_only_gives_the_bits_of_training(lens, D):
+    """Forward only, the one-CTA scan keeps its bf16 operands in tensor memory and reads a chunk's o out under the next chunk; in training they go
+    through shared memory.  The same sums: a single chunk, full and ragged last chunks, an empty sequence, narrow heads."""
+    N = len(lens)
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32) if N > 1 else None
+    d = make_inputs(1, sum(lens), 3, D, D, torch.bfloat16, seed=990 + sum(lens) + D, h0_std=0.02, n_states=N, backward=True)
+    train, infer = _run(d, cu, 1), _run(d, cu, 1, backward=False)
+    assert torch.equal(train["o"], infer["o"]) and torch.equal(train["ht"], infer["ht"])
