@@ -237,3 +237,25 @@ def test_fp32_backward_twice_through_one_forward():
     a = torch.autograd.grad(o, lv, d["do"], retain_graph=True)
     b = torch.autograd.grad(o, lv, d["do"])
     assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+def _backward_us(B, T, H):
+    from kda_b200 import chunk_kda
+    d = {n: t.cuda() for n, t in make_inputs(B, T, H, 128, 128, torch.float32, seed=53, backward=True).items() if t is not None}
+    lv = [d[n].requires_grad_(True) for n in ("q", "k", "v", "g", "beta")]
+    o, _ = chunk_kda(*lv)
+    times = []
+    for _ in range(8):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        torch.autograd.grad(o, lv, d["do"], retain_graph=True)
+        b.record()
+        torch.cuda.synchronize()
+        times.append(a.elapsed_time(b) * 1e3)
+    return min(times)
+
+
+def test_fp32_backward_of_short_sequences_does_not_cost_32_tokens():
+    """The middle works on pieces of 32 tokens and stops behind the last token of a shorter one.  4,096 states of one token against the same
+    of 32: 424 of 1,742 us (the states' traffic remains); with every piece walked to its end 1,231 of 1,832."""
+    assert _backward_us(128, 1, 32) < 0.5 * _backward_us(128, 32, 32)
