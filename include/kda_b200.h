@@ -148,7 +148,10 @@ typedef struct kda_recurrent_bwd_args {
 size_t kda_recurrent_bwd_workspace_bytes(int64_t tokens, int32_t N, int32_t H, int32_t K, int32_t V);
 int kda_recurrent_bwd(const kda_recurrent_bwd_args* args, void* stream);
 
-/* The same pair for a caller that runs the forward anyway: kda_recurrent_train_fwd is kda_recurrent_fwd for fp32, K, V in {32, 64, 128},
+/* The forward that belongs to kda_recurrent_bwd: kda_recurrent_train_fwd below that leaves nothing (o and ht are the same bits). */
+int kda_recurrent_walk_fwd(const kda_recurrent_args* args, void* stream);
+
+/* The same pair for a caller that runs the forward anyway and has the memory (2.5 KB per token and head of 128 from forward to backward): kda_recurrent_train_fwd is kda_recurrent_fwd for fp32, K, V in {32, 64, 128},
  * whole sequences, activated g and beta, [K, V] states and ht != h0 (KDA_E_SHAPE otherwise), and leaves in `saved` (256-byte
  * aligned, kda_recurrent_saved_bytes(..)) what kda_recurrent_train_bwd, called with the same tensors, then need not compute
  * again.  `saved` is only read by the backward; its results are those of kda_recurrent_bwd, bit for bit, and its workspace

@@ -152,6 +152,7 @@ struct RecurrentCall {
   Tensor q, k, v, g, beta, A_log, dt_bias, h0, cu, slots, accepted, out;
   std::optional<double> scale, lower_bound;
   bool output_final = false, inplace = false, l2norm = false, gate = false, beta_sigmoid = false, transposed = false;
+  bool training = false;      // float32 with gradients: the forward that the replaying backward belongs to
 };
 
 std::pair<Tensor, Tensor> recurrent_fwd(RecurrentCall& c) {
@@ -220,6 +221,10 @@ std::pair<Tensor, Tensor> recurrent_fwd(RecurrentCall& c) {
   a.K = static_cast<int32_t>(s.K); a.V = static_cast<int32_t>(s.V); a.HQ = static_cast<int32_t>(s.HQ);
   a.io_dtype = dtype_code(q); a.use_qk_l2norm = c.l2norm; a.transpose_state = c.transposed;
   a.scale = static_cast<float>(c.scale ? *c.scale : 1.0 / std::sqrt(static_cast<double>(s.K)));
+  if (c.training) {
+    check_rc(kda_recurrent_walk_fwd(&a, stream_of(dev)), "kda_recurrent_walk_fwd");
+    return {o, ht};
+  }
   check_rc(kda_recurrent_fwd(&a, stream_of(dev)), "kda_recurrent_fwd");
   if (checked_mode()) {
     uint32_t st = 0;
@@ -512,7 +517,7 @@ PyObject* wrap(const Tensor& t) {
 
 PyObject* py_recurrent_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   KDA_BEGIN
-  KDA_REQUIRE(n == 20, PyExc_TypeError, "recurrent_fwd takes 20 arguments");
+  KDA_REQUIRE(n == 20 || n == 21, PyExc_TypeError, "recurrent_fwd takes 20 or 21 arguments");
   RecurrentCall c;
   c.q = need_arg(a[0], "q"); c.k = need_arg(a[1], "k"); c.v = need_arg(a[2], "v"); c.g = need_arg(a[3], "g"); c.beta = need_arg(a[4], "beta");
   c.A_log = tensor_arg(a[5], "A_log"); c.dt_bias = tensor_arg(a[6], "dt_bias"); c.h0 = tensor_arg(a[7], "initial_state");
@@ -520,6 +525,7 @@ PyObject* py_recurrent_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   c.slots = tensor_arg(a[12], "ssm_state_indices"); c.accepted = tensor_arg(a[13], "num_accepted_tokens"); c.l2norm = bool_arg(a[14]);
   c.gate = bool_arg(a[15]); c.beta_sigmoid = bool_arg(a[16]); c.lower_bound = double_arg(a[17]); c.out = tensor_arg(a[18], "out");
   c.transposed = bool_arg(a[19]);
+  c.training = n == 21 && bool_arg(a[20]);
   std::pair<Tensor, Tensor> r;
   {
     GilRelease nogil;

@@ -191,6 +191,7 @@ __global__ void __launch_bounds__(128, CPL == 8 ? 2 : 4) kda_recurrent_walk_kern
   const int V = p.V, cg = lane & 3, rg = lane >> 2, lcol = 4 * CPL * warp + 4 * cg, col = part * ncols + lcol;
   const Seq sq = sequence(p, n);
   const int stages = static_cast<int>((sq.len + TS - 1) / TS);
+  const bool keeps = !FWD || p.ckpt;      // (a forward that leaves nothing: no states, no r, no norms)
   float* const kept = (FWD ? p.ckpt : p.dckpt) + ((sq.bos / TC + n) * p.H + h) * static_cast<size_t>(K) * V + col;
   const size_t sbase = (static_cast<size_t>(n) * p.H + h) * K * V + col;
 
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(128, CPL == 8 ? 2 : 4) kda_recurrent_walk_kern
             ssk += kf[e] * kf[e];
           }
           const float rq = rsqrtf(warp_sum(ssq) + L2NORM_EPS), rk = rsqrtf(warp_sum(ssk) + L2NORM_EPS);
-          if (lane == 0 && part == 0) *reinterpret_cast<float2*>(p.norms + 2 * row) = make_float2(rq, rk);
+          if (lane == 0 && part == 0 && p.norms) *reinterpret_cast<float2*>(p.norms + 2 * row) = make_float2(rq, rk);
           qs *= rq;
           ks = rk;
         } else {
@@ -272,7 +273,7 @@ __global__ void __launch_bounds__(128, CPL == 8 ? 2 : 4) kda_recurrent_walk_kern
     __syncthreads();      // stage st has arrived; everybody is done with the other buffer
     if (it + 1 < stages) issue(FWD ? st + 1 : st - 1);
     activate(st);
-    if (FWD ? st % (TC / TS) == 0 : (it == 0 || st % (TC / TS) == TC / TS - 1))
+    if (keeps && (FWD ? st % (TC / TS) == 0 : (it == 0 || st % (TC / TS) == TC / TS - 1)))
       S.store(kept + static_cast<size_t>(st / (TC / TS)) * p.H * K * V, rg, V);
     __syncthreads();
     // (running pointers: the products of 64-bit indices cost more than a tenth of a token's instructions)
@@ -318,7 +319,7 @@ __global__ void __launch_bounds__(128, CPL == 8 ? 2 : 4) kda_recurrent_walk_kern
           w2[c] = pair(beta * x[c], beta * x[c]);
           acc[0][c] = acc[P - 1][c] = 0ull;
         }
-        if (rg < CPL / 4)
+        if (keeps && rg < CPL / 4)
           *reinterpret_cast<float4*>(out) =
               CPL == 8 && rg ? make_float4(x[CPL - 4], x[CPL - 3], x[CPL - 2], x[CPL - 1]) : make_float4(x[0], x[1], x[2], x[3]);
 #pragma unroll
@@ -879,7 +880,8 @@ extern "C" size_t kda_recurrent_bwd_workspace_bytes(int64_t tokens, int32_t N, i
   return work_layout(tokens, N, H, K, V).total + saved_layout(tokens, N, H, K, V).total;
 }
 
-extern "C" int kda_recurrent_train_fwd(const kda_recurrent_args* a, void* saved, size_t saved_bytes, void* stream) {
+// the forward walk; with_saved: leaves what a backward then need not compute again
+static int forward(const kda_recurrent_args* a, void* saved, size_t saved_bytes, bool with_saved, void* stream) {
   if (!a) return KDA_E_NULL;
   if (a->N < 0 || a->H <= 0 || a->tokens < 0 || (!a->cu_seqlens && a->T < 0)) return KDA_E_SHAPE;
   if (!head_size_ok(a->K) || !head_size_ok(a->V)) return KDA_E_SHAPE;
@@ -888,11 +890,11 @@ extern "C" int kda_recurrent_train_fwd(const kda_recurrent_args* a, void* saved,
   // whole sequences, activated gates, [K, V] states
   if (a->state_indices || a->num_accepted_tokens || a->transpose_state || a->A_log || a->beta_sigmoid || (a->ht && a->ht == a->h0)) return KDA_E_SHAPE;
   if (a->N == 0 || a->tokens == 0) return kda_recurrent_fwd(a, stream);      // nothing to walk: the final state is the initial one
-  if (!a->q || !a->k || !a->v || !a->g || !a->beta || !a->o || !saved) return KDA_E_NULL;
+  if (!a->q || !a->k || !a->v || !a->g || !a->beta || !a->o || (with_saved && !saved)) return KDA_E_NULL;
   if (a->io_dtype != KDA_FP32) return KDA_E_DTYPE;
   if (!a->cu_seqlens && static_cast<int64_t>(a->N) * a->T != a->tokens) return KDA_E_SHAPE;
   const SavedLayout sl = saved_layout(a->tokens, a->N, a->H, a->K, a->V);
-  if (saved_bytes < sl.total) return KDA_E_WORKSPACE;
+  if (with_saved && saved_bytes < sl.total) return KDA_E_WORKSPACE;
   if (reinterpret_cast<uintptr_t>(saved) & 255) return KDA_E_ALIGN;
   const void* sixteen[] = {a->q, a->k, a->v, a->g, a->o, a->h0, a->ht};      // as kda_recurrent_fwd
   for (const void* p : sixteen)
@@ -904,9 +906,15 @@ extern "C" int kda_recurrent_train_fwd(const kda_recurrent_args* a, void* saved,
   p.T = a->T; p.slots = static_cast<long long>(kept_states(a->tokens, a->N));
   p.N = a->N; p.H = a->H; p.HQ = HQ; p.V = a->V; p.use_l2 = a->use_qk_l2norm; p.scale = a->scale;
   p.wide = wide(a->q, a->k, a->g);
-  use_saved(p, saved, sl);
+  if (with_saved) use_saved(p, saved, sl);
   return launch_walk<true>(p, a->K, true, static_cast<cudaStream_t>(stream));
 }
+
+extern "C" int kda_recurrent_train_fwd(const kda_recurrent_args* args, void* saved, size_t saved_bytes, void* stream) {
+  return forward(args, saved, saved_bytes, true, stream);
+}
+
+extern "C" int kda_recurrent_walk_fwd(const kda_recurrent_args* args, void* stream) { return forward(args, nullptr, 0, false, stream); }
 
 extern "C" int kda_recurrent_bwd(const kda_recurrent_bwd_args* args, void* stream) { return backward(args, nullptr, 0, false, stream); }
 

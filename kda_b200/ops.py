@@ -269,29 +269,36 @@ def fused_recurrent_kda(q, k, v, g, beta, A_log=None, dt_bias=None, scale=None, 
 
 
 class RecurrentKDAFunction(torch.autograd.Function):
-    """float32 path of chunk_kda with gradients: token-recurrent forward that keeps the state of every 32nd token, and its exact
-    reverse mode (`kda_recurrent_train_fwd`, `kda_recurrent_train_bwd`, fla/ops/kda/naive.py:12-66 differentiated).  K, V in
-    {32, 64, 128}."""
+    """float32 path of chunk_kda with gradients: token-recurrent forward and its exact reverse mode (fla/ops/kda/naive.py:12-66
+    differentiated).  K, V in {32, 64, 128}.  A call keeps its inputs and the backward replays the forward (`kda_recurrent_walk_fwd`,
+    `kda_recurrent_bwd`); with `keep` the forward also leaves the state of every 32nd token and a row per token until the backward, which is
+    then shorter (`kda_recurrent_train_fwd`, `kda_recurrent_train_bwd`): the same bits."""
 
     @staticmethod
-    def forward(ctx, q, k, v, g, beta, scale, initial_state, output_final_state, use_l2norm, cu_seqlens):
+    def forward(ctx, q, k, v, g, beta, scale, initial_state, output_final_state, use_l2norm, cu_seqlens, keep):
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
         g32, beta32 = g.contiguous().float(), beta.contiguous().float()
         h0 = initial_state.contiguous().float() if initial_state is not None else None
         cu = _as_i32(cu_seqlens, q.device) if cu_seqlens is not None else None
-        B, T, HQ, K = q.shape
-        H, V = v.shape[-2], v.shape[-1]
-        N = B if cu is None else cu.numel() - 1
-        dev = q.device
-        lib = _lib.load()
-        o = torch.empty_like(v)
-        ht = torch.empty(N, H, K, V, dtype=torch.float32, device=dev) if output_final_state else None
-        saved = torch.empty(lib.kda_recurrent_saved_bytes(B * T, N, H, K, V), dtype=torch.uint8, device=dev)
-        args = _lib.RecurrentArgs(
-            q=_ptr(q), k=_ptr(k), v=_ptr(v), g=_ptr(g32), beta=_ptr(beta32), h0=_ptr(h0), ht=_ptr(ht), o=_ptr(o), cu_seqlens=_ptr(cu),
-            tokens=B * T, N=N, T=T, H=H, K=K, V=V, HQ=HQ, io_dtype=_lib.KDA_FP32, use_qk_l2norm=int(use_l2norm), scale=scale)
-        with torch.cuda.device(dev):
-            _lib.check(lib.kda_recurrent_train_fwd(C.byref(args), _ptr(saved), saved.numel(), _stream(dev)), "kda_recurrent_train_fwd")
+        if keep:
+            B, T, HQ, K = q.shape
+            H, V = v.shape[-2], v.shape[-1]
+            N = B if cu is None else cu.numel() - 1
+            dev = q.device
+            lib = _lib.load()
+            o = torch.empty_like(v)
+            ht = torch.empty(N, H, K, V, dtype=torch.float32, device=dev) if output_final_state else None
+            saved = torch.empty(lib.kda_recurrent_saved_bytes(B * T, N, H, K, V), dtype=torch.uint8, device=dev)
+            args = _lib.RecurrentArgs(
+                q=_ptr(q), k=_ptr(k), v=_ptr(v), g=_ptr(g32), beta=_ptr(beta32), h0=_ptr(h0), ht=_ptr(ht), o=_ptr(o), cu_seqlens=_ptr(cu),
+                tokens=B * T, N=N, T=T, H=H, K=K, V=V, HQ=HQ, io_dtype=_lib.KDA_FP32, use_qk_l2norm=int(use_l2norm), scale=scale)
+            with torch.cuda.device(dev):
+                _lib.check(lib.kda_recurrent_train_fwd(C.byref(args), _ptr(saved), saved.numel(), _stream(dev)), "kda_recurrent_train_fwd")
+        else:
+            saved = None
+            o, ht = (_lib._native or _lib.native()).recurrent_fwd(
+                q, k, v, g32, beta32, None, None, h0, scale, output_final_state, False, cu, None, None, use_l2norm, False, False, None, None, False,
+                True)
         ctx.save_for_backward(q, k, v, g32, beta32, h0, cu, saved)
         ctx.meta = (float(scale), bool(use_l2norm), g.dtype, beta.dtype)
         return o, ht
@@ -311,15 +318,19 @@ class RecurrentKDAFunction(torch.autograd.Function):
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         dg, dbeta = torch.empty_like(g32), torch.empty_like(beta32)
         dh0 = torch.empty(N, H, K, V, dtype=torch.float32, device=dev) if h0 is not None else None
-        ws = torch.empty(lib.kda_recurrent_bwd_workspace_bytes(B * T, N, H, K, V) - saved.numel(), dtype=torch.uint8, device=dev)
+        ws = torch.empty(lib.kda_recurrent_bwd_workspace_bytes(B * T, N, H, K, V) - (saved.numel() if saved is not None else 0), dtype=torch.uint8,
+                         device=dev)
         args = _lib.RecurrentBwdArgs(
             q=_ptr(q), k=_ptr(k), v=_ptr(v), g=_ptr(g32), beta=_ptr(beta32), h0=_ptr(h0), cu_seqlens=_ptr(cu),
             d_o=_ptr(do), d_ht=_ptr(dht), dq=_ptr(dq), dk=_ptr(dk), dv=_ptr(dv), dg=_ptr(dg), dbeta=_ptr(dbeta), dh0=_ptr(dh0),
             workspace=_ptr(ws), workspace_bytes=ws.numel(), tokens=B * T, N=N, T=T, H=H, K=K, V=V, HQ=HQ,
             io_dtype=_lib.KDA_FP32, use_qk_l2norm=int(use_l2norm), scale=scale)
         with torch.cuda.device(dev):
-            _lib.check(lib.kda_recurrent_train_bwd(C.byref(args), _ptr(saved), saved.numel(), _stream(dev)), "kda_recurrent_train_bwd")
-        return dq, dk, dv, dg.to(g_dtype), dbeta.to(beta_dtype), None, dh0, None, None, None
+            if saved is not None:
+                _lib.check(lib.kda_recurrent_train_bwd(C.byref(args), _ptr(saved), saved.numel(), _stream(dev)), "kda_recurrent_train_bwd")
+            else:
+                _lib.check(lib.kda_recurrent_bwd(C.byref(args), _stream(dev)), "kda_recurrent_bwd")
+        return dq, dk, dv, dg.to(g_dtype), dbeta.to(beta_dtype), None, dh0, None, None, None, None
 
 
 # =================================================================================================
@@ -493,8 +504,9 @@ def chunk_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_sta
     token-recurrent fp32 kernels: forward for K in {32, 64, 128, 256}, with gradients for K, V in {32, 64, 128}.  `safe_gate=True` is the caller's promise that every gate value is at least
     -5 (fla/ops/kda/chunk.py:235-246); the forward then computes the diagonal 16 x 16 blocks of the intra-chunk products on
     tensor cores as well (factored around each block's middle row) instead of pairwise, which is faster and only safe under
-    that bound; without it the kernels are range-safe for any gate.  `disable_recompute` only selects a variant of the
-    same computation upstream and is accepted as a no-op; `chunk_size` (32 or
+    that bound; without it the kernels are range-safe for any gate.  `disable_recompute=True` lets a float32
+    call with gradients keep intermediates for its backward (2.5 KB per token and head of 128) instead of replaying the forward there: faster, the
+    same bits; the bf16 kernels always keep theirs; `chunk_size` (32 or
     64) changes nothing but the spacing of the intermediate states (the kernels always tile by 64 tokens); options
     that change results and are not built raise.
     """
@@ -523,7 +535,7 @@ def chunk_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_sta
                 raise NotImplementedError(f"kda_b200: float32 gradients need K, V in {{32, 64, 128}}, got K={K}, V={V}")
             tr = (lambda t: t.transpose(-1, -2)) if transpose_state_layout else (lambda t: t)
             o, ht = RecurrentKDAFunction.apply(q, k, v, g, beta, float(scale), tr(initial_state) if initial_state is not None else None,
-                                               bool(output_final_state), bool(use_qk_l2norm_in_kernel), cu_seqlens)
+                                               bool(output_final_state), bool(use_qk_l2norm_in_kernel), cu_seqlens, bool(disable_recompute))
             return o, (tr(ht).contiguous() if (transpose_state_layout and ht is not None) else ht)
         return fused_recurrent_kda_fwd(q, k, v, g, beta, initial_state=initial_state, scale=scale,
                                        output_final_state=output_final_state, inplace_final_state=False,

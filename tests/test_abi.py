@@ -164,3 +164,12 @@ def test_training_pair_refuses_what_it_does_not_take(lib):
     assert back(saved=None) == -1 and back(n=size - 1) == -5 and back(saved=272) == -4
     assert back(workspace_bytes=bwd["workspace_bytes"] - 1) == -5 and back(d_o=260) == -4
     assert lib.kda_recurrent_bwd(C.byref(_lib.RecurrentBwdArgs(**bwd)), None) == -5      # without the saved states the workspace holds them too
+
+
+def test_walk_forward_refuses_what_the_training_forward_refuses(lib):
+    """kda_recurrent_walk_fwd: the checks of kda_recurrent_train_fwd, without a buffer to leave anything in."""
+    from kda_b200 import _lib
+    ok = dict(q=256, k=256, v=256, g=256, beta=256, o=256, N=1, T=64, tokens=64, H=2, K=64, V=64, HQ=2, io_dtype=_lib.KDA_FP32)
+    call = lambda **kw: lib.kda_recurrent_walk_fwd(C.byref(_lib.RecurrentArgs(**{**ok, **kw})), None)      # noqa: E731
+    assert call(K=96) == -2 and call(tokens=63) == -2 and call(h0=512, ht=512) == -2 and call(transpose_state=1) == -2 and call(A_log=256) == -2
+    assert call(io_dtype=_lib.KDA_BF16) == -3 and call(o=None) == -1 and call(v=260) == -4 and call(q=260) == -4

@@ -259,3 +259,23 @@ def test_fp32_backward_of_short_sequences_does_not_cost_32_tokens():
     """The middle works on pieces of 32 tokens and stops behind the last token of a shorter one.  4,096 states of one token against the same
     of 32: 424 of 1,742 us (the states' traffic remains); with every piece walked to its end 1,231 of 1,832."""
     assert _backward_us(128, 1, 32) < 0.5 * _backward_us(128, 32, 32)
+
+
+@pytest.mark.parametrize("l2,states", [(False, True), (True, False)])
+def test_fp32_training_call_keeps_only_its_inputs(l2, states):
+    """Between forward and backward a float32 call holds no memory but its results, unless it is asked to (`disable_recompute`): gradients, o and the
+    final state are the same bits either way."""
+    from kda_b200 import chunk_kda
+    d = {n: t.cuda() for n, t in make_inputs(2, 333, 4, 128, 128, torch.float32, seed=54, h0_std=0.1, backward=True).items() if t is not None}
+    lv = [d[n].requires_grad_(True) for n in ("q", "k", "v", "g", "beta", "h0")[:6 if states else 5]]
+    got, kept = [], []
+    for keep in (False, True):
+        before = torch.cuda.memory_allocated()
+        o, ht = chunk_kda(*lv[:5], initial_state=lv[5] if states else None, output_final_state=states, use_qk_l2norm_in_kernel=l2,
+                          disable_recompute=keep)
+        kept.append(torch.cuda.memory_allocated() - before - o.numel() * 4 - (ht.numel() * 4 if states else 0))
+        grads = torch.autograd.grad([o, ht][:1 + states], lv, [d["do"], d["dht"]][:1 + states])
+        got.append([o, *([ht] if states else []), *grads])
+    # nothing but rounding; a state per 32 tokens, and r (blocks of the allocator above 1 MB may be up to 1 MB larger than asked for)
+    assert kept[0] < 4096 and kept[1] > 2 * (333 // 32) * 4 * 65536 + 2 * 333 * 4 * 512
+    assert all(torch.equal(a, b) for a, b in zip(*got))
