@@ -143,10 +143,16 @@ typedef struct kda_recurrent_bwd_args {
   float scale;
 } kda_recurrent_bwd_args;
 
-/* Scratch for kda_recurrent_bwd: per-value-head dq, dk, the state and its gradient every 32 tokens
- * (2 x (tokens / 32 + N) x H x K x V x 4 bytes), and one row per token. */
+/* Scratch for kda_recurrent_bwd, whatever its options: per-value-head dq, dk, the state and its gradient at every 32nd token of a sequence
+ * (2 x tokens / 32 x H x K x V x 4 bytes), r of every token, and copies of h0 and d_ht, which dh0 may overwrite. */
 size_t kda_recurrent_bwd_workspace_bytes(int64_t tokens, int32_t N, int32_t H, int32_t K, int32_t V);
 int kda_recurrent_bwd(const kda_recurrent_bwd_args* args, void* stream);
+
+/* The same with the scratch that these very arguments need (their workspace fields are not read by the query): without per-value-head dq, dk
+ * where heads are not grouped and rows not normalised, without copies unless dh0 overlaps h0 or d_ht.  saved: as in kda_recurrent_train_bwd
+ * below (with_saved != 0), or NULL. */
+size_t kda_recurrent_bwd_scratch_bytes(const kda_recurrent_bwd_args* args, int32_t with_saved);
+int kda_recurrent_bwd_scratch(const kda_recurrent_bwd_args* args, const void* saved, size_t saved_bytes, void* stream);
 
 /* The forward that belongs to kda_recurrent_bwd: kda_recurrent_train_fwd below that leaves nothing (o and ht are the same bits). */
 int kda_recurrent_walk_fwd(const kda_recurrent_args* args, void* stream);

@@ -73,6 +73,7 @@ EXPORTS = (
     "kda_b200_abi_version", "kda_b200_strerror", "kda_recurrent_fwd", "kda_recurrent_status",
     "kda_recurrent_bwd_workspace_bytes", "kda_recurrent_bwd",
     "kda_recurrent_saved_bytes", "kda_recurrent_train_fwd", "kda_recurrent_train_bwd", "kda_recurrent_walk_fwd",
+    "kda_recurrent_bwd_scratch_bytes", "kda_recurrent_bwd_scratch",
     "kda_chunk_max_chunks", "kda_chunk_workspace_bytes", "kda_chunk_bwd_workspace_bytes",
     "kda_chunk_fwd", "kda_chunk_bwd", "kda_chunk_status", "kda_chunk_fwd_noalloc", "kda_chunk_export_states",
     "kda_gate_bwd_workspace_bytes", "kda_gate_fwd", "kda_gate_bwd",
@@ -107,6 +108,10 @@ def load() -> C.CDLL:
     lib.kda_recurrent_bwd.argtypes = [C.POINTER(RecurrentBwdArgs), C.c_void_p]
     lib.kda_recurrent_train_fwd.restype = C.c_int
     lib.kda_recurrent_train_fwd.argtypes = [C.POINTER(RecurrentArgs), C.c_void_p, C.c_size_t, C.c_void_p]
+    lib.kda_recurrent_bwd_scratch_bytes.restype = C.c_size_t
+    lib.kda_recurrent_bwd_scratch_bytes.argtypes = [C.POINTER(RecurrentBwdArgs), C.c_int32]
+    lib.kda_recurrent_bwd_scratch.restype = C.c_int
+    lib.kda_recurrent_bwd_scratch.argtypes = [C.POINTER(RecurrentBwdArgs), C.c_void_p, C.c_size_t, C.c_void_p]
     lib.kda_recurrent_walk_fwd.restype = C.c_int
     lib.kda_recurrent_walk_fwd.argtypes = [C.POINTER(RecurrentArgs), C.c_void_p]
     lib.kda_recurrent_train_bwd.restype = C.c_int

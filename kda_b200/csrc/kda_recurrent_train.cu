@@ -49,10 +49,10 @@ struct TrainParams {
   float *o, *ht;
   float *dqh, *dkh;            // [tokens, H, K] per value head, w.r.t. the normalised rows
   float *dv, *dg, *dbeta, *dh0;
-  float *ckpt;                 // [tokens / 32 + N][H][K][V] states at the start of every 32 tokens
+  float *ckpt;                 // [tokens / 32][H][K][V] states at the borders of a sequence's 32-token pieces (its ends are h0 and ht)
   float *resid;                // [tokens, H, V] r
   float *norms;                // [tokens, H, 2] reciprocal norms of q, k (only with use_l2)
-  float *dckpt;                // like ckpt: dS at the end of every 32 tokens
+  float *dckpt;                // like ckpt: dS at the same borders
   float *dbp;                  // [tokens, H, V / 16] dbeta over 16 columns
   long long T, slots;
   int N, H, HQ, V;
@@ -60,7 +60,8 @@ struct TrainParams {
   float scale, dq_scale;       // dq_scale: what dqh still gets (without grouped heads and norms dqh, dkh are dq, dk themselves)
 };
 
-// first token and length of sequence n; the states of its 32-token pieces start at slot bos / 32 + n (disjoint for any lengths)
+// first token and length of sequence n.  Its 32-token pieces are numbered from bos / 32 + n (disjoint for any lengths), the borders between them from
+// bos / 32: ceil(len / 32) - 1 of them, at most floor((bos + len - 1) / 32) - floor(bos / 32).
 struct Seq { long long bos, len; };
 __device__ __forceinline__ long long seq_start(const TrainParams& p, long long n) { return p.cu ? p.cu[n] : n * p.T; }
 __device__ __forceinline__ Seq sequence(const TrainParams& p, int n) {
@@ -192,7 +193,7 @@ __global__ void __launch_bounds__(128, CPL == 8 ? 2 : 4) kda_recurrent_walk_kern
   const Seq sq = sequence(p, n);
   const int stages = static_cast<int>((sq.len + TS - 1) / TS);
   const bool keeps = !FWD || p.ckpt;      // (a forward that leaves nothing: no states, no r, no norms)
-  float* const kept = (FWD ? p.ckpt : p.dckpt) + ((sq.bos / TC + n) * p.H + h) * static_cast<size_t>(K) * V + col;
+  float* const kept = (FWD ? p.ckpt : p.dckpt) + ((sq.bos / TC) * p.H + h) * static_cast<size_t>(K) * V + col;
   const size_t sbase = (static_cast<size_t>(n) * p.H + h) * K * V + col;
 
   const long long out_step = (FWD ? 1LL : -1LL) * p.H * V, aux_step = FWD ? out_step : -1LL * p.H * (V / 16);
@@ -273,8 +274,8 @@ __global__ void __launch_bounds__(128, CPL == 8 ? 2 : 4) kda_recurrent_walk_kern
     __syncthreads();      // stage st has arrived; everybody is done with the other buffer
     if (it + 1 < stages) issue(FWD ? st + 1 : st - 1);
     activate(st);
-    if (keeps && (FWD ? st % (TC / TS) == 0 : (it == 0 || st % (TC / TS) == TC / TS - 1)))
-      S.store(kept + static_cast<size_t>(st / (TC / TS)) * p.H * K * V, rg, V);
+    if (keeps && it > 0 && st % (TC / TS) == (FWD ? 0 : TC / TS - 1))      // behind piece st / 4 - 1 (forward), st / 4
+      S.store(kept + static_cast<size_t>(st / (TC / TS) - (FWD ? 1 : 0)) * p.H * K * V, rg, V);
     __syncthreads();
     // (running pointers: the products of 64-bit indices cost more than a tenth of a token's instructions)
     const size_t row0 = (static_cast<size_t>(sq.bos + static_cast<long long>(st) * TS + (FWD ? 0 : cnt - 1))) * p.H + h;
@@ -451,14 +452,14 @@ __global__ void __launch_bounds__(Mid<K, V>::NT, 2) kda_recurrent_mid_kernel(con
   if (warp == 0) umma::tmem_alloc(&s.tmem_slot, 256);
   // ---- this thread's eight columns of four rows of S and dS; the tokens' rows -------------------------------------------------------
   const int l = lane % LPR, lrow = warp * M::RPW + 4 * (lane / LPR);
-  const size_t sbase = ((static_cast<size_t>(slot) * p.H + h) * K + slice * ROWS + lrow) * V + 4 * l;
   using Tile = f32x2[4][4];      // [row][pair of columns]
-  auto load_state = [&](Tile& x, const float* base) {
+  auto load_state = [&](Tile& x, const float* base, size_t index) {      // of [..][H][K][V]; no base: zeros
+    const float* const from = base + ((index * p.H + h) * K + slice * ROWS + lrow) * V + 4 * l;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
-        const F4 y = lds4(base + sbase + i * V + 4 * LPR * m);
+        const F4 y = base ? lds4(from + i * V + 4 * LPR * m) : F4{0ull, 0ull};
         x[i][2 * m] = y.a;
         x[i][2 * m + 1] = y.b;
       }
@@ -474,8 +475,10 @@ __global__ void __launch_bounds__(Mid<K, V>::NT, 2) kda_recurrent_mid_kernel(con
   cp_async_commit();
   if (tid < TC) s.beta[tid] = tid < cnt ? p.beta[(tok0 + tid) * p.H + h] : 0.f;
   Tile dS, S;
-  load_state(S, p.ckpt);
-  load_state(dS, p.dckpt);
+  // a sequence's own ends are where the caller has them: short sequences move no other states
+  const bool head = c == 0, tail = (c + 1) * TC >= sq.len;
+  load_state(S, head ? p.h0 : p.ckpt, head ? static_cast<size_t>(n) : static_cast<size_t>(sq.bos / TC + c - 1));
+  load_state(dS, tail ? p.d_ht : p.dckpt, tail ? static_cast<size_t>(n) : static_cast<size_t>(sq.bos / TC + c));
   for (int i = tid; i < rows * ROWS; i += NT) {      // tokens beyond the sequence leave S and dS as they are
     const int t = i / ROWS, row = i % ROWS;
     const bool ok = t < cnt;
@@ -722,33 +725,48 @@ __global__ void __launch_bounds__(256) kda_recurrent_bwd_finish_kernel(const Tra
 // buffers and launches
 // ---------------------------------------------------------------------------------------------------------------------
 size_t up256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
-size_t kept_states(int64_t tokens, int N) { return static_cast<size_t>(tokens) / TC + static_cast<size_t>(N); }
+size_t kept_states(int64_t tokens) { return static_cast<size_t>(tokens) / TC; }
 
 struct SavedLayout {      // what the forward leaves for the backward
   size_t ckpt, resid, norms, total;
 };
-SavedLayout saved_layout(int64_t tokens, int N, int H, int K, int V) {
+SavedLayout saved_layout(int64_t tokens, int H, int K, int V, bool l2) {
   SavedLayout l{};
   size_t off = 0;
-  l.ckpt = off; off = up256(off + kept_states(tokens, N) * H * K * V * 4);
+  l.ckpt = off; off = up256(off + kept_states(tokens) * H * K * V * 4);
   l.resid = off; off = up256(off + static_cast<size_t>(tokens) * H * V * 4);
-  l.norms = off; off = up256(off + static_cast<size_t>(tokens) * H * 2 * 4);
+  l.norms = off; off = up256(off + (l2 ? static_cast<size_t>(tokens) * H * 2 * 4 : 0));
   l.total = off;
   return l;
 }
-struct WorkLayout {      // the backward's own scratch; kda_recurrent_bwd's workspace continues with a SavedLayout
-  size_t dqh, dkh, dckpt, dbp, total;
+struct WorkLayout {      // the backward's scratch; a replaying backward's continues with a SavedLayout
+  size_t dqh, dkh, dckpt, dbp, h0, d_ht, total;
 };
-WorkLayout work_layout(int64_t tokens, int N, int H, int K, int V) {
+// What a call does without: dq^, dk^ when they are dq, dk; copies of h0 and d_ht, which the last kernel still reads, unless dh0 overwrites them
+struct Skip { bool dqk, h0, d_ht; };
+WorkLayout work_layout(int64_t tokens, int N, int H, int K, int V, const Skip& skip) {
   WorkLayout l{};
   size_t off = 0;
-  l.dqh = off; off = up256(off + static_cast<size_t>(tokens) * H * K * 4);
-  l.dkh = off; off = up256(off + static_cast<size_t>(tokens) * H * K * 4);
-  l.dckpt = off; off = up256(off + kept_states(tokens, N) * H * K * V * 4);
+  const size_t rows = skip.dqk ? 0 : static_cast<size_t>(tokens) * H * K * 4, states = static_cast<size_t>(N) * H * K * V * 4;
+  l.dqh = off; off = up256(off + rows);
+  l.dkh = off; off = up256(off + rows);
+  l.dckpt = off; off = up256(off + kept_states(tokens) * H * K * V * 4);
   l.dbp = off; off = up256(off + static_cast<size_t>(tokens) * H * (V / 16) * 4);
+  l.h0 = off; off = up256(off + (skip.h0 ? 0 : states));
+  l.d_ht = off; off = up256(off + (skip.d_ht ? 0 : states));
   l.total = off;
   return l;
 }
+bool overlap(const void* a, const void* b, size_t bytes) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return a && b && (x < y ? y - x : x - y) < bytes;
+}
+size_t state_bytes(const kda_recurrent_bwd_args& a) { return static_cast<size_t>(a.N) * a.H * a.K * a.V * 4; }
+Skip skips(const kda_recurrent_bwd_args& a) {
+  const int HQ = a.HQ > 0 ? a.HQ : a.H;
+  return {HQ == a.H && !a.use_qk_l2norm, !overlap(a.dh0, a.h0, state_bytes(a)), !overlap(a.dh0, a.d_ht, state_bytes(a))};
+}
+constexpr Skip NOTHING{false, false, false};
 bool head_size_ok(int d) { return d == 32 || d == 64 || d == 128; }
 void use_saved(TrainParams& p, void* saved, const SavedLayout& l) {
   unsigned char* const b = static_cast<unsigned char*>(saved);
@@ -811,19 +829,24 @@ int launch_finish(const TrainParams& p, float* dq, float* dk, long long rows, cu
   return static_cast<int>(launch_chained(kda_recurrent_bwd_finish_kernel<K>, static_cast<unsigned>((rows + 7) / 8), 256, 0, st, p, dq, dk, rows));
 }
 
-// saved == NULL: the forward walk runs here first, into the end of the workspace
-int backward(const kda_recurrent_bwd_args* a, const void* saved, size_t saved_bytes, bool with_saved, void* stream) {
+int check_backward(const kda_recurrent_bwd_args* a) {
   if (!a) return KDA_E_NULL;
   if (!a->q || !a->k || !a->v || !a->g || !a->beta || !a->d_o || !a->dq || !a->dk || !a->dv || !a->dg || !a->dbeta || !a->workspace)
     return KDA_E_NULL;
-  if (with_saved && !saved) return KDA_E_NULL;
   if (a->io_dtype != KDA_FP32) return KDA_E_DTYPE;
   if (a->N < 0 || a->H <= 0 || a->tokens < 0 || (!a->cu_seqlens && a->T < 0)) return KDA_E_SHAPE;
   if (!head_size_ok(a->K) || !head_size_ok(a->V)) return KDA_E_SHAPE;
+  if (a->H % (a->HQ > 0 ? a->HQ : a->H)) return KDA_E_SHAPE;
+  return KDA_OK;
+}
+
+// saved == NULL: the forward walk runs here first, into the end of the workspace
+int backward(const kda_recurrent_bwd_args* a, const void* saved, size_t saved_bytes, void* stream) {
+  const bool with_saved = saved != nullptr;
   const int HQ = a->HQ > 0 ? a->HQ : a->H;
-  if (a->H % HQ) return KDA_E_SHAPE;
-  const WorkLayout l = work_layout(a->tokens, a->N, a->H, a->K, a->V);
-  const SavedLayout sl = saved_layout(a->tokens, a->N, a->H, a->K, a->V);
+  const Skip skip = skips(*a);
+  const WorkLayout l = work_layout(a->tokens, a->N, a->H, a->K, a->V, skip);
+  const SavedLayout sl = saved_layout(a->tokens, a->H, a->K, a->V, with_saved || a->use_qk_l2norm);
   if (a->workspace_bytes < l.total + (with_saved ? 0 : sl.total)) return KDA_E_WORKSPACE;
   if (with_saved && saved_bytes < sl.total) return KDA_E_WORKSPACE;
   if ((reinterpret_cast<uintptr_t>(a->workspace) | reinterpret_cast<uintptr_t>(saved)) & 255) return KDA_E_ALIGN;
@@ -846,15 +869,23 @@ int backward(const kda_recurrent_bwd_args* a, const void* saved, size_t saved_by
   p.dqh = reinterpret_cast<float*>(ws + l.dqh); p.dkh = reinterpret_cast<float*>(ws + l.dkh);
   p.dckpt = reinterpret_cast<float*>(ws + l.dckpt); p.dbp = reinterpret_cast<float*>(ws + l.dbp);
   p.dv = static_cast<float*>(a->dv); p.dg = a->dg; p.dbeta = a->dbeta; p.dh0 = a->dh0;
-  p.T = a->T; p.slots = static_cast<long long>(kept_states(a->tokens, a->N));
+  p.T = a->T; p.slots = a->tokens / TC + a->N;
   p.N = a->N; p.H = a->H; p.HQ = HQ; p.V = a->V; p.use_l2 = a->use_qk_l2norm; p.scale = a->scale;
   p.wide = wide(a->q, a->k, a->g);
-  const bool direct = HQ == a->H && !p.use_l2;      // nothing to sum or to take back: no pass of its own (0.27 ms at 8 x 2048 x 32)
+  const bool direct = skip.dqk;      // nothing to sum or to take back: no pass of its own (0.27 ms at 8 x 2048 x 32)
   float *const dq = static_cast<float*>(a->dq), *const dk = static_cast<float*>(a->dk);
   if (direct) p.dqh = dq, p.dkh = dk;
   p.dq_scale = direct ? p.scale : 1.f;
   use_saved(p, with_saved ? const_cast<void*>(saved) : ws + l.total, sl);
   int rc = KDA_OK;
+  auto keep = [&](bool not_needed, const float*& x, size_t at) {
+    if (not_needed || rc != KDA_OK) return;
+    rc = static_cast<int>(cudaMemcpyAsync(ws + at, x, state_bytes(*a), cudaMemcpyDeviceToDevice, st));
+    x = reinterpret_cast<const float*>(ws + at);
+  };
+  keep(skip.h0, p.h0, l.h0);
+  keep(skip.d_ht, p.d_ht, l.d_ht);
+  if (rc != KDA_OK) return rc;
   if (!with_saved) rc = launch_walk<true>(p, a->K, true, st);
   if (rc == KDA_OK) rc = launch_walk<false>(p, a->K, with_saved, st);
   const long long rows = a->tokens * HQ;
@@ -872,12 +903,19 @@ using namespace kda;
 
 extern "C" size_t kda_recurrent_saved_bytes(int64_t tokens, int32_t N, int32_t H, int32_t K, int32_t V) {
   if (tokens < 0 || N < 0 || H <= 0 || K <= 0 || V <= 0) return 0;
-  return saved_layout(tokens, N, H, K, V).total;
+  return saved_layout(tokens, H, K, V, true).total;
 }
 
+// (an upper bound over all options; kda_recurrent_bwd_scratch_bytes knows them)
 extern "C" size_t kda_recurrent_bwd_workspace_bytes(int64_t tokens, int32_t N, int32_t H, int32_t K, int32_t V) {
   if (tokens < 0 || N < 0 || H <= 0 || K <= 0 || V <= 0) return 0;
-  return work_layout(tokens, N, H, K, V).total + saved_layout(tokens, N, H, K, V).total;
+  return work_layout(tokens, N, H, K, V, NOTHING).total + saved_layout(tokens, H, K, V, true).total;
+}
+
+extern "C" size_t kda_recurrent_bwd_scratch_bytes(const kda_recurrent_bwd_args* a, int32_t with_saved) {
+  if (!a || a->tokens < 0 || a->N < 0 || a->H <= 0 || !head_size_ok(a->K) || !head_size_ok(a->V)) return 0;
+  return work_layout(a->tokens, a->N, a->H, a->K, a->V, skips(*a)).total +
+         (with_saved ? 0 : saved_layout(a->tokens, a->H, a->K, a->V, a->use_qk_l2norm != 0).total);
 }
 
 // the forward walk; with_saved: leaves what a backward then need not compute again
@@ -893,7 +931,7 @@ static int forward(const kda_recurrent_args* a, void* saved, size_t saved_bytes,
   if (!a->q || !a->k || !a->v || !a->g || !a->beta || !a->o || (with_saved && !saved)) return KDA_E_NULL;
   if (a->io_dtype != KDA_FP32) return KDA_E_DTYPE;
   if (!a->cu_seqlens && static_cast<int64_t>(a->N) * a->T != a->tokens) return KDA_E_SHAPE;
-  const SavedLayout sl = saved_layout(a->tokens, a->N, a->H, a->K, a->V);
+  const SavedLayout sl = saved_layout(a->tokens, a->H, a->K, a->V, true);
   if (with_saved && saved_bytes < sl.total) return KDA_E_WORKSPACE;
   if (reinterpret_cast<uintptr_t>(saved) & 255) return KDA_E_ALIGN;
   const void* sixteen[] = {a->q, a->k, a->v, a->g, a->o, a->h0, a->ht};      // as kda_recurrent_fwd
@@ -903,7 +941,7 @@ static int forward(const kda_recurrent_args* a, void* saved, size_t saved_bytes,
   p.q = static_cast<const float*>(a->q); p.k = static_cast<const float*>(a->k); p.v = static_cast<const float*>(a->v);
   p.g = a->g; p.beta = a->beta; p.h0 = a->h0; p.ht = a->ht; p.o = static_cast<float*>(a->o);
   p.cu = a->cu_seqlens;
-  p.T = a->T; p.slots = static_cast<long long>(kept_states(a->tokens, a->N));
+  p.T = a->T;
   p.N = a->N; p.H = a->H; p.HQ = HQ; p.V = a->V; p.use_l2 = a->use_qk_l2norm; p.scale = a->scale;
   p.wide = wide(a->q, a->k, a->g);
   if (with_saved) use_saved(p, saved, sl);
@@ -916,8 +954,22 @@ extern "C" int kda_recurrent_train_fwd(const kda_recurrent_args* args, void* sav
 
 extern "C" int kda_recurrent_walk_fwd(const kda_recurrent_args* args, void* stream) { return forward(args, nullptr, 0, false, stream); }
 
-extern "C" int kda_recurrent_bwd(const kda_recurrent_bwd_args* args, void* stream) { return backward(args, nullptr, 0, false, stream); }
+extern "C" int kda_recurrent_bwd_scratch(const kda_recurrent_bwd_args* args, const void* saved, size_t saved_bytes, void* stream) {
+  const int rc = check_backward(args);
+  return rc != KDA_OK ? rc : backward(args, saved, saved_bytes, stream);
+}
+
+extern "C" int kda_recurrent_bwd(const kda_recurrent_bwd_args* args, void* stream) {
+  const int rc = check_backward(args);
+  if (rc != KDA_OK) return rc;
+  if (args->workspace_bytes < kda_recurrent_bwd_workspace_bytes(args->tokens, args->N, args->H, args->K, args->V)) return KDA_E_WORKSPACE;
+  return backward(args, nullptr, 0, stream);
+}
 
 extern "C" int kda_recurrent_train_bwd(const kda_recurrent_bwd_args* args, const void* saved, size_t saved_bytes, void* stream) {
-  return backward(args, saved, saved_bytes, true, stream);
+  const int rc = check_backward(args);
+  if (rc != KDA_OK) return rc;
+  if (!saved) return KDA_E_NULL;
+  if (args->workspace_bytes < work_layout(args->tokens, args->N, args->H, args->K, args->V, NOTHING).total) return KDA_E_WORKSPACE;
+  return backward(args, saved, saved_bytes, stream);
 }

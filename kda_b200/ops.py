@@ -270,9 +270,9 @@ def fused_recurrent_kda(q, k, v, g, beta, A_log=None, dt_bias=None, scale=None, 
 
 class RecurrentKDAFunction(torch.autograd.Function):
     """float32 path of chunk_kda with gradients: token-recurrent forward and its exact reverse mode (fla/ops/kda/naive.py:12-66
-    differentiated).  K, V in {32, 64, 128}.  A call keeps its inputs and the backward replays the forward (`kda_recurrent_walk_fwd`,
-    `kda_recurrent_bwd`); with `keep` the forward also leaves the state of every 32nd token and a row per token until the backward, which is
-    then shorter (`kda_recurrent_train_fwd`, `kda_recurrent_train_bwd`): the same bits."""
+    differentiated).  K, V in {32, 64, 128}.  A call keeps its inputs and the backward (`kda_recurrent_bwd_scratch`) replays the forward
+    (`kda_recurrent_walk_fwd`); with `keep` the forward (`kda_recurrent_train_fwd`) also leaves the state of every 32nd token and a row per token
+    until the backward, which is then shorter: the same bits."""
 
     @staticmethod
     def forward(ctx, q, k, v, g, beta, scale, initial_state, output_final_state, use_l2norm, cu_seqlens, keep):
@@ -318,18 +318,15 @@ class RecurrentKDAFunction(torch.autograd.Function):
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         dg, dbeta = torch.empty_like(g32), torch.empty_like(beta32)
         dh0 = torch.empty(N, H, K, V, dtype=torch.float32, device=dev) if h0 is not None else None
-        ws = torch.empty(lib.kda_recurrent_bwd_workspace_bytes(B * T, N, H, K, V) - (saved.numel() if saved is not None else 0), dtype=torch.uint8,
-                         device=dev)
         args = _lib.RecurrentBwdArgs(
             q=_ptr(q), k=_ptr(k), v=_ptr(v), g=_ptr(g32), beta=_ptr(beta32), h0=_ptr(h0), cu_seqlens=_ptr(cu),
             d_o=_ptr(do), d_ht=_ptr(dht), dq=_ptr(dq), dk=_ptr(dk), dv=_ptr(dv), dg=_ptr(dg), dbeta=_ptr(dbeta), dh0=_ptr(dh0),
-            workspace=_ptr(ws), workspace_bytes=ws.numel(), tokens=B * T, N=N, T=T, H=H, K=K, V=V, HQ=HQ,
-            io_dtype=_lib.KDA_FP32, use_qk_l2norm=int(use_l2norm), scale=scale)
+            tokens=B * T, N=N, T=T, H=H, K=K, V=V, HQ=HQ, io_dtype=_lib.KDA_FP32, use_qk_l2norm=int(use_l2norm), scale=scale)
+        ws = torch.empty(lib.kda_recurrent_bwd_scratch_bytes(C.byref(args), saved is not None), dtype=torch.uint8, device=dev)
+        args.workspace, args.workspace_bytes = _ptr(ws), ws.numel()
         with torch.cuda.device(dev):
-            if saved is not None:
-                _lib.check(lib.kda_recurrent_train_bwd(C.byref(args), _ptr(saved), saved.numel(), _stream(dev)), "kda_recurrent_train_bwd")
-            else:
-                _lib.check(lib.kda_recurrent_bwd(C.byref(args), _stream(dev)), "kda_recurrent_bwd")
+            _lib.check(lib.kda_recurrent_bwd_scratch(C.byref(args), _ptr(saved), saved.numel() if saved is not None else 0, _stream(dev)),
+                       "kda_recurrent_bwd_scratch")
         return dq, dk, dv, dg.to(g_dtype), dbeta.to(beta_dtype), None, dh0, None, None, None, None
 
 

@@ -173,3 +173,31 @@ def test_walk_forward_refuses_what_the_training_forward_refuses(lib):
     call = lambda **kw: lib.kda_recurrent_walk_fwd(C.byref(_lib.RecurrentArgs(**{**ok, **kw})), None)      # noqa: E731
     assert call(K=96) == -2 and call(tokens=63) == -2 and call(h0=512, ht=512) == -2 and call(transpose_state=1) == -2 and call(A_log=256) == -2
     assert call(io_dtype=_lib.KDA_BF16) == -3 and call(o=None) == -1 and call(v=260) == -4 and call(q=260) == -4
+
+
+def _bwd_args(**kw):
+    from kda_b200 import _lib
+    a = dict(q=256, k=256, v=256, g=256, beta=256, d_o=256, dq=256, dk=256, dv=256, dg=256, dbeta=256, N=8, T=2048, tokens=16384, H=32, K=128, V=128,
+             HQ=32, io_dtype=_lib.KDA_FP32, workspace=256)
+    return _lib.RecurrentBwdArgs(**{**a, **kw})
+
+
+def test_float32_backward_scratch_holds_what_the_call_needs(lib):
+    """kda_recurrent_bwd_scratch_bytes: two rows per token for per-value-head dq, dk only with grouped heads or normalised rows, norms only with
+    normalised rows, copies of h0 and d_ht only where dh0 overlaps them, and no states per sequence."""
+    size = lambda saved=0, **kw: lib.kda_recurrent_bwd_scratch_bytes(C.byref(_bwd_args(**kw)), saved)      # noqa: E731
+    rows, states = 16384 * 32 * 128 * 4, 8 * 32 * 128 * 128 * 4
+    assert size() < 16384 // 32 * 32 * 65536 * 2 + 1.2 * rows                 # the kept states and r, dbeta's parts
+    assert size(use_qk_l2norm=1) - size() == 2 * rows + 16384 * 32 * 8
+    assert size(HQ=8) - size() == 2 * rows
+    assert size(h0=256, d_ht=1 << 40, dh0=1 << 45) == size()
+    assert size(d_ht=1 << 40, dh0=1 << 40) - size() == size(h0=(1 << 40) + states - 16, dh0=1 << 40) - size() == states
+    assert size(h0=(1 << 40) + states, dh0=1 << 40) == size()
+    assert size(1) == size() - 16384 // 32 * 32 * 65536 - rows
+    assert size(N=2000, T=5, tokens=10000, H=8, HQ=8) < 10000 * 8 * (2048 * 2 + 512 + 32) + 4096
+    # the upper bound covers every call
+    bound = lib.kda_recurrent_bwd_workspace_bytes(16384, 8, 32, 128, 128)
+    assert bound == size(use_qk_l2norm=1, HQ=8, h0=1 << 40, d_ht=1 << 40, dh0=1 << 40)
+    run = lambda n, **kw: lib.kda_recurrent_bwd_scratch(C.byref(_bwd_args(workspace_bytes=n, **kw)), None, 0, None)      # noqa: E731
+    assert run(size() - 1) == -5 and run(size(HQ=8) - 1, HQ=8) == -5
+    assert run(1 << 40, K=96) == -2 and run(1 << 40, io_dtype=0) == -3 and run(1 << 40, dq=None) == -1 and run(1 << 40, d_o=260) == -4

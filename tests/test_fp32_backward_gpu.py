@@ -279,3 +279,55 @@ def test_fp32_training_call_keeps_only_its_inputs(l2, states):
     # nothing but rounding; a state per 32 tokens, and r (blocks of the allocator above 1 MB may be up to 1 MB larger than asked for)
     assert kept[0] < 4096 and kept[1] > 2 * (333 // 32) * 4 * 65536 + 2 * 333 * 4 * 512
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("lens", [[1, 1, 1], [32, 64, 31, 33], [3, 0, 96, 5, 32, 40]])
+@pytest.mark.parametrize("over", ["nothing", "d_ht", "h0"])
+@pytest.mark.parametrize("saved", [False, True])
+def test_fp32_backward_scratch_bits_margins_and_states_in_place(lens, over, saved):
+    """kda_recurrent_bwd_scratch with exactly the scratch it asks for, between sentinel margins, after either forward; dh0 over d_ht or h0, which the
+    last kernel reads after the walk has written dh0.  The bits of the operator's autograd path, pieces that end on and off a multiple of 32."""
+    import ctypes as C
+    from _abi import guarded_like
+    from kda_b200 import _lib, chunk_kda
+    lib = _lib.load()
+    tokens, N, H, D = sum(lens), len(lens), 2, 128
+    d = make_inputs(1, tokens, H, D, D, torch.float32, seed=55 + tokens, h0_std=0.1, n_states=N, backward=True)
+    d = {n: t.cuda().contiguous() for n, t in d.items()}
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device="cuda")
+    lv = {n: d[n].clone().requires_grad_(True) for n in ("q", "k", "v", "g", "beta", "h0")}
+    o, ht = chunk_kda(*(lv[n] for n in ("q", "k", "v", "g", "beta")), initial_state=lv["h0"], output_final_state=True, cu_seqlens=cu,
+                      use_qk_l2norm_in_kernel=True)
+    torch.autograd.backward([o, ht], [d["do"], d["dht"]])
+    guards, out = [], {}
+    for n in ("q", "k", "v", "g", "beta", "h0"):
+        g, out[n] = guarded_like(tuple(d[n].shape), torch.float32)
+        guards.append((n, g))
+    h0, dht = d["h0"], d["dht"]
+    if over == "d_ht":
+        dht = out["h0"].copy_(dht)
+    elif over == "h0":
+        h0 = out["h0"].copy_(h0)
+    p = lambda t: C.c_void_p(t.data_ptr())      # noqa: E731
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    sizes = dict(tokens=tokens, N=N, T=0, H=H, K=D, V=D, HQ=H, io_dtype=_lib.KDA_FP32, use_qk_l2norm=1, scale=D ** -0.5)
+    kept = None
+    if saved:
+        sg, kept = guarded_like((lib.kda_recurrent_saved_bytes(tokens, N, H, D, D),), torch.uint8)
+        og, o2 = guarded_like(tuple(d["v"].shape), torch.float32)
+        guards += [("saved", sg), ("o", og)]
+        f = _lib.RecurrentArgs(q=p(d["q"]), k=p(d["k"]), v=p(d["v"]), g=p(d["g"]), beta=p(d["beta"]), h0=p(h0), o=p(o2), cu_seqlens=p(cu), **sizes)
+        _lib.check(lib.kda_recurrent_train_fwd(C.byref(f), p(kept), kept.numel(), st), "kda_recurrent_train_fwd")
+        assert torch.equal(o2, o)
+    a = _lib.RecurrentBwdArgs(q=p(d["q"]), k=p(d["k"]), v=p(d["v"]), g=p(d["g"]), beta=p(d["beta"]), h0=p(h0), cu_seqlens=p(cu), d_o=p(d["do"]),
+                              d_ht=p(dht), dq=p(out["q"]), dk=p(out["k"]), dv=p(out["v"]), dg=p(out["g"]), dbeta=p(out["beta"]), dh0=p(out["h0"]),
+                              **sizes)
+    wg, ws = guarded_like((lib.kda_recurrent_bwd_scratch_bytes(C.byref(a), saved),), torch.uint8)
+    a.workspace, a.workspace_bytes = p(ws), ws.numel()
+    _lib.check(lib.kda_recurrent_bwd_scratch(C.byref(a), p(kept) if saved else None, kept.numel() if saved else 0, st), "kda_recurrent_bwd_scratch")
+    torch.cuda.synchronize()
+    for n, g in [*guards, ("scratch", wg)]:
+        assert g.margins_intact(), n
+    for n in out:
+        assert torch.equal(out[n], lv[n].grad), n
+
