@@ -109,7 +109,7 @@ def load() -> C.CDLL:
     lib.kda_recurrent_train_fwd.restype = C.c_int
     lib.kda_recurrent_train_fwd.argtypes = [C.POINTER(RecurrentArgs), C.c_void_p, C.c_size_t, C.c_void_p]
     lib.kda_recurrent_bwd_scratch_bytes.restype = C.c_size_t
-    lib.kda_recurrent_bwd_scratch_bytes.argtypes = [C.POINTER(RecurrentBwdArgs), C.c_int32]
+    lib.kda_recurrent_bwd_scratch_bytes.argtypes = [C.POINTER(RecurrentBwdArgs), C.c_int32, C.c_int32]
     lib.kda_recurrent_bwd_scratch.restype = C.c_int
     lib.kda_recurrent_bwd_scratch.argtypes = [C.POINTER(RecurrentBwdArgs), C.c_void_p, C.c_size_t, C.c_void_p]
     lib.kda_recurrent_walk_fwd.restype = C.c_int

@@ -55,7 +55,9 @@ struct TrainParams {
   float *dckpt;                // like ckpt: dS at the same borders
   float *dbp;                  // [tokens, H, V / 16] dbeta over 16 columns
   long long T, slots;
-  int N, H, HQ, V;
+  int N, H, HQ, V;             // H, HQ: heads of the tensors
+  int HL;                      // value heads of this launch: every pointer starts at the first of them
+  int HS, HD, HW;              // heads per token or border in ckpt, resid, norms; in dqh, dkh; in dckpt, dbp
   int use_l2, wide;            // wide: q, k, g start on 16-byte boundaries
   float scale, dq_scale;       // dq_scale: what dqh still gets (without grouped heads and norms dqh, dkh are dq, dk themselves)
 };
@@ -188,15 +190,16 @@ __global__ void __launch_bounds__(128, CPL == 8 ? 2 : 4) kda_recurrent_walk_kern
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5, nt = blockDim.x;
   const int ncols = 4 * CPL * nw, parts = p.V / ncols;
   const int unit = blockIdx.x / parts, part = blockIdx.x % parts;
-  const int n = unit / p.H, h = unit % p.H, hq = h / (p.H / p.HQ);
+  const int n = unit / p.HL, h = unit % p.HL, hq = h / (p.H / p.HQ);
   const int V = p.V, cg = lane & 3, rg = lane >> 2, lcol = 4 * CPL * warp + 4 * cg, col = part * ncols + lcol;
   const Seq sq = sequence(p, n);
   const int stages = static_cast<int>((sq.len + TS - 1) / TS);
   const bool keeps = !FWD || p.ckpt;      // (a forward that leaves nothing: no states, no r, no norms)
-  float* const kept = (FWD ? p.ckpt : p.dckpt) + ((sq.bos / TC) * p.H + h) * static_cast<size_t>(K) * V + col;
+  const int HK = FWD ? p.HS : p.HW;
+  float* const kept = (FWD ? p.ckpt : p.dckpt) + ((sq.bos / TC) * HK + h) * static_cast<size_t>(K) * V + col;
   const size_t sbase = (static_cast<size_t>(n) * p.H + h) * K * V + col;
 
-  const long long out_step = (FWD ? 1LL : -1LL) * p.H * V, aux_step = FWD ? out_step : -1LL * p.H * (V / 16);
+  const long long out_step = FWD ? 1LL * p.HS * V : -1LL * p.H * V, aux_step = FWD ? 1LL * p.H * V : -1LL * p.HW * (V / 16);
   const int oc = CPL == 8 ? rg : rg >> 1, ocol = col + 16 * (oc >> 2) + (oc & 3);      // the column whose o this lane ends with
 
   auto tokens_of = [&](int st) { return static_cast<int>(min(static_cast<long long>(TS), sq.len - static_cast<long long>(st) * TS)); };
@@ -214,7 +217,7 @@ __global__ void __launch_bounds__(128, CPL == 8 ? 2 : 4) kda_recurrent_walk_kern
       const int j = i / (ncols / 4), c = 4 * (i % (ncols / 4));
       const size_t row = ((tok0 + j) * p.H + h) * V + part * ncols + c;
       cp_async16(&s.x[b][j][c], (FWD ? p.v : p.d_o) + row, true);
-      if (!FWD) cp_async16(&s.y[b][j][c], p.resid + row, true);
+      if (!FWD) cp_async16(&s.y[b][j][c], p.resid + ((tok0 + j) * p.HS + h) * V + part * ncols + c, true);
     }
     if (tid < cnt) cp_async4(&s.beta[b][tid], p.beta + (tok0 + tid) * p.H + h, true);
     cp_async_commit();
@@ -229,7 +232,7 @@ __global__ void __launch_bounds__(128, CPL == 8 ? 2 : 4) kda_recurrent_walk_kern
       if (!FWD || p.o) row_get<E>(qf, &s.q[b][j][lane * E]);
       float qs = p.scale, ks = 1.f;
       if (p.use_l2) {
-        const size_t tok = static_cast<size_t>(sq.bos + static_cast<long long>(st) * TS + j), row = tok * p.H + h;
+        const size_t tok = static_cast<size_t>(sq.bos + static_cast<long long>(st) * TS + j), row = tok * p.HS + h;
         if (FWD) {
           if (!p.o) {      // (replay in front of a backward: q is only here for its norm)
 #pragma unroll
@@ -275,12 +278,12 @@ __global__ void __launch_bounds__(128, CPL == 8 ? 2 : 4) kda_recurrent_walk_kern
     if (it + 1 < stages) issue(FWD ? st + 1 : st - 1);
     activate(st);
     if (keeps && it > 0 && st % (TC / TS) == (FWD ? 0 : TC / TS - 1))      // behind piece st / 4 - 1 (forward), st / 4
-      S.store(kept + static_cast<size_t>(st / (TC / TS) - (FWD ? 1 : 0)) * p.H * K * V, rg, V);
+      S.store(kept + static_cast<size_t>(st / (TC / TS) - (FWD ? 1 : 0)) * HK * K * V, rg, V);
     __syncthreads();
     // (running pointers: the products of 64-bit indices cost more than a tenth of a token's instructions)
-    const size_t row0 = (static_cast<size_t>(sq.bos + static_cast<long long>(st) * TS + (FWD ? 0 : cnt - 1))) * p.H + h;
-    float* out = (FWD ? p.resid : p.dv) + row0 * V + col + 16 * rg;                    // r, dv: row groups 0 (and 1) store
-    float* aux = FWD ? p.o + row0 * V + ocol : p.dbp + row0 * (V / 16) + col / 16;      // o, dbeta's parts
+    const size_t tok1 = static_cast<size_t>(sq.bos + static_cast<long long>(st) * TS + (FWD ? 0 : cnt - 1));
+    float* out = (FWD ? p.resid + (tok1 * p.HS + h) * V : p.dv + (tok1 * p.H + h) * V) + col + 16 * rg;                // r, dv: row groups 0 (and 1) store
+    float* aux = FWD ? p.o + (tok1 * p.H + h) * V + ocol : p.dbp + (tok1 * p.HW + h) * (V / 16) + col / 16;      // o, dbeta's parts
     for (int jj = 0; jj < cnt; ++jj, out += out_step, aux += aux_step) {
       const int j = FWD ? jj : cnt - 1 - jj;
       const float* const kr = &s.k[b][j][4 * rg];
@@ -427,8 +430,8 @@ __global__ void __launch_bounds__(Mid<K, V>::NT, 2) kda_recurrent_mid_kernel(con
   extern __shared__ __align__(16) unsigned char smem_raw[];
   typename M::Smem& s = *reinterpret_cast<typename M::Smem*>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-  const int slice = blockIdx.x % M::SLICES, h = blockIdx.x / M::SLICES % p.H, hq = h / (p.H / p.HQ);
-  const long long slot = blockIdx.x / M::SLICES / p.H;
+  const int slice = blockIdx.x % M::SLICES, h = blockIdx.x / M::SLICES % p.HL, hq = h / (p.H / p.HQ);
+  const long long slot = blockIdx.x / M::SLICES / p.HL;
   if (tid == 0) {      // the last sequence whose first slot is not behind this one
     int lo = 0, hi = p.N - 1;
     while (lo < hi) {
@@ -453,8 +456,8 @@ __global__ void __launch_bounds__(Mid<K, V>::NT, 2) kda_recurrent_mid_kernel(con
   // ---- this thread's eight columns of four rows of S and dS; the tokens' rows -------------------------------------------------------
   const int l = lane % LPR, lrow = warp * M::RPW + 4 * (lane / LPR);
   using Tile = f32x2[4][4];      // [row][pair of columns]
-  auto load_state = [&](Tile& x, const float* base, size_t index) {      // of [..][H][K][V]; no base: zeros
-    const float* const from = base + ((index * p.H + h) * K + slice * ROWS + lrow) * V + 4 * l;
+  auto load_state = [&](Tile& x, const float* base, size_t index, int heads) {      // of [..][heads][K][V]; no base: zeros
+    const float* const from = base + ((index * heads + h) * K + slice * ROWS + lrow) * V + 4 * l;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -467,8 +470,8 @@ __global__ void __launch_bounds__(Mid<K, V>::NT, 2) kda_recurrent_mid_kernel(con
   for (int i = tid; i < rows * (V / 4); i += NT) {
     const int t = i / (V / 4), cc = 4 * (i % (V / 4));
     const bool ok = t < cnt;
-    const size_t row = ((tok0 + (ok ? t : 0)) * p.H + h) * V + cc;
-    cp_async16(&s.w[t][cc], p.resid + row, ok);
+    const size_t tok = tok0 + (ok ? t : 0), row = (tok * p.H + h) * V + cc;
+    cp_async16(&s.w[t][cc], p.resid + (tok * p.HS + h) * V + cc, ok);
     cp_async16(&s.d_o[t][cc], p.d_o + row, ok);
     cp_async16(&s.dr[t][cc], p.dv + row, ok);
   }
@@ -477,20 +480,20 @@ __global__ void __launch_bounds__(Mid<K, V>::NT, 2) kda_recurrent_mid_kernel(con
   Tile dS, S;
   // a sequence's own ends are where the caller has them: short sequences move no other states
   const bool head = c == 0, tail = (c + 1) * TC >= sq.len;
-  load_state(S, head ? p.h0 : p.ckpt, head ? static_cast<size_t>(n) : static_cast<size_t>(sq.bos / TC + c - 1));
-  load_state(dS, tail ? p.d_ht : p.dckpt, tail ? static_cast<size_t>(n) : static_cast<size_t>(sq.bos / TC + c));
+  load_state(S, head ? p.h0 : p.ckpt, head ? static_cast<size_t>(n) : static_cast<size_t>(sq.bos / TC + c - 1), head ? p.H : p.HS);
+  load_state(dS, tail ? p.d_ht : p.dckpt, tail ? static_cast<size_t>(n) : static_cast<size_t>(sq.bos / TC + c), tail ? p.H : p.HW);
   for (int i = tid; i < rows * ROWS; i += NT) {      // tokens beyond the sequence leave S and dS as they are
     const int t = i / ROWS, row = i % ROWS;
     const bool ok = t < cnt;
     const size_t tok = tok0 + (ok ? t : 0), rq = (tok * p.HQ + hq) * K + slice * ROWS + row, rv = tok * p.H + h;
     float2 r = make_float2(1.f, 1.f);
-    if (p.use_l2) r = *reinterpret_cast<const float2*>(p.norms + 2 * rv);
+    if (p.use_l2) r = *reinterpret_cast<const float2*>(p.norms + 2 * (tok * p.HS + h));
     s.q[t][row] = ok ? p.q[rq] * (p.scale * r.x) : 0.f;
     s.k[t][row] = ok ? p.k[rq] * r.y : 0.f;
     s.a[t][row] = ok ? expf(p.g[rv * K + slice * ROWS + row]) : 1.f;
   }
   if (slice == 0 && tid < cnt) {
-    const float* const part = p.dbp + ((tok0 + tid) * p.H + h) * (V / 16);
+    const float* const part = p.dbp + ((tok0 + tid) * p.HW + h) * (V / 16);
     float sum = 0.f;
 #pragma unroll
     for (int i = 0; i < V / 16; ++i) sum += part[i];
@@ -671,10 +674,11 @@ __global__ void __launch_bounds__(Mid<K, V>::NT, 2) kda_recurrent_mid_kernel(con
   __syncthreads();
   for (int i = tid; i < cnt * ROWS; i += NT) {
     const int t = i / ROWS, row = i % ROWS;
-    const size_t o = ((tok0 + t) * p.H + h) * K + slice * ROWS + row;
+    const int at = slice * ROWS + row;
+    const size_t o = ((tok0 + t) * p.HD + h) * K + at;
     p.dqh[o] = s.q[t][row] * p.dq_scale;
     p.dkh[o] = s.k[t][row];
-    p.dg[o] = s.a[t][row];
+    p.dg[((tok0 + t) * p.H + h) * K + at] = s.a[t][row];
   }
   if (warp == 0) umma::tmem_dealloc(s.tmem_slot, 256);
 }
@@ -686,16 +690,17 @@ __global__ void __launch_bounds__(256) kda_recurrent_bwd_finish_kernel(const Tra
                                                                        long long rows) {
   chain_point();
   constexpr int E = K / 32;
-  const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);      // token * HQ + q head
+  const long long item = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);      // token, q head of this launch
   const int lane = threadIdx.x & 31;
-  if (row >= rows) return;
-  const int grp = p.H / p.HQ;
-  const long long tok = row / p.HQ;
-  const int hq = static_cast<int>(row % p.HQ);
+  if (item >= rows) return;
+  const int grp = p.H / p.HQ, heads = p.HL / grp;
+  const long long tok = item / heads;
+  const int hq = static_cast<int>(item % heads);
+  const long long row = tok * p.HQ + hq;
 #pragma unroll
   for (int which = 0; which < 2; ++which) {
     const float* x = (which ? p.k : p.q) + row * K + lane * E;
-    const float* src = (which ? p.dkh : p.dqh) + (tok * p.H + static_cast<long long>(hq) * grp) * K + lane * E;
+    const float* src = (which ? p.dkh : p.dqh) + (tok * p.HD + static_cast<long long>(hq) * grp) * K + lane * E;
     float d[E], xf[E];
     float ss = 0.f;
 #pragma unroll
@@ -744,10 +749,10 @@ struct WorkLayout {      // the backward's scratch; a replaying backward's conti
 };
 // What a call does without: dq^, dk^ when they are dq, dk; copies of h0 and d_ht, which the last kernel still reads, unless dh0 overwrites them
 struct Skip { bool dqk, h0, d_ht; };
-WorkLayout work_layout(int64_t tokens, int N, int H, int K, int V, const Skip& skip) {
+WorkLayout work_layout(int64_t tokens, int N, int H, int all_heads, int K, int V, const Skip& skip) {
   WorkLayout l{};
   size_t off = 0;
-  const size_t rows = skip.dqk ? 0 : static_cast<size_t>(tokens) * H * K * 4, states = static_cast<size_t>(N) * H * K * V * 4;
+  const size_t rows = skip.dqk ? 0 : static_cast<size_t>(tokens) * H * K * 4, states = static_cast<size_t>(N) * all_heads * K * V * 4;
   l.dqh = off; off = up256(off + rows);
   l.dkh = off; off = up256(off + rows);
   l.dckpt = off; off = up256(off + kept_states(tokens) * H * K * V * 4);
@@ -767,6 +772,21 @@ Skip skips(const kda_recurrent_bwd_args& a) {
   return {HQ == a.H && !a.use_qk_l2norm, !overlap(a.dh0, a.h0, state_bytes(a)), !overlap(a.dh0, a.d_ht, state_bytes(a))};
 }
 constexpr Skip NOTHING{false, false, false};
+
+// The heads may be worked on in groups, one after another, in the scratch of one group.
+int heads_of(const kda_recurrent_bwd_args& a, int passes) {      // value heads a pass, evened out; whole groups of value heads
+  const int HQ = a.HQ > 0 ? a.HQ : a.H;
+  return (HQ + passes - 1) / passes * (a.H / HQ);
+}
+size_t scratch_bytes(const kda_recurrent_bwd_args& a, int heads, bool with_saved) {
+  return work_layout(a.tokens, a.N, heads, a.H, a.K, a.V, skips(a)).total + (with_saved ? 0 : saved_layout(a.tokens, heads, a.K, a.V, a.use_qk_l2norm != 0).total);
+}
+// the fewest passes whose scratch `bytes` holds; 0: not even one group fits
+int heads_per_pass(const kda_recurrent_bwd_args& a, bool with_saved, size_t bytes) {
+  for (int passes = 1; passes <= (a.HQ > 0 ? a.HQ : a.H); ++passes)
+    if (scratch_bytes(a, heads_of(a, passes), with_saved) <= bytes) return heads_of(a, passes);
+  return 0;
+}
 bool head_size_ok(int d) { return d == 32 || d == 64 || d == 128; }
 void use_saved(TrainParams& p, void* saved, const SavedLayout& l) {
   unsigned char* const b = static_cast<unsigned char*>(saved);
@@ -786,7 +806,7 @@ int launch_walk(const TrainParams& p, bool first, cudaStream_t st) {
   const int rc = once.run([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
   if (rc != KDA_OK) return rc;
   const int cols = std::min(p.V, WalkSmem<K, CPL>::COLS);
-  const long long grid = static_cast<long long>(p.N) * p.H * (p.V / cols);
+  const long long grid = static_cast<long long>(p.N) * p.HL * (p.V / cols);
   if (grid > 0x7fffffffLL) return KDA_E_SHAPE;
   const unsigned threads = static_cast<unsigned>(cols / (4 * CPL) * 32);
   if (!first) return static_cast<int>(launch_chained(kernel, static_cast<unsigned>(grid), threads, smem, st, p));
@@ -794,7 +814,8 @@ int launch_walk(const TrainParams& p, bool first, cudaStream_t st) {
   return static_cast<int>(cudaGetLastError());
 }
 // 32 columns a warp read a row of q, k, exp g for 128 state values instead of 64, and two warps a scheduler are enough to keep the FP32
-// pipe fed; while there are fewer than that, more and narrower warps shorten the chain
+// pipe fed; while there are fewer than that, more and narrower warps shorten the chain.  (Of the call, not of a pass over some of its heads: the two
+// add up in another order, and a pass gives the bits that the whole call gives.)
 bool wide_slices(const TrainParams& p) { return static_cast<long long>(p.N) * p.H * p.V > 32LL * 4 * sm_count(); }
 template <bool FWD>
 int launch_walk(const TrainParams& p, int K, bool first, cudaStream_t st) {
@@ -812,7 +833,7 @@ int launch_mid(const TrainParams& p, cudaStream_t st) {
   const int smem = static_cast<int>(sizeof(typename Mid<K, V>::Smem));
   const int rc = once.run([&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
   if (rc != KDA_OK) return rc;
-  const long long grid = p.slots * p.H * Mid<K, V>::SLICES;
+  const long long grid = p.slots * p.HL * Mid<K, V>::SLICES;
   if (grid > 0x7fffffffLL) return KDA_E_SHAPE;
   return static_cast<int>(launch_chained(kernel, static_cast<unsigned>(grid), Mid<K, V>::NT, smem, st, p));
 }
@@ -843,12 +864,11 @@ int check_backward(const kda_recurrent_bwd_args* a) {
 // saved == NULL: the forward walk runs here first, into the end of the workspace
 int backward(const kda_recurrent_bwd_args* a, const void* saved, size_t saved_bytes, void* stream) {
   const bool with_saved = saved != nullptr;
-  const int HQ = a->HQ > 0 ? a->HQ : a->H;
+  const int HQ = a->HQ > 0 ? a->HQ : a->H, grp = a->H / HQ, K = a->K, V = a->V;
   const Skip skip = skips(*a);
-  const WorkLayout l = work_layout(a->tokens, a->N, a->H, a->K, a->V, skip);
-  const SavedLayout sl = saved_layout(a->tokens, a->H, a->K, a->V, with_saved || a->use_qk_l2norm);
-  if (a->workspace_bytes < l.total + (with_saved ? 0 : sl.total)) return KDA_E_WORKSPACE;
-  if (with_saved && saved_bytes < sl.total) return KDA_E_WORKSPACE;
+  const int most = heads_per_pass(*a, with_saved, a->workspace_bytes);
+  if (!most) return KDA_E_WORKSPACE;
+  if (with_saved && saved_bytes < saved_layout(a->tokens, a->H, K, V, true).total) return KDA_E_WORKSPACE;
   if ((reinterpret_cast<uintptr_t>(a->workspace) | reinterpret_cast<uintptr_t>(saved)) & 255) return KDA_E_ALIGN;
   const void* sixteen[] = {a->v, a->h0, a->d_o, a->d_ht, a->dv, a->dh0};      // 16-byte loads and stores
   for (const void* p : sixteen)
@@ -857,41 +877,51 @@ int backward(const kda_recurrent_bwd_args* a, const void* saved, size_t saved_by
   if (a->N == 0) return KDA_OK;
   if (a->tokens == 0) {      // empty sequences: the initial state is the final state
     if (!a->dh0) return KDA_OK;
-    const size_t bytes = static_cast<size_t>(a->N) * a->H * a->K * a->V * sizeof(float);
-    return static_cast<int>(a->d_ht ? cudaMemcpyAsync(a->dh0, a->d_ht, bytes, cudaMemcpyDeviceToDevice, st) : cudaMemsetAsync(a->dh0, 0, bytes, st));
+    return static_cast<int>(a->d_ht ? cudaMemcpyAsync(a->dh0, a->d_ht, state_bytes(*a), cudaMemcpyDeviceToDevice, st)
+                                    : cudaMemsetAsync(a->dh0, 0, state_bytes(*a), st));
   }
   if (!a->cu_seqlens && static_cast<int64_t>(a->N) * a->T != a->tokens) return KDA_E_SHAPE;
   unsigned char* const ws = static_cast<unsigned char*>(a->workspace);
-  TrainParams p{};
-  p.q = static_cast<const float*>(a->q); p.k = static_cast<const float*>(a->k); p.v = static_cast<const float*>(a->v);
-  p.g = a->g; p.beta = a->beta; p.h0 = a->h0; p.d_o = static_cast<const float*>(a->d_o); p.d_ht = a->d_ht;
-  p.cu = a->cu_seqlens;
-  p.dqh = reinterpret_cast<float*>(ws + l.dqh); p.dkh = reinterpret_cast<float*>(ws + l.dkh);
-  p.dckpt = reinterpret_cast<float*>(ws + l.dckpt); p.dbp = reinterpret_cast<float*>(ws + l.dbp);
-  p.dv = static_cast<float*>(a->dv); p.dg = a->dg; p.dbeta = a->dbeta; p.dh0 = a->dh0;
-  p.T = a->T; p.slots = a->tokens / TC + a->N;
-  p.N = a->N; p.H = a->H; p.HQ = HQ; p.V = a->V; p.use_l2 = a->use_qk_l2norm; p.scale = a->scale;
-  p.wide = wide(a->q, a->k, a->g);
-  const bool direct = skip.dqk;      // nothing to sum or to take back: no pass of its own (0.27 ms at 8 x 2048 x 32)
-  float *const dq = static_cast<float*>(a->dq), *const dk = static_cast<float*>(a->dk);
-  if (direct) p.dqh = dq, p.dkh = dk;
-  p.dq_scale = direct ? p.scale : 1.f;
-  use_saved(p, with_saved ? const_cast<void*>(saved) : ws + l.total, sl);
+  const WorkLayout l = work_layout(a->tokens, a->N, most, a->H, K, V, skip);
+  const float *h0 = a->h0, *d_ht = a->d_ht;
   int rc = KDA_OK;
   auto keep = [&](bool not_needed, const float*& x, size_t at) {
     if (not_needed || rc != KDA_OK) return;
     rc = static_cast<int>(cudaMemcpyAsync(ws + at, x, state_bytes(*a), cudaMemcpyDeviceToDevice, st));
     x = reinterpret_cast<const float*>(ws + at);
   };
-  keep(skip.h0, p.h0, l.h0);
-  keep(skip.d_ht, p.d_ht, l.d_ht);
-  if (rc != KDA_OK) return rc;
-  if (!with_saved) rc = launch_walk<true>(p, a->K, true, st);
-  if (rc == KDA_OK) rc = launch_walk<false>(p, a->K, with_saved, st);
-  const long long rows = a->tokens * HQ;
-  if (rc == KDA_OK) rc = a->K == 32 ? launch_mid<32>(p, st) : (a->K == 64 ? launch_mid<64>(p, st) : launch_mid<128>(p, st));
-  if (rc == KDA_OK && !direct)
-    rc = a->K == 32 ? launch_finish<32>(p, dq, dk, rows, st) : (a->K == 64 ? launch_finish<64>(p, dq, dk, rows, st) : launch_finish<128>(p, dq, dk, rows, st));
+  keep(skip.h0, h0, l.h0);
+  keep(skip.d_ht, d_ht, l.d_ht);
+  for (int h = 0; h < a->H && rc == KDA_OK; h += most) {
+    TrainParams p{};
+    p.N = a->N; p.H = a->H; p.HQ = HQ; p.V = V; p.T = a->T; p.slots = a->tokens / TC + a->N; p.cu = a->cu_seqlens;
+    p.HL = std::min(most, a->H - h); p.HS = with_saved ? a->H : p.HL; p.HW = p.HL;
+    p.use_l2 = a->use_qk_l2norm; p.scale = a->scale; p.wide = wide(a->q, a->k, a->g);
+    auto from = [&](auto* x, int per_head) { return x ? x + static_cast<size_t>(h) * per_head : x; };
+    const size_t qk = static_cast<size_t>(h / grp) * K;
+    p.q = static_cast<const float*>(a->q) + qk; p.k = static_cast<const float*>(a->k) + qk;
+    p.v = from(static_cast<const float*>(a->v), V); p.d_o = from(static_cast<const float*>(a->d_o), V); p.dv = from(static_cast<float*>(a->dv), V);
+    p.g = from(a->g, K); p.dg = from(a->dg, K); p.beta = from(a->beta, 1); p.dbeta = from(a->dbeta, 1);
+    p.h0 = from(h0, K * V); p.d_ht = from(d_ht, K * V); p.dh0 = from(a->dh0, K * V);
+    p.dckpt = reinterpret_cast<float*>(ws + l.dckpt); p.dbp = reinterpret_cast<float*>(ws + l.dbp);
+    float *const dq = static_cast<float*>(a->dq) + qk, *const dk = static_cast<float*>(a->dk) + qk;
+    const bool direct = skip.dqk;      // nothing to sum or to take back: no pass of its own (0.27 ms at 8 x 2048 x 32)
+    p.dqh = direct ? dq : reinterpret_cast<float*>(ws + l.dqh); p.dkh = direct ? dk : reinterpret_cast<float*>(ws + l.dkh);
+    p.HD = direct ? a->H : p.HL;
+    p.dq_scale = direct ? p.scale : 1.f;
+    if (with_saved) {
+      use_saved(p, const_cast<void*>(saved), saved_layout(a->tokens, a->H, K, V, true));
+      p.ckpt = from(p.ckpt, K * V); p.resid = from(p.resid, V); p.norms = from(p.norms, 2);
+    } else {
+      use_saved(p, ws + l.total, saved_layout(a->tokens, most, K, V, p.use_l2 != 0));
+      rc = launch_walk<true>(p, K, h == 0, st);
+    }
+    if (rc == KDA_OK) rc = launch_walk<false>(p, K, with_saved && h == 0, st);
+    if (rc == KDA_OK) rc = K == 32 ? launch_mid<32>(p, st) : (K == 64 ? launch_mid<64>(p, st) : launch_mid<128>(p, st));
+    const long long rows = a->tokens * (p.HL / grp);
+    if (rc == KDA_OK && !direct)
+      rc = K == 32 ? launch_finish<32>(p, dq, dk, rows, st) : (K == 64 ? launch_finish<64>(p, dq, dk, rows, st) : launch_finish<128>(p, dq, dk, rows, st));
+  }
   return rc;
 }
 
@@ -909,13 +939,14 @@ extern "C" size_t kda_recurrent_saved_bytes(int64_t tokens, int32_t N, int32_t H
 // (an upper bound over all options; kda_recurrent_bwd_scratch_bytes knows them)
 extern "C" size_t kda_recurrent_bwd_workspace_bytes(int64_t tokens, int32_t N, int32_t H, int32_t K, int32_t V) {
   if (tokens < 0 || N < 0 || H <= 0 || K <= 0 || V <= 0) return 0;
-  return work_layout(tokens, N, H, K, V, NOTHING).total + saved_layout(tokens, H, K, V, true).total;
+  return work_layout(tokens, N, H, H, K, V, NOTHING).total + saved_layout(tokens, H, K, V, true).total;
 }
 
-extern "C" size_t kda_recurrent_bwd_scratch_bytes(const kda_recurrent_bwd_args* a, int32_t with_saved) {
+extern "C" size_t kda_recurrent_bwd_scratch_bytes(const kda_recurrent_bwd_args* a, int32_t with_saved, int32_t passes) {
   if (!a || a->tokens < 0 || a->N < 0 || a->H <= 0 || !head_size_ok(a->K) || !head_size_ok(a->V)) return 0;
-  return work_layout(a->tokens, a->N, a->H, a->K, a->V, skips(*a)).total +
-         (with_saved ? 0 : saved_layout(a->tokens, a->H, a->K, a->V, a->use_qk_l2norm != 0).total);
+  const int HQ = a->HQ > 0 ? a->HQ : a->H;
+  if (a->H % HQ) return 0;
+  return scratch_bytes(*a, heads_of(*a, std::max(1, std::min(passes, HQ))), with_saved != 0);
 }
 
 // the forward walk; with_saved: leaves what a backward then need not compute again
@@ -942,7 +973,7 @@ static int forward(const kda_recurrent_args* a, void* saved, size_t saved_bytes,
   p.g = a->g; p.beta = a->beta; p.h0 = a->h0; p.ht = a->ht; p.o = static_cast<float*>(a->o);
   p.cu = a->cu_seqlens;
   p.T = a->T;
-  p.N = a->N; p.H = a->H; p.HQ = HQ; p.V = a->V; p.use_l2 = a->use_qk_l2norm; p.scale = a->scale;
+  p.N = a->N; p.H = p.HL = p.HS = a->H; p.HQ = HQ; p.V = a->V; p.use_l2 = a->use_qk_l2norm; p.scale = a->scale;
   p.wide = wide(a->q, a->k, a->g);
   if (with_saved) use_saved(p, saved, sl);
   return launch_walk<true>(p, a->K, true, static_cast<cudaStream_t>(stream));
@@ -970,6 +1001,6 @@ extern "C" int kda_recurrent_train_bwd(const kda_recurrent_bwd_args* args, const
   const int rc = check_backward(args);
   if (rc != KDA_OK) return rc;
   if (!saved) return KDA_E_NULL;
-  if (args->workspace_bytes < work_layout(args->tokens, args->N, args->H, args->K, args->V, NOTHING).total) return KDA_E_WORKSPACE;
+  if (args->workspace_bytes < work_layout(args->tokens, args->N, args->H, args->H, args->K, args->V, NOTHING).total) return KDA_E_WORKSPACE;
   return backward(args, saved, saved_bytes, stream);
 }

@@ -268,6 +268,18 @@ def fused_recurrent_kda(q, k, v, g, beta, A_log=None, dt_bias=None, scale=None, 
                                    transpose_state_layout=transpose_state_layout)
 
 
+def _bwd_scratch(lib, args, with_saved, q_heads, dev):
+    """Scratch of the float32 backward: all heads at once, or, on a device that has no room for that, as many of them as fit."""
+    passes = 1
+    while True:
+        try:
+            return torch.empty(lib.kda_recurrent_bwd_scratch_bytes(C.byref(args), with_saved, passes), dtype=torch.uint8, device=dev)
+        except torch.OutOfMemoryError:
+            if passes >= q_heads:
+                raise
+            passes = min(2 * passes, q_heads)
+
+
 class RecurrentKDAFunction(torch.autograd.Function):
     """float32 path of chunk_kda with gradients: token-recurrent forward and its exact reverse mode (fla/ops/kda/naive.py:12-66
     differentiated).  K, V in {32, 64, 128}.  A call keeps its inputs and the backward (`kda_recurrent_bwd_scratch`) replays the forward
@@ -322,7 +334,7 @@ class RecurrentKDAFunction(torch.autograd.Function):
             q=_ptr(q), k=_ptr(k), v=_ptr(v), g=_ptr(g32), beta=_ptr(beta32), h0=_ptr(h0), cu_seqlens=_ptr(cu),
             d_o=_ptr(do), d_ht=_ptr(dht), dq=_ptr(dq), dk=_ptr(dk), dv=_ptr(dv), dg=_ptr(dg), dbeta=_ptr(dbeta), dh0=_ptr(dh0),
             tokens=B * T, N=N, T=T, H=H, K=K, V=V, HQ=HQ, io_dtype=_lib.KDA_FP32, use_qk_l2norm=int(use_l2norm), scale=scale)
-        ws = torch.empty(lib.kda_recurrent_bwd_scratch_bytes(C.byref(args), saved is not None), dtype=torch.uint8, device=dev)
+        ws = _bwd_scratch(lib, args, saved is not None, HQ, dev)
         args.workspace, args.workspace_bytes = _ptr(ws), ws.numel()
         with torch.cuda.device(dev):
             _lib.check(lib.kda_recurrent_bwd_scratch(C.byref(args), _ptr(saved), saved.numel() if saved is not None else 0, _stream(dev)),

@@ -185,7 +185,7 @@ def _bwd_args(**kw):
 def test_float32_backward_scratch_holds_what_the_call_needs(lib):
     """kda_recurrent_bwd_scratch_bytes: two rows per token for per-value-head dq, dk only with grouped heads or normalised rows, norms only with
     normalised rows, copies of h0 and d_ht only where dh0 overlaps them, and no states per sequence."""
-    size = lambda saved=0, **kw: lib.kda_recurrent_bwd_scratch_bytes(C.byref(_bwd_args(**kw)), saved)      # noqa: E731
+    size = lambda saved=0, passes=1, **kw: lib.kda_recurrent_bwd_scratch_bytes(C.byref(_bwd_args(**kw)), saved, passes)      # noqa: E731
     rows, states = 16384 * 32 * 128 * 4, 8 * 32 * 128 * 128 * 4
     assert size() < 16384 // 32 * 32 * 65536 * 2 + 1.2 * rows                 # the kept states and r, dbeta's parts
     assert size(use_qk_l2norm=1) - size() == 2 * rows + 16384 * 32 * 8
@@ -199,5 +199,11 @@ def test_float32_backward_scratch_holds_what_the_call_needs(lib):
     bound = lib.kda_recurrent_bwd_workspace_bytes(16384, 8, 32, 128, 128)
     assert bound == size(use_qk_l2norm=1, HQ=8, h0=1 << 40, d_ht=1 << 40, dh0=1 << 40)
     run = lambda n, **kw: lib.kda_recurrent_bwd_scratch(C.byref(_bwd_args(workspace_bytes=n, **kw)), None, 0, None)      # noqa: E731
-    assert run(size() - 1) == -5 and run(size(HQ=8) - 1, HQ=8) == -5
+    # in passes over the heads: a whole number of q/k heads each; the call takes what holds one (the next check after the scratch is of the alignment)
+    row = 16384 * (2 * 2048 + 512 + 32)
+    assert [size(passes=n) for n in (0, 1, 2, 3, 32, 99)] == [row * n for n in (32, 32, 16, 11, 1, 1)]
+    assert size(passes=4, HQ=4) == (row + 16384 * 1024) * 8 == size(passes=99, HQ=4)
+    assert run(size(), d_o=260) == run(size() - 1, d_o=260) == run(row, d_o=260) == -4 and run(row - 1) == -5
+    assert run(size(passes=4, HQ=4), HQ=4, d_o=260) == -4 and run(size(passes=4, HQ=4) - 1, HQ=4) == -5
+    assert run(size(HQ=1), HQ=1, d_o=260) == -4 and run(size(HQ=1) - 1, HQ=1) == -5
     assert run(1 << 40, K=96) == -2 and run(1 << 40, io_dtype=0) == -3 and run(1 << 40, dq=None) == -1 and run(1 << 40, d_o=260) == -4

@@ -322,7 +322,7 @@ def test_fp32_backward_scratch_bits_margins_and_states_in_place(lens, over, save
     a = _lib.RecurrentBwdArgs(q=p(d["q"]), k=p(d["k"]), v=p(d["v"]), g=p(d["g"]), beta=p(d["beta"]), h0=p(h0), cu_seqlens=p(cu), d_o=p(d["do"]),
                               d_ht=p(dht), dq=p(out["q"]), dk=p(out["k"]), dv=p(out["v"]), dg=p(out["g"]), dbeta=p(out["beta"]), dh0=p(out["h0"]),
                               **sizes)
-    wg, ws = guarded_like((lib.kda_recurrent_bwd_scratch_bytes(C.byref(a), saved),), torch.uint8)
+    wg, ws = guarded_like((lib.kda_recurrent_bwd_scratch_bytes(C.byref(a), saved, 1),), torch.uint8)
     a.workspace, a.workspace_bytes = p(ws), ws.numel()
     _lib.check(lib.kda_recurrent_bwd_scratch(C.byref(a), p(kept) if saved else None, kept.numel() if saved else 0, st), "kda_recurrent_bwd_scratch")
     torch.cuda.synchronize()
@@ -331,3 +331,76 @@ def test_fp32_backward_scratch_bits_margins_and_states_in_place(lens, over, save
     for n in out:
         assert torch.equal(out[n], lv[n].grad), n
 
+
+@pytest.mark.parametrize("K,V,HQ,H,l2,lens", [(128, 128, 5, 5, False, [70, 32, 5]), (64, 128, 2, 6, False, [33, 64]), (128, 32, 3, 3, True, [200]),
+                                              (128, 128, 3, 6, True, [1, 96, 40])])
+@pytest.mark.parametrize("saved", [False, True])
+def test_fp32_backward_over_groups_of_heads(K, V, HQ, H, l2, lens, saved):
+    """A scratch that does not hold all heads: they are worked on in groups (of one q/k head, and of as many as two thirds of the scratch hold),
+    between sentinel margins; the bits of the whole call."""
+    import ctypes as C
+    from _abi import guarded_like
+    from kda_b200 import _lib
+    lib = _lib.load()
+    tokens, N = sum(lens), len(lens)
+    d = make_inputs(1, tokens, H, K, V, torch.float32, seed=56 + tokens, h0_std=0.1, n_states=N, backward=True)
+    d = {n: t.cuda().contiguous() for n, t in d.items()}
+    d["q"], d["k"] = (d[n][:, :, :HQ].contiguous() for n in ("q", "k"))
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device="cuda")
+    p = lambda t: C.c_void_p(t.data_ptr())      # noqa: E731
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    sizes = dict(tokens=tokens, N=N, T=0, H=H, K=K, V=V, HQ=HQ, io_dtype=_lib.KDA_FP32, use_qk_l2norm=int(l2), scale=K ** -0.5)
+    inputs = dict(q=p(d["q"]), k=p(d["k"]), v=p(d["v"]), g=p(d["g"]), beta=p(d["beta"]), h0=p(d["h0"]), cu_seqlens=p(cu))
+    kept, kept_bytes = None, 0
+    if saved:
+        kept = torch.empty(lib.kda_recurrent_saved_bytes(tokens, N, H, K, V), dtype=torch.uint8, device="cuda")
+        kept_bytes, o = kept.numel(), torch.empty_like(d["v"])
+        f = _lib.RecurrentArgs(**inputs, o=p(o), **sizes)
+        _lib.check(lib.kda_recurrent_train_fwd(C.byref(f), p(kept), kept_bytes, st), "kda_recurrent_train_fwd")
+    got = []
+    for part in (1.0, 2 / 3, 1 / HQ):
+        guards, out = [], {}
+        for n in ("q", "k", "v", "g", "beta", "h0"):
+            g, out[n] = guarded_like(tuple(d[n].shape), torch.float32)
+            guards.append((n, g))
+        a = _lib.RecurrentBwdArgs(**inputs, d_o=p(d["do"]), d_ht=p(d["dht"]), dq=p(out["q"]), dk=p(out["k"]), dv=p(out["v"]), dg=p(out["g"]),
+                                  dbeta=p(out["beta"]), dh0=p(out["h0"]), **sizes)
+        whole = lib.kda_recurrent_bwd_scratch_bytes(C.byref(a), saved, 1)
+        size = whole if part == 1 else int(part * whole) + 7 * 256      # (each of the buffers is rounded up to 256 bytes)
+        wg, ws = guarded_like((size,), torch.uint8)
+        a.workspace, a.workspace_bytes = p(ws), size
+        _lib.check(lib.kda_recurrent_bwd_scratch(C.byref(a), p(kept) if saved else None, kept_bytes, st), "kda_recurrent_bwd_scratch")
+        torch.cuda.synchronize()
+        for n, g in [*guards, ("scratch", wg)]:
+            assert g.margins_intact(), n
+        got.append(out)
+    for n in got[0]:
+        assert torch.equal(got[0][n], got[1][n]) and torch.equal(got[0][n], got[2][n]), n
+    ref = recurrent_kda_grads(d["q"].repeat_interleave(H // HQ, 2), d["k"].repeat_interleave(H // HQ, 2), *(d[n] for n in ("v", "g", "beta", "do", "dht")),
+                              initial_state=d["h0"], cu_seqlens=cu, use_qk_l2norm=l2)
+    assert max_norm_err(got[0]["v"], ref["dv"]) <= TOL and max_norm_err(got[0]["g"], ref["dg"]) <= TOL
+    for n in ("q", "k"):
+        assert max_norm_err(got[0][n], ref["d" + n].view(1, tokens, HQ, H // HQ, K).sum(3)) <= TOL, n
+
+
+def test_fp32_backward_takes_the_memory_that_is_there():
+    """The scratch for all heads at once (152 MB here) does not fit what the allocator may still hand out: the call makes do with a part, same bits."""
+    from kda_b200 import chunk_kda
+    d = {n: t.cuda() for n, t in make_inputs(1, 4096, 8, 128, 128, torch.float32, seed=57, backward=True).items() if t is not None}
+    lv = [d[n].requires_grad_(True) for n in ("q", "k", "v", "g", "beta")]
+    o, _ = chunk_kda(*lv)
+    first = torch.autograd.grad(o, lv, d["do"], retain_graph=True)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    grads = sum(t.numel() * 4 for t in first)
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + grads + (100 << 20)) / total)
+    try:
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        second = torch.autograd.grad(o, lv, d["do"])
+        torch.cuda.synchronize()
+        assert torch.cuda.max_memory_allocated() - before - grads < 100 << 20
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert all(torch.equal(a, b) for a, b in zip(first, second))
