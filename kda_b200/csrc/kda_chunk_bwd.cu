@@ -157,7 +157,7 @@ extern "C" int kda_chunk_bwd(const kda_chunk_args* args, void* stream) {
   rp.map = chunk_map(w, a.cu_seqlens, a.tokens, a.N);
   rp.W = w.W; rp.KG = w.KG; rp.QG = w.QG; rp.AQK = w.AQK; rp.GL = w.GL;
   rp.DH = w.DH; rp.DVNEWT = w.DVNEWT;
-  rp.d_o = static_cast<const __nv_bfloat16*>(a.d_o); rp.d_ht = a.d_ht; rp.dh0 = a.dh0; rp.status = w.status; rp.dbg = g_dbg_clocks;
+  rp.d_ht = a.d_ht; rp.dh0 = a.dh0; rp.status = w.status; rp.dbg = g_dbg_clocks;
   rp.H = a.H; rp.kc = kc; rp.vc = vc;
   if (make_rows_tmap(&rp.tm_do, a.d_o, false, a.tokens, a.H, vc, 64, C, true)) return KDA_E_TMAP;
   const int slices = scan_slices_for(a.N * a.H, a.scan_slices);
@@ -165,21 +165,21 @@ extern "C" int kda_chunk_bwd(const kda_chunk_args* args, void* stream) {
   prof_mark(prof, KDA_STAGE_BWD_SCAN, st);
 
   MainParams mp{};
-  mp.q = q; mp.k = k; mp.v = static_cast<const __nv_bfloat16*>(a.v); mp.d_o = static_cast<const __nv_bfloat16*>(a.d_o);
-  mp.g = a.g; mp.beta = a.beta; mp.map = rp.map;
+  mp.beta = a.beta; mp.map = rp.map;
   mp.TI = w.TI; mp.RKK = w.RKK; mp.HS = w.HS; mp.VNEWT = w.VNEWT; mp.DH = w.DH; mp.DVNEWT = w.DVNEWT;
   mp.dv = static_cast<__nv_bfloat16*>(a.dv);
   // grouped value heads: every value head writes its own dq, dk; a second kernel sums each group
   mp.dq = grp > 1 ? w.DQH : static_cast<__nv_bfloat16*>(a.dq);
   mp.dk = grp > 1 ? w.DKH : static_cast<__nv_bfloat16*>(a.dk);
-  mp.kc = kc; mp.vc = vc; mp.qc = l2 ? KD : kc; mp.dqc = grp > 1 ? KD : kc;
+  mp.kc = kc; mp.vc = vc; mp.dqc = grp > 1 ? KD : kc;
   mp.dbeta = a.dbeta; mp.dg = a.dg; mp.status = w.status; mp.dbg = g_dbg_clocks;
-  if (make_rows_tmap(&mp.tm_q, q, false, a.tokens, HQ, mp.qc, KD, C, false) || make_rows_tmap(&mp.tm_k, k, false, a.tokens, HQ, mp.qc, KD, C, false) ||
+  const int qc = l2 ? KD : kc;      // columns of a row of q, k (the kept normalised rows have 128)
+  if (make_rows_tmap(&mp.tm_q, q, false, a.tokens, HQ, qc, KD, C, false) || make_rows_tmap(&mp.tm_k, k, false, a.tokens, HQ, qc, KD, C, false) ||
       make_rows_tmap(&mp.tm_g, a.g, true, a.tokens, a.H, kc, KD, C, false) ||
       make_rows_tmap(&mp.tm_v, a.v, false, a.tokens, a.H, vc, 64, C, true) ||
       make_rows_tmap(&mp.tm_do, a.d_o, false, a.tokens, a.H, vc, 64, C, true) ||
       make_rows_tmap(&mp.tm_dq, mp.dq, false, a.tokens, a.H, mp.dqc, KD, C, false) || make_rows_tmap(&mp.tm_dk, mp.dk, false, a.tokens, a.H, mp.dqc, KD, C, false) ||
-      (reinterpret_cast<uintptr_t>(a.dg) & 15) || make_rows_tmap(&mp.tm_dv, a.dv, false, a.tokens, a.H, vc, 32, C, false))
+      make_rows_tmap(&mp.tm_dv, a.dv, false, a.tokens, a.H, vc, 32, C, false))
     return KDA_E_TMAP;
   mp.H = a.H; mp.scale = a.scale; mp.grp = grp;
   // without grouped heads the normalisation's backward is applied by bwd_main's own epilogue

@@ -7,8 +7,7 @@
 namespace kda {
 
 struct MainParams {
-  const __nv_bfloat16 *q, *k, *v, *d_o;
-  const float *g, *beta;
+  const float* beta;
   ChunkMap map;
   const unsigned char *TI, *RKK, *HS, *VNEWT, *DH, *DVNEWT;
   __nv_bfloat16 *dv, *dq, *dk;
@@ -17,11 +16,10 @@ struct MainParams {
   long long* dbg;
   int H;
   int kc, vc;       // key and value columns of the tensors (<= 128; tiles are 128 wide, zero beyond)
-  int qc;           // columns of a row of q, k as the kernel reads them (kc, or 128 for the kept normalised rows)
   int dqc;          // columns of a row of dq, dk as the kernel writes them (kc, or 128 for the per-value-head scratch)
   float scale;
   int grp;          // value heads per q/k head (grouped value heads): the q, k maps have H / grp heads
-  const float* rstd;    // [2][qrows] reciprocal norms of the q, k rows, or NULL.  Not NULL (only with grp == 1): q, k are the
+  const float* rstd;    // [2][qrows] reciprocal norms of the q, k rows, or NULL.  Not NULL (only with grp == 1): tm_q, tm_k are of the
   long long qrows;      // L2-normalised rows and the kernel applies the normalisation's backward to dq, dk before storing them
   // tiled-load maps of the [tokens, H, 128] operator tensors (64-token boxes of one head)
   alignas(64) CUtensorMap tm_q, tm_k, tm_g;   // plain row-major boxes [64][128]
@@ -33,7 +31,6 @@ struct RScanParams {
   ChunkMap map;
   const unsigned char *W, *KG, *QG, *AQK, *GL;
   unsigned char *DH, *DVNEWT;
-  const __nv_bfloat16* d_o;
   const float* d_ht;
   float* dh0;
   unsigned* status;
