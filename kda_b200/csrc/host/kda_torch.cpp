@@ -152,7 +152,8 @@ struct RecurrentCall {
   Tensor q, k, v, g, beta, A_log, dt_bias, h0, cu, slots, accepted, out;
   std::optional<double> scale, lower_bound;
   bool output_final = false, inplace = false, l2norm = false, gate = false, beta_sigmoid = false, transposed = false;
-  bool training = false;      // float32 with gradients: the forward that the replaying backward belongs to
+  bool training = false;      // float32 with gradients: the forward that the backward belongs to,
+  Tensor saved;               // and what it leaves for it (undefined: nothing)
 };
 
 std::pair<Tensor, Tensor> recurrent_fwd(RecurrentCall& c) {
@@ -222,7 +223,8 @@ std::pair<Tensor, Tensor> recurrent_fwd(RecurrentCall& c) {
   a.io_dtype = dtype_code(q); a.use_qk_l2norm = c.l2norm; a.transpose_state = c.transposed;
   a.scale = static_cast<float>(c.scale ? *c.scale : 1.0 / std::sqrt(static_cast<double>(s.K)));
   if (c.training) {
-    check_rc(kda_recurrent_walk_fwd(&a, stream_of(dev)), "kda_recurrent_walk_fwd");
+    if (c.saved.defined()) check_rc(kda_recurrent_train_fwd(&a, c.saved.data_ptr(), static_cast<size_t>(c.saved.numel()), stream_of(dev)), "kda_recurrent_train_fwd");
+    else check_rc(kda_recurrent_walk_fwd(&a, stream_of(dev)), "kda_recurrent_walk_fwd");
     return {o, ht};
   }
   check_rc(kda_recurrent_fwd(&a, stream_of(dev)), "kda_recurrent_fwd");
@@ -525,7 +527,8 @@ PyObject* py_recurrent_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   c.slots = tensor_arg(a[12], "ssm_state_indices"); c.accepted = tensor_arg(a[13], "num_accepted_tokens"); c.l2norm = bool_arg(a[14]);
   c.gate = bool_arg(a[15]); c.beta_sigmoid = bool_arg(a[16]); c.lower_bound = double_arg(a[17]); c.out = tensor_arg(a[18], "out");
   c.transposed = bool_arg(a[19]);
-  c.training = n == 21 && bool_arg(a[20]);
+  c.training = n == 21;
+  if (c.training) c.saved = tensor_arg(a[20], "saved");
   std::pair<Tensor, Tensor> r;
   {
     GilRelease nogil;

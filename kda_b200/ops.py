@@ -9,8 +9,11 @@ CPU tensors, a missing shared library or an unsupported option raise.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import math
 import os
+import threading
+import weakref
 
 import torch
 
@@ -268,6 +271,33 @@ def fused_recurrent_kda(q, k, v, g, beta, A_log=None, dt_bias=None, scale=None, 
                                    transpose_state_layout=transpose_state_layout)
 
 
+# Bytes that float32 calls waiting for their backward keep on each device: (device index, bytes) by a weak reference to each buffer, which takes its
+# entry out when the buffer is freed (after the backward, with the graph, or by a hook that moves saved tensors elsewhere).
+_kept: dict = {}
+_kept_lock = threading.Lock()
+
+
+@functools.lru_cache(maxsize=None)
+def _keep_limit(index: int) -> int:
+    """What those calls may keep together: 1/128 of the device, 1.5 of 180 GB.  8 x 2048 x 32 heads of 128 keep 1.35 GB and their step takes 8.8 instead
+    of 10.6 ms; a model of many layers holds no more than this for all of them, which is about the scratch that one backward takes anyway."""
+    return torch.cuda.get_device_properties(index).total_memory // 128
+
+
+def _keep(n: int, dev, asked: bool):
+    """A buffer of n bytes for what a forward leaves for its backward, or None: the backward replays the forward."""
+    with _kept_lock:
+        held = sum(b for d, b in list(_kept.values()) if d == dev.index)
+        if not asked and held + n > _keep_limit(dev.index):
+            return None
+        try:
+            saved = torch.empty(n, dtype=torch.uint8, device=dev)
+        except torch.OutOfMemoryError:
+            return None
+        _kept[weakref.ref(saved, lambda r: _kept.pop(r, None))] = (dev.index, n)
+    return saved
+
+
 def _bwd_scratch(lib, args, with_saved, q_heads, dev):
     """Scratch of the float32 backward: all heads at once, or, on a device that has no room for that, as many of them as fit."""
     passes = 1
@@ -282,9 +312,9 @@ def _bwd_scratch(lib, args, with_saved, q_heads, dev):
 
 class RecurrentKDAFunction(torch.autograd.Function):
     """float32 path of chunk_kda with gradients: token-recurrent forward and its exact reverse mode (fla/ops/kda/naive.py:12-66
-    differentiated).  K, V in {32, 64, 128}.  A call keeps its inputs and the backward (`kda_recurrent_bwd_scratch`) replays the forward
-    (`kda_recurrent_walk_fwd`); with `keep` the forward (`kda_recurrent_train_fwd`) also leaves the state of every 32nd token and a row per token
-    until the backward, which is then shorter: the same bits."""
+    differentiated).  K, V in {32, 64, 128}.  The forward (`kda_recurrent_train_fwd`) leaves the state of every 32nd token and a row per token for
+    the backward (`kda_recurrent_bwd_scratch`) where there is room for that (`_keep`, or the caller asked for it); otherwise the call keeps its inputs
+    alone and the backward replays the forward (`kda_recurrent_walk_fwd`).  The same bits."""
 
     @staticmethod
     def forward(ctx, q, k, v, g, beta, scale, initial_state, output_final_state, use_l2norm, cu_seqlens, keep):
@@ -292,25 +322,14 @@ class RecurrentKDAFunction(torch.autograd.Function):
         g32, beta32 = g.contiguous().float(), beta.contiguous().float()
         h0 = initial_state.contiguous().float() if initial_state is not None else None
         cu = _as_i32(cu_seqlens, q.device) if cu_seqlens is not None else None
-        if keep:
-            B, T, HQ, K = q.shape
-            H, V = v.shape[-2], v.shape[-1]
-            N = B if cu is None else cu.numel() - 1
-            dev = q.device
-            lib = _lib.load()
-            o = torch.empty_like(v)
-            ht = torch.empty(N, H, K, V, dtype=torch.float32, device=dev) if output_final_state else None
-            saved = torch.empty(lib.kda_recurrent_saved_bytes(B * T, N, H, K, V), dtype=torch.uint8, device=dev)
-            args = _lib.RecurrentArgs(
-                q=_ptr(q), k=_ptr(k), v=_ptr(v), g=_ptr(g32), beta=_ptr(beta32), h0=_ptr(h0), ht=_ptr(ht), o=_ptr(o), cu_seqlens=_ptr(cu),
-                tokens=B * T, N=N, T=T, H=H, K=K, V=V, HQ=HQ, io_dtype=_lib.KDA_FP32, use_qk_l2norm=int(use_l2norm), scale=scale)
-            with torch.cuda.device(dev):
-                _lib.check(lib.kda_recurrent_train_fwd(C.byref(args), _ptr(saved), saved.numel(), _stream(dev)), "kda_recurrent_train_fwd")
-        else:
-            saved = None
-            o, ht = (_lib._native or _lib.native()).recurrent_fwd(
-                q, k, v, g32, beta32, None, None, h0, scale, output_final_state, False, cu, None, None, use_l2norm, False, False, None, None, False,
-                True)
+        B, T, _, K = q.shape
+        H, V = v.shape[-2:]
+        # (up to 48 tokens the device waits for the host, which takes 10 us over the buffer and 4 over the replay: one token x 8 heads 145 and 134 us)
+        saved = None
+        if keep or B * T > 48:
+            saved = _keep(_lib.load().kda_recurrent_saved_bytes(B * T, B if cu is None else cu.numel() - 1, H, K, V), q.device, keep)
+        o, ht = (_lib._native or _lib.native()).recurrent_fwd(
+            q, k, v, g32, beta32, None, None, h0, scale, output_final_state, False, cu, None, None, use_l2norm, False, False, None, None, False, saved)
         ctx.save_for_backward(q, k, v, g32, beta32, h0, cu, saved)
         ctx.meta = (float(scale), bool(use_l2norm), g.dtype, beta.dtype)
         return o, ht
@@ -513,9 +532,10 @@ def chunk_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_sta
     token-recurrent fp32 kernels: forward for K in {32, 64, 128, 256}, with gradients for K, V in {32, 64, 128}.  `safe_gate=True` is the caller's promise that every gate value is at least
     -5 (fla/ops/kda/chunk.py:235-246); the forward then computes the diagonal 16 x 16 blocks of the intra-chunk products on
     tensor cores as well (factored around each block's middle row) instead of pairwise, which is faster and only safe under
-    that bound; without it the kernels are range-safe for any gate.  `disable_recompute=True` lets a float32
-    call with gradients keep intermediates for its backward (2.5 KB per token and head of 128) instead of replaying the forward there: faster, the
-    same bits; the bf16 kernels always keep theirs; `chunk_size` (32 or
+    that bound; without it the kernels are range-safe for any gate.  `disable_recompute=True` makes a
+    float32 call with gradients keep intermediates for its backward (2.5 KB per token and head of 128) whatever the room; by default it does so
+    while all calls that wait for their backward keep at most 1/128 of the device's memory, and the backward replays the forward otherwise: the same
+    bits.  The bf16 kernels always keep theirs.  `chunk_size` (32 or
     64) changes nothing but the spacing of the intermediate states (the kernels always tile by 64 tokens); options
     that change results and are not built raise.
     """

@@ -262,23 +262,37 @@ def test_fp32_backward_of_short_sequences_does_not_cost_32_tokens():
 
 
 @pytest.mark.parametrize("l2,states", [(False, True), (True, False)])
-def test_fp32_training_call_keeps_only_its_inputs(l2, states):
-    """Between forward and backward a float32 call holds no memory but its results, unless it is asked to (`disable_recompute`): gradients, o and the
-    final state are the same bits either way."""
-    from kda_b200 import chunk_kda
+def test_fp32_training_calls_keep_no_more_than_their_share(l2, states, monkeypatch):
+    """Between forward and backward float32 calls keep intermediates up to a bound for all of them together; a call beyond it holds no memory but its
+    results, unless it is asked to (`disable_recompute`).  What one call kept is given back with its backward.  The same bits either way."""
+    from kda_b200 import chunk_kda, ops
     d = {n: t.cuda() for n, t in make_inputs(2, 333, 4, 128, 128, torch.float32, seed=54, h0_std=0.1, backward=True).items() if t is not None}
     lv = [d[n].requires_grad_(True) for n in ("q", "k", "v", "g", "beta", "h0")[:6 if states else 5]]
-    got, kept = [], []
-    for keep in (False, True):
+    one = 2 * (333 // 32) * 4 * 65536 + 2 * 333 * 4 * 512      # a state per 32 tokens and r, at least
+    monkeypatch.setattr(ops, "_keep_limit", lambda index: 3 * one)
+
+    def forward(**kw):
         before = torch.cuda.memory_allocated()
-        o, ht = chunk_kda(*lv[:5], initial_state=lv[5] if states else None, output_final_state=states, use_qk_l2norm_in_kernel=l2,
-                          disable_recompute=keep)
-        kept.append(torch.cuda.memory_allocated() - before - o.numel() * 4 - (ht.numel() * 4 if states else 0))
-        grads = torch.autograd.grad([o, ht][:1 + states], lv, [d["do"], d["dht"]][:1 + states])
-        got.append([o, *([ht] if states else []), *grads])
-    # nothing but rounding; a state per 32 tokens, and r (blocks of the allocator above 1 MB may be up to 1 MB larger than asked for)
-    assert kept[0] < 4096 and kept[1] > 2 * (333 // 32) * 4 * 65536 + 2 * 333 * 4 * 512
-    assert all(torch.equal(a, b) for a, b in zip(*got))
+        o, ht = chunk_kda(*lv[:5], initial_state=lv[5] if states else None, output_final_state=states, use_qk_l2norm_in_kernel=l2, **kw)
+        kept = torch.cuda.memory_allocated() - before - o.numel() * 4 - (ht.numel() * 4 if states else 0)
+        return [o, ht][:1 + states], kept
+
+    def backward(r, **kw):
+        return [*r, *torch.autograd.grad(r, lv, [d["do"], d["dht"]][:1 + states], **kw)]
+
+    calls = [forward() for _ in range(4)]                       # two have room, then none, then one that is asked to
+    calls.append(forward(disable_recompute=True))
+    assert [k >= one for _, k in calls] == [True, True, False, False, True]
+    assert all(k < 4096 for _, k in calls[2:4])
+    got = [backward(r, retain_graph=i == 0) for i, (r, _) in enumerate(calls)]
+    assert forward()[1] >= one                                  # (its graph goes at once)
+    assert [forward()[1] >= one for _ in range(3)] == [True] * 3
+    got.append(backward(calls[0][0]))
+    assert not ops._kept
+    o, _ = chunk_kda(*(t[:1, :48] for t in lv[:5]))            # a short call replays
+    assert o.requires_grad and not ops._kept
+    for other in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0], other))
 
 
 @pytest.mark.parametrize("lens", [[1, 1, 1], [32, 64, 31, 33], [3, 0, 96, 5, 32, 40]])
@@ -383,9 +397,12 @@ def test_fp32_backward_over_groups_of_heads(K, V, HQ, H, l2, lens, saved):
         assert max_norm_err(got[0][n], ref["d" + n].view(1, tokens, HQ, H // HQ, K).sum(3)) <= TOL, n
 
 
-def test_fp32_backward_takes_the_memory_that_is_there(monkeypatch):
-    """An allocator that has no room for the scratch of all heads at once (152 MB here): the call makes do with a part, same bits."""
-    from kda_b200 import chunk_kda
+@pytest.mark.parametrize("kept", [True, False])
+def test_fp32_backward_takes_the_memory_that_is_there(kept, monkeypatch):
+    """An allocator that has no room for the scratch of all heads at once (68 MB here, 152 with the replay): the call makes do with a part, same bits."""
+    from kda_b200 import chunk_kda, ops
+    if not kept:
+        monkeypatch.setattr(ops, "_keep_limit", lambda index: 0)
     d = {n: t.cuda() for n, t in make_inputs(1, 4096, 8, 128, 128, torch.float32, seed=57, backward=True).items() if t is not None}
     lv = [d[n].requires_grad_(True) for n in ("q", "k", "v", "g", "beta")]
     o, _ = chunk_kda(*lv)
@@ -395,12 +412,12 @@ def test_fp32_backward_takes_the_memory_that_is_there(monkeypatch):
     def empty(*size, **kw):
         if kw.get("dtype") == torch.uint8:
             asked.append(size[0])
-            if size[0] > 50 << 20:
+            if size[0] > 25 << 20:
                 raise torch.OutOfMemoryError("no room")
         return real(*size, **kw)
 
     monkeypatch.setattr(torch, "empty", empty)
     second = torch.autograd.grad(o, lv, d["do"])
-    row = 4096 * (2 * 2048 + 512 + 32)
-    assert asked == [8 * row, 4 * row, 2 * row]
+    row = 4096 * (2048 + 32 + (0 if kept else 2048 + 512))
+    assert asked == [n * row for n in ((8, 4, 2) if kept else (8, 4, 2, 1))]
     assert all(torch.equal(a, b) for a, b in zip(first, second))
