@@ -1,5 +1,5 @@
-"""GPU parity of the float32 training path (token-recurrent forward + its exact reverse-mode backward,
-`kda_recurrent_bwd`) against float64 autograd through the token-by-token oracle: max-normalised error <= 1e-4 for
+"""GPU parity of the float32 training path (token-recurrent forward and its exact reverse mode: two walks over the tokens and
+32-token pieces between them, `kda_recurrent_train.cu`) against float64 autograd through the token-by-token oracle: max-normalised error <= 1e-4 for
 o, the final state and every gradient (the fp32-mode bar)."""
 import numpy as np
 import pytest
@@ -185,22 +185,54 @@ EXACT = 5e-7
 
 @pytest.mark.parametrize("T", [7, 8, 9, 31, 32, 33, 40, 61])
 def test_fp32_training_at_the_edges_of_stages_and_kept_states(T):
-    """The walks stage eight tokens at a time and keep a state every 32; the middle works on four tokens at a time, replayed from every eighth."""
+    """The walks stage eight tokens at a time and keep a state every 32; the middle works on four tokens at a time, with the states between them in tensor memory."""
     d = make_inputs(2, T, 2, 128, 128, torch.float32, seed=600 + T, h0_std=0.1, backward=True)
     ref = recurrent_kda_grads(d["q"], d["k"], d["v"], d["g"], d["beta"], d["do"], d["dht"], initial_state=d["h0"])
     _errors(_run(d), ref, EXACT)
 
 
-@pytest.mark.parametrize("K,V", [(32, 32), (32, 64), (32, 128), (64, 32), (64, 64), (64, 128), (128, 32), (128, 64)])
+def _wide_batch(V, H):
+    """Sequences that make enough (sequence, head) units for the walks with 32 columns a warp: units * V / 32 > 4 warps per SM."""
+    return 4 * torch.cuda.get_device_properties(0).multi_processor_count * 32 // (V * H) + 1
+
+
+@pytest.mark.parametrize("K,V", [(32, 32), (32, 64), (32, 128), (64, 32), (64, 64), (64, 128), (128, 32), (128, 64), (128, 128)])
 @pytest.mark.parametrize("wide", [False, True])
-def test_fp32_training_of_both_walks(K, V, wide):
-    """Enough (sequence, head) units for the walks with 32 columns a warp (units * V / 32 > 4 warps per SM), and few units."""
-    sms = torch.cuda.get_device_properties(0).multi_processor_count
+@pytest.mark.parametrize("l2", [True, False])
+def test_fp32_training_of_both_walks(K, V, wide, l2):
+    """Many and few (sequence, head) units; with normalised rows (dq, dk through the last kernel) and without (dq, dk straight from the middle)."""
     H = 4
-    B = 4 * sms * 32 // (V * H) + 1 if wide else 1
+    B = _wide_batch(V, H) if wide else 1
     d = make_inputs(B, 37, H, K, V, torch.float32, seed=700 + K + V, h0_std=0.1, backward=True)
-    ref = recurrent_kda_grads(*(d[n].cuda() for n in ("q", "k", "v", "g", "beta", "do", "dht")), initial_state=d["h0"].cuda(), use_qk_l2norm=True)
-    _errors(_run(d, l2=True), ref, EXACT)
+    ref = recurrent_kda_grads(*(d[n].cuda() for n in ("q", "k", "v", "g", "beta", "do", "dht")), initial_state=d["h0"].cuda(), use_qk_l2norm=l2)
+    _errors(_run(d, l2=l2), ref, EXACT)
+
+
+@pytest.mark.parametrize("l2", [False, True])
+@pytest.mark.parametrize("HQ", [4, 2])
+@pytest.mark.parametrize("kept", [True, False])
+def test_fp32_training_of_many_uneven_sequences(l2, HQ, kept, monkeypatch):
+    """The walks with 32 columns a warp over packed sequences of 0 to 70 tokens, with and without grouped value heads, from what the forward kept and
+    replayed."""
+    from kda_b200 import chunk_kda, ops
+    monkeypatch.setattr(ops, "_keep_limit", lambda index: (1 << 30) if kept else 0)
+    H, D = 4, 128
+    lens = [(0, 1, 37, 32, 5, 70, 33)[i % 7] for i in range(_wide_batch(D, H))]
+    tokens, N = sum(lens), len(lens)
+    cu = torch.tensor(np.concatenate([[0], np.cumsum(lens)]), dtype=torch.int32, device="cuda")
+    d = {n: t.cuda() for n, t in make_inputs(1, tokens, H, D, D, torch.float32, seed=58 + HQ, h0_std=0.1, n_states=N, backward=True).items()
+         if t is not None}
+    d["q"], d["k"] = (d[n][:, :, :HQ].contiguous() for n in ("q", "k"))
+    each = lambda t: t.repeat_interleave(H // HQ, 2)      # noqa: E731
+    ref = recurrent_kda_grads(each(d["q"]), each(d["k"]), *(d[n] for n in ("v", "g", "beta", "do", "dht")), initial_state=d["h0"], cu_seqlens=cu,
+                              use_qk_l2norm=l2)
+    for n in ("dq", "dk"):
+        ref[n] = ref[n].view(1, tokens, HQ, H // HQ, D).sum(3)
+    lv = [d[n].requires_grad_(True) for n in ("q", "k", "v", "g", "beta", "h0")]
+    o, ht = chunk_kda(*lv[:5], initial_state=lv[5], output_final_state=True, cu_seqlens=cu, use_qk_l2norm_in_kernel=l2)
+    assert bool(ops._kept) == kept
+    grads = torch.autograd.grad([o, ht], lv, [d["do"], d["dht"]])
+    _errors(dict(zip(NAMES, (o.detach(), ht.detach(), *grads))), ref, EXACT)
 
 
 def test_recurrent_bwd_takes_q_k_g_at_odd_addresses():
