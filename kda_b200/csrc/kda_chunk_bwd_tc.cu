@@ -27,9 +27,9 @@
 // instruction for both sides.  Row numbers are left to the uniform registers.
 // 8 x 8192 tokens x 32 heads, whole step: 6.05 ms with 61 k instructions -> 5.91; operands handed over 5.81; dg from registers and the next q, k early
 // 5.73.  Packed documents with the L2 norm 7.13 -> 6.78 ms (its epilogue reads q and k where they are instead of from global memory); 2 x 1000 x 8
-// heads of 64: 108 -> 94 us, of which 9 are the code's size: 135 KB with every issue loop and wait unrolled, 85 now, and a short step fetches
-// all of it anew.  Kept as they were: the points where operands are rounded to bf16 (one scaled copy of each row instead of one per reference row
-// halves the builds and moves dA_log by 4 %).
+// heads of 64: 108 -> 98 us, of which 9 are the code's size: 135 KB with every issue loop and wait unrolled, 85 now, and a short step fetches
+// all of it anew.  (One scaled copy of each operand row instead of one per reference row halves the builds, 5 %.  It rounds to bf16 at other points:
+// nearer to fp32, but dA_log moves by 4 % of itself, and a gradient of the layer's call may move by 2 % from one build to the next.)
 #include "kda_chunk_bwd.cuh"
 #include "kda_device.cuh"
 #include "kda_f32x2.cuh"

@@ -90,7 +90,7 @@ __device__ __forceinline__ float butterfly(float (&v)[N], int lane) {
   return v[0];
 }
 
-// Four adjacent key columns in fp32: F4.
+// A thread's four adjacent key columns of a row are an F4.
 __device__ __forceinline__ F4 mul4c(const F4& x, const F4& y) { return {mul2(x.a, y.a), mul2(x.b, y.b)}; }
 __device__ __forceinline__ f32x2 widen2(uint32_t u) {      // two bf16 -> two fp32
   f32x2 d;

@@ -130,7 +130,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
 // hardware suspends for a short while, plus the sleep) takes about 4 microseconds on B200, so 2^18 polls are
 // about one second -- four orders of magnitude above the longest wait of a healthy run.
 constexpr unsigned MBAR_WAIT_POLLS = 1u << 18;
-// mbar_wait's loop is not unrolled, which keeps a kernel's code small: the copies made 30 of the 120 KB of the per-chunk backward, and code
+// mbar_wait's loop is not unrolled, which keeps a kernel's code small: the copies made 30 KB of the per-chunk backward (85 without), and code
 // is fetched anew whenever kernels alternate (one short training step: 104.7 -> 95.5 us with this and its issue loops rolled).  The decode
 // kernel, which runs at the copy rate of the memory, is 0.3 % better off with the copies (1,024 x 32: 655.9 against 657.6 us).
 __device__ __forceinline__ bool mbar_wait_unrolled(uint64_t* bar, unsigned parity) {

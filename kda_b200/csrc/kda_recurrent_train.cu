@@ -10,21 +10,24 @@
 //
 // Only two chains run through a whole sequence, and both fall apart into the state's columns: S forward (its sums run over k) and dS
 // backward (needs q, k, g, beta, do, but no S).  So three kernels:
-//   walk forward    S alone.  Leaves the state at the start of every 32 tokens and r of every token.
-//   walk backward   dS alone.  Leaves dS at the end of every 32 tokens, dv, and dbeta summed over 16 columns.
-//   middle          every (32 tokens, 32 rows of the state) on its own.  With r and beta dw known a step needs no sum over k: S and dS of
-//                   a row follow from that row's q, k, g, and its dq^, dk^, dg are sums along the row.
+//   walk forward    S alone.  Leaves the state at every border of a sequence's 32-token pieces and r of every token.
+//   walk backward   dS alone.  Leaves dS at the same borders, dv, and dbeta summed over 16 columns.
+//   middle          every piece (32 tokens or the rest of the sequence, 32 rows of the state) on its own.  With r and beta dw known a step needs no sum over
+//                   k: S and dS of a row follow from that row's q, k, g, and its dq^, dk^, dg are sums along the row.
+// What the forward walk leaves (2.5 KB per token and head of 128) is kept until the backward where the caller has the memory; otherwise the backward
+// replays the walk.  Heads may be worked on in groups, one after another, in a part of the scratch.  Neither changes a bit.
 // Walks: a warp holds 16 or 32 columns of all K rows (a lane 16 rows x 4 or 8 columns, packed two rows to a register pair), and nothing is
 // shared between warps but the staged q, k, exp g.
 // Middle: a thread holds 8 columns of 4 rows of S and dS.  S' of four tokens lives in registers; the states between are replayed once and kept as they
 // are, every fourth token, in tensor memory (256 columns a CTA, which nothing else here uses): 10.5 multiply-adds per element and token, and no
-// per-token state through memory (128 KB per token: what a CTA per sequence waited for).  Every eighth token's in shared memory, replayed
-// further from there: 9.33 -> 9.03 ms for the whole step.  The tile's shape is set by shared-memory bandwidth, which is 128 bytes per cycle
-// delivered to registers, broadcast or not: with 16 columns of one row a thread read 90 floats per 16 elements and token (92 % of the LSU's rate,
-// 7.5 ms), with 4 x 8 it reads 36 (5.0 ms, with the states in tensor memory 4.7).
-// What bounds them: the FP32 pipe (60 % busy; one CTA's load of its rows and states under the other's arithmetic) and, in the walks,
-// the 256 units' uneven share of 148 SMs.  8 x 2048 tokens x 32 heads of 128: forward walk 2.14, backward walk 2.11, middle 4.7 ms; 25.7 ms for
-// the whole step as a CTA per sequence -> 9.03.  One sequence x 32 heads: 12.8 -> 2.39 ms; 2 x 200 tokens x 8 heads: 1.23 -> 0.23.
+// per-token state through memory (128 KB per token: what a CTA per sequence waited for).  The tile's shape is set by shared-memory bandwidth, which is
+// 128 bytes per cycle delivered to registers, broadcast or not: with 16 columns of one row a thread reads 90 floats per 16 elements and token (92 % of
+// the LSU's rate, 7.5 ms), with 4 x 8 it reads 36.  With every eighth token's state in shared memory, replayed further from there: 5.0 ms; every fourth
+// in tensor memory 4.7; loops that end with the piece's tokens instead of unrolled to 32 4.5.
+// What bounds them: the FP32 pipe (61 % busy in the middle, 50 % in the walks; one CTA's load of its rows and states under the other's arithmetic) and,
+// in the walks, the 256 units' uneven share of 148 SMs.  8 x 2048 tokens x 32 heads of 128: forward walk 2.11, backward walk 2.11, middle 4.5 ms; the
+// whole step 25.7 ms as a CTA per sequence, 8.77 with what the forward kept, 10.6 with the replay.  One sequence x 32 heads: 12.8 -> 2.4 (3.1) ms;
+// 2 x 200 tokens x 8 heads: 1.25 -> 0.27 (0.33); 2,000 sequences of five tokens x 8: 3.5 -> 2.3 (2.6).
 // (Walks of two tokens a step, seven multiply-adds instead of eight and one reduction: 1 % less at 256 units, 5 % more at 32.)
 // dq^, dk^ (gradients w.r.t. the possibly L2-normalised rows, per VALUE head) go to the workspace; a last kernel sums grouped value
 // heads, applies the normalisation's backward (fla/modules/l2norm.py:190-240) and writes dq, dk; with neither they are dq, dk.  Every sum has a
