@@ -162,15 +162,10 @@ struct Slice {
   }
 };
 // sums over the rows of a lane's columns: the pairs' halves, then the eight row groups of the warp (lane bits 2..4); every lane gets all
-template <int CPL, int P>
-__device__ __forceinline__ float row_sum(const f32x2 (&h)[P][CPL], int c) {
-  const float2 x = halves(h[0][c]), y = halves(h[P - 1][c]);
-  return P == 1 ? x.x + x.y : (x.x + x.y) + (y.x + y.y);
-}
-template <int CPL, int P>
-__device__ __forceinline__ void column_sums(const f32x2 (&h)[P][CPL], float (&s)[CPL]) {
+template <int CPL>
+__device__ __forceinline__ void column_sums(const f32x2 (&h)[CPL], float (&s)[CPL]) {
 #pragma unroll
-  for (int c = 0; c < CPL; ++c) s[c] = row_sum<CPL, P>(h, c);
+  for (int c = 0; c < CPL; ++c) s[c] = halves(h[c]).x + halves(h[c]).y;
 #pragma unroll
   for (int o = 4; o < 32; o <<= 1)
 #pragma unroll
@@ -187,7 +182,6 @@ template <int K, int CPL, bool FWD>
 __global__ void __launch_bounds__(128, CPL == 8 ? 2 : 4) kda_recurrent_walk_kernel(const TrainParams p) {
   chain_point();
   constexpr int I = K / 32, E = K / 32;
-  constexpr int P = CPL == 8 ? 1 : 2;      // sums in flight per column: eight chains a lane
   extern __shared__ __align__(16) unsigned char smem_raw[];
   WalkSmem<K, CPL>& s = *reinterpret_cast<WalkSmem<K, CPL>*>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5, nt = blockDim.x;
@@ -299,12 +293,13 @@ __global__ void __launch_bounds__(128, CPL == 8 ? 2 : 4) kda_recurrent_walk_kern
         x[4 * m] = y.x; x[4 * m + 1] = y.y; x[4 * m + 2] = y.z; x[4 * m + 3] = y.w;
       }
       const float beta = s.beta[b][j];
-      f32x2 acc[P][CPL];
+      // (one sum a column, whatever the lane's number of columns: every sequence gets the same bits alone and in a large batch)
+      f32x2 acc[CPL];
       F4 k[I];
 #pragma unroll
       for (int i = 0; i < I; ++i) k[i] = lds4(kr + 32 * i);
 #pragma unroll
-      for (int c = 0; c < CPL; ++c) acc[0][c] = acc[P - 1][c] = 0ull;
+      for (int c = 0; c < CPL; ++c) acc[c] = 0ull;
       if constexpr (FWD) {
 #pragma unroll
         for (int i = 0; i < I; ++i) {
@@ -313,18 +308,18 @@ __global__ void __launch_bounds__(128, CPL == 8 ? 2 : 4) kda_recurrent_walk_kern
           for (int c = 0; c < CPL; ++c) {
             S.v[i][0][c] = mul2(S.v[i][0][c], a.a);
             S.v[i][1][c] = mul2(S.v[i][1][c], a.b);
-            acc[0][c] = fma2(S.v[i][0][c], k[i].a, acc[0][c]);
-            acc[P - 1][c] = fma2(S.v[i][1][c], k[i].b, acc[P - 1][c]);
+            acc[c] = fma2(S.v[i][0][c], k[i].a, acc[c]);
+            acc[c] = fma2(S.v[i][1][c], k[i].b, acc[c]);
           }
         }
         float hk[CPL];
-        column_sums<CPL, P>(acc, hk);
+        column_sums(acc, hk);
         f32x2 w2[CPL];
 #pragma unroll
         for (int c = 0; c < CPL; ++c) {
           x[c] -= hk[c];      // r
           w2[c] = pair(beta * x[c], beta * x[c]);
-          acc[0][c] = acc[P - 1][c] = 0ull;
+          acc[c] = 0ull;
         }
         if (keeps && rg < CPL / 4)
           *reinterpret_cast<float4*>(out) =
@@ -336,14 +331,14 @@ __global__ void __launch_bounds__(128, CPL == 8 ? 2 : 4) kda_recurrent_walk_kern
           for (int c = 0; c < CPL; ++c) {
             S.v[i][0][c] = fma2(k[i].a, w2[c], S.v[i][0][c]);
             S.v[i][1][c] = fma2(k[i].b, w2[c], S.v[i][1][c]);
-            acc[0][c] = fma2(S.v[i][0][c], q.a, acc[0][c]);
-            acc[P - 1][c] = fma2(S.v[i][1][c], q.b, acc[P - 1][c]);
+            acc[c] = fma2(S.v[i][0][c], q.a, acc[c]);
+            acc[c] = fma2(S.v[i][1][c], q.b, acc[c]);
           }
         }
         if (p.o) {      // summed off the chain: a lane ends with one column
           float y[CPL];
 #pragma unroll
-          for (int c = 0; c < CPL; ++c) y[c] = row_sum<CPL, P>(acc, c);
+          for (int c = 0; c < CPL; ++c) y[c] = halves(acc[c]).x + halves(acc[c]).y;
           int o = 16;
 #pragma unroll
           for (int half = CPL / 2; half >= 1; half >>= 1, o >>= 1)
@@ -363,12 +358,12 @@ __global__ void __launch_bounds__(128, CPL == 8 ? 2 : 4) kda_recurrent_walk_kern
           for (int c = 0; c < CPL; ++c) {
             S.v[i][0][c] = fma2(q.a, d2[c], S.v[i][0][c]);
             S.v[i][1][c] = fma2(q.b, d2[c], S.v[i][1][c]);
-            acc[0][c] = fma2(S.v[i][0][c], k[i].a, acc[0][c]);
-            acc[P - 1][c] = fma2(S.v[i][1][c], k[i].b, acc[P - 1][c]);
+            acc[c] = fma2(S.v[i][0][c], k[i].a, acc[c]);
+            acc[c] = fma2(S.v[i][1][c], k[i].b, acc[c]);
           }
         }
         float dw[CPL], dr[CPL];
-        column_sums<CPL, P>(acc, dw);
+        column_sums(acc, dw);
 #pragma unroll
         for (int c = 0; c < CPL; ++c) {
           dr[c] = beta * dw[c];
@@ -817,9 +812,8 @@ int launch_walk(const TrainParams& p, bool first, cudaStream_t st) {
   return static_cast<int>(cudaGetLastError());
 }
 // 32 columns a warp read a row of q, k, exp g for 128 state values instead of 64, and two warps a scheduler are enough to keep the FP32
-// pipe fed; while there are fewer than that, more and narrower warps shorten the chain.  (Of the call, not of a pass over some of its heads: the two
-// add up in another order, and a pass gives the bits that the whole call gives.)
-bool wide_slices(const TrainParams& p) { return static_cast<long long>(p.N) * p.H * p.V > 32LL * 4 * sm_count(); }
+// pipe fed; while there are fewer than that, more and narrower warps shorten the chain.  Both add up in the same order
+bool wide_slices(const TrainParams& p) { return static_cast<long long>(p.N) * p.HL * p.V > 32LL * 4 * sm_count(); }
 template <bool FWD>
 int launch_walk(const TrainParams& p, int K, bool first, cudaStream_t st) {
   const bool w = wide_slices(p);

@@ -453,3 +453,20 @@ def test_fp32_backward_takes_the_memory_that_is_there(kept, monkeypatch):
     row = 4096 * (2048 + 32 + (0 if kept else 2048 + 512))
     assert asked == [n * row for n in ((8, 4, 2) if kept else (8, 4, 2, 1))]
     assert all(torch.equal(a, b) for a, b in zip(first, second))
+
+
+@pytest.mark.parametrize("K,V,l2", [(128, 128, False), (64, 128, True), (32, 32, False)])
+def test_fp32_training_of_packed_sequences_gives_each_one_its_own_bits(K, V, l2):
+    """A batch that takes the walks with 32 columns a warp, and its sequences alone, which take those with 16: o, states and gradients are equal."""
+    H = 4
+    lens = [(70, 1, 37, 32, 9)[i % 5] for i in range(_wide_batch(V, H))]
+    d = {n: t.cuda() for n, t in make_inputs(1, sum(lens), H, K, V, torch.float32, seed=59, h0_std=0.1, n_states=len(lens), backward=True).items()
+         if t is not None}
+    starts = np.concatenate([[0], np.cumsum(lens)])
+    packed = _run({n: t.clone() for n, t in d.items()}, cu=torch.tensor(starts, dtype=torch.int32), l2=l2)
+    for i in (0, 1, 2, 3, 4, len(lens) - 1):
+        s, e = int(starts[i]), int(starts[i + 1])
+        alone = _run({n: (t[i:i + 1] if n in ("h0", "dht") else t[:, s:e]).clone() for n, t in d.items()}, l2=l2)
+        for n in NAMES:
+            assert torch.equal(alone[n], packed[n][i:i + 1] if n in ("ht", "dh0") else packed[n][:, s:e]), (n, i)
+
