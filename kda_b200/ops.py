@@ -272,7 +272,7 @@ def fused_recurrent_kda(q, k, v, g, beta, A_log=None, dt_bias=None, scale=None, 
 
 
 # Bytes that float32 calls waiting for their backward keep on each device: (device index, bytes) by a weak reference to each buffer, which takes its
-# entry out when the buffer is freed (after the backward, with the graph, or by a hook that moves saved tensors elsewhere).
+# entry out when the buffer is freed (after the backward, or with the graph).
 _kept: dict = {}
 _kept_lock = threading.Lock()
 
@@ -284,11 +284,11 @@ def _keep_limit(index: int) -> int:
     return torch.cuda.get_device_properties(index).total_memory // 128
 
 
-def _keep(n: int, dev, asked: bool):
+def _keep(n: int, dev):
     """A buffer of n bytes for what a forward leaves for its backward, or None: the backward replays the forward."""
     with _kept_lock:
         held = sum(b for d, b in list(_kept.values()) if d == dev.index)
-        if not asked and held + n > _keep_limit(dev.index):
+        if held + n > _keep_limit(dev.index):
             return None
         try:
             saved = torch.empty(n, dtype=torch.uint8, device=dev)
@@ -327,16 +327,22 @@ class RecurrentKDAFunction(torch.autograd.Function):
         # (up to 48 tokens the device waits for the host, which takes 10 us over the buffer and 4 over the replay: one token x 8 heads 145 and 134 us)
         saved = None
         if keep or B * T > 48:
-            saved = _keep(_lib.load().kda_recurrent_saved_bytes(B * T, B if cu is None else cu.numel() - 1, H, K, V), q.device, keep)
+            n = _lib.load().kda_recurrent_saved_bytes(B * T, B if cu is None else cu.numel() - 1, H, K, V)
+            saved = torch.empty(n, dtype=torch.uint8, device=q.device) if keep else _keep(n, q.device)
         o, ht = (_lib._native or _lib.native()).recurrent_fwd(
             q, k, v, g32, beta32, None, None, h0, scale, output_final_state, False, cu, None, None, use_l2norm, False, False, None, None, False, saved)
-        ctx.save_for_backward(q, k, v, g32, beta32, h0, cu, saved)
+        # Whether there was room may differ when a checkpointed segment is run again, the list of saved tensors may not: the buffer is among them only
+        # where the caller asked for it, and otherwise goes with the first backward.
+        ctx.save_for_backward(q, k, v, g32, beta32, h0, cu, saved if keep else None)
+        ctx.kept = None if keep else saved
         ctx.meta = (float(scale), bool(use_l2norm), g.dtype, beta.dtype)
         return o, ht
 
     @staticmethod
     def backward(ctx, do, dht):
         q, k, v, g32, beta32, h0, cu, saved = ctx.saved_tensors
+        if saved is None:
+            saved, ctx.kept = ctx.kept, None
         scale, use_l2norm, g_dtype, beta_dtype = ctx.meta
         B, T, HQ, K = q.shape
         H, V = v.shape[-2], v.shape[-1]

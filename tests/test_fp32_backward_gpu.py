@@ -437,8 +437,8 @@ def test_fp32_backward_takes_the_memory_that_is_there(kept, monkeypatch):
         monkeypatch.setattr(ops, "_keep_limit", lambda index: 0)
     d = {n: t.cuda() for n, t in make_inputs(1, 4096, 8, 128, 128, torch.float32, seed=57, backward=True).items() if t is not None}
     lv = [d[n].requires_grad_(True) for n in ("q", "k", "v", "g", "beta")]
+    first = torch.autograd.grad(chunk_kda(*lv)[0], lv, d["do"])
     o, _ = chunk_kda(*lv)
-    first = torch.autograd.grad(o, lv, d["do"], retain_graph=True)
     asked, real = [], torch.empty
 
     def empty(*size, **kw):
@@ -470,3 +470,24 @@ def test_fp32_training_of_packed_sequences_gives_each_one_its_own_bits(K, V, l2)
         for n in NAMES:
             assert torch.equal(alone[n], packed[n][i:i + 1] if n in ("ht", "dh0") else packed[n][:, s:e]), (n, i)
 
+
+@pytest.mark.parametrize("keep", [False, True])
+def test_fp32_calls_in_a_checkpointed_segment(keep, monkeypatch):
+    """Room for the intermediates of one call of three: in a checkpointed segment all three find it, since nothing is held between, and when the segment
+    is run again for its backward only the first does.  The saved tensors must be the same ones both times."""
+    from torch.utils.checkpoint import checkpoint
+    from kda_b200 import chunk_kda, ops
+    d = {n: t.cuda() for n, t in make_inputs(1, 200, 2, 64, 64, torch.float32, seed=60, backward=True).items() if t is not None}
+    lv = [d[n].requires_grad_(True) for n in ("q", "k", "v", "g", "beta")]
+    monkeypatch.setattr(ops, "_keep_limit", lambda index: 200 * 2 * 64 * 4 * 2 + 200 // 32 * 2 * 64 * 64 * 4)
+
+    def segment(q, k, v, g, beta):
+        for _ in range(3):
+            v = chunk_kda(q, k, v, g, beta, disable_recompute=keep)[0]
+        return v
+
+    plain = torch.autograd.grad(segment(*lv), lv, d["do"])
+    out = checkpoint(segment, *lv, use_reentrant=False)
+    assert all(torch.equal(a, b) for a, b in zip(plain, torch.autograd.grad(out, lv, d["do"])))
+    del out
+    assert not ops._kept
